@@ -20,7 +20,7 @@ SYMBOLS = (
     "evoattn_bwd", "evoattn_bwd_static_scratch", "evoattn_last_path", "evoattn_last_launch_count",
     "evoattn_peer_data_bytes", "evoattn_peer_flag_bytes", "evoattn_peer_buffer_create", "evoattn_peer_buffer_open",
     "evoattn_peer_buffer_close", "evoattn_peer_buffer_destroy", "evoattn_peer_allreduce_f32",
-    "evoattn_bias_to_heads_first", "evoattn_dbias_to_heads_last",
+    "evoattn_bias_to_heads_first", "evoattn_bias_to_heads_first_ld", "evoattn_dbias_to_heads_last", "evoattn_bias_pad_rows",
 )
 STATIC_SCRATCH_BYTES = 64 << 20
 
@@ -114,6 +114,10 @@ def load() -> C.CDLL:
             fn = getattr(lib, name)
             fn.restype = C.c_int
             fn.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p]
+        lib.evoattn_bias_to_heads_first_ld.restype = C.c_int
+        lib.evoattn_bias_to_heads_first_ld.argtypes = [C.c_void_p, C.c_void_p] + [C.c_int] * 5 + [C.c_void_p]
+        lib.evoattn_bias_pad_rows.restype = C.c_int
+        lib.evoattn_bias_pad_rows.argtypes = [C.c_void_p, C.POINTER(C.c_int64), C.c_void_p] + [C.c_int] * 5 + [C.c_void_p]
         lib.evoattn_peer_allreduce_f32.restype = C.c_int
         lib.evoattn_peer_allreduce_f32.argtypes = [C.POINTER(PeerAllReduceParams), C.c_void_p]
         if lib.evoattn_abi_version() != ABI_VERSION:

@@ -188,18 +188,44 @@ def attention_backward(q, k, v, o, lse, mask, bias, scale, d_o, want_dbias=True,
     return dq, dk, dv, dbias, dgate, dmask
 
 
+def _rows_of_16_bytes(R: int, dtype: torch.dtype) -> int:
+    """``R`` rounded up so that a row of that many elements is a whole number of 16-byte pieces."""
+    per = 16 // dtype.itemsize
+    return (R + per - 1) // per * per
+
+
+def pad_bias_rows(bias: torch.Tensor) -> torch.Tensor:
+    """A ``[B, H, R, R]`` pair bias whose rows a tensor map cannot read (their stride is not a multiple
+    of 16 bytes, as for most odd ``R``) copied into padded rows; any other bias as it is.  One pass
+    over the bias, which the MSA rows share, instead of the CUDA-core kernels for the whole call."""
+    es = bias.element_size()
+    if bias.data_ptr() % 16 == 0 and all(st * es % 16 == 0 for st in bias.stride()[:3]):
+        return bias
+    lib = _lib.load()
+    B, H, R, _ = bias.shape
+    ld = _rows_of_16_bytes(R, bias.dtype)
+    dst = torch.empty((B, H, R, ld), dtype=bias.dtype, device=bias.device)
+    stream = torch.cuda.current_stream(bias.device).cuda_stream
+    with torch.cuda.device(bias.device):
+        _lib.check(lib.evoattn_bias_pad_rows(bias.data_ptr(), (C.c_int64 * 3)(*bias.stride()[:3]), dst.data_ptr(),
+                                             _DTYPES[bias.dtype], B, H, R, ld, C.c_void_p(stream)), "evoattn_bias_pad_rows")
+    return dst[..., :R]
+
+
 def bias_to_heads_first(bias_brrh: torch.Tensor) -> torch.Tensor:
     """``[B, R, R, H]`` (as a linear layer emits a pair bias) -> ``[B, H, R, R]``, same dtype, one
-    device pass (the reference's layout, evoformer.py:638,652, makes its caller permute and copy)."""
+    device pass (the reference's layout, evoformer.py:638,652, makes its caller permute and copy);
+    rows padded to whole 16-byte pieces."""
     lib = _lib.load()
     B, R, R2, H = bias_brrh.shape
     src = bias_brrh.contiguous()
-    dst = torch.empty((B, H, R, R), dtype=src.dtype, device=src.device)
+    ld = _rows_of_16_bytes(R, src.dtype)
+    dst = torch.empty((B, H, R, ld), dtype=src.dtype, device=src.device)
     stream = torch.cuda.current_stream(src.device).cuda_stream
     with torch.cuda.device(src.device):
-        _lib.check(lib.evoattn_bias_to_heads_first(src.data_ptr(), dst.data_ptr(), _DTYPES[src.dtype], B, H, R,
-                                                   C.c_void_p(stream)), "evoattn_bias_to_heads_first")
-    return dst
+        _lib.check(lib.evoattn_bias_to_heads_first_ld(src.data_ptr(), dst.data_ptr(), _DTYPES[src.dtype], B, H, R, ld,
+                                                      C.c_void_p(stream)), "evoattn_bias_to_heads_first_ld")
+    return dst[..., :R]
 
 
 def dbias_to_heads_last(dbias_bhrr: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -277,6 +303,8 @@ class _EvoformerAttentionBase(torch.autograd.Function):
                 bias = bias.float()
             if bias.stride(-1) != 1:
                 bias = bias.contiguous()
+            if Q.dtype != torch.float32 and D <= 64 and D % 8 == 0 and R <= 2048:  # what the tensor-core kernels cover
+                bias = pad_bias_rows(bias)
         o, lse = attention_forward(q, k, v, mask, bias, scale, g)
         ctx.save_for_backward(q, k, v, mask, bias, o, lse, g)  # evoformer.py:729
         ctx.softmax_scale = scale

@@ -115,8 +115,9 @@ bool use_sm100_bwd(const evoattn_bwd_params* p, const evo::Args& a) {
   if (!stride_ok16(p->do_stride, es) || !stride_ok16(p->dq_stride, es) || !stride_ok16(p->dk_stride, es) ||
       !stride_ok16(p->dv_stride, es))
     return false;
-  // d(pair_bias) leaves through a tensor map over its dense [B,H,R,R] layout: 16-byte base and rows
-  if (p->fwd.bias && p->dbias && ((((uintptr_t)p->dbias) & 15) != 0 || (p->fwd.R % 4) != 0)) return false;
+  // A dense d(pair_bias) whose rows are not whole 16-byte pieces costs the tensor-core path a padded
+  // buffer and one more pass; a handful of score rows is done sooner on the CUDA cores.
+  if (p->fwd.bias && p->dbias && p->fwd.R % 4 != 0 && (long long)a.B * a.H * a.S * a.R <= 512) return false;
   return evo::sm100_bwd_supported(p->fwd.dtype, a);
 }
 
@@ -148,10 +149,14 @@ int static_scratch_address(void** out) {
   return EVOATTN_OK;
 }
 
+// Row stride of the statistics the tensor-core backward reads through tensor maps: whole 16-byte pieces.
+int stats_ld(const evo::Args& a) { return (a.R + 3) / 4 * 4; }
+
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 // Scratch of a backward call: what the kernel family needs, then (gated output) the effective dO.
-size_t path_scratch_need(const evoattn_bwd_params* p, const evo::Args& a, bool fast) {
+size_t path_scratch_need(const evoattn_bwd_params* p, evo::Args a, bool fast) {
+  a.delta_ld = fast ? stats_ld(a) : a.R;
   return align256(fast ? evo::sm100_bwd_workspace_bytes(p->fwd.dtype, a) : generic_bwd_workspace(a));
 }
 size_t bwd_scratch_need(const evoattn_bwd_params* p, const evo::Args& a, bool fast) {
@@ -161,6 +166,7 @@ size_t bwd_scratch_need(const evoattn_bwd_params* p, const evo::Args& a, bool fa
 // The backward with its scratch at `scratch` (caller-provided or the static array).
 int run_bwd(const evoattn_bwd_params* p, evo::Args& a, bool fast, void* scratch, cudaStream_t st) {
   const size_t path_bytes = path_scratch_need(p, a, fast);
+  a.delta_ld = fast ? stats_ld(a) : a.R;
   a.delta = reinterpret_cast<float*>(scratch);  // every kernel family keeps delta at the start of its scratch
   if (p->fwd.gate) {
     const int rc = evo::launch_gate_backward(p->fwd.dtype, &a, reinterpret_cast<unsigned char*>(scratch) + path_bytes, p->dgate,

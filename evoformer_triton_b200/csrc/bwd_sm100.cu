@@ -126,9 +126,10 @@ __global__ void __launch_bounds__(256) prep_kernel(Args a, float* __restrict__ n
 #pragma unroll
     for (int u = 0; u < 8; ++u) acc += to_float<T>(op[u]) * to_float<T>(gp[u]);
   }
-  if (!a.delta_ready) a.delta[row] = acc;
+  const long long at = (row / a.R) * a.delta_ld + i;
+  if (!a.delta_ready) a.delta[at] = acc;
   const float lse = a.lse[row];
-  nl[row] = (lse == -FLT_MAX) ? __int_as_float(0x7f800000) : -lse * kLog2e;
+  nl[at] = (lse == -FLT_MAX) ? __int_as_float(0x7f800000) : -lse * kLog2e;
 }
 
 // dq = scale * dq_acc, cast to the storage type (dq_acc: contiguous fp32 [B,H,S,R,D]).
@@ -697,18 +698,30 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 
 size_t align_up(size_t x, size_t al) { return (x + al - 1) / al * al; }
 
+// One vector of row statistics: [B,H,S,delta_ld] fp32.
+size_t stats_bytes(const Args& a) { return align_up((size_t)a.B * a.H * a.S * a.delta_ld * sizeof(float), 256); }
+bool dbias_needs_padding(const Args& a) {
+  return a.dbias && (a.R % 4 != 0 || (reinterpret_cast<uintptr_t>(a.dbias) & 15) != 0);
+}
+
 template <class T, int DP>
 int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* launches) {
   constexpr int G = RowsPerItem<DP>::G;
   using L = SmemT<DP>;
   Args a = a0;
   const size_t rows = (size_t)a.B * a.H * a.S * a.R;
-  const size_t vec_bytes = align_up(rows * sizeof(float), 256);
-  const size_t dq_bytes = rows * a.D * sizeof(float);
-  if (ws_bytes < 2 * vec_bytes + dq_bytes) return EVOATTN_ERR_WORKSPACE;
+  const size_t vec_bytes = stats_bytes(a);
+  const size_t dq_bytes = align_up(rows * a.D * sizeof(float), 256);
+  if (ws_bytes < sm100_bwd_workspace_bytes(0, a)) return EVOATTN_ERR_WORKSPACE;
   a.delta = reinterpret_cast<float*>(ws);
   float* nl = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + vec_bytes);
   float* dq_acc = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + 2 * vec_bytes);
+  // A dense d(pair_bias) whose rows are not whole 16-byte pieces cannot be the target of tensor
+  // reductions: it is summed in a padded copy and written out at the end.
+  float* const dbias_dense = a.dbias;
+  const bool padded = dbias_needs_padding(a);
+  const int ld = padded ? a.delta_ld : a.R;
+  if (padded) a.dbias = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + 2 * vec_bytes + dq_bytes);
 
   CUtensorMap tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl;
   if (!make_qkv_map(&tq, a.q, a.sq, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
@@ -716,18 +729,18 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   if (!make_qkv_map(&tv, a.v, a.sv, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tdo, a.d_o, a.sdo, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_rows_f32_plain_map(&tdq, dq_acc, a.D, a.R, (long long)a.B * a.H * a.S, DP / 4, 32)) return EVOATTN_ERR_CUDA;
-  if (!make_stats_map(&tnl, nl, a.B * a.H, a.S, a.R, BT)) return EVOATTN_ERR_CUDA;
-  if (!make_stats_map(&tdl, a.delta, a.B * a.H, a.S, a.R, BT)) return EVOATTN_ERR_CUDA;
+  if (!make_stats_map(&tnl, nl, a.B * a.H, a.S, a.R, a.delta_ld, BT)) return EVOATTN_ERR_CUDA;
+  if (!make_stats_map(&tdl, a.delta, a.B * a.H, a.S, a.R, a.delta_ld, BT)) return EVOATTN_ERR_CUDA;
   tb = tq;
   tdb = tq;
   if (a.bias) {
     const bool ok = a.bias16 ? make_bias16_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT, /*swizzle=*/false)
                              : make_bias_plain_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT);
     if (!ok) return EVOATTN_ERR_CUDA;
-    const Str3 dense{(long long)a.H * a.R * a.R, (long long)a.R * a.R, (long long)a.R};
+    const Str3 dense{(long long)a.H * a.R * ld, (long long)a.R * ld, (long long)ld};
     if (a.dbias && !make_bias_plain_map(&tdb, a.dbias, dense, a.B, a.H, a.R, 16, 32)) return EVOATTN_ERR_CUDA;
   }
-  if (a.dbias && cudaMemsetAsync(a.dbias, 0, (size_t)a.B * a.H * a.R * a.R * sizeof(float), st) != cudaSuccess)
+  if (a.dbias && cudaMemsetAsync(a.dbias, 0, (size_t)a.B * a.H * a.R * ld * sizeof(float), st) != cudaSuccess)
     return EVOATTN_ERR_CUDA;
   prep_kernel<T><<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(a, nl, dq_acc);
 
@@ -747,6 +760,10 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)L::bytes, &num_regs)) return EVOATTN_ERR_CUDA;
   if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
   kern<<<(unsigned)ctas, kThreadsT, L::bytes, st>>>(a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
+  if (padded) {
+    launch_dbias_dense(a.dbias, ld, dbias_dense, (long long)a.B * a.H * a.R, a.R, st);
+    *launches += 1;
+  }
   // d(pair_bias) is complete: its sum over the GPUs of the node, if the caller asked for one, runs on
   // a stream of its own next to the dQ store below; the caller's stream waits for it at the end
   cudaStream_t side = nullptr;
@@ -778,7 +795,8 @@ bool sm100_bwd_supported(int dtype, const Args& a) {
 
 size_t sm100_bwd_workspace_bytes(int, const Args& a) {
   const size_t rows = (size_t)a.B * a.H * a.S * a.R;
-  return 2 * align_up(rows * sizeof(float), 256) + rows * a.D * sizeof(float);
+  const size_t dbias = dbias_needs_padding(a) ? (size_t)a.B * a.H * a.R * a.delta_ld * sizeof(float) : 0;
+  return 2 * stats_bytes(a) + align_up(rows * a.D * sizeof(float), 256) + dbias;
 }
 
 int launch_sm100_bwd(int dtype, const Args& a, void* workspace, size_t workspace_bytes, cudaStream_t st,

@@ -48,7 +48,8 @@ struct Args {
   void* dk;
   void* dv;
   float* dbias;     // [B,H,R,R] contiguous
-  float* delta;     // [B,H,S,R] (workspace)
+  float* delta;     // [B,H,S,delta_ld] (workspace)
+  int delta_ld;     // R, or R rounded up to whole 16-byte rows where a tensor map reads it
   Str4 sdo, sdq, sdk, sdv;
   int* status;
   // gated output (optional): forward multiplies O by sigmoid(gate); backward gets dO of the gated output

@@ -40,13 +40,14 @@ __global__ void __launch_bounds__(256) gate_backward_kernel(Args a, T* __restric
     dg[d] = from_float<T>(G * O * (1.f - sg));
   }
   acc = warp_sum(acc);
-  if (lane == 0) a.delta[row] = acc;
+  if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
 }
 
-// [B,R,R,H] -> [B,H,R,R]: a block takes 128 keys of one (b, i) row: 128*H contiguous elements in,
+// [B,R,R,H] -> [B,H,R,ld >= R]: a block takes 128 keys of one (b, i) row: 128*H contiguous elements in,
 // H runs of 128 contiguous elements out.
 template <class E>
-__global__ void __launch_bounds__(256) heads_first_kernel(const E* __restrict__ src, E* __restrict__ dst, int H, int R) {
+__global__ void __launch_bounds__(256) heads_first_kernel(const E* __restrict__ src, E* __restrict__ dst, int H, int R,
+                                                          int ld) {
   extern __shared__ unsigned char sm_raw[];
   E* sm = reinterpret_cast<E*>(sm_raw);
   const int j0 = blockIdx.x * 128, i = blockIdx.y, b = blockIdx.z;
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(256) heads_first_kernel(const E* __restrict__ 
   __syncthreads();
   for (int e = threadIdx.x; e < nj * H; e += 256) {
     const int h = e / nj, j = e - h * nj;
-    dst[(((long long)b * H + h) * R + i) * R + j0 + j] = sm[j * H + h];
+    dst[(((long long)b * H + h) * R + i) * ld + j0 + j] = sm[j * H + h];
   }
 }
 
@@ -76,7 +77,32 @@ __global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict
   for (int e = threadIdx.x; e < nj * H; e += 256) out[e] = from_float<E>(sm[e]);
 }
 
+// A pair bias with arbitrary (b, h, i) strides -> rows of R values with a row stride of `ld`, the form
+// the tensor maps can read (whole 16-byte pieces).  One read and one write of the bias, no more: at
+// [4, 32, 300, 300] bf16 it moves 46 MB.  The last ld - R columns are never read and stay unwritten.
+template <class E>
+__global__ void __launch_bounds__(256) pad_rows_kernel(const E* __restrict__ src, Str3 st, E* __restrict__ dst, int H,
+                                                       int R, int ld) {
+  const int h = blockIdx.y % H, b = blockIdx.y / H;
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < R; i += gridDim.x * 8) {  // a warp per row
+    const E* in = src + (long long)b * st.a + (long long)h * st.b + (long long)i * st.c;
+    E* out = dst + ((long long)blockIdx.y * R + i) * ld;
+    for (int j = threadIdx.x & 31; j < R; j += 32) out[j] = in[j];
+  }
+}
+
+__global__ void __launch_bounds__(256) dbias_dense_kernel(const float* __restrict__ src, int ld, float* __restrict__ dst,
+                                                          long long rows, int cols) {
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  for (int j = threadIdx.x & 31; j < cols; j += 32) dst[row * cols + j] = src[row * ld + j];
+}
+
 }  // namespace
+
+void launch_dbias_dense(const float* src, int ld, float* dst, long long rows, int cols, cudaStream_t st) {
+  dbias_dense_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(src, ld, dst, rows, cols);
+}
 
 size_t gate_backward_scratch_bytes(int dtype, const Args& a) {
   const size_t es = dtype == EVOATTN_FP32 ? 4 : 2;
@@ -104,14 +130,35 @@ int launch_gate_backward(int dtype, Args* a, void* scratch, void* dgate, const S
 extern "C" {
 
 int evoattn_bias_to_heads_first(const void* src, void* dst, int dtype, int B, int H, int R, void* cuda_stream) {
+  return evoattn_bias_to_heads_first_ld(src, dst, dtype, B, H, R, R, cuda_stream);
+}
+
+int evoattn_bias_pad_rows(const void* src, const int64_t* stride, void* dst, int dtype, int B, int H, int R, int ld,
+                          void* cuda_stream) {
+  if (!src || !dst || !stride) return EVOATTN_ERR_NULL;
+  if (B <= 0 || H <= 0 || R <= 0 || ld < R || (long long)B * H > 65535) return EVOATTN_ERR_SHAPE;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
+  const evo::Str3 s{stride[0], stride[1], stride[2]};
+  dim3 grid((R + 7) / 8, B * H);
+  if (dtype == EVOATTN_FP32)
+    evo::pad_rows_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(src), s, static_cast<float*>(dst), H, R, ld);
+  else if (dtype == EVOATTN_BF16 || dtype == EVOATTN_FP16)
+    evo::pad_rows_kernel<uint16_t><<<grid, 256, 0, st>>>(static_cast<const uint16_t*>(src), s, static_cast<uint16_t*>(dst), H, R, ld);
+  else
+    return EVOATTN_ERR_DTYPE;
+  return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
+}
+
+int evoattn_bias_to_heads_first_ld(const void* src, void* dst, int dtype, int B, int H, int R, int ld, void* cuda_stream) {
   if (!src || !dst) return EVOATTN_ERR_NULL;
+  if (ld < R) return EVOATTN_ERR_SHAPE;
   if (B <= 0 || H <= 0 || R <= 0 || H > 96 || B > 65535 || R > 65535) return EVOATTN_ERR_SHAPE;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   dim3 grid((R + 127) / 128, R, B);
   if (dtype == EVOATTN_FP32)
-    evo::heads_first_kernel<float><<<grid, 256, (size_t)128 * H * 4, st>>>(static_cast<const float*>(src), static_cast<float*>(dst), H, R);
+    evo::heads_first_kernel<float><<<grid, 256, (size_t)128 * H * 4, st>>>(static_cast<const float*>(src), static_cast<float*>(dst), H, R, ld);
   else if (dtype == EVOATTN_BF16 || dtype == EVOATTN_FP16)
-    evo::heads_first_kernel<uint16_t><<<grid, 256, (size_t)128 * H * 2, st>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), H, R);
+    evo::heads_first_kernel<uint16_t><<<grid, 256, (size_t)128 * H * 2, st>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), H, R, ld);
   else
     return EVOATTN_ERR_DTYPE;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;

@@ -622,7 +622,6 @@ bool sm100_fwd_supported(int dtype, const Args& a) {
     const int es = a.bias16 ? 2 : 4;
     if ((reinterpret_cast<uintptr_t>(a.bias) & 15) != 0) return false;
     if ((a.sbias.a * es) % 16 || (a.sbias.b * es) % 16 || (a.sbias.c * es) % 16) return false;
-    if ((a.R * es) % 16 != 0) return false;  // rows of the bias tensor map are whole 16-byte pieces
   }
   if ((long long)a.B * a.H * a.S * ((a.R + BM - 1) / BM) > 2147483647LL) return false;
   return true;

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(GW * 32) generic_delta_kernel(Args a) {
   float acc = 0.f;
   for (int d = lane; d < a.D; d += 32) acc += to_float<T>(o[d]) * to_float<T>(g[d]);
   acc = warp_sum(acc);
-  if (lane == 0) a.delta[row] = acc;
+  if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
 }
 
 // dQ: one warp per query row, lanes over keys.
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(GW * 32) generic_dq_kernel(Args a) {
     Gs[warp * DP + d] = to_float<T>(g[d]);
   }
   const float lse = a.lse[(long long)blockIdx.x * a.R + ic];
-  const float delta = a.delta[(long long)blockIdx.x * a.R + ic];
+  const float delta = a.delta[(long long)blockIdx.x * a.delta_ld + ic];
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
   for (int j0 = 0; j0 < a.R; j0 += GT) {
     __syncthreads();
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(GW * 32) generic_dkdv_kernel(Args a) {
     if (threadIdx.x < GT) {
       const int i = i0 + threadIdx.x;
       Ls[threadIdx.x] = (i < a.R) ? a.lse[(long long)blockIdx.x * a.R + i] : 0.f;
-      Ds[threadIdx.x] = (i < a.R) ? a.delta[(long long)blockIdx.x * a.R + i] : 0.f;
+      Ds[threadIdx.x] = (i < a.R) ? a.delta[(long long)blockIdx.x * a.delta_ld + i] : 0.f;
     }
     __syncthreads();
     const int i = i0 + lane;
@@ -298,8 +298,8 @@ __global__ void __launch_bounds__(GW * 32) generic_dbias_kernel(Args a) {
         Gw[d] = to_float<T>(g[d]);
       }
       __syncwarp();
-      const long long row = (((long long)b * a.H + h) * a.S + s) * a.R + i;
-      const float lse = a.lse[row], delta = a.delta[row];
+      const long long slab = ((long long)b * a.H + h) * a.S + s;
+      const float lse = a.lse[slab * a.R + i], delta = a.delta[slab * a.delta_ld + i];
       if (j < a.R) {
         const T* k = reinterpret_cast<const T*>(a.k) + off4(a.sk, b, h, s, j);
         const T* v = reinterpret_cast<const T*>(a.v) + off4(a.sv, b, h, s, j);

@@ -57,6 +57,10 @@ int launch_sm100_bwd(int dtype, const Args& a, void* workspace, size_t workspace
 int launch_peer_allreduce(const evoattn_peer_allreduce_params* p, cudaStream_t st);
 bool exchange_lane(cudaStream_t* side, cudaEvent_t* fork, cudaEvent_t* join);
 
+// fp32 rows of `cols` values with a row stride of `ld` -> dense rows (extras.cu): d(pair_bias) leaving
+// the padded buffer it was summed in.
+void launch_dbias_dense(const float* src, int ld, float* dst, long long rows, int cols, cudaStream_t st);
+
 // Backward half of the gated output (extras.cu): writes delta, the effective dO (into `scratch`) and
 // dgate, and redirects `a` to the effective dO.
 size_t gate_backward_scratch_bytes(int dtype, const Args& a);

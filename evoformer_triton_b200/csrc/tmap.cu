@@ -50,7 +50,7 @@ bool make_qkv_map(CUtensorMap* out, const void* base, const Str4& st, int B, int
 bool make_bias_map(CUtensorMap* out, const float* base, const Str3& st, int B, int H, int R, int box_i, int box_j) {
   std::call_once(g_once, resolve);
   if (!g_encode) return false;
-  const uint64_t row = static_cast<uint64_t>(R) * 4;
+  const uint64_t row = (static_cast<uint64_t>(R) * 4 + 15) / 16 * 16;  // (a stride that is never used must still be legal)
   cuuint64_t dims[4] = {(cuuint64_t)R, (cuuint64_t)R, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[3] = {fix_stride(st.c, 4, row, R), fix_stride(st.b, 4, row, H), fix_stride(st.a, 4, row, B)};
   cuuint32_t box[4] = {(cuuint32_t)box_j, (cuuint32_t)box_i, 1, 1};
@@ -59,23 +59,6 @@ bool make_bias_map(CUtensorMap* out, const float* base, const Str3& st, int B, i
                         CU_TENSOR_MAP_INTERLEAVE_NONE,
                         box_j == 32 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
-bool make_rows_f32_map(CUtensorMap* out, const float* base, int D, int R, long long slabs, int box_d, int box_r) {
-  std::call_once(g_once, resolve);
-  if (!g_encode) return false;
-  cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)R, (cuuint64_t)slabs};
-  cuuint64_t strides[2] = {(cuuint64_t)D * 4, (cuuint64_t)D * 4 * (cuuint64_t)R};
-  cuuint32_t box[3] = {(cuuint32_t)box_d, (cuuint32_t)box_r, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const int row_bytes = box_d * 4;
-  CUtensorMapSwizzle swz = row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
-                           : row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
-                                             : CU_TENSOR_MAP_SWIZZLE_32B;
-  CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
 
@@ -96,7 +79,7 @@ bool make_bias_plain_map(CUtensorMap* out, const float* base, const Str3& st, in
                          int box_j) {
   std::call_once(g_once, resolve);
   if (!g_encode) return false;
-  const uint64_t row = static_cast<uint64_t>(R) * 4;
+  const uint64_t row = (static_cast<uint64_t>(R) * 4 + 15) / 16 * 16;  // (a stride that is never used must still be legal)
   cuuint64_t dims[4] = {(cuuint64_t)R, (cuuint64_t)R, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[3] = {fix_stride(st.c, 4, row, R), fix_stride(st.b, 4, row, H), fix_stride(st.a, 4, row, B)};
   cuuint32_t box[4] = {(cuuint32_t)box_j, (cuuint32_t)box_i, 1, 1};
@@ -111,7 +94,7 @@ bool make_bias16_map(CUtensorMap* out, const void* base, const Str3& st, int B, 
                      bool swizzle) {
   std::call_once(g_once, resolve);
   if (!g_encode) return false;
-  const uint64_t row = static_cast<uint64_t>(R) * 2;
+  const uint64_t row = (static_cast<uint64_t>(R) * 2 + 15) / 16 * 16;
   cuuint64_t dims[4] = {(cuuint64_t)R, (cuuint64_t)R, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[3] = {fix_stride(st.c, 2, row, R), fix_stride(st.b, 2, row, H), fix_stride(st.a, 2, row, B)};
   cuuint32_t box[4] = {(cuuint32_t)box_j, (cuuint32_t)box_i, 1, 1};
@@ -127,11 +110,11 @@ bool make_bias16_map(CUtensorMap* out, const void* base, const Str3& st, int B, 
   return r == CUDA_SUCCESS;
 }
 
-bool make_stats_map(CUtensorMap* out, const float* base, int BH, int S, int R, int box_r) {
+bool make_stats_map(CUtensorMap* out, const float* base, int BH, int S, int R, int ld, int box_r) {
   std::call_once(g_once, resolve);
   if (!g_encode) return false;
   cuuint64_t dims[3] = {(cuuint64_t)R, (cuuint64_t)S, (cuuint64_t)BH};
-  cuuint64_t strides[2] = {(cuuint64_t)R * 4, (cuuint64_t)R * 4 * (cuuint64_t)S};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)ld * 4 * (cuuint64_t)S};
   cuuint32_t box[3] = {(cuuint32_t)box_r, 1, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,

@@ -19,10 +19,9 @@ bool make_qkv_map(CUtensorMap* out, const void* base, const Str4& stride_elems, 
 bool make_bias_map(CUtensorMap* out, const float* base, const Str3& stride_elems, int B, int H, int R, int box_i,
                    int box_j);
 
-// Contiguous fp32 [slabs, R, D] (the dQ accumulator: one slab per (b,h,s)) as a 3-D map
-// (D, R, slabs) with box (box_d, box_r, 1); rows and columns beyond R and D are clipped.
-bool make_rows_f32_map(CUtensorMap* out, const float* base, int D, int R, long long slabs, int box_d, int box_r);
-// The same tensor with an unswizzled box (rows of box_d floats land back to back in shared memory).
+// Contiguous fp32 [slabs, R, D] (the dQ accumulator: one slab per (b,h,s)) as a 3-D map (D, R, slabs)
+// with an unswizzled box (box_d, box_r, 1): rows of box_d floats land back to back in shared memory;
+// rows and columns beyond R and D are clipped.
 bool make_rows_f32_plain_map(CUtensorMap* out, const float* base, int D, int R, long long slabs, int box_d, int box_r);
 
 // fp32 [B,H,R,R] pair bias (or its dense gradient) as a 4-D map (R_j, R_i, H, B) with an
@@ -36,8 +35,8 @@ bool make_bias_plain_map(CUtensorMap* out, const float* base, const Str3& stride
 bool make_bias16_map(CUtensorMap* out, const void* base, const Str3& stride_elems, int B, int H, int R, int box_i,
                      int box_j, bool swizzle = true);
 
-// Contiguous fp32 per-row statistics [B*H, S, R] as a 3-D map (R, S, B*H) with box (box_r, 1, 1);
-// rows beyond R and MSA rows beyond S read as zero.
-bool make_stats_map(CUtensorMap* out, const float* base, int BH, int S, int R, int box_r);
+// fp32 per-row statistics [B*H, S, ld] (ld = R rounded up to whole 16-byte pieces) as a 3-D map
+// (R, S, B*H) with box (box_r, 1, 1); rows beyond R and MSA rows beyond S read as zero.
+bool make_stats_map(CUtensorMap* out, const float* base, int BH, int S, int R, int ld, int box_r);
 
 }  // namespace evo

@@ -223,7 +223,18 @@ int evoattn_peer_allreduce_f32(const evoattn_peer_allreduce_params* p, void* cud
  * kernels do that conversion on the device in one pass each; the second also casts the fp32
  * gradient to the bias type on the way.  `dtype` is the element type of the 16/32-bit side. */
 int evoattn_bias_to_heads_first(const void* src_brrh, void* dst_bhrr, int dtype, int B, int H, int R, void* cuda_stream);
+/* The same with a row stride of ld >= R elements in dst ([B,H,R,ld]). */
+int evoattn_bias_to_heads_first_ld(const void* src_brrh, void* dst_bhrr, int dtype, int B, int H, int R, int ld, void* cuda_stream);
 int evoattn_dbias_to_heads_last(const float* src_bhrr, void* dst_brrh, int dtype, int B, int H, int R, void* cuda_stream);
+
+/* ---- Pair bias of an arbitrary number of residues.
+ *
+ * The tensor-core kernels read the bias through tensor maps, whose row stride must be a multiple of 16
+ * bytes.  This copies a bias [B,H,R,R] with element strides stride[3] of (b,h,i) into rows of ld
+ * elements ([B,H,R,ld], ld >= R), which evoattn_fwd / evoattn_bwd then take with those strides.
+ * d(pair_bias) needs no such step: the backward writes it densely for any R. */
+int evoattn_bias_pad_rows(const void* src, const int64_t* stride, void* dst, int dtype, int B, int H, int R, int ld,
+                          void* cuda_stream);
 
 /* EVOATTN_PATH_* of the most recent forward / backward call made by this thread. */
 int evoattn_last_path(void);
