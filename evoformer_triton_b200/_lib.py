@@ -8,7 +8,7 @@ import threading
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libevoattn.so")
 
-ABI_VERSION = 3
+ABI_VERSION = 4
 BF16, FP16, FP32 = 0, 1, 2
 MASK_NONE, MASK_BOOL, MASK_ADD_F32, MASK_ADD_SAME = 0, 1, 2, 3
 FLAG_FORCE_GENERIC = 1
@@ -66,6 +66,8 @@ class BwdParams(C.Structure):
         ("dgate_stride", C.c_int64 * 4),
         ("dmask", C.c_void_p),
         ("exchange", C.POINTER(PeerAllReduceParams)),
+        ("dbias_cast", C.c_void_p),
+        ("dbias_cast_dtype", C.c_int32), ("dbias_cast_heads_last", C.c_int32),
     ]
 
 
@@ -124,6 +126,25 @@ def load() -> C.CDLL:
             raise RuntimeError("libevoattn.so ABI version mismatch; rebuild it")
         _lib = lib
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native autograd boundary (csrc/host.cpp); built together with the library."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _evohost
+        except ImportError as e:
+            raise RuntimeError("evoformer_triton_b200/_evohost.so is missing or was built against another torch: build it "
+                               "with `python -m evoformer_triton_b200.build`. There is no Python fallback.") from e
+        if _evohost.abi_version() != ABI_VERSION:
+            raise RuntimeError("_evohost.so ABI version mismatch; rebuild it")
+        _host = _evohost
+    return _host
 
 
 def strerror(rc: int) -> str:

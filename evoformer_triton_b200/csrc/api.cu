@@ -72,6 +72,11 @@ int validate_bwd(const evoattn_bwd_params* p) {
   if (rc) return rc;
   if (!p->d_o || !p->dq || !p->dk || !p->dv) return EVOATTN_ERR_NULL;
   if (p->fwd.gate && !p->dgate) return EVOATTN_ERR_NULL;
+  if (p->dbias_cast) {
+    if (p->dbias || p->exchange) return EVOATTN_ERR_SHAPE;  // one destination
+    if (p->dbias_cast_dtype < EVOATTN_BF16 || p->dbias_cast_dtype > EVOATTN_FP32) return EVOATTN_ERR_DTYPE;
+    if (p->dbias_cast_heads_last && (p->fwd.H > 96 || p->fwd.R > 65535 || p->fwd.B > 65535)) return EVOATTN_ERR_SHAPE;
+  }
   if (p->exchange) {  // the in-call sum of d(pair_bias) over the node's GPUs works on the caller's exchange buffer
     const evoattn_peer_allreduce_params* x = p->exchange;
     if (!p->fwd.bias || !p->dbias || !x->bufs) return EVOATTN_ERR_NULL;
@@ -86,6 +91,16 @@ void fill_bwd_args(const evoattn_bwd_params* p, evo::Args* a) {
   fill_args(&p->fwd, a);
   a->d_o = p->d_o; a->dq = p->dq; a->dk = p->dk; a->dv = p->dv;
   a->dbias = p->fwd.bias ? p->dbias : nullptr;
+  a->dbias_ld = a->R;
+  if (p->fwd.bias && p->dbias_cast) {
+    a->dbias_out = p->dbias_cast;
+    a->dbias_out_dtype = p->dbias_cast_dtype;
+    a->dbias_out_last = p->dbias_cast_heads_last;
+  }
+  if (p->fwd.gate) {
+    a->dgate = p->dgate;
+    a->sdgate = str4(p->dgate_stride);
+  }
   a->sdo = str4(p->do_stride); a->sdq = str4(p->dq_stride); a->sdk = str4(p->dk_stride); a->sdv = str4(p->dv_stride);
   a->dmask = p->dmask;
   a->exchange = p->exchange;
@@ -115,9 +130,10 @@ bool use_sm100_bwd(const evoattn_bwd_params* p, const evo::Args& a) {
   if (!stride_ok16(p->do_stride, es) || !stride_ok16(p->dq_stride, es) || !stride_ok16(p->dk_stride, es) ||
       !stride_ok16(p->dv_stride, es))
     return false;
+  if (p->fwd.gate && ((((uintptr_t)p->dgate) & 15) || !stride_ok16(p->dgate_stride, es))) return false;
   // A dense d(pair_bias) whose rows are not whole 16-byte pieces costs the tensor-core path a padded
   // buffer and one more pass; a handful of score rows is done sooner on the CUDA cores.
-  if (p->fwd.bias && p->dbias && p->fwd.R % 4 != 0 && (long long)a.B * a.H * a.S * a.R <= 512) return false;
+  if (p->fwd.bias && (p->dbias || p->dbias_cast) && p->fwd.R % 4 != 0 && (long long)a.B * a.H * a.S * a.R <= 512) return false;
   return evo::sm100_bwd_supported(p->fwd.dtype, a);
 }
 
@@ -154,34 +170,50 @@ int stats_ld(const evo::Args& a) { return (a.R + 3) / 4 * 4; }
 
 size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Scratch of a backward call: what the kernel family needs, then (gated output) the effective dO.
-size_t path_scratch_need(const evoattn_bwd_params* p, evo::Args a, bool fast) {
-  a.delta_ld = fast ? stats_ld(a) : a.R;
-  return align256(fast ? evo::sm100_bwd_workspace_bytes(p->fwd.dtype, a) : generic_bwd_workspace(a));
-}
-size_t bwd_scratch_need(const evoattn_bwd_params* p, const evo::Args& a, bool fast) {
-  return path_scratch_need(p, a, fast) + (p->fwd.gate ? evo::gate_backward_scratch_bytes(p->fwd.dtype, a) : 0);
+// Scratch of a backward call, in this order: what the kernel family needs (delta first), the effective
+// dO of a gated output, and the fp32 buffer d(pair_bias) is summed in where the caller's own cannot be
+// it: another type or layout, or (tensor reductions) rows that are not whole 16-byte pieces.
+struct Scratch {
+  size_t path, gate, dbias;
+  size_t total() const { return path + gate + dbias; }
+};
+Scratch plan_scratch(const evoattn_bwd_params* p, evo::Args* a, bool fast) {
+  a->delta_ld = fast ? stats_ld(*a) : a->R;
+  Scratch s{};
+  s.path = align256(fast ? evo::sm100_bwd_workspace_bytes(p->fwd.dtype, *a) : generic_bwd_workspace(*a));
+  if (p->fwd.gate) s.gate = align256((size_t)a->B * a->H * a->S * a->R * a->D * esize_of(p->fwd.dtype));
+  const bool direct = a->dbias && (!fast || (a->R % 4 == 0 && (reinterpret_cast<uintptr_t>(a->dbias) & 15) == 0));
+  if (a->dbias && !direct) {
+    a->dbias_out = a->dbias;
+    a->dbias_out_dtype = EVOATTN_FP32;
+    a->dbias_out_last = 0;
+  }
+  if (a->dbias_out) {
+    a->dbias_ld = fast ? stats_ld(*a) : a->R;
+    s.dbias = align256((size_t)a->B * a->H * a->R * a->dbias_ld * sizeof(float));
+  }
+  return s;
 }
 
 // The backward with its scratch at `scratch` (caller-provided or the static array).
-int run_bwd(const evoattn_bwd_params* p, evo::Args& a, bool fast, void* scratch, cudaStream_t st) {
-  const size_t path_bytes = path_scratch_need(p, a, fast);
-  a.delta_ld = fast ? stats_ld(a) : a.R;
-  a.delta = reinterpret_cast<float*>(scratch);  // every kernel family keeps delta at the start of its scratch
-  if (p->fwd.gate) {
-    const int rc = evo::launch_gate_backward(p->fwd.dtype, &a, reinterpret_cast<unsigned char*>(scratch) + path_bytes, p->dgate,
-                                             str4(p->dgate_stride), st, &g_last_launches);
-    if (rc) return rc;
-  }
+int run_bwd(const evoattn_bwd_params* p, evo::Args& a, const Scratch& plan, bool fast, void* scratch, cudaStream_t st) {
+  unsigned char* base = reinterpret_cast<unsigned char*>(scratch);
+  a.delta = reinterpret_cast<float*>(base);  // every kernel family keeps delta at the start of its scratch
+  if (plan.gate) a.d_o_eff = base + plan.path;
+  if (plan.dbias) a.dbias = reinterpret_cast<float*>(base + plan.path + plan.gate);
   if (a.dmask &&
       cudaMemsetAsync(a.dmask, 0, (size_t)a.B * a.S * a.R * sizeof(float), st) != cudaSuccess)
     return EVOATTN_ERR_CUDA;
   if (fast) {
     g_last_path = EVOATTN_PATH_TCGEN05;
-    return evo::launch_sm100_bwd(p->fwd.dtype, a, scratch, path_bytes, st, &g_last_launches);
+    return evo::launch_sm100_bwd(p->fwd.dtype, a, scratch, plan.path, st, &g_last_launches);
   }
   g_last_path = EVOATTN_PATH_GENERIC;
   if (evo::launch_generic_bwd(p->fwd.dtype, a, st, &g_last_launches) != cudaSuccess) return EVOATTN_ERR_CUDA;
+  if (a.dbias_out) {
+    const int rc = evo::launch_dbias_out(a, st, &g_last_launches);
+    if (rc) return rc;
+  }
   if (p->exchange) {  // (the CUDA-core kernels have nothing to run the exchange next to)
     const int rc = evo::launch_peer_allreduce(p->exchange, st);
     if (rc) return rc;
@@ -232,7 +264,7 @@ size_t evoattn_bwd_workspace_bytes(const evoattn_bwd_params* p) {
   if (validate_bwd(p)) return 0;
   evo::Args a;
   fill_bwd_args(p, &a);
-  return bwd_scratch_need(p, a, use_sm100_bwd(p, a));
+  return plan_scratch(p, &a, use_sm100_bwd(p, a)).total();
 }
 
 int evoattn_bwd(const evoattn_bwd_params* p, void* cuda_stream) {
@@ -244,10 +276,11 @@ int evoattn_bwd(const evoattn_bwd_params* p, void* cuda_stream) {
   fill_bwd_args(p, &a);
   bind_context_once();
   const bool fast = use_sm100_bwd(p, a);
-  const size_t need = bwd_scratch_need(p, a, fast);
+  const Scratch plan = plan_scratch(p, &a, fast);
+  const size_t need = plan.total();
   if (need && (!p->workspace || p->workspace_bytes < need)) return EVOATTN_ERR_WORKSPACE;
   if (need && ((uintptr_t)p->workspace & 255)) return EVOATTN_ERR_ALIGN;
-  return run_bwd(p, a, fast, p->workspace, reinterpret_cast<cudaStream_t>(cuda_stream));
+  return run_bwd(p, a, plan, fast, p->workspace, reinterpret_cast<cudaStream_t>(cuda_stream));
 }
 
 int evoattn_bwd_static_scratch(const evoattn_bwd_params* p, void* cuda_stream) {
@@ -258,13 +291,14 @@ int evoattn_bwd_static_scratch(const evoattn_bwd_params* p, void* cuda_stream) {
   evo::Args a;
   fill_bwd_args(p, &a);
   const bool fast = use_sm100_bwd(p, a);
-  if (bwd_scratch_need(p, a, fast) > EVOATTN_STATIC_SCRATCH_BYTES) return EVOATTN_ERR_WORKSPACE;
+  const Scratch plan = plan_scratch(p, &a, fast);
+  if (plan.total() > EVOATTN_STATIC_SCRATCH_BYTES) return EVOATTN_ERR_WORKSPACE;
   // Looking the symbol up (done on every call) also makes the device's primary context current
   // on this thread, which the tensor-map encoder needs; nothing here allocates.
   void* scratch = nullptr;
   rc = static_scratch_address(&scratch);
   if (rc) return rc;
-  return run_bwd(p, a, fast, scratch, reinterpret_cast<cudaStream_t>(cuda_stream));
+  return run_bwd(p, a, plan, fast, scratch, reinterpret_cast<cudaStream_t>(cuda_stream));
 }
 
 int evoattn_last_path(void) { return g_last_path; }

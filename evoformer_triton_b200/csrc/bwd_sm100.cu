@@ -96,40 +96,84 @@ __device__ __forceinline__ void mbar_expect_tx(Bar b, uint32_t bytes) { mbar_exp
 __device__ __forceinline__ void mma_commit_if(uint32_t leader, Bar b) { mma_commit_if_s(leader, b.a); }
 
 
-// delta[b,h,s,i] = <dO_i, O_i> (evoformer.py:299-326) and nl = -lse*log2e, one thread per row.
+// The first pass of a backward call: delta[b,h,s,i] = <dO_i, O_i> (evoformer.py:299-326), nl = -lse*log2e,
+// and zeros in the buffers that the fused kernel adds to (the fp32 dQ accumulator, d(pair_bias)).
 // A row whose keys were all dropped carries lse = -FLT_MAX from the forward; its nl is +inf, which
-// the fused kernel recognises.  The block also clears its 256 rows of the fp32 dQ accumulator
-// (contiguous in memory), which saves a separate pass over that buffer.
-template <class T>
-__global__ void __launch_bounds__(256) prep_kernel(Args a, float* __restrict__ nl, float* __restrict__ dq_acc) {
-  const long long rows = (long long)a.B * a.H * a.S * a.R;
-  {
-    const long long f4_first = (long long)blockIdx.x * 256 * (a.D / 4);
-    const long long f4_end = min(rows, (long long)(blockIdx.x + 1) * 256) * (a.D / 4);
-    float4* dst = reinterpret_cast<float4*>(dq_acc);
-    for (long long e = f4_first + threadIdx.x; e < f4_end; e += 256) dst[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  const long long row = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (row >= rows) return;
-  const int i = (int)(row % a.R);
-  long long sl = row / a.R;
-  const int s = (int)(sl % a.S); sl /= a.S;
-  const int h = (int)(sl % a.H);
-  const int b = (int)(sl / a.H);
-  const uint4* o = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.o) + off4(a.so, b, h, s, i));
-  const uint4* g = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, b, h, s, i));
+// the fused kernel recognises.  With a gate (Og = sigmoid(gate) O is the output, G its gradient):
+//   dO    = G * sigmoid(gate)                      (what the attention backward needs; into scratch)
+//   delta = sum_d dO * O = sum_d G * Og            (so the un-gated O is never needed)
+//   dgate = G * O * sigmoid'(gate) = G * Og * (1 - sigmoid(gate))
+// Bound by memory.  1 << LG lanes share a row, 16 bytes of each tensor per lane, so every access of a
+// warp is a run of whole sectors whatever D is.
+template <class T, int LG, bool GATE>
+__global__ void __launch_bounds__(256) prep_kernel(const Args a, float* __restrict__ nl, float* __restrict__ dq_acc,
+                                                   const uint32_t dbias_f4) {
+  const uint32_t gid = blockIdx.x * 256 + threadIdx.x;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t e = gid; e < dbias_f4; e += gridDim.x * 256) reinterpret_cast<float4*>(a.dbias)[e] = zero;
+  const uint32_t row = gid >> LG, c = gid & ((1u << LG) - 1u);
+  const uint32_t slab = row / (uint32_t)a.R, i = row - slab * (uint32_t)a.R;
+  const uint32_t bh = slab / (uint32_t)a.S, s = slab - bh * (uint32_t)a.S;
+  const uint32_t b = bh / (uint32_t)a.H, h = bh - b * (uint32_t)a.H;
+  const bool ok = (int)b < a.B;
   float acc = 0.f;
-  for (int d8 = 0; d8 < a.D / 8; ++d8) {
-    const uint4 ov = o[d8], gv = g[d8];
+  if (ok && (int)c * 8 < a.D) {
+    const int d = (int)c * 8;
+    const uint4 ov = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.o) + off4(a.so, b, h, s, i) + d);
+    const uint4 gv = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, b, h, s, i) + d);
     const T* op = reinterpret_cast<const T*>(&ov);
     const T* gp = reinterpret_cast<const T*>(&gv);
+    const size_t at = (size_t)row * a.D + d;
+    if constexpr (GATE) {
+      const uint4 tv = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(a.gate) + off4(a.sgate, b, h, s, i) + d);
+      const T* tp = reinterpret_cast<const T*>(&tv);
+      uint32_t eff[4], dg[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc += to_float<T>(op[u]) * to_float<T>(gp[u]);
+      for (int u = 0; u < 4; ++u) {
+        float x[2], y[2];
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          const float G = to_float<T>(gp[2 * u + w]), go = G * to_float<T>(op[2 * u + w]);
+          const float sg = sigmoidf_fast(to_float<T>(tp[2 * u + w]));
+          acc += go;
+          x[w] = G * sg;
+          y[w] = go * (1.f - sg);
+        }
+        eff[u] = Pack2<T>::pack(x[0], x[1]);
+        dg[u] = Pack2<T>::pack(y[0], y[1]);
+      }
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.d_o_eff) + at) = make_uint4(eff[0], eff[1], eff[2], eff[3]);
+      *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.dgate) + off4(a.sdgate, b, h, s, i) + d) = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += to_float<T>(op[u]) * to_float<T>(gp[u]);
+    }
+    reinterpret_cast<float4*>(dq_acc + at)[0] = zero;
+    reinterpret_cast<float4*>(dq_acc + at)[1] = zero;
   }
-  const long long at = (row / a.R) * a.delta_ld + i;
-  if (!a.delta_ready) a.delta[at] = acc;
-  const float lse = a.lse[row];
-  nl[at] = (lse == -FLT_MAX) ? __int_as_float(0x7f800000) : -lse * kLog2e;
+#pragma unroll
+  for (int o = (1 << LG) >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (ok && c == 0) {
+    const size_t at = (size_t)slab * a.delta_ld + i;
+    a.delta[at] = acc;
+    const float lse = a.lse[row];
+    nl[at] = (lse == -FLT_MAX) ? __int_as_float(0x7f800000) : -lse * kLog2e;
+  }
+}
+
+template <class T, bool GATE>
+void launch_prep(const Args& a, float* nl, float* dq_acc, cudaStream_t st) {
+  const int chunks = a.D / 8;
+  const int lg = chunks > 4 ? 3 : chunks > 2 ? 2 : chunks > 1 ? 1 : 0;
+  const size_t threads = ((size_t)a.B * a.H * a.S * a.R) << lg;
+  const uint32_t f4 = a.dbias ? (uint32_t)((size_t)a.B * a.H * a.R * a.dbias_ld / 4) : 0u;
+  const unsigned grid = (unsigned)((threads + 255) / 256);
+  switch (lg) {
+    case 3: prep_kernel<T, 3, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
+    case 2: prep_kernel<T, 2, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
+    case 1: prep_kernel<T, 1, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
+    default: prep_kernel<T, 0, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
+  }
 }
 
 // dq = scale * dq_acc, cast to the storage type (dq_acc: contiguous fp32 [B,H,S,R,D]).
@@ -700,9 +744,6 @@ size_t align_up(size_t x, size_t al) { return (x + al - 1) / al * al; }
 
 // One vector of row statistics: [B,H,S,delta_ld] fp32.
 size_t stats_bytes(const Args& a) { return align_up((size_t)a.B * a.H * a.S * a.delta_ld * sizeof(float), 256); }
-bool dbias_needs_padding(const Args& a) {
-  return a.dbias && (a.R % 4 != 0 || (reinterpret_cast<uintptr_t>(a.dbias) & 15) != 0);
-}
 
 template <class T, int DP>
 int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* launches) {
@@ -711,17 +752,16 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   Args a = a0;
   const size_t rows = (size_t)a.B * a.H * a.S * a.R;
   const size_t vec_bytes = stats_bytes(a);
-  const size_t dq_bytes = align_up(rows * a.D * sizeof(float), 256);
   if (ws_bytes < sm100_bwd_workspace_bytes(0, a)) return EVOATTN_ERR_WORKSPACE;
   a.delta = reinterpret_cast<float*>(ws);
   float* nl = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + vec_bytes);
   float* dq_acc = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + 2 * vec_bytes);
-  // A dense d(pair_bias) whose rows are not whole 16-byte pieces cannot be the target of tensor
-  // reductions: it is summed in a padded copy and written out at the end.
-  float* const dbias_dense = a.dbias;
-  const bool padded = dbias_needs_padding(a);
-  const int ld = padded ? a.delta_ld : a.R;
-  if (padded) a.dbias = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws) + 2 * vec_bytes + dq_bytes);
+  if (a.dgate) {
+    launch_prep<T, true>(a, nl, dq_acc, st);
+    use_effective_d_o(&a);
+  } else {
+    launch_prep<T, false>(a, nl, dq_acc, st);
+  }
 
   CUtensorMap tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl;
   if (!make_qkv_map(&tq, a.q, a.sq, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
@@ -737,13 +777,9 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
     const bool ok = a.bias16 ? make_bias16_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT, /*swizzle=*/false)
                              : make_bias_plain_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT);
     if (!ok) return EVOATTN_ERR_CUDA;
-    const Str3 dense{(long long)a.H * a.R * ld, (long long)a.R * ld, (long long)ld};
+    const Str3 dense{(long long)a.H * a.R * a.dbias_ld, (long long)a.R * a.dbias_ld, (long long)a.dbias_ld};
     if (a.dbias && !make_bias_plain_map(&tdb, a.dbias, dense, a.B, a.H, a.R, 16, 32)) return EVOATTN_ERR_CUDA;
   }
-  if (a.dbias && cudaMemsetAsync(a.dbias, 0, (size_t)a.B * a.H * a.R * ld * sizeof(float), st) != cudaSuccess)
-    return EVOATTN_ERR_CUDA;
-  prep_kernel<T><<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(a, nl, dq_acc);
-
   const int NT = (a.R + BT - 1) / BT;
   const long long items = (long long)a.B * a.H * NT * ((a.S + G - 1) / G);
   if (items > 0x7fffffffLL / (G * NT)) return EVOATTN_ERR_SHAPE;
@@ -760,9 +796,9 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)L::bytes, &num_regs)) return EVOATTN_ERR_CUDA;
   if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
   kern<<<(unsigned)ctas, kThreadsT, L::bytes, st>>>(a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
-  if (padded) {
-    launch_dbias_dense(a.dbias, ld, dbias_dense, (long long)a.B * a.H * a.R, a.R, st);
-    *launches += 1;
+  if (a.dbias_out) {
+    const int rc = launch_dbias_out(a, st, launches);
+    if (rc) return rc;
   }
   // d(pair_bias) is complete: its sum over the GPUs of the node, if the caller asked for one, runs on
   // a stream of its own next to the dQ store below; the caller's stream waits for it at the end
@@ -795,8 +831,7 @@ bool sm100_bwd_supported(int dtype, const Args& a) {
 
 size_t sm100_bwd_workspace_bytes(int, const Args& a) {
   const size_t rows = (size_t)a.B * a.H * a.S * a.R;
-  const size_t dbias = dbias_needs_padding(a) ? (size_t)a.B * a.H * a.R * a.delta_ld * sizeof(float) : 0;
-  return 2 * stats_bytes(a) + align_up(rows * a.D * sizeof(float), 256) + dbias;
+  return 2 * stats_bytes(a) + align_up(rows * a.D * sizeof(float), 256);
 }
 
 int launch_sm100_bwd(int dtype, const Args& a, void* workspace, size_t workspace_bytes, cudaStream_t st,

@@ -47,7 +47,12 @@ struct Args {
   void* dq;
   void* dk;
   void* dv;
-  float* dbias;     // [B,H,R,R] contiguous
+  float* dbias;     // [B,H,R,dbias_ld] fp32: where the kernels sum d(pair_bias), or null
+  int dbias_ld;
+  // where it goes from there, if it is not the caller's own fp32 buffer already
+  void* dbias_out;      // [B,H,R,R], or [B,R,R,H] if dbias_out_last
+  int dbias_out_dtype;
+  int dbias_out_last;
   float* delta;     // [B,H,S,delta_ld] (workspace)
   int delta_ld;     // R, or R rounded up to whole 16-byte rows where a tensor map reads it
   Str4 sdo, sdq, sdk, sdv;
@@ -55,7 +60,11 @@ struct Args {
   // gated output (optional): forward multiplies O by sigmoid(gate); backward gets dO of the gated output
   const void* gate;
   Str4 sgate;
-  int delta_ready;  // backward: delta has been written already (gated path), the kernels must not recompute it
+  // backward of a gated output: d_o and o are the gated ones; the first kernel of a family writes the
+  // gradient of the gate and the effective dO (contiguous), which the later ones read
+  void* dgate;
+  Str4 sdgate;
+  void* d_o_eff;
   const void* exchange;  // backward: evoattn_peer_allreduce_params of the d(pair_bias) exchange, or null
   float* dmask;     // backward (CUDA-core kernels only): gradient of an additive mask, [B,S,R] fp32
 };

@@ -1,7 +1,6 @@
-// Small device passes around the attention kernels: the backward half of the gated output, and the
-// conversion of a pair bias (and its gradient) between the layout a linear layer emits,
+// Small device passes around the attention kernels: the conversion of a pair bias (and its gradient) between the layout a linear layer emits,
 // [B, R, R, H], and the [B, H, R, R] the kernels (and dsevoformer-triton/evoformer.py:638,652) use.
-// None of this exists in the reference: its op ends at O and takes the bias heads-first.
+// None of this exists in the reference: it takes the bias heads-first.
 #include <string.h>
 
 #include "common.cuh"
@@ -9,39 +8,6 @@
 
 namespace evo {
 namespace {
-
-// Gated output Og = sigmoid(gate) * O.  With G = dOg (gradient of the gated output):
-//   dO    = G * sigmoid(gate)                      (what the attention backward needs)
-//   delta = sum_d dO * O = sum_d G * Og            (so the un-gated O is never needed)
-//   dgate = G * O * sigmoid'(gate) = G * Og * (1 - sigmoid(gate))
-// One warp per (b,h,s,i) row.  dO is written contiguously ([rows][D]) into scratch.
-template <class T>
-__global__ void __launch_bounds__(256) gate_backward_kernel(Args a, T* __restrict__ d_o_eff, void* __restrict__ dgate,
-                                                            Str4 sdgate) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * 8 + warp;
-  const long long rows = (long long)a.B * a.H * a.S * a.R;
-  if (row >= rows) return;
-  const int i = (int)(row % a.R);
-  long long sl = row / a.R;
-  const int s = (int)(sl % a.S); sl /= a.S;
-  const int h = (int)(sl % a.H);
-  const int b = (int)(sl / a.H);
-  const T* og = reinterpret_cast<const T*>(a.o) + off4(a.so, b, h, s, i);
-  const T* g = reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, b, h, s, i);
-  const T* gt = reinterpret_cast<const T*>(a.gate) + off4(a.sgate, b, h, s, i);
-  T* dg = reinterpret_cast<T*>(dgate) + off4(sdgate, b, h, s, i);
-  float acc = 0.f;
-  for (int d = lane; d < a.D; d += 32) {
-    const float G = to_float<T>(g[d]), O = to_float<T>(og[d]);
-    const float sg = sigmoidf_fast(to_float<T>(gt[d]));
-    acc += G * O;
-    d_o_eff[row * a.D + d] = from_float<T>(G * sg);
-    dg[d] = from_float<T>(G * O * (1.f - sg));
-  }
-  acc = warp_sum(acc);
-  if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
-}
 
 // [B,R,R,H] -> [B,H,R,ld >= R]: a block takes 128 keys of one (b, i) row: 128*H contiguous elements in,
 // H runs of 128 contiguous elements out.
@@ -61,16 +27,17 @@ __global__ void __launch_bounds__(256) heads_first_kernel(const E* __restrict__ 
   }
 }
 
-// fp32 [B,H,R,R] -> [B,R,R,H] in type E (the one cast of the gradient happens here).
+// fp32 [B,H,R,ld] -> [B,R,R,H] in type E (the one cast of the gradient happens here).
 template <class E>
-__global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict__ src, E* __restrict__ dst, int H, int R) {
+__global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict__ src, int ld, E* __restrict__ dst, int H,
+                                                         int R) {
   extern __shared__ unsigned char sm_raw[];
   float* sm = reinterpret_cast<float*>(sm_raw);
   const int j0 = blockIdx.x * 128, i = blockIdx.y, b = blockIdx.z;
   const int nj = min(128, R - j0);
   for (int e = threadIdx.x; e < nj * H; e += 256) {
     const int h = e / nj, j = e - h * nj;
-    sm[j * H + h] = src[(((long long)b * H + h) * R + i) * R + j0 + j];
+    sm[j * H + h] = src[(((long long)b * H + h) * R + i) * ld + j0 + j];
   }
   __syncthreads();
   E* out = dst + (((long long)b * R + i) * R + j0) * H;
@@ -91,37 +58,35 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(const E* __restrict__ src
   }
 }
 
-__global__ void __launch_bounds__(256) dbias_dense_kernel(const float* __restrict__ src, int ld, float* __restrict__ dst,
+template <class E>
+__global__ void __launch_bounds__(256) dbias_dense_kernel(const float* __restrict__ src, int ld, E* __restrict__ dst,
                                                           long long rows, int cols) {
-  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // a warp per row
   if (row >= rows) return;
-  for (int j = threadIdx.x & 31; j < cols; j += 32) dst[row * cols + j] = src[row * ld + j];
+  for (int j = threadIdx.x & 31; j < cols; j += 32) dst[row * cols + j] = from_float<E>(src[row * ld + j]);
+}
+
+template <class E>
+void dbias_out_t(const Args& a, cudaStream_t st) {
+  E* dst = reinterpret_cast<E*>(a.dbias_out);
+  if (a.dbias_out_last) {
+    dim3 grid((a.R + 127) / 128, a.R, a.B);
+    heads_last_kernel<E><<<grid, 256, (size_t)128 * a.H * 4, st>>>(a.dbias, a.dbias_ld, dst, a.H, a.R);
+  } else {
+    const long long rows = (long long)a.B * a.H * a.R;
+    dbias_dense_kernel<E><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a.dbias, a.dbias_ld, dst, rows, a.R);
+  }
 }
 
 }  // namespace
 
-void launch_dbias_dense(const float* src, int ld, float* dst, long long rows, int cols, cudaStream_t st) {
-  dbias_dense_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(src, ld, dst, rows, cols);
-}
-
-size_t gate_backward_scratch_bytes(int dtype, const Args& a) {
-  const size_t es = dtype == EVOATTN_FP32 ? 4 : 2;
-  return ((size_t)a.B * a.H * a.S * a.R * a.D * es + 255) / 256 * 256;
-}
-
-// Runs the gate pass and redirects `a` to the effective dO; `scratch` holds gate_backward_scratch_bytes().
-int launch_gate_backward(int dtype, Args* a, void* scratch, void* dgate, const Str4& sdgate, cudaStream_t st, int* launches) {
-  const long long rows = (long long)a->B * a->H * a->S * a->R;
-  const unsigned grid = (unsigned)((rows + 7) / 8);
-  switch (dtype) {
-    case EVOATTN_BF16: gate_backward_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(*a, reinterpret_cast<__nv_bfloat16*>(scratch), dgate, sdgate); break;
-    case EVOATTN_FP16: gate_backward_kernel<__half><<<grid, 256, 0, st>>>(*a, reinterpret_cast<__half*>(scratch), dgate, sdgate); break;
-    default: gate_backward_kernel<float><<<grid, 256, 0, st>>>(*a, reinterpret_cast<float*>(scratch), dgate, sdgate); break;
+int launch_dbias_out(const Args& a, cudaStream_t st, int* launches) {
+  switch (a.dbias_out_dtype) {
+    case EVOATTN_BF16: dbias_out_t<__nv_bfloat16>(a, st); break;
+    case EVOATTN_FP16: dbias_out_t<__half>(a, st); break;
+    default: dbias_out_t<float>(a, st); break;
   }
   *launches += 1;
-  a->d_o = scratch;
-  a->sdo = Str4{(long long)a->H * a->S * a->R * a->D, (long long)a->S * a->R * a->D, (long long)a->R * a->D, (long long)a->D};
-  a->delta_ready = 1;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }
 
@@ -170,9 +135,9 @@ int evoattn_dbias_to_heads_last(const float* src, void* dst, int dtype, int B, i
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   dim3 grid((R + 127) / 128, R, B);
   const size_t smem = (size_t)128 * H * 4;
-  if (dtype == EVOATTN_FP32) evo::heads_last_kernel<float><<<grid, 256, smem, st>>>(src, static_cast<float*>(dst), H, R);
-  else if (dtype == EVOATTN_BF16) evo::heads_last_kernel<__nv_bfloat16><<<grid, 256, smem, st>>>(src, static_cast<__nv_bfloat16*>(dst), H, R);
-  else if (dtype == EVOATTN_FP16) evo::heads_last_kernel<__half><<<grid, 256, smem, st>>>(src, static_cast<__half*>(dst), H, R);
+  if (dtype == EVOATTN_FP32) evo::heads_last_kernel<float><<<grid, 256, smem, st>>>(src, R, static_cast<float*>(dst), H, R);
+  else if (dtype == EVOATTN_BF16) evo::heads_last_kernel<__nv_bfloat16><<<grid, 256, smem, st>>>(src, R, static_cast<__nv_bfloat16*>(dst), H, R);
+  else if (dtype == EVOATTN_FP16) evo::heads_last_kernel<__half><<<grid, 256, smem, st>>>(src, R, static_cast<__half*>(dst), H, R);
   else return EVOATTN_ERR_DTYPE;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }

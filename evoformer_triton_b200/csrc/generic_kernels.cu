@@ -135,6 +135,39 @@ __global__ void __launch_bounds__(GW * 32) generic_delta_kernel(Args a) {
   if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
 }
 
+// Gated output Og = sigmoid(gate) * O.  With G = dOg (gradient of the gated output):
+//   dO    = G * sigmoid(gate)                      (what the attention backward needs)
+//   delta = sum_d dO * O = sum_d G * Og            (so the un-gated O is never needed)
+//   dgate = G * O * sigmoid'(gate) = G * Og * (1 - sigmoid(gate))
+// One warp per (b,h,s,i) row.  dO is written contiguously ([rows][D]) into scratch.
+template <class T>
+__global__ void __launch_bounds__(256) generic_gate_backward_kernel(Args a) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long row = (long long)blockIdx.x * 8 + warp;
+  T* d_o_eff = reinterpret_cast<T*>(a.d_o_eff);
+  const long long rows = (long long)a.B * a.H * a.S * a.R;
+  if (row >= rows) return;
+  const int i = (int)(row % a.R);
+  long long sl = row / a.R;
+  const int s = (int)(sl % a.S); sl /= a.S;
+  const int h = (int)(sl % a.H);
+  const int b = (int)(sl / a.H);
+  const T* og = reinterpret_cast<const T*>(a.o) + off4(a.so, b, h, s, i);
+  const T* g = reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, b, h, s, i);
+  const T* gt = reinterpret_cast<const T*>(a.gate) + off4(a.sgate, b, h, s, i);
+  T* dg = reinterpret_cast<T*>(a.dgate) + off4(a.sdgate, b, h, s, i);
+  float acc = 0.f;
+  for (int d = lane; d < a.D; d += 32) {
+    const float G = to_float<T>(g[d]), O = to_float<T>(og[d]);
+    const float sg = sigmoidf_fast(to_float<T>(gt[d]));
+    acc += G * O;
+    d_o_eff[row * a.D + d] = from_float<T>(G * sg);
+    dg[d] = from_float<T>(G * O * (1.f - sg));
+  }
+  acc = warp_sum(acc);
+  if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
+}
+
 // dQ: one warp per query row, lanes over keys.
 template <class T>
 __global__ void __launch_bounds__(GW * 32) generic_dq_kernel(Args a) {
@@ -329,10 +362,15 @@ static cudaError_t launch_fwd_t(const Args& a, cudaStream_t st, int* launches) {
 }
 
 template <class T>
-static cudaError_t launch_bwd_t(const Args& a, cudaStream_t st, int* launches) {
+static cudaError_t launch_bwd_t(Args a, cudaStream_t st, int* launches) {
   const int DP = a.D + 1;
   const long long rows = (long long)a.B * a.H * a.S * a.R;
-  if (!a.delta_ready) generic_delta_kernel<T><<<(unsigned)((rows + GW - 1) / GW), GW * 32, 0, st>>>(a);
+  if (a.dgate) {
+    generic_gate_backward_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a);
+    use_effective_d_o(&a);
+  } else {
+    generic_delta_kernel<T><<<(unsigned)((rows + GW - 1) / GW), GW * 32, 0, st>>>(a);
+  }
   dim3 grid(a.B * a.H * a.S, (a.R + GW - 1) / GW);
   generic_dq_kernel<T><<<grid, GW * 32, (size_t)(2 * GT + 2 * GW) * DP * sizeof(float), st>>>(a);
   generic_dkdv_kernel<T><<<grid, GW * 32, ((size_t)(2 * GT + 2 * GW) * DP + 2 * GT) * sizeof(float), st>>>(a);

@@ -57,13 +57,13 @@ int launch_sm100_bwd(int dtype, const Args& a, void* workspace, size_t workspace
 int launch_peer_allreduce(const evoattn_peer_allreduce_params* p, cudaStream_t st);
 bool exchange_lane(cudaStream_t* side, cudaEvent_t* fork, cudaEvent_t* join);
 
-// fp32 rows of `cols` values with a row stride of `ld` -> dense rows (extras.cu): d(pair_bias) leaving
-// the padded buffer it was summed in.
-void launch_dbias_dense(const float* src, int ld, float* dst, long long rows, int cols, cudaStream_t st);
+// d(pair_bias) from the fp32 buffer it was summed in to a.dbias_out, in its type and layout (extras.cu).
+int launch_dbias_out(const Args& a, cudaStream_t st, int* launches);
 
-// Backward half of the gated output (extras.cu): writes delta, the effective dO (into `scratch`) and
-// dgate, and redirects `a` to the effective dO.
-size_t gate_backward_scratch_bytes(int dtype, const Args& a);
-int launch_gate_backward(int dtype, Args* a, void* scratch, void* dgate, const Str4& sdgate, cudaStream_t st, int* launches);
+// From here on `a` reads the effective dO of a gated output (contiguous, in scratch).
+inline void use_effective_d_o(Args* a) {
+  a->d_o = a->d_o_eff;
+  a->sdo = Str4{(long long)a->H * a->S * a->R * a->D, (long long)a->S * a->R * a->D, (long long)a->R * a->D, (long long)a->D};
+}
 
 }  // namespace evo

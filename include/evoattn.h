@@ -25,7 +25,7 @@
 extern "C" {
 #endif
 
-#define EVOATTN_ABI_VERSION 3
+#define EVOATTN_ABI_VERSION 4
 
 /* status codes (0 = success). */
 enum {
@@ -130,6 +130,11 @@ typedef struct evoattn_bwd_params {
                              launched as soon as d(pair_bias) is complete, on a stream of the library's
                              own, next to the call's remaining kernel; the call's stream then waits
                              for it, so everything the call returns is ordered on `cuda_stream` as usual */
+  void* dbias_cast;       /* optional (null: none), instead of dbias: d(pair_bias) in the type and layout the
+                             caller wants it in.  The sum stays fp32 (in the workspace) until this one
+                             conversion, which is the call's last step for it */
+  int32_t dbias_cast_dtype;       /* EVOATTN_BF16 / FP16 / FP32 */
+  int32_t dbias_cast_heads_last;  /* 0: [B,H,R,R]; otherwise [B,R,R,H] */
 } evoattn_bwd_params;
 
 /* ABI version of the loaded library; compare with EVOATTN_ABI_VERSION. */
