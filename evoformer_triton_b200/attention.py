@@ -5,9 +5,12 @@ name, same ``apply(Q, K, V, res_mask, pair_bias)`` call on ``[B, N_seq, N_res, H
 tensors, same reinterpretation of those tensors as ``[B, H, N_seq, N_res, D]``
 (evoformer.py:648-650), same ``(dQ, dK, dV, None, d_pair_bias)`` gradients.  The device
 work is done by libevoattn.so through its C ABI; torch is used for memory and streams.
+A call goes through the native boundary (csrc/host.cpp); the raw forward and backward below are the
+same steps in Python, for the N_seq-sharded op and for callers that hold attention-view tensors.
 """
 from __future__ import annotations
 
+import collections.abc
 import contextlib
 import ctypes as C
 import os
@@ -20,47 +23,62 @@ from . import _lib
 
 _DTYPES = {torch.bfloat16: _lib.BF16, torch.float16: _lib.FP16, torch.float32: _lib.FP32}
 
-# Launch counters the benchmark reads (kernels of this library only).
-launches = {"fwd": 0, "bwd": 0}
-last_path = {"fwd": _lib.PATH_NONE, "bwd": _lib.PATH_NONE}
-_force_generic = bool(int(os.environ.get("EVOATTN_FORCE_GENERIC", "0")))
-_status_words = {}
+
+class _LastCall(collections.abc.Mapping):
+    """What the most recent forward and backward call of the process reported."""
+
+    def __init__(self, read):
+        self._read = read
+
+    def __getitem__(self, key):
+        return dict(zip(("fwd", "bwd"), self._read(_lib.host())))[key]
+
+    def __iter__(self):
+        return iter(("fwd", "bwd"))
+
+    def __len__(self):
+        return 2
+
+    def __repr__(self):
+        return repr(dict(self))
+
+
+# Launch counters the benchmark reads (kernels of this library only), and which kernel family ran.
+launches = _LastCall(lambda h: h.launch_counts())
+last_path = _LastCall(lambda h: h.paths())
+_force_generic = False
 
 
 def force_generic(on: bool) -> None:
     """Route every call to the CUDA-core kernels (used by tests to cross-check)."""
     global _force_generic
     _force_generic = bool(on)
+    _lib.host().force_generic(_force_generic)
+
+
+if int(os.environ.get("EVOATTN_FORCE_GENERIC", "0")):
+    force_generic(True)
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
     """One int32 per device that kernels set when they give up a bounded wait."""
-    t = _status_words.get(device)
-    if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=device)
-        _status_words[device] = t
-    return t
+    return _lib.host().status_word(torch.cuda.current_device() if device.index is None else device.index)
 
 
 def check_device_status(device=None) -> None:
     """Synchronise and raise if any kernel reported a timed-out wait."""
-    for dev, t in list(_status_words.items()):
-        if device is not None and torch.device(device) != dev:
+    for t in _lib.host().status_words():
+        if device is not None and torch.device(device) != t.device:
             continue
         v = int(t.item())
         if v != 0:
             t.zero_()
-            raise RuntimeError(f"evoattn kernel on {dev} gave up a bounded wait (device status {v})")
+            raise RuntimeError(f"evoattn kernel on {t.device} gave up a bounded wait (device status {v})")
 
 
 def _strides4(t: torch.Tensor):
     st = t.stride()
     return (C.c_int64 * 4)(st[0], st[1], st[2], st[3])
-
-
-def _require_cuda(t: torch.Tensor):
-    if not t.is_cuda:
-        raise RuntimeError("EvoformerAttention runs on CUDA tensors only; there is no CPU fallback")
 
 
 def _fill_fwd(p: "_lib.FwdParams", q, k, v, o, lse, mask, bias, scale, gate=None):
@@ -135,8 +153,7 @@ def attention_forward(q, k, v, mask, bias, scale, gate=None):
     stream = torch.cuda.current_stream(q.device).cuda_stream
     with torch.cuda.device(q.device):
         _lib.check(lib.evoattn_fwd(C.byref(p), C.c_void_p(stream)), "evoattn_fwd")
-    launches["fwd"] = lib.evoattn_last_launch_count()
-    last_path["fwd"] = lib.evoattn_last_path()
+    _lib.host().note_fwd(lib.evoattn_last_launch_count(), lib.evoattn_last_path())
     return o, lse
 
 
@@ -181,8 +198,7 @@ def attention_backward(q, k, v, o, lse, mask, bias, scale, d_o, want_dbias=True,
     stream = torch.cuda.current_stream(q.device).cuda_stream
     with torch.cuda.device(q.device):
         _lib.check(lib.evoattn_bwd(C.byref(p), C.c_void_p(stream)), "evoattn_bwd")
-    launches["bwd"] = lib.evoattn_last_launch_count()
-    last_path["bwd"] = lib.evoattn_last_path()
+    _lib.host().note_bwd(lib.evoattn_last_launch_count(), lib.evoattn_last_path())
     if gate is None and not want_dmask:
         return dq, dk, dv, dbias
     return dq, dk, dv, dbias, dgate, dmask
@@ -261,7 +277,9 @@ def pair_bias_grad_summed_over(group, peer_reducer=None):
 
 
 class _EvoformerAttentionBase(torch.autograd.Function):
-    """Shared implementation; ``layout`` (how heads are found in Q/K/V) and ``bias_layout``
+    """What the public classes share.  A call goes to the native boundary (csrc/host.cpp); inside
+    :func:`pair_bias_grad_summed_over` it is this Function itself, whose backward sums d(pair_bias)
+    over the ranks.  ``layout`` (how heads are found in Q/K/V) and ``bias_layout``
     (``"b1hrr"``: the reference's ``[B, 1, H, R, R]``; ``"brrh"``: ``[B, R, R, H]`` as a linear
     layer emits it) are fixed by the public subclasses."""
 
@@ -269,9 +287,17 @@ class _EvoformerAttentionBase(torch.autograd.Function):
     bias_layout = "b1hrr"
 
     @classmethod
+    def apply(cls, Q, K, V, res_mask=None, pair_bias=None, *gate):
+        if getattr(_pending, "group", None) is not None:
+            return super().apply(Q, K, V, res_mask, pair_bias, *gate)
+        return _lib.host().attention(Q, K, V, res_mask, pair_bias, gate[0] if gate else None,
+                                     cls.layout == "true", cls.bias_layout == "brrh")
+
+    @classmethod
     def _forward(cls, ctx, Q, K, V, res_mask, pair_bias, gate=None):
         for t in (Q, K, V):
-            _require_cuda(t)
+            if not t.is_cuda:
+                raise RuntimeError("EvoformerAttention runs on CUDA tensors only; there is no CPU fallback")
         if not (Q.shape[-1] == K.shape[-1] == V.shape[-1]):
             raise AssertionError("Q, K, V must share the head dimension")  # evoformer.py:642-643
         if Q.dtype not in _DTYPES or K.dtype != Q.dtype or V.dtype != Q.dtype:
@@ -309,8 +335,7 @@ class _EvoformerAttentionBase(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, mask, bias, o, lse, g)  # evoformer.py:729
         ctx.softmax_scale = scale
         ctx.bias_meta = None if pair_bias is None else (pair_bias.dtype, tuple(pair_bias.shape))
-        ctx.mask_meta = None if res_mask is None else (res_mask.dtype, tuple(res_mask.shape))
-        ctx.reduce_group = getattr(_pending, "group", None)
+        ctx.reduce_group = _pending.group
         return _unview(o, cls.layout)
 
     @classmethod
@@ -322,23 +347,22 @@ class _EvoformerAttentionBase(torch.autograd.Function):
         if d_o.dtype != q.dtype:
             d_o = d_o.to(q.dtype)
         want_dbias = bias is not None and ctx.needs_input_grad[4]
-        # an additive mask that asks for a gradient gets one (DS4Sci returns gradients for both
-        # biases; the reference returns None, evoformer.py:862)
-        want_dmask = mask is not None and mask.is_floating_point() and ctx.needs_input_grad[3]
-        reducer = ctx.reduce_group[1] if (ctx.reduce_group is not None and want_dbias) else None
+        if mask is not None and mask.is_floating_point() and ctx.needs_input_grad[3]:
+            raise RuntimeError("a mask gradient is not available in the N_seq-sharded op (the mask rows are sharded)")
+        reducer = ctx.reduce_group[1] if want_dbias else None
         dbias_out = reducer.buffer(bias.numel()) if reducer is not None else None
         # (with a peer reducer the call sums d(pair_bias) over the ranks itself, next to its last kernel)
         res = attention_backward(q, k, v, o, lse, mask, bias, ctx.softmax_scale, d_o, want_dbias=want_dbias,
-                                 dbias_out=dbias_out, gate=g, want_dmask=want_dmask,
+                                 dbias_out=dbias_out, gate=g,
                                  exchange=None if reducer is None else reducer.exchange_params(bias.numel()))
         dq, dk, dv, dbias = res[:4]
-        dgate, dmask = (res[4], res[5]) if len(res) > 4 else (None, None)
+        dgate = res[4] if len(res) > 4 else None
         d_pair_bias = None
         if dbias is not None:
             dtype, shape = ctx.bias_meta
             if reducer is not None:  # N_seq is sharded: the other ranks' rows belong to the sum
                 pass                 # (summed inside the backward call)
-            elif ctx.reduce_group is not None:
+            else:
                 import torch.distributed as dist
                 dist.all_reduce(dbias, op=dist.ReduceOp.SUM, group=ctx.reduce_group[0])
             # the sum over N_seq stays in fp32 until this single cast (evoformer.py:860 casts to dO's dtype)
@@ -348,14 +372,7 @@ class _EvoformerAttentionBase(torch.autograd.Function):
                 d_pair_bias = dbias.reshape(shape).to(dtype)
                 if reducer is not None and d_pair_bias.data_ptr() == dbias.data_ptr():
                     d_pair_bias = d_pair_bias.clone()  # the exchange buffer is reused by the next call
-        d_mask = None
-        if dmask is not None:
-            if ctx.reduce_group is None:
-                mdtype, mshape = ctx.mask_meta
-                d_mask = dmask.reshape(mshape).to(mdtype)
-            else:
-                raise RuntimeError("a mask gradient is not available in the N_seq-sharded op (the mask rows are sharded)")
-        grads = (_unview(dq, cls.layout), _unview(dk, cls.layout), _unview(dv, cls.layout), d_mask, d_pair_bias)
+        grads = (_unview(dq, cls.layout), _unview(dk, cls.layout), _unview(dv, cls.layout), None, d_pair_bias)
         if g is not None:
             grads = grads + (_unview(dgate, cls.layout),)
         return grads
@@ -454,5 +471,7 @@ def evoformer_attention(Q, K, V, biases: Optional[Sequence[Optional[torch.Tensor
     biases = list(biases or [])
     while len(biases) < 2:
         biases.append(None)
+    if getattr(_pending, "group", None) is None:
+        return _lib.host().attention(Q, K, V, biases[0], biases[1], gate, layout == "true", pair_bias_layout == "brrh")
     fn = _variant("true" if layout == "true" else "reinterpret", pair_bias_layout, gate is not None)
     return fn.apply(Q, K, V, biases[0], biases[1], gate)
