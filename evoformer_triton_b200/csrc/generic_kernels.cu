@@ -1,23 +1,36 @@
 // CUDA-core Evoformer attention kernels: any dtype (fp32 included), any D <= 128, any R.
 //
-// These serve fp32 inputs (tensor cores would lose bits there) and every shape the
-// tcgen05 kernels do not cover.  They are written for clarity and determinism, not
-// speed: one warp owns one score row, every sum has a fixed order, and the pair-bias
-// gradient is produced by one owner per element instead of the reference's fp32
-// atomics (dsevoformer-triton/evoformer.py:458).
+// These serve fp32 inputs (tensor cores would lose bits there) and every shape the tcgen05 kernels do
+// not cover.  fp32 math throughout, every sum in a fixed order: the pair-bias gradient is produced by
+// one owner per element instead of the reference's fp32 atomics (dsevoformer-triton/evoformer.py:458),
+// and dQ, dK/dV and d(pair_bias) each recompute the scores, so results are the same bits on every run.
 //
-// Math (evoformer.py:68-89 forward, :450-462 and :594-614 backward), fp32 throughout:
+// Math (evoformer.py:68-89 forward, :450-462 and :594-614 backward):
 //   x_ij = scale * <q_i,k_j> + bias_ij ;  mask ;  P = softmax_j(x) ;  O = P V
 //   delta_i = <dO_i,O_i> ; dP_ij = <dO_i,v_j> ; dS = P (dP - delta)
 //   dV_j = sum_i P_ij dO_i ; dQ_i = scale sum_j dS_ij k_j ; dK_j = scale sum_i dS_ij q_i
 //   dBias_ij = sum_s dS_ij
+//
+// Bound by the fp32 FMA rate.  A block of 256 threads works on 64 x 64 scores, 4 x 4 per thread, so that
+// a 16-byte shared load feeds 16 multiply-adds: rows are strided over the threads (i = ty + 16 r,
+// j = tx + 16 c) and a staged row has DP + 4 floats, which makes the 16-byte loads of eight
+// neighbouring lanes hit all 32 banks once without transposing anything on the way in.
 #include "common.cuh"
 #include "launch.h"
+#include "ptx.cuh"
 
 namespace evo {
+namespace {
 
-constexpr int GW = 8;   // warps per CTA = score rows per CTA
-constexpr int GT = 32;  // rows staged in shared memory per step (one per lane)
+using ptx::F2;
+using ptx::f2_fma;
+using ptx::f2_get;
+using ptx::f2_make;
+
+constexpr int TT = 64;        // rows of a tile (queries and keys)
+constexpr int TB = 32;        // ... of a d(pair_bias) tile
+constexpr int NTH = 256;
+constexpr int PLD = TT + 4;   // row stride of a staged score tile
 
 struct Slab {
   int b, h, s;
@@ -30,26 +43,126 @@ __device__ __forceinline__ Slab slab_of(int idx, const Args& a) {
   return r;
 }
 
-template <class T>
-__device__ __forceinline__ void stage_rows(float* dst, int DP, const T* base, const Str4& st, int b, int h, int s,
-                                           int r0, int R, int D) {
-  for (int idx = threadIdx.x; idx < GT * D; idx += blockDim.x) {
-    int rr = idx / D, d = idx - rr * D;
-    int r = r0 + rr;
-    dst[rr * DP + d] = (r < R) ? to_float<T>(base[off4(st, b, h, s, r) + d]) : 0.f;
+// `n` rows r0.. of slab (b,h,s) -> shared memory, widened, rows of DP + 4 floats; zeros beyond R and D.
+// `t` of `nt` threads take part.
+template <class T, int DP>
+__device__ __forceinline__ void stage_rows(float* dst, const T* x, const Str4& st, const Slab& sl, int r0, int n, int R, int D,
+                                           bool vec, int t, int nt) {
+  constexpr int LD = DP + 4, C4 = DP / 4;
+  const T* base = x + off4(st, sl.b, sl.h, sl.s, 0);
+  for (int e = t; e < n * C4; e += nt) {
+    const int rr = e / C4, d = (e - rr * C4) * 4, r = r0 + rr;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < R) {
+      const T* p = base + (long long)r * st.r + d;
+      if (vec && d + 4 <= D) {
+        if constexpr (sizeof(T) == 4) {
+          v = *reinterpret_cast<const float4*>(p);
+        } else {
+          const uint2 w = *reinterpret_cast<const uint2*>(p);
+          const T* h = reinterpret_cast<const T*>(&w);
+          v = make_float4(to_float<T>(h[0]), to_float<T>(h[1]), to_float<T>(h[2]), to_float<T>(h[3]));
+        }
+      } else {
+        if (d < D) v.x = to_float<T>(p[0]);
+        if (d + 1 < D) v.y = to_float<T>(p[1]);
+        if (d + 2 < D) v.z = to_float<T>(p[2]);
+        if (d + 3 < D) v.w = to_float<T>(p[3]);
+      }
+    }
+    *reinterpret_cast<float4*>(dst + rr * LD + d) = v;
   }
 }
 
-// Score of (i, j) before the softmax, with mask applied.  `replaced` tells the caller
-// that the score is a constant (boolean mask dropped the key).
+// acc[r][c] = <A row ty + W r, B row tx + W c> over DP columns.  Two columns per instruction: the even
+// and the odd ones are summed apart and added at the end.
+template <int DP, int W>
+__device__ __forceinline__ void dots(float (&acc)[4][4], const float* A, const float* B, int ty, int tx) {
+  constexpr int LD = DP + 4;
+  F2 s[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) s[r][c] = f2_make(0.f, 0.f);
+#pragma unroll 4
+  for (int d = 0; d < DP; d += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + (ty + W * r) * LD + d);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) b[c] = *reinterpret_cast<const float4*>(B + (tx + W * c) * LD + d);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        s[r][c] = f2_fma(f2_make(a[r].x, a[r].y), f2_make(b[c].x, b[c].y), s[r][c]);
+        s[r][c] = f2_fma(f2_make(a[r].z, a[r].w), f2_make(b[c].z, b[c].w), s[r][c]);
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float lo, hi;
+      f2_get(s[r][c], lo, hi);
+      acc[r][c] = lo + hi;
+    }
+}
+
+// The columns of a [rows][DP] product that a thread owns: NC of them, in runs of VEC.
+template <int DP>
+struct Cols {
+  static constexpr int NC = DP / 16, VEC = NC < 4 ? NC : 4;
+  static __device__ __forceinline__ int at(int tx, int n) { return (n / VEC) * (16 * VEC) + tx * VEC + n % VEC; }
+};
+
+// acc[r][n] += sum_j P[ty + 16 r][j] * V[j][col n] over the 64 rows of V.
+template <int DP>
+__device__ __forceinline__ void weighted_rows(float (&acc)[4][DP / 16], const float* P, const float* V, int ty, int tx) {
+  using C = Cols<DP>;
+  constexpr int LD = DP + 4;
+#pragma unroll 4
+  for (int j = 0; j < TT; j += 4) {
+    float p[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float4 t = *reinterpret_cast<const float4*>(P + (ty + 16 * r) * PLD + j);
+      p[r][0] = t.x; p[r][1] = t.y; p[r][2] = t.z; p[r][3] = t.w;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      float v[C::NC];
+#pragma unroll
+      for (int n = 0; n < C::NC; n += C::VEC) {
+        const float* src = V + (j + u) * LD + C::at(tx, n);
+        if constexpr (C::VEC == 4) {
+          const float4 t = *reinterpret_cast<const float4*>(src);
+          v[n] = t.x; v[n + 1] = t.y; v[n + 2] = t.z; v[n + 3] = t.w;
+        } else if constexpr (C::VEC == 2) {
+          const float2 t = *reinterpret_cast<const float2*>(src);
+          v[n] = t.x; v[n + 1] = t.y;
+        } else {
+          v[n] = *src;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int n = 0; n < C::NC; ++n) acc[r][n] += p[r][u] * v[n];
+    }
+  }
+}
+
+// Score of (i, j) before the softmax, with mask applied.  `replaced` tells the caller that the score is a
+// constant (boolean mask dropped the key).
 template <class T>
-__device__ __forceinline__ float score(const Args& a, int b, int h, int s, int i, int j, float dot, bool& replaced) {
+__device__ __forceinline__ float score(const Args& a, const Slab& sl, int i, int j, float dot, bool& replaced) {
   float x = dot * a.scale;
-  if (a.bias) x += load_bias<T>(a, b, h, i, j);
+  if (a.bias) x += load_bias<T>(a, sl.b, sl.h, i, j);
   replaced = false;
   if (a.mask_kind != EVOATTN_MASK_NONE)
-    x = apply_mask<T>(x, a.mask, a.mask_kind, (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c,
-                      replaced);
+    x = apply_mask<T>(x, a.mask, a.mask_kind,
+                      (long long)sl.b * a.smask.a + (long long)sl.s * a.smask.b + (long long)j * a.smask.c, replaced);
   return x;
 }
 
@@ -60,69 +173,89 @@ __device__ __forceinline__ float prob_from_lse(float x, float lse, int R) {
   return expf(x - lse);
 }
 
-template <class T>
-__global__ void __launch_bounds__(GW * 32) generic_fwd_kernel(Args a) {
-  extern __shared__ float sm[];
-  const int D = a.D, DP = D + 1;
-  float* Ks = sm;
-  float* Vs = Ks + GT * DP;
-  float* Qs = Vs + GT * DP;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Which loads of a tensor may take 16 bytes (fp32) or 8 (16-bit) at a time.
+enum : int { VEC_Q = 1, VEC_K = 2, VEC_V = 4, VEC_DO = 8 };
+
+template <class T, int DP>
+__global__ void __launch_bounds__(NTH, DP <= 64 ? 2 : 1) generic_fwd_kernel(const Args a, const int vec) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int LD = DP + 4;
+  float* Qs = sm;
+  float* Ks = Qs + TT * LD;
+  float* Vs = Ks + TT * LD;
+  float* Ps = Vs + TT * LD;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const Slab sl = slab_of(blockIdx.x, a);
-  const int i = blockIdx.y * GW + warp;
-  const bool row_ok = i < a.R;
-  const int ic = row_ok ? i : 0;
-  const T* q = reinterpret_cast<const T*>(a.q) + off4(a.sq, sl.b, sl.h, sl.s, ic);
-  for (int d = lane; d < D; d += 32) Qs[warp * DP + d] = to_float<T>(q[d]);
-  float m = -INFINITY, l = 0.f;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int j0 = 0; j0 < a.R; j0 += GT) {
-    __syncthreads();
-    stage_rows<T>(Ks, DP, reinterpret_cast<const T*>(a.k), a.sk, sl.b, sl.h, sl.s, j0, a.R, D);
-    stage_rows<T>(Vs, DP, reinterpret_cast<const T*>(a.v), a.sv, sl.b, sl.h, sl.s, j0, a.R, D);
-    __syncthreads();
-    const int j = j0 + lane;
-    float x = -INFINITY;
-    if (j < a.R) {
-      float dot = 0.f;
-      for (int d = 0; d < D; ++d) dot += Qs[warp * DP + d] * Ks[lane * DP + d];
-      bool rep;
-      x = score<T>(a, sl.b, sl.h, sl.s, ic, j, dot, rep);
-    }
-    const float mn = fmaxf(m, warp_max(x));
-    const float alpha = expf(m - mn);
-    const float p = (j < a.R) ? expf(x - mn) : 0.f;
-    l = l * alpha + warp_sum(p);
+  const int i0 = blockIdx.y * TT;
+  stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
+  float m[4], l[4], acc[4][DP / 16];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) acc[t] *= alpha;
-    for (int jj = 0; jj < GT; ++jj) {
-      const float pj = __shfl_sync(0xffffffffu, p, jj);
+  for (int r = 0; r < 4; ++r) {
+    m[r] = -INFINITY;
+    l[r] = 0.f;
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int d = lane + 32 * t;
-        if (d < D) acc[t] += pj * Vs[jj * DP + d];
-      }
-    }
-    m = mn;
+    for (int n = 0; n < DP / 16; ++n) acc[r][n] = 0.f;
   }
-  if (row_ok) {
+  for (int j0 = 0; j0 < a.R; j0 += TT) {
+    __syncthreads();
+    stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
+    stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
+    __syncthreads();
+    float x[4][4];
+    dots<DP, 16>(x, Qs, Ks, ty, tx);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = min(i0 + ty + 16 * r, a.R - 1);
+      float mx = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int j = j0 + tx + 16 * c;
+        bool rep;
+        x[r][c] = j < a.R ? score<T>(a, sl, i, j, x[r][c], rep) : -INFINITY;
+        mx = fmaxf(mx, x[r][c]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const float mn = fmaxf(m[r], mx), alpha = expf(m[r] - mn);
+      float sum = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const float p = (j0 + tx + 16 * c < a.R) ? expf(x[r][c] - mn) : 0.f;
+        sum += p;
+        Ps[(ty + 16 * r) * PLD + tx + 16 * c] = p;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l[r] = l[r] * alpha + sum;
+      m[r] = mn;
+#pragma unroll
+      for (int n = 0; n < DP / 16; ++n) acc[r][n] *= alpha;
+    }
+    __syncwarp();  // (a row of P is written and read by the same half-warp)
+    weighted_rows<DP>(acc, Ps, Vs, ty, tx);
+    __syncwarp();
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + ty + 16 * r;
+    if (i >= a.R) continue;
     T* o = reinterpret_cast<T*>(a.o) + off4(a.so, sl.b, sl.h, sl.s, i);
     const T* gate = a.gate ? reinterpret_cast<const T*>(a.gate) + off4(a.sgate, sl.b, sl.h, sl.s, i) : nullptr;
-    const float inv = 1.f / l;
+    const float inv = 1.f / l[r];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int d = lane + 32 * t;
-      if (d < D) o[d] = from_float<T>(acc[t] * inv * (gate ? sigmoidf_fast(to_float<T>(gate[d])) : 1.f));
+    for (int n = 0; n < DP / 16; ++n) {
+      const int d = Cols<DP>::at(tx, n);
+      if (d < a.D) o[d] = from_float<T>(acc[r][n] * inv * (gate ? sigmoidf_fast(to_float<T>(gate[d])) : 1.f));
     }
-    if (lane == 0) a.lse[((long long)blockIdx.x) * a.R + i] = m + logf(l);
+    if (tx == 0) a.lse[((long long)blockIdx.x) * a.R + i] = m[r] + logf(l[r]);
   }
 }
 
 // delta[b,h,s,i] = <dO_i, O_i>   (evoformer.py:299-326)
 template <class T>
-__global__ void __launch_bounds__(GW * 32) generic_delta_kernel(Args a) {
+__global__ void __launch_bounds__(256) generic_delta_kernel(Args a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * GW + warp;
+  const long long row = (long long)blockIdx.x * 8 + warp;
   const long long rows = (long long)a.B * a.H * a.S * a.R;
   if (row >= rows) return;
   const int i = (int)(row % a.R);
@@ -168,234 +301,280 @@ __global__ void __launch_bounds__(256) generic_gate_backward_kernel(Args a) {
   if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
 }
 
-// dQ: one warp per query row, lanes over keys.
-template <class T>
-__global__ void __launch_bounds__(GW * 32) generic_dq_kernel(Args a) {
-  extern __shared__ float sm[];
-  const int D = a.D, DP = D + 1;
-  float* Ks = sm;
-  float* Vs = Ks + GT * DP;
-  float* Qs = Vs + GT * DP;
-  float* Gs = Qs + GW * DP;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Slab sl = slab_of(blockIdx.x, a);
-  const int i = blockIdx.y * GW + warp;
-  const bool row_ok = i < a.R;
-  const int ic = row_ok ? i : 0;
-  const T* q = reinterpret_cast<const T*>(a.q) + off4(a.sq, sl.b, sl.h, sl.s, ic);
-  const T* g = reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, sl.b, sl.h, sl.s, ic);
-  for (int d = lane; d < D; d += 32) {
-    Qs[warp * DP + d] = to_float<T>(q[d]);
-    Gs[warp * DP + d] = to_float<T>(g[d]);
-  }
-  const float lse = a.lse[(long long)blockIdx.x * a.R + ic];
-  const float delta = a.delta[(long long)blockIdx.x * a.delta_ld + ic];
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int j0 = 0; j0 < a.R; j0 += GT) {
-    __syncthreads();
-    stage_rows<T>(Ks, DP, reinterpret_cast<const T*>(a.k), a.sk, sl.b, sl.h, sl.s, j0, a.R, D);
-    stage_rows<T>(Vs, DP, reinterpret_cast<const T*>(a.v), a.sv, sl.b, sl.h, sl.s, j0, a.R, D);
-    __syncthreads();
-    const int j = j0 + lane;
-    float ds = 0.f;
-    if (j < a.R) {
-      float dot = 0.f, dp = 0.f;
-      for (int d = 0; d < D; ++d) {
-        dot += Qs[warp * DP + d] * Ks[lane * DP + d];
-        dp += Gs[warp * DP + d] * Vs[lane * DP + d];
-      }
+// P and dS of a 4 x 4 patch from its two dot products; both 0 outside the R x R scores.
+template <class T, int W>
+__device__ __forceinline__ void probs(const Args& a, const Slab& sl, long long slab, int i0, int j0, int ty, int tx,
+                                      float (&p)[4][4], float (&ds)[4][4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + ty + W * r, ic = min(i, a.R - 1);
+    const float lse = a.lse[slab * a.R + ic], delta = a.delta[slab * a.delta_ld + ic];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int j = j0 + tx + W * c;
       bool rep;
-      const float x = score<T>(a, sl.b, sl.h, sl.s, ic, j, dot, rep);
-      const float p = prob_from_lse(x, lse, a.R);
-      ds = rep ? 0.f : p * (dp - delta);
-    }
-    for (int jj = 0; jj < GT; ++jj) {
-      const float dj = __shfl_sync(0xffffffffu, ds, jj);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int d = lane + 32 * t;
-        if (d < D) acc[t] += dj * Ks[jj * DP + d];
-      }
-    }
-  }
-  if (row_ok) {
-    T* o = reinterpret_cast<T*>(a.dq) + off4(a.sdq, sl.b, sl.h, sl.s, i);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int d = lane + 32 * t;
-      if (d < D) o[d] = from_float<T>(acc[t] * a.scale);
+      const float x = score<T>(a, sl, ic, min(j, a.R - 1), p[r][c], rep);
+      const bool in = i < a.R && j < a.R;
+      p[r][c] = in ? prob_from_lse(x, lse, a.R) : 0.f;
+      ds[r][c] = (in && !rep) ? p[r][c] * (ds[r][c] - delta) : 0.f;
     }
   }
 }
 
-// dK, dV: one warp per key row, lanes over queries.
-template <class T>
-__global__ void __launch_bounds__(GW * 32) generic_dkdv_kernel(Args a) {
-  extern __shared__ float sm[];
-  const int D = a.D, DP = D + 1;
-  float* Qs = sm;                  // [GT][DP]
-  float* Gs = Qs + GT * DP;        // [GT][DP]
-  float* Kw = Gs + GT * DP;        // [GW][DP]
-  float* Vw = Kw + GW * DP;        // [GW][DP]
-  float* Ls = Vw + GW * DP;        // [GT] lse
-  float* Ds = Ls + GT;             // [GT] delta
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Slab sl = slab_of(blockIdx.x, a);
-  const int j = blockIdx.y * GW + warp;
-  const bool row_ok = j < a.R;
-  const int jc = row_ok ? j : 0;
-  const T* k = reinterpret_cast<const T*>(a.k) + off4(a.sk, sl.b, sl.h, sl.s, jc);
-  const T* v = reinterpret_cast<const T*>(a.v) + off4(a.sv, sl.b, sl.h, sl.s, jc);
-  for (int d = lane; d < D; d += 32) {
-    Kw[warp * DP + d] = to_float<T>(k[d]);
-    Vw[warp * DP + d] = to_float<T>(v[d]);
-  }
-  float accK[4] = {0.f, 0.f, 0.f, 0.f}, accV[4] = {0.f, 0.f, 0.f, 0.f};
-  float dmask_acc = 0.f;  // this lane's share of sum_i dS_ij (gradient of an additive mask)
-  for (int i0 = 0; i0 < a.R; i0 += GT) {
+// dQ of 64 queries: walks the keys.
+template <class T, int DP>
+__device__ __forceinline__ void dq_role(const Args& a, int vec, float* sm, int slab, int i0) {
+  constexpr int LD = DP + 4;
+  float* Qs = sm;
+  float* Gs = Qs + TT * LD;
+  float* Ks = Gs + TT * LD;
+  float* Vs = Ks + TT * LD;
+  float* Ds = Vs + TT * LD;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const Slab sl = slab_of(slab, a);
+  stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
+  stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO, threadIdx.x, NTH);
+  float acc[4][DP / 16] = {};
+  for (int j0 = 0; j0 < a.R; j0 += TT) {
     __syncthreads();
-    stage_rows<T>(Qs, DP, reinterpret_cast<const T*>(a.q), a.sq, sl.b, sl.h, sl.s, i0, a.R, D);
-    stage_rows<T>(Gs, DP, reinterpret_cast<const T*>(a.d_o), a.sdo, sl.b, sl.h, sl.s, i0, a.R, D);
-    if (threadIdx.x < GT) {
-      const int i = i0 + threadIdx.x;
-      Ls[threadIdx.x] = (i < a.R) ? a.lse[(long long)blockIdx.x * a.R + i] : 0.f;
-      Ds[threadIdx.x] = (i < a.R) ? a.delta[(long long)blockIdx.x * a.delta_ld + i] : 0.f;
-    }
+    stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
+    stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
     __syncthreads();
-    const int i = i0 + lane;
-    float p = 0.f, ds = 0.f;
-    if (i < a.R) {
-      float dot = 0.f, dp = 0.f;
-      for (int d = 0; d < D; ++d) {
-        dot += Qs[lane * DP + d] * Kw[warp * DP + d];
-        dp += Gs[lane * DP + d] * Vw[warp * DP + d];
-      }
-      bool rep;
-      const float x = score<T>(a, sl.b, sl.h, sl.s, i, jc, dot, rep);
-      p = prob_from_lse(x, Ls[lane], a.R);
-      ds = rep ? 0.f : p * (dp - Ds[lane]);
-      dmask_acc += ds;
-    }
-    for (int ii = 0; ii < GT; ++ii) {
-      const float pi = __shfl_sync(0xffffffffu, p, ii);
-      const float di = __shfl_sync(0xffffffffu, ds, ii);
+    float p[4][4], ds[4][4];
+    dots<DP, 16>(p, Qs, Ks, ty, tx);
+    dots<DP, 16>(ds, Gs, Vs, ty, tx);
+    probs<T, 16>(a, sl, slab, i0, j0, ty, tx, p, ds);
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int d = lane + 32 * t;
-        if (d < D) {
-          accV[t] += pi * Gs[ii * DP + d];
-          accK[t] += di * Qs[ii * DP + d];
-        }
-      }
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) Ds[(ty + 16 * r) * PLD + tx + 16 * c] = ds[r][c];
+    __syncwarp();  // (a row of dS is written and read by the same half-warp)
+    weighted_rows<DP>(acc, Ds, Ks, ty, tx);
+    __syncwarp();
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + ty + 16 * r;
+    if (i >= a.R) continue;
+    T* o = reinterpret_cast<T*>(a.dq) + off4(a.sdq, sl.b, sl.h, sl.s, i);
+#pragma unroll
+    for (int n = 0; n < DP / 16; ++n) {
+      const int d = Cols<DP>::at(tx, n);
+      if (d < a.D) o[d] = from_float<T>(acc[r][n] * a.scale);
     }
+  }
+}
+
+// dK, dV of 64 keys (and their share of an additive mask's gradient): walks the queries.
+template <class T, int DP>
+__device__ __forceinline__ void dkdv_role(const Args& a, int vec, float* sm, int slab, int j0) {
+  constexpr int LD = DP + 4;
+  float* Qs = sm;
+  float* Gs = Qs + TT * LD;
+  float* Ks = Gs + TT * LD;
+  float* Vs = Ks + TT * LD;
+  float* Pt = Vs + TT * LD;  // P^T and dS^T: [key][query]
+  float* Dt = Pt + TT * PLD;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const Slab sl = slab_of(slab, a);
+  stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
+  stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
+  float accK[4][DP / 16] = {}, accV[4][DP / 16] = {}, dm[4] = {};
+  for (int i0 = 0; i0 < a.R; i0 += TT) {
+    __syncthreads();
+    stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
+    stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO, threadIdx.x, NTH);
+    __syncthreads();
+    float p[4][4], ds[4][4];
+    dots<DP, 16>(p, Qs, Ks, ty, tx);
+    dots<DP, 16>(ds, Gs, Vs, ty, tx);
+    probs<T, 16>(a, sl, slab, i0, j0, ty, tx, p, ds);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        Pt[(tx + 16 * c) * PLD + ty + 16 * r] = p[r][c];
+        Dt[(tx + 16 * c) * PLD + ty + 16 * r] = ds[r][c];
+        dm[c] += ds[r][c];
+      }
+    __syncthreads();
+    weighted_rows<DP>(accV, Pt, Gs, ty, tx);
+    weighted_rows<DP>(accK, Dt, Qs, ty, tx);
   }
   if (a.dmask != nullptr) {  // one addition per (b,h,s,j): the sum over heads
-    const float tot = warp_sum(dmask_acc);
-    if (row_ok && lane == 0) atomicAdd(a.dmask + ((long long)sl.b * a.S + sl.s) * a.R + j, tot);
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) Pt[(tx + 16 * c) * PLD + ty] = dm[c];
+    __syncthreads();
+    if (threadIdx.x < TT && j0 + threadIdx.x < a.R) {
+      float tot = 0.f;
+      for (int u = 0; u < 16; ++u) tot += Pt[threadIdx.x * PLD + u];
+      atomicAdd(a.dmask + ((long long)sl.b * a.S + sl.s) * a.R + j0 + threadIdx.x, tot);
+    }
   }
-  if (row_ok) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int j = j0 + ty + 16 * r;
+    if (j >= a.R) continue;
     T* ok = reinterpret_cast<T*>(a.dk) + off4(a.sdk, sl.b, sl.h, sl.s, j);
     T* ov = reinterpret_cast<T*>(a.dv) + off4(a.sdv, sl.b, sl.h, sl.s, j);
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int d = lane + 32 * t;
-      if (d < D) {
-        ok[d] = from_float<T>(accK[t] * a.scale);
-        ov[d] = from_float<T>(accV[t]);
+    for (int n = 0; n < DP / 16; ++n) {
+      const int d = Cols<DP>::at(tx, n);
+      if (d < a.D) {
+        ok[d] = from_float<T>(accK[r][n] * a.scale);
+        ov[d] = from_float<T>(accV[r][n]);
       }
     }
   }
 }
 
-// dBias[b,h,i,j] = sum over the S rows of dS_ij.  One warp owns one (b,h,i) row and
-// walks s in order, so the sum order is fixed.
-template <class T>
-__global__ void __launch_bounds__(GW * 32) generic_dbias_kernel(Args a) {
-  extern __shared__ float sm[];
-  const int D = a.D, DP = D + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* Qw = sm + warp * 2 * DP;
-  float* Gw = Qw + DP;
-  const int i = blockIdx.y * GW + warp;
-  if (i >= a.R) return;  // warps are independent here (only __syncwarp below)
-  const int h = blockIdx.x % a.H, b = blockIdx.x / a.H;
-  for (int j0 = 0; j0 < a.R; j0 += 32) {
-    const int j = j0 + lane;
-    float acc = 0.f;
-    for (int s = 0; s < a.S; ++s) {
-      __syncwarp();
-      const T* q = reinterpret_cast<const T*>(a.q) + off4(a.sq, b, h, s, i);
-      const T* g = reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, b, h, s, i);
-      for (int d = lane; d < D; d += 32) {
-        Qw[d] = to_float<T>(q[d]);
-        Gw[d] = to_float<T>(g[d]);
-      }
-      __syncwarp();
-      const long long slab = ((long long)b * a.H + h) * a.S + s;
-      const float lse = a.lse[slab * a.R + i], delta = a.delta[slab * a.delta_ld + i];
-      if (j < a.R) {
-        const T* k = reinterpret_cast<const T*>(a.k) + off4(a.sk, b, h, s, j);
-        const T* v = reinterpret_cast<const T*>(a.v) + off4(a.sv, b, h, s, j);
-        float dot = 0.f, dp = 0.f;
-        for (int d = 0; d < D; ++d) {
-          dot += Qw[d] * to_float<T>(k[d]);
-          dp += Gw[d] * to_float<T>(v[d]);
-        }
-        bool rep;
-        const float x = score<T>(a, b, h, s, i, j, dot, rep);
-        const float p = prob_from_lse(x, lse, a.R);
-        acc += rep ? 0.f : p * (dp - delta);
-      }
+// dBias of 32 x 32 scores of one (b,h): the MSA rows are dealt out to the groups of 64 threads of the
+// block, whose sums are added in a fixed order at the end.
+template <int DP> constexpr int kGroups = DP <= 64 ? 4 : 2;
+template <class T, int DP>
+__device__ __forceinline__ void dbias_role(const Args& a, int vec, float* sm, int bh, int i0, int j0) {
+  constexpr int LD = DP + 4, NG = kGroups<DP>;
+  const int grp = threadIdx.x >> 6, t = threadIdx.x & 63, tx = t & 7, ty = t >> 3;
+  float acc[4][4] = {};
+  if (grp < NG) {
+    float* Qs = sm + grp * 4 * TB * LD;
+    float* Gs = Qs + TB * LD;
+    float* Ks = Gs + TB * LD;
+    float* Vs = Ks + TB * LD;
+    for (int s = grp; s < a.S; s += NG) {
+      const Slab sl{bh / a.H, bh % a.H, s};
+      ptx::named_bar_sync(1 + grp, 64);
+      stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TB, a.R, a.D, vec & VEC_Q, t, 64);
+      stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TB, a.R, a.D, vec & VEC_DO, t, 64);
+      stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TB, a.R, a.D, vec & VEC_K, t, 64);
+      stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TB, a.R, a.D, vec & VEC_V, t, 64);
+      ptx::named_bar_sync(1 + grp, 64);
+      float p[4][4], ds[4][4];
+      dots<DP, 8>(p, Qs, Ks, ty, tx);
+      dots<DP, 8>(ds, Gs, Vs, ty, tx);
+      probs<T, 8>(a, sl, (long long)bh * a.S + s, i0, j0, ty, tx, p, ds);
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][c] += ds[r][c];
     }
-    if (j < a.R) a.dbias[(((long long)b * a.H + h) * a.R + i) * a.R + j] = acc;
+  }
+  __syncthreads();
+  float* part = sm;  // [group][32][32]
+  if (grp < NG) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) part[grp * TB * TB + (ty + 8 * r) * TB + tx + 8 * c] = acc[r][c];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < TB * TB; e += NTH) {
+    const int i = i0 + e / TB, j = j0 + e % TB;
+    float tot = part[e];
+#pragma unroll
+    for (int g = 1; g < NG; ++g) tot += part[g * TB * TB + e];
+    if (i < a.R && j < a.R) a.dbias[((long long)bh * a.R + i) * a.dbias_ld + j] = tot;
   }
 }
 
+// The three parts of a backward call read the same inputs and write different outputs: one launch, the
+// d(pair_bias) blocks (which walk all MSA rows) first.
+template <class T, int DP>
+__global__ void __launch_bounds__(NTH, DP <= 32 ? 2 : 1) generic_bwd_kernel(const Args a, const int vec, const long long n_dbias,
+                                                                          const long long n_total) {
+  extern __shared__ __align__(16) float sm[];
+  long long idx = (long long)blockIdx.y * gridDim.x + blockIdx.x;
+  if (idx >= n_total) return;
+  if (idx < n_dbias) {
+    const int nb = (a.R + TB - 1) / TB;
+    const int tj = (int)(idx % nb), ti = (int)(idx / nb % nb), bh = (int)(idx / nb / nb);
+    dbias_role<T, DP>(a, vec, sm, bh, ti * TB, tj * TB);
+    return;
+  }
+  idx -= n_dbias;
+  const long long half = (n_total - n_dbias) / 2;
+  const int nt = (a.R + TT - 1) / TT;
+  if (idx < half) dkdv_role<T, DP>(a, vec, sm, (int)(idx / nt), (int)(idx % nt) * TT);
+  else dq_role<T, DP>(a, vec, sm, (int)((idx - half) / nt), (int)((idx - half) % nt) * TT);
+}
+
+template <int DP> constexpr int fwd_smem() { return (3 * TT * (DP + 4) + TT * PLD) * 4; }
+template <int DP> constexpr int bwd_smem() {
+  constexpr int tiles = (4 * TT * (DP + 4) + 2 * TT * PLD) * 4, groups = kGroups<DP> * 4 * TB * (DP + 4) * 4;
+  return tiles > groups ? tiles : groups;
+}
+
 template <class T>
-static cudaError_t launch_fwd_t(const Args& a, cudaStream_t st, int* launches) {
-  const int DP = a.D + 1;
-  dim3 grid(a.B * a.H * a.S, (a.R + GW - 1) / GW);
-  size_t smem = (size_t)(2 * GT + GW) * DP * sizeof(float);
-  generic_fwd_kernel<T><<<grid, GW * 32, smem, st>>>(a);
+bool vec_ok(const void* p, const Str4& s) {
+  const long long n = 4;  // elements of a vector load
+  return reinterpret_cast<uintptr_t>(p) % (n * sizeof(T)) == 0 && s.b % n == 0 && s.h % n == 0 && s.s % n == 0 && s.r % n == 0;
+}
+template <class T>
+int vec_flags(const Args& a, bool bwd) {
+  return (vec_ok<T>(a.q, a.sq) ? VEC_Q : 0) | (vec_ok<T>(a.k, a.sk) ? VEC_K : 0) | (vec_ok<T>(a.v, a.sv) ? VEC_V : 0) |
+         (bwd && vec_ok<T>(a.d_o, a.sdo) ? VEC_DO : 0);
+}
+
+template <class T, int DP>
+cudaError_t launch_fwd_t(const Args& a, cudaStream_t st, int* launches) {
+  auto kern = generic_fwd_kernel<T, DP>;
+  if (!kernel_ready(reinterpret_cast<const void*>(kern), fwd_smem<DP>(), nullptr)) return cudaErrorUnknown;
+  kern<<<dim3(a.B * a.H * a.S, (a.R + TT - 1) / TT), NTH, fwd_smem<DP>(), st>>>(a, vec_flags<T>(a, false));
   *launches += 1;
   return cudaGetLastError();
 }
 
-template <class T>
-static cudaError_t launch_bwd_t(Args a, cudaStream_t st, int* launches) {
-  const int DP = a.D + 1;
+template <class T, int DP>
+cudaError_t launch_bwd_t(Args a, cudaStream_t st, int* launches) {
   const long long rows = (long long)a.B * a.H * a.S * a.R;
   if (a.dgate) {
     generic_gate_backward_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a);
     use_effective_d_o(&a);
   } else {
-    generic_delta_kernel<T><<<(unsigned)((rows + GW - 1) / GW), GW * 32, 0, st>>>(a);
+    generic_delta_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a);
   }
-  dim3 grid(a.B * a.H * a.S, (a.R + GW - 1) / GW);
-  generic_dq_kernel<T><<<grid, GW * 32, (size_t)(2 * GT + 2 * GW) * DP * sizeof(float), st>>>(a);
-  generic_dkdv_kernel<T><<<grid, GW * 32, ((size_t)(2 * GT + 2 * GW) * DP + 2 * GT) * sizeof(float), st>>>(a);
-  *launches += 3;
-  if (a.dbias) {
-    dim3 g2(a.B * a.H, (a.R + GW - 1) / GW);
-    generic_dbias_kernel<T><<<g2, GW * 32, (size_t)GW * 2 * DP * sizeof(float), st>>>(a);
-    *launches += 1;
-  }
+  auto kern = generic_bwd_kernel<T, DP>;
+  if (!kernel_ready(reinterpret_cast<const void*>(kern), bwd_smem<DP>(), nullptr)) return cudaErrorUnknown;
+  const long long nt = (a.R + TT - 1) / TT, nb = (a.R + TB - 1) / TB;
+  const long long n_dbias = a.dbias ? (long long)a.B * a.H * nb * nb : 0;
+  const long long n_total = n_dbias + 2 * (long long)a.B * a.H * a.S * nt;
+  const long long gx = n_total < (1 << 30) ? n_total : (1 << 30);
+  kern<<<dim3((unsigned)gx, (unsigned)((n_total + gx - 1) / gx)), NTH, bwd_smem<DP>(), st>>>(a, vec_flags<T>(a, true), n_dbias, n_total);
+  *launches += 2;
   return cudaGetLastError();
 }
 
+template <class T>
+cudaError_t launch_fwd_d(const Args& a, cudaStream_t st, int* launches) {
+  if (a.D <= 16) return launch_fwd_t<T, 16>(a, st, launches);
+  if (a.D <= 32) return launch_fwd_t<T, 32>(a, st, launches);
+  if (a.D <= 64) return launch_fwd_t<T, 64>(a, st, launches);
+  return launch_fwd_t<T, 128>(a, st, launches);
+}
+template <class T>
+cudaError_t launch_bwd_d(const Args& a, cudaStream_t st, int* launches) {
+  if (a.D <= 16) return launch_bwd_t<T, 16>(a, st, launches);
+  if (a.D <= 32) return launch_bwd_t<T, 32>(a, st, launches);
+  if (a.D <= 64) return launch_bwd_t<T, 64>(a, st, launches);
+  return launch_bwd_t<T, 128>(a, st, launches);
+}
+
+}  // namespace
+
 cudaError_t launch_generic_fwd(int dtype, const Args& a, cudaStream_t st, int* launches) {
   switch (dtype) {
-    case EVOATTN_BF16: return launch_fwd_t<__nv_bfloat16>(a, st, launches);
-    case EVOATTN_FP16: return launch_fwd_t<__half>(a, st, launches);
-    default: return launch_fwd_t<float>(a, st, launches);
+    case EVOATTN_BF16: return launch_fwd_d<__nv_bfloat16>(a, st, launches);
+    case EVOATTN_FP16: return launch_fwd_d<__half>(a, st, launches);
+    default: return launch_fwd_d<float>(a, st, launches);
   }
 }
 
 cudaError_t launch_generic_bwd(int dtype, const Args& a, cudaStream_t st, int* launches) {
   switch (dtype) {
-    case EVOATTN_BF16: return launch_bwd_t<__nv_bfloat16>(a, st, launches);
-    case EVOATTN_FP16: return launch_bwd_t<__half>(a, st, launches);
-    default: return launch_bwd_t<float>(a, st, launches);
+    case EVOATTN_BF16: return launch_bwd_d<__nv_bfloat16>(a, st, launches);
+    case EVOATTN_FP16: return launch_bwd_d<__half>(a, st, launches);
+    default: return launch_bwd_d<float>(a, st, launches);
   }
 }
 
