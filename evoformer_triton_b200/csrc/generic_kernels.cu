@@ -84,7 +84,7 @@ __device__ __forceinline__ void dots(float (&acc)[4][4], const float* A, const f
   for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) s[r][c] = f2_make(0.f, 0.f);
-#pragma unroll 4
+#pragma unroll 1
   for (int d = 0; d < DP; d += 4) {
     float4 a[4], b[4];
 #pragma unroll
@@ -121,7 +121,7 @@ template <int DP>
 __device__ __forceinline__ void weighted_rows(float (&acc)[4][DP / 16], const float* P, const float* V, int ty, int tx) {
   using C = Cols<DP>;
   constexpr int LD = DP + 4;
-#pragma unroll 4
+#pragma unroll 2
   for (int j = 0; j < TT; j += 4) {
     float p[4][4];
 #pragma unroll
@@ -153,17 +153,30 @@ __device__ __forceinline__ void weighted_rows(float (&acc)[4][DP / 16], const fl
   }
 }
 
-// Score of (i, j) before the softmax, with mask applied.  `replaced` tells the caller that the score is a
-// constant (boolean mask dropped the key).
-template <class T>
-__device__ __forceinline__ float score(const Args& a, const Slab& sl, int i, int j, float dot, bool& replaced) {
-  float x = dot * a.scale;
-  if (a.bias) x += load_bias<T>(a, sl.b, sl.h, i, j);
-  replaced = false;
-  if (a.mask_kind != EVOATTN_MASK_NONE)
-    x = apply_mask<T>(x, a.mask, a.mask_kind,
-                      (long long)sl.b * a.smask.a + (long long)sl.s * a.smask.b + (long long)j * a.smask.c, replaced);
-  return x;
+// What is added to the 4 x 4 scores of a thread (i = i0 + ty + W r, j = j0 + tx + W c) before the softmax.
+// Read ahead of the dot products, whose arithmetic covers the latency of these loads.
+struct Terms {
+  float bias[4][4], add[4];
+  unsigned replaced;  // bit c: a boolean mask dropped column c (its scores are constants)
+};
+template <class T, int W>
+__device__ __forceinline__ void load_terms(Terms& t, const Args& a, const Slab& sl, int i0, int j0, int ty, int tx) {
+  t.replaced = 0;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int j = min(j0 + tx + W * c, a.R - 1);
+    const long long mi = (long long)sl.b * a.smask.a + (long long)sl.s * a.smask.b + (long long)j * a.smask.c;
+    t.add[c] = 0.f;
+    if (a.mask_kind == EVOATTN_MASK_BOOL) t.replaced |= (reinterpret_cast<const unsigned char*>(a.mask)[mi] == 0 ? 1u : 0u) << c;
+    else if (a.mask_kind == EVOATTN_MASK_ADD_F32) t.add[c] = reinterpret_cast<const float*>(a.mask)[mi];
+    else if (a.mask_kind == EVOATTN_MASK_ADD_SAME) t.add[c] = to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]);
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      t.bias[r][c] = a.bias ? load_bias<T>(a, sl.b, sl.h, min(i0 + ty + W * r, a.R - 1), j) : 0.f;
+  }
+}
+__device__ __forceinline__ float score(const Terms& t, float scale, float dot, int r, int c) {
+  return (t.replaced >> c & 1u) ? -FLT_MAX : (dot * scale + t.bias[r][c]) + t.add[c];
 }
 
 // P_ij from a stored log-sum-exp.  A row whose keys were all dropped has lse == -FLT_MAX
@@ -201,17 +214,16 @@ __global__ void __launch_bounds__(NTH, DP <= 64 ? 2 : 1) generic_fwd_kernel(cons
     stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
     stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
     __syncthreads();
+    Terms terms;
+    load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
     float x[4][4];
     dots<DP, 16>(x, Qs, Ks, ty, tx);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const int i = min(i0 + ty + 16 * r, a.R - 1);
       float mx = -INFINITY;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const int j = j0 + tx + 16 * c;
-        bool rep;
-        x[r][c] = j < a.R ? score<T>(a, sl, i, j, x[r][c], rep) : -INFINITY;
+        x[r][c] = j0 + tx + 16 * c < a.R ? score(terms, a.scale, x[r][c], r, c) : -INFINITY;
         mx = fmaxf(mx, x[r][c]);
       }
 #pragma unroll
@@ -251,21 +263,23 @@ __global__ void __launch_bounds__(NTH, DP <= 64 ? 2 : 1) generic_fwd_kernel(cons
   }
 }
 
-// delta[b,h,s,i] = <dO_i, O_i>   (evoformer.py:299-326)
+// delta[b,h,s,i] = <dO_i, O_i>   (evoformer.py:299-326), eight lanes per row.
 template <class T>
-__global__ void __launch_bounds__(256) generic_delta_kernel(Args a) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long row = (long long)blockIdx.x * 8 + warp;
+__global__ void __launch_bounds__(256) generic_delta_kernel(const Args a) {
+  const int lane = threadIdx.x & 7;
+  const long long row = (long long)blockIdx.x * 32 + (threadIdx.x >> 3);
   const long long rows = (long long)a.B * a.H * a.S * a.R;
-  if (row >= rows) return;
-  const int i = (int)(row % a.R);
-  const Slab sl = slab_of((int)(row / a.R), a);
+  const long long rc = row < rows ? row : rows - 1;
+  const long long slab = rc / a.R;
+  const int i = (int)(rc - slab * a.R);
+  const Slab sl = slab_of((int)slab, a);
   const T* o = reinterpret_cast<const T*>(a.o) + off4(a.so, sl.b, sl.h, sl.s, i);
   const T* g = reinterpret_cast<const T*>(a.d_o) + off4(a.sdo, sl.b, sl.h, sl.s, i);
   float acc = 0.f;
-  for (int d = lane; d < a.D; d += 32) acc += to_float<T>(o[d]) * to_float<T>(g[d]);
-  acc = warp_sum(acc);
-  if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
+  for (int d = lane; d < a.D; d += 8) acc += to_float<T>(o[d]) * to_float<T>(g[d]);
+#pragma unroll
+  for (int m = 4; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+  if (row < rows && lane == 0) a.delta[slab * a.delta_ld + i] = acc;
 }
 
 // Gated output Og = sigmoid(gate) * O.  With G = dOg (gradient of the gated output):
@@ -301,24 +315,29 @@ __global__ void __launch_bounds__(256) generic_gate_backward_kernel(Args a) {
   if (lane == 0) a.delta[(row / a.R) * a.delta_ld + i] = acc;
 }
 
-// P and dS of a 4 x 4 patch from its two dot products; both 0 outside the R x R scores.
-template <class T, int W>
-__device__ __forceinline__ void probs(const Args& a, const Slab& sl, long long slab, int i0, int j0, int ty, int tx,
-                                      float (&p)[4][4], float (&ds)[4][4]) {
+// The row statistics of a thread's four query rows.
+template <int W>
+__device__ __forceinline__ void load_stats(float (&lse)[4], float (&delta)[4], const Args& a, long long slab, int i0, int ty) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty + W * r, ic = min(i, a.R - 1);
-    const float lse = a.lse[slab * a.R + ic], delta = a.delta[slab * a.delta_ld + ic];
+    const int i = min(i0 + ty + W * r, a.R - 1);
+    lse[r] = a.lse[slab * a.R + i];
+    delta[r] = a.delta[slab * a.delta_ld + i];
+  }
+}
+
+// P and dS of a 4 x 4 patch from its two dot products; both 0 outside the R x R scores.
+template <int W>
+__device__ __forceinline__ void probs(const Args& a, const Terms& t, const float (&lse)[4], const float (&delta)[4], int i0, int j0,
+                                      int ty, int tx, float (&p)[4][4], float (&ds)[4][4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      const int j = j0 + tx + W * c;
-      bool rep;
-      const float x = score<T>(a, sl, ic, min(j, a.R - 1), p[r][c], rep);
-      const bool in = i < a.R && j < a.R;
-      p[r][c] = in ? prob_from_lse(x, lse, a.R) : 0.f;
-      ds[r][c] = (in && !rep) ? p[r][c] * (ds[r][c] - delta) : 0.f;
+      const bool in = i0 + ty + W * r < a.R && j0 + tx + W * c < a.R;
+      p[r][c] = in ? prob_from_lse(score(t, a.scale, p[r][c], r, c), lse[r], a.R) : 0.f;
+      ds[r][c] = (in && !(t.replaced >> c & 1u)) ? p[r][c] * (ds[r][c] - delta[r]) : 0.f;
     }
-  }
 }
 
 // dQ of 64 queries: walks the keys.
@@ -334,16 +353,19 @@ __device__ __forceinline__ void dq_role(const Args& a, int vec, float* sm, int s
   const Slab sl = slab_of(slab, a);
   stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
   stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO, threadIdx.x, NTH);
-  float acc[4][DP / 16] = {};
+  float acc[4][DP / 16] = {}, lse[4], delta[4];
+  load_stats<16>(lse, delta, a, slab, i0, ty);
   for (int j0 = 0; j0 < a.R; j0 += TT) {
     __syncthreads();
     stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
     stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
     __syncthreads();
+    Terms terms;
+    load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
     float p[4][4], ds[4][4];
     dots<DP, 16>(p, Qs, Ks, ty, tx);
     dots<DP, 16>(ds, Gs, Vs, ty, tx);
-    probs<T, 16>(a, sl, slab, i0, j0, ty, tx, p, ds);
+    probs<16>(a, terms, lse, delta, i0, j0, ty, tx, p, ds);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -385,10 +407,13 @@ __device__ __forceinline__ void dkdv_role(const Args& a, int vec, float* sm, int
     stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
     stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO, threadIdx.x, NTH);
     __syncthreads();
-    float p[4][4], ds[4][4];
+    Terms terms;
+    load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
+    float p[4][4], ds[4][4], lse[4], delta[4];
+    load_stats<16>(lse, delta, a, slab, i0, ty);
     dots<DP, 16>(p, Qs, Ks, ty, tx);
     dots<DP, 16>(ds, Gs, Vs, ty, tx);
-    probs<T, 16>(a, sl, slab, i0, j0, ty, tx, p, ds);
+    probs<16>(a, terms, lse, delta, i0, j0, ty, tx, p, ds);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -449,11 +474,14 @@ __device__ __forceinline__ void dbias_role(const Args& a, int vec, float* sm, in
       stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TB, a.R, a.D, vec & VEC_DO, t, 64);
       stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TB, a.R, a.D, vec & VEC_K, t, 64);
       stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TB, a.R, a.D, vec & VEC_V, t, 64);
+      float p[4][4], ds[4][4], lse[4], delta[4];
+      load_stats<8>(lse, delta, a, (long long)bh * a.S + s, i0, ty);
+      Terms terms;
+      load_terms<T, 8>(terms, a, sl, i0, j0, ty, tx);
       ptx::named_bar_sync(1 + grp, 64);
-      float p[4][4], ds[4][4];
       dots<DP, 8>(p, Qs, Ks, ty, tx);
       dots<DP, 8>(ds, Gs, Vs, ty, tx);
-      probs<T, 8>(a, sl, (long long)bh * a.S + s, i0, j0, ty, tx, p, ds);
+      probs<8>(a, terms, lse, delta, i0, j0, ty, tx, p, ds);
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -532,7 +560,7 @@ cudaError_t launch_bwd_t(Args a, cudaStream_t st, int* launches) {
     generic_gate_backward_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a);
     use_effective_d_o(&a);
   } else {
-    generic_delta_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a);
+    generic_delta_kernel<T><<<(unsigned)((rows + 31) / 32), 256, 0, st>>>(a);
   }
   auto kern = generic_bwd_kernel<T, DP>;
   if (!kernel_ready(reinterpret_cast<const void*>(kern), bwd_smem<DP>(), nullptr)) return cudaErrorUnknown;
