@@ -94,6 +94,18 @@ template <> struct Pack2<__half> {
   }
 };
 
+// The two 16-bit values of a 32-bit word, widened.
+template <class T> __device__ __forceinline__ void unpack2(uint32_t w, float& lo, float& hi);
+template <> __device__ __forceinline__ void unpack2<__nv_bfloat16>(uint32_t w, float& lo, float& hi) {
+  lo = __uint_as_float(w << 16);
+  hi = __uint_as_float(w & 0xffff0000u);
+}
+template <> __device__ __forceinline__ void unpack2<__half>(uint32_t w, float& lo, float& hi) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  lo = f.x;
+  hi = f.y;
+}
+
 __device__ __forceinline__ long long off4(const Str4& s, int b, int h, int ss, int r) {
   return (long long)b * s.b + (long long)h * s.h + (long long)ss * s.s + (long long)r * s.r;
 }
@@ -112,19 +124,6 @@ __device__ __forceinline__ float apply_mask(float x, const void* mask, int kind,
   if (kind == EVOATTN_MASK_ADD_F32) return x + reinterpret_cast<const float*>(mask)[idx];
   if (kind == EVOATTN_MASK_ADD_SAME) return x + to_float<T>(reinterpret_cast<const T*>(mask)[idx]);
   return x;
-}
-
-// Residue mask of key j for batch b, MSA row s as the float the tcgen05 kernels combine with a
-// score: MIN mode (boolean keep-mask or none) gives +FLT_MAX (keep) or -FLT_MAX (drop) for
-// `min(score, m)`; ADD mode gives the additive value.  Keys beyond R are always dropped.
-template <class T, int MIN_MODE>
-__device__ __forceinline__ float mask_value(const Args& a, int b, int s, int j) {
-  if (j >= a.R) return -FLT_MAX;
-  if (a.mask_kind == EVOATTN_MASK_NONE) return MIN_MODE ? FLT_MAX : 0.f;
-  const long long mi = (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c;
-  if (MIN_MODE) return reinterpret_cast<const unsigned char*>(a.mask)[mi] ? FLT_MAX : -FLT_MAX;
-  if (a.mask_kind == EVOATTN_MASK_ADD_F32) return reinterpret_cast<const float*>(a.mask)[mi];
-  return to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]);
 }
 
 // Pair-bias element (b, h, i, j) in either storage type.

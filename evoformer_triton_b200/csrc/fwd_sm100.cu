@@ -270,31 +270,57 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     } else if (warp == 3) {
       // =============================== residue-mask stager ===============================
       // One float per key for each warpgroup's MSA row, one item ahead of the softmax warps.
-      // Keys beyond R are always excluded.
+      // Keys beyond R are always excluded.  A lane takes eight consecutive keys: one address, then
+      // independent loads.  (A chain of test, load and convert per key, as the compiler made of a branching
+      // helper, took 18 000 cycles an item and set the pace of the whole kernel.)
+      constexpr bool kMin = MASKMODE == MASK_MIN;
+      const int kind = a.mask_kind;
+      const int es = kind == EVOATTN_MASK_BOOL ? 1 : kind == EVOATTN_MASK_ADD_F32 ? 4 : 2;
+      const long long step = a.smask.c * es;  // bytes from key to key
       uint32_t n = 0;
       for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
         const Item it = decode_item<QP>(item, n_inner, n_outer, a.H);
         const int st = n & 1;
         for (int w = 0; w < 2; ++w) {
-          const int s = min(it.s[w], a.S - 1);
+          const unsigned char* ptr = reinterpret_cast<const unsigned char*>(a.mask) +
+                                     ((long long)it.b * a.smask.a + (long long)min(it.s[w], a.S - 1) * a.smask.b) * es;
           mbar_wait(m_empty(w, st), ((n >> 1) & 1) ^ 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
           float* dst = sMask + (w * 2 + st) * r_pad;
           uint32_t* dirty = sDirty + (w * 2 + st) * 32;
-          dirty[lane] = 0u;
-          __syncwarp();
-          // eight loads in flight per lane: a dependent load-convert-store chain per key would
-          // make this warp the slowest stage of the pipeline
           for (int j0 = 0; j0 < r_pad; j0 += 256) {
-            float m[8];
+            const int j = j0 + lane * 8;
+            const unsigned char* q = ptr + j * step;
+            uint32_t raw[8];
+            if (kind == EVOATTN_MASK_BOOL) {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) m[u] = mask_value<T, MASKMODE == MASK_MIN>(a, it.b, s, j0 + u * 32 + lane);
+              for (int u = 0; u < 8; ++u) raw[u] = ldg_u8_if(q + u * step, j + u < a.R);
+            } else if (kind == EVOATTN_MASK_ADD_F32) {
+#pragma unroll
+              for (int u = 0; u < 8; ++u) raw[u] = ldg_u32_if(q + u * step, j + u < a.R);
+            } else if (kind == EVOATTN_MASK_ADD_SAME) {
+#pragma unroll
+              for (int u = 0; u < 8; ++u) raw[u] = ldg_u16_if(q + u * step, j + u < a.R);
+            }
+            float m[8];
+            bool any = false;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-              const bool in = j0 + u * 32 + lane < r_pad;
-              if (in) dst[j0 + u * 32 + lane] = m[u];
-              const uint32_t any = __ballot_sync(0xffffffffu, in && m[u] < 0.f);
-              if (lane == 0 && any != 0u) dirty[(j0 + u * 32) / BN] = 1u;
+              float v = kMin ? FLT_MAX : 0.f;
+              if constexpr (kMin) {
+                if (kind == EVOATTN_MASK_BOOL && raw[u] == 0) v = -FLT_MAX;
+              } else {
+                if (kind == EVOATTN_MASK_ADD_F32) v = __uint_as_float(raw[u]);
+                else unpack2<T>(raw[u], v, m[u]);
+              }
+              m[u] = j + u < a.R ? v : -FLT_MAX;
+              any |= m[u] < 0.f;
             }
+            if (j < r_pad) {
+              *reinterpret_cast<float4*>(dst + j) = make_float4(m[0], m[1], m[2], m[3]);
+              *reinterpret_cast<float4*>(dst + j + 4) = make_float4(m[4], m[5], m[6], m[7]);
+            }
+            const uint32_t lanes_any = __ballot_sync(0xffffffffu, any);  // eight lanes to a key tile
+            if (lane < 4) dirty[j0 / BN + lane] = (lanes_any >> (8 * lane)) & 0xffu;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(m_full(w, st));
