@@ -592,15 +592,17 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     StepT cur = decode(0), prv = cur;
     uint32_t mraw = mask_fetch(cur.b, cur.s, cur.j0 + jrow, total_steps > 0);
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
-    float bacc[32];
+    const F2 l2e2 = f2_make(kLog2e, kLog2e), c12 = f2_make(c1, c1), neg1 = f2_make(-1.f, -1.f);
+    F2 bacc[16];  // d(pair_bias) of this thread's key and its 32 queries, summed over the rows of a group
 #pragma unroll
-    for (int e = 0; e < 32; ++e) bacc[e] = 0.f;
+    for (int e = 0; e < 16; ++e) bacc[e] = f2_make(0.f, 0.f);
 
     for (int n = 0; n < total_steps; ++n) {
       const StepT nxt = advance(cur, n + 1);
       const bool more = n + 1 < total_steps;
       const int g = cur.g;
       const float mj = mask_decode(mraw, cur.s, cur.j0 + jrow);
+      const F2 mj2 = f2_make(mj, mj);
       mraw = mask_fetch(nxt.b, nxt.s, nxt.j0 + jrow, more);  // in flight during this step
       const int stg = n % kStages;
       const uint32_t vec_s = sStage_s + stg * L::kStage + 2 * L::kTile;
@@ -631,38 +633,38 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           for (int c4 = 0; c4 < 4; ++c4) {
             const float4 nl = lds_v4f(vnl + 16 * c4);
             const float4 dl = lds_v4f(vdl + 16 * c4);
-            float t[4] = {nl.x, nl.y, nl.z, nl.w};
-            const float de[4] = {dl.x, dl.y, dl.z, dl.w};
+            // two queries per instruction (the pairs lie side by side in every operand)
+            F2 t[2] = {f2_make(nl.x, nl.y), f2_make(nl.z, nl.w)};
+            const F2 de[2] = {f2_make(dl.x, dl.y), f2_make(dl.z, dl.w)};
             if (has_bias) {
+              float bv[4];
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
-                float bv;
                 if constexpr (kBias16) {
                   const uint16_t raw = lds_u16(brow + (4 * c4 + u) * kBRow);
-                  bv = to_float<T>(*reinterpret_cast<const T*>(&raw));
+                  bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
                 } else {
-                  bv = lds_f32(brow + (4 * c4 + u) * kBRow);
+                  bv[u] = lds_f32(brow + (4 * c4 + u) * kBRow);
                 }
-                t[u] = fmaf(bv, kLog2e, t[u]);
               }
+              t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
+              t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
             }
-            float p[4], ds[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
+            for (int u = 0; u < 2; ++u) {
+              const int e = 4 * c4 + 2 * u;
               // x = S*(scale*log2e) + (bias*log2e - lse*log2e) + mask
-              const float x = fmaf(__uint_as_float(sr[4 * c4 + u]), c1, t[u]) + mj;
-              p[u] = ex2(x);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
+              float x0, x1;
+              f2_get(f2_add(f2_fma(f2_from_bits(sr[e], sr[e + 1]), c12, t[u]), mj2), x0, x1);
+              const float p0 = ex2(x0), p1 = ex2(x1);
               // dS = P (dP - delta); d_bias_acc += dS
-              ds[u] = p[u] * (__uint_as_float(dr[4 * c4 + u]) - de[u]);
-              bacc[sub * 16 + 4 * c4 + u] += ds[u];
+              const F2 ds = f2_mul(f2_make(p0, p1), f2_fma(de[u], neg1, f2_from_bits(dr[e], dr[e + 1])));
+              bacc[(sub * 16 + e) / 2] = f2_add(bacc[(sub * 16 + e) / 2], ds);
+              float d0, d1;
+              f2_get(ds, d0, d1);
+              pk[2 * c4 + u] = Pack2<T>::pack(p0, p1);
+              dk[sub * 8 + 2 * c4 + u] = Pack2<T>::pack(d0, d1);
             }
-            pk[2 * c4] = Pack2<T>::pack(p[0], p[1]);
-            pk[2 * c4 + 1] = Pack2<T>::pack(p[2], p[3]);
-            dk[sub * 8 + 2 * c4] = Pack2<T>::pack(ds[0], ds[1]);
-            dk[sub * 8 + 2 * c4 + 1] = Pack2<T>::pack(ds[2], ds[3]);
           }
         } else {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
@@ -688,9 +690,12 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           // memory by a bulk tensor reduction that the warp issues itself.
           staging_free();
 #pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            sts_f32(out_s + c * 128 + lane * 4, bacc[sub * 16 + c]);
-            bacc[sub * 16 + c] = 0.f;
+          for (int c = 0; c < 16; c += 2) {
+            float b0, b1;
+            f2_get(bacc[(sub * 16 + c) / 2], b0, b1);
+            sts_f32(out_s + c * 128 + lane * 4, b0);
+            sts_f32(out_s + (c + 1) * 128 + lane * 4, b1);
+            bacc[(sub * 16 + c) / 2] = f2_make(0.f, 0.f);
           }
           fence_async_shared();
           __syncwarp();
