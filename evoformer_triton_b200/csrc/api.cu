@@ -106,10 +106,6 @@ void fill_bwd_args(const evoattn_bwd_params* p, evo::Args* a) {
   a->exchange = p->exchange;
 }
 
-size_t generic_bwd_workspace(const evo::Args& a) {
-  return (size_t)a.B * a.H * a.S * a.R * sizeof(float);  // delta
-}
-
 bool use_sm100_fwd(const evoattn_fwd_params* p, const evo::Args& a) {
   if (p->flags & EVOATTN_FLAG_FORCE_GENERIC) return false;
   if (p->dtype == EVOATTN_FP32) return false;
@@ -180,8 +176,15 @@ struct Scratch {
 Scratch plan_scratch(const evoattn_bwd_params* p, evo::Args* a, bool fast) {
   a->delta_ld = fast ? stats_ld(*a) : a->R;
   Scratch s{};
-  s.path = align256(fast ? evo::sm100_bwd_workspace_bytes(p->fwd.dtype, *a) : generic_bwd_workspace(*a));
   if (p->fwd.gate) s.gate = align256((size_t)a->B * a->H * a->S * a->R * a->D * esize_of(p->fwd.dtype));
+  if (fast) {
+    s.path = evo::sm100_bwd_workspace_bytes(p->fwd.dtype, *a);
+  } else {
+    evo::Args want = *a;
+    if (want.dbias_out) want.dbias = reinterpret_cast<float*>(want.dbias_out);  // (only whether there is one)
+    s.path = evo::generic_bwd_workspace_bytes(want);
+  }
+  s.path = align256(s.path);
   const bool direct = a->dbias && (!fast || (a->R % 4 == 0 && (reinterpret_cast<uintptr_t>(a->dbias) & 15) == 0));
   if (a->dbias && !direct) {
     a->dbias_out = a->dbias;

@@ -3,7 +3,7 @@
 // These serve fp32 inputs (tensor cores would lose bits there) and every shape the tcgen05 kernels do
 // not cover.  fp32 math throughout, every sum in a fixed order: the pair-bias gradient is produced by
 // one owner per element instead of the reference's fp32 atomics (dsevoformer-triton/evoformer.py:458),
-// and dQ, dK/dV and d(pair_bias) each recompute the scores, so results are the same bits on every run.
+// and dQ and dK/dV each compute the scores, so results are the same bits on every run.
 //
 // Math (evoformer.py:68-89 forward, :450-462 and :594-614 backward):
 //   x_ij = scale * <q_i,k_j> + bias_ij ;  mask ;  P = softmax_j(x) ;  O = P V
@@ -28,7 +28,6 @@ using ptx::f2_get;
 using ptx::f2_make;
 
 constexpr int TT = 64;        // rows of a tile (queries and keys)
-constexpr int TB = 32;        // ... of a d(pair_bias) tile
 constexpr int NTH = 256;
 constexpr int PLD = TT + 4;   // row stride of a staged score tile
 
@@ -73,6 +72,33 @@ __device__ __forceinline__ void stage_rows(float* dst, const T* x, const Str4& s
     *reinterpret_cast<float4*>(dst + rr * LD + d) = v;
   }
 }
+
+// The same without waiting for the loads where they can be asynchronous (fp32 rows read 16 bytes at a time):
+// the caller waits with async_wait() before the barrier that makes the rows visible.
+template <class T, int DP>
+__device__ __forceinline__ void stage_rows_ahead(float* dst, const T* x, const Str4& st, const Slab& sl, int r0, int n, int R, int D,
+                                                 bool vec) {
+  if constexpr (sizeof(T) == 4) {
+    if (vec && D == DP) {
+      constexpr int LD = DP + 4, C4 = DP / 4;
+      const T* base = x + off4(st, sl.b, sl.h, sl.s, 0);
+      for (int e = threadIdx.x; e < n * C4; e += NTH) {
+        const int rr = e / C4, d = (e - rr * C4) * 4, r = r0 + rr;
+        const int bytes = r < R ? 16 : 0;  // (rows beyond R are filled with zeros)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst + rr * LD + d)),
+                     "l"(base + (long long)min(r, R - 1) * st.r + d), "r"(bytes)
+                     : "memory");
+      }
+      return;
+    }
+  }
+  stage_rows<T, DP>(dst, x, st, sl, r0, n, R, D, vec, threadIdx.x, NTH);
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Whether the tiles of the inner loop are double-buffered: the next pair is loaded under the arithmetic
+// of this one (at DP = 128 two pairs do not fit).
+template <int DP> constexpr bool kAhead = DP <= 64;
 
 // acc[r][c] = <A row ty + W r, B row tx + W c> over DP columns.  Two columns per instruction: the even
 // and the odd ones are summed apart and added at the end.
@@ -162,6 +188,7 @@ struct Terms {
 template <class T, int W>
 __device__ __forceinline__ void load_terms(Terms& t, const Args& a, const Slab& sl, int i0, int j0, int ty, int tx) {
   t.replaced = 0;
+  const bool full = i0 + 4 * W <= a.R && j0 + 4 * W <= a.R;  // (one address per row, the same for the whole block)
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const int j = min(j0 + tx + W * c, a.R - 1);
@@ -170,9 +197,24 @@ __device__ __forceinline__ void load_terms(Terms& t, const Args& a, const Slab& 
     if (a.mask_kind == EVOATTN_MASK_BOOL) t.replaced |= (reinterpret_cast<const unsigned char*>(a.mask)[mi] == 0 ? 1u : 0u) << c;
     else if (a.mask_kind == EVOATTN_MASK_ADD_F32) t.add[c] = reinterpret_cast<const float*>(a.mask)[mi];
     else if (a.mask_kind == EVOATTN_MASK_ADD_SAME) t.add[c] = to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]);
+  }
+  if (!a.bias) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
-      t.bias[r][c] = a.bias ? load_bias<T>(a, sl.b, sl.h, min(i0 + ty + W * r, a.R - 1), j) : 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) t.bias[r][c] = 0.f;
+  } else if (full && !a.bias16) {
+    const float* p = a.bias + (long long)sl.b * a.sbias.a + (long long)sl.h * a.sbias.b + (long long)(i0 + ty) * a.sbias.c + j0 + tx;
+#pragma unroll
+    for (int r = 0; r < 4; ++r, p += W * a.sbias.c)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) t.bias[r][c] = __ldg(p + W * c);
+  } else {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        t.bias[r][c] = load_bias<T>(a, sl.b, sl.h, min(i0 + ty + W * r, a.R - 1), min(j0 + tx + W * c, a.R - 1));
   }
 }
 __device__ __forceinline__ float score(const Terms& t, float scale, float dot, int r, int c) {
@@ -194,12 +236,17 @@ __global__ void __launch_bounds__(NTH, DP <= 64 ? 2 : 1) generic_fwd_kernel(cons
   extern __shared__ __align__(16) float sm[];
   constexpr int LD = DP + 4;
   float* Qs = sm;
-  float* Ks = Qs + TT * LD;
-  float* Vs = Ks + TT * LD;
-  float* Ps = Vs + TT * LD;
+  float* KV = Qs + TT * LD;  // one or two pairs of K and V tiles
+  float* Ps = KV + (kAhead<DP> ? 4 : 2) * TT * LD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const Slab sl = slab_of(blockIdx.x, a);
   const int i0 = blockIdx.y * TT;
+  auto stage = [&](int j0) {
+    float* dst = KV + (kAhead<DP> ? (j0 / TT & 1) * 2 * TT * LD : 0);
+    stage_rows_ahead<T, DP>(dst, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K);
+    stage_rows_ahead<T, DP>(dst + TT * LD, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V);
+  };
+  if (kAhead<DP>) stage(0);
   stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
   float m[4], l[4], acc[4][DP / 16];
 #pragma unroll
@@ -210,10 +257,15 @@ __global__ void __launch_bounds__(NTH, DP <= 64 ? 2 : 1) generic_fwd_kernel(cons
     for (int n = 0; n < DP / 16; ++n) acc[r][n] = 0.f;
   }
   for (int j0 = 0; j0 < a.R; j0 += TT) {
+    if (!kAhead<DP>) {
+      __syncthreads();
+      stage(j0);
+    }
+    async_wait();
     __syncthreads();
-    stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
-    stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
-    __syncthreads();
+    if (kAhead<DP> && j0 + TT < a.R) stage(j0 + TT);  // (the pair the last iteration read)
+    const float* Ks = KV + (kAhead<DP> ? (j0 / TT & 1) * 2 * TT * LD : 0);
+    const float* Vs = Ks + TT * LD;
     Terms terms;
     load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
     float x[4][4];
@@ -340,49 +392,76 @@ __device__ __forceinline__ void probs(const Args& a, const Terms& t, const float
     }
 }
 
-// dQ of 64 queries: walks the keys.
+// dQ of 64 queries of the MSA rows s0 .. s1: walks the keys.  dS is at hand here, so d(pair_bias) of these
+// queries and rows is summed on the way, in a buffer that no other block touches (`part`, [R][R] of this
+// (b,h) and run of rows): the first row stores, the others add in turn.  That read and write of L2 costs a
+// tenth of what a pass of its own did, which had to compute every score and dP once more.
 template <class T, int DP>
-__device__ __forceinline__ void dq_role(const Args& a, int vec, float* sm, int slab, int i0) {
+__device__ __forceinline__ void dq_role(const Args& a, int vec, float* sm, int bh, int s0, int s1, int i0, float* part, int ld) {
   constexpr int LD = DP + 4;
   float* Qs = sm;
   float* Gs = Qs + TT * LD;
-  float* Ks = Gs + TT * LD;
-  float* Vs = Ks + TT * LD;
-  float* Ds = Vs + TT * LD;
+  float* KV = Gs + TT * LD;
+  float* Ds = KV + (kAhead<DP> ? 4 : 2) * TT * LD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const Slab sl = slab_of(slab, a);
-  stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
-  stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO, threadIdx.x, NTH);
-  float acc[4][DP / 16] = {}, lse[4], delta[4];
-  load_stats<16>(lse, delta, a, slab, i0, ty);
-  for (int j0 = 0; j0 < a.R; j0 += TT) {
-    __syncthreads();
-    stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
-    stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
-    __syncthreads();
-    Terms terms;
-    load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
-    float p[4][4], ds[4][4];
-    dots<DP, 16>(p, Qs, Ks, ty, tx);
-    dots<DP, 16>(ds, Gs, Vs, ty, tx);
-    probs<16>(a, terms, lse, delta, i0, j0, ty, tx, p, ds);
+  for (int srow = s0; srow < s1; ++srow) {
+    const Slab sl{bh / a.H, bh % a.H, srow};
+    const long long slab = (long long)bh * a.S + srow;
+    auto stage = [&](int j0) {
+      float* dst = KV + (kAhead<DP> ? (j0 / TT & 1) * 2 * TT * LD : 0);
+      stage_rows_ahead<T, DP>(dst, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K);
+      stage_rows_ahead<T, DP>(dst + TT * LD, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V);
+    };
+    if (srow > s0) __syncthreads();  // the tiles of the row before have been read
+    if (kAhead<DP>) stage(0);
+    stage_rows_ahead<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q);
+    stage_rows_ahead<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO);
+    float acc[4][DP / 16] = {}, lse[4], delta[4];
+    load_stats<16>(lse, delta, a, slab, i0, ty);
+    for (int j0 = 0; j0 < a.R; j0 += TT) {
+      if (!kAhead<DP>) {
+        __syncthreads();
+        stage(j0);
+      }
+      async_wait();
+      __syncthreads();
+      if (kAhead<DP> && j0 + TT < a.R) stage(j0 + TT);
+      const float* Ks = KV + (kAhead<DP> ? (j0 / TT & 1) * 2 * TT * LD : 0);
+      const float* Vs = Ks + TT * LD;
+      Terms terms;
+      load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
+      float p[4][4], ds[4][4];
+      dots<DP, 16>(p, Qs, Ks, ty, tx);
+      dots<DP, 16>(ds, Gs, Vs, ty, tx);
+      probs<16>(a, terms, lse, delta, i0, j0, ty, tx, p, ds);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) Ds[(ty + 16 * r) * PLD + tx + 16 * c] = ds[r][c];
-    __syncwarp();  // (a row of dS is written and read by the same half-warp)
-    weighted_rows<DP>(acc, Ds, Ks, ty, tx);
-    __syncwarp();
-  }
+        for (int c = 0; c < 4; ++c) Ds[(ty + 16 * r) * PLD + tx + 16 * c] = ds[r][c];
+      if (part != nullptr) {
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = i0 + ty + 16 * r;
-    if (i >= a.R) continue;
-    T* o = reinterpret_cast<T*>(a.dq) + off4(a.sdq, sl.b, sl.h, sl.s, i);
+        for (int r = 0; r < 4; ++r) {
+          const int i = i0 + ty + 16 * r;
+          float* out = part + (long long)i * ld + j0 + tx;
 #pragma unroll
-    for (int n = 0; n < DP / 16; ++n) {
-      const int d = Cols<DP>::at(tx, n);
-      if (d < a.D) o[d] = from_float<T>(acc[r][n] * a.scale);
+          for (int c = 0; c < 4; ++c)
+            if (i < a.R && j0 + tx + 16 * c < a.R) out[16 * c] = srow == s0 ? ds[r][c] : out[16 * c] + ds[r][c];
+        }
+      }
+      __syncwarp();  // (a row of dS is written and read by the same half-warp)
+      weighted_rows<DP>(acc, Ds, Ks, ty, tx);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int i = i0 + ty + 16 * r;
+      if (i >= a.R) continue;
+      T* o = reinterpret_cast<T*>(a.dq) + off4(a.sdq, sl.b, sl.h, sl.s, i);
+#pragma unroll
+      for (int n = 0; n < DP / 16; ++n) {
+        const int d = Cols<DP>::at(tx, n);
+        if (d < a.D) o[d] = from_float<T>(acc[r][n] * a.scale);
+      }
     }
   }
 }
@@ -391,22 +470,32 @@ __device__ __forceinline__ void dq_role(const Args& a, int vec, float* sm, int s
 template <class T, int DP>
 __device__ __forceinline__ void dkdv_role(const Args& a, int vec, float* sm, int slab, int j0) {
   constexpr int LD = DP + 4;
-  float* Qs = sm;
-  float* Gs = Qs + TT * LD;
-  float* Ks = Gs + TT * LD;
+  float* Ks = sm;
   float* Vs = Ks + TT * LD;
-  float* Pt = Vs + TT * LD;  // P^T and dS^T: [key][query]
+  float* QG = Vs + TT * LD;
+  float* Pt = QG + (kAhead<DP> ? 4 : 2) * TT * LD;  // P^T and dS^T: [key][query]
   float* Dt = Pt + TT * PLD;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const Slab sl = slab_of(slab, a);
+  auto stage = [&](int i0) {
+    float* dst = QG + (kAhead<DP> ? (i0 / TT & 1) * 2 * TT * LD : 0);
+    stage_rows_ahead<T, DP>(dst, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q);
+    stage_rows_ahead<T, DP>(dst + TT * LD, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO);
+  };
+  if (kAhead<DP>) stage(0);
   stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TT, a.R, a.D, vec & VEC_K, threadIdx.x, NTH);
   stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TT, a.R, a.D, vec & VEC_V, threadIdx.x, NTH);
   float accK[4][DP / 16] = {}, accV[4][DP / 16] = {}, dm[4] = {};
   for (int i0 = 0; i0 < a.R; i0 += TT) {
+    if (!kAhead<DP>) {
+      __syncthreads();
+      stage(i0);
+    }
+    async_wait();
     __syncthreads();
-    stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TT, a.R, a.D, vec & VEC_Q, threadIdx.x, NTH);
-    stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TT, a.R, a.D, vec & VEC_DO, threadIdx.x, NTH);
-    __syncthreads();
+    if (kAhead<DP> && i0 + TT < a.R) stage(i0 + TT);
+    const float* Qs = QG + (kAhead<DP> ? (i0 / TT & 1) * 2 * TT * LD : 0);
+    const float* Gs = Qs + TT * LD;
     Terms terms;
     load_terms<T, 16>(terms, a, sl, i0, j0, ty, tx);
     float p[4][4], ds[4][4], lse[4], delta[4];
@@ -454,84 +543,55 @@ __device__ __forceinline__ void dkdv_role(const Args& a, int vec, float* sm, int
   }
 }
 
-// dBias of 32 x 32 scores of one (b,h): the MSA rows are dealt out to the groups of 64 threads of the
-// block, whose sums are added in a fixed order at the end.
-template <int DP> constexpr int kGroups = DP <= 64 ? 4 : 2;
-template <class T, int DP>
-__device__ __forceinline__ void dbias_role(const Args& a, int vec, float* sm, int bh, int i0, int j0) {
-  constexpr int LD = DP + 4, NG = kGroups<DP>;
-  const int grp = threadIdx.x >> 6, t = threadIdx.x & 63, tx = t & 7, ty = t >> 3;
-  float acc[4][4] = {};
-  if (grp < NG) {
-    float* Qs = sm + grp * 4 * TB * LD;
-    float* Gs = Qs + TB * LD;
-    float* Ks = Gs + TB * LD;
-    float* Vs = Ks + TB * LD;
-    for (int s = grp; s < a.S; s += NG) {
-      const Slab sl{bh / a.H, bh % a.H, s};
-      ptx::named_bar_sync(1 + grp, 64);
-      stage_rows<T, DP>(Qs, reinterpret_cast<const T*>(a.q), a.sq, sl, i0, TB, a.R, a.D, vec & VEC_Q, t, 64);
-      stage_rows<T, DP>(Gs, reinterpret_cast<const T*>(a.d_o), a.sdo, sl, i0, TB, a.R, a.D, vec & VEC_DO, t, 64);
-      stage_rows<T, DP>(Ks, reinterpret_cast<const T*>(a.k), a.sk, sl, j0, TB, a.R, a.D, vec & VEC_K, t, 64);
-      stage_rows<T, DP>(Vs, reinterpret_cast<const T*>(a.v), a.sv, sl, j0, TB, a.R, a.D, vec & VEC_V, t, 64);
-      float p[4][4], ds[4][4], lse[4], delta[4];
-      load_stats<8>(lse, delta, a, (long long)bh * a.S + s, i0, ty);
-      Terms terms;
-      load_terms<T, 8>(terms, a, sl, i0, j0, ty, tx);
-      ptx::named_bar_sync(1 + grp, 64);
-      dots<DP, 8>(p, Qs, Ks, ty, tx);
-      dots<DP, 8>(ds, Gs, Vs, ty, tx);
-      probs<8>(a, terms, lse, delta, i0, j0, ty, tx, p, ds);
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] += ds[r][c];
-    }
-  }
-  __syncthreads();
-  float* part = sm;  // [group][32][32]
-  if (grp < NG) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) part[grp * TB * TB + (ty + 8 * r) * TB + tx + 8 * c] = acc[r][c];
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < TB * TB; e += NTH) {
-    const int i = i0 + e / TB, j = j0 + e % TB;
-    float tot = part[e];
-#pragma unroll
-    for (int g = 1; g < NG; ++g) tot += part[g * TB * TB + e];
-    if (i < a.R && j < a.R) a.dbias[((long long)bh * a.R + i) * a.dbias_ld + j] = tot;
-  }
+// How the MSA rows are dealt out to the blocks that compute dQ and d(pair_bias): runs of `rows`, each run
+// with a partial d(pair_bias) of its own unless there is only one.  Long enough that the partial sums
+// stay few, short enough for some four blocks per SM.
+struct Runs {
+  int rows, n;
+};
+Runs plan_runs(const Args& a) {
+  if (!a.dbias) return Runs{1, a.S};
+  const long long tiles = (long long)a.B * a.H * ((a.R + TT - 1) / TT);
+  const int want = (int)min((long long)a.S, (600 + tiles - 1) / tiles);
+  const int rows = (a.S + want - 1) / want;
+  return Runs{rows, (a.S + rows - 1) / rows};
 }
 
-// The three parts of a backward call read the same inputs and write different outputs: one launch, the
-// d(pair_bias) blocks (which walk all MSA rows) first.
+// The two parts of a backward call read the same inputs and write different outputs: one launch, the
+// blocks that walk several MSA rows first.
 template <class T, int DP>
-__global__ void __launch_bounds__(NTH, DP <= 32 ? 2 : 1) generic_bwd_kernel(const Args a, const int vec, const long long n_dbias,
-                                                                          const long long n_total) {
+__global__ void __launch_bounds__(NTH, DP <= 32 ? 2 : 1) generic_bwd_kernel(const Args a, const int vec, const Runs runs, float* part,
+                                                                          const long long n_dq, const long long n_total) {
   extern __shared__ __align__(16) float sm[];
   long long idx = (long long)blockIdx.y * gridDim.x + blockIdx.x;
   if (idx >= n_total) return;
-  if (idx < n_dbias) {
-    const int nb = (a.R + TB - 1) / TB;
-    const int tj = (int)(idx % nb), ti = (int)(idx / nb % nb), bh = (int)(idx / nb / nb);
-    dbias_role<T, DP>(a, vec, sm, bh, ti * TB, tj * TB);
+  const int nt = (a.R + TT - 1) / TT;
+  const int i0 = (int)(idx % nt) * TT;
+  if (idx >= n_dq) {
+    idx -= n_dq;
+    dkdv_role<T, DP>(a, vec, sm, (int)(idx / nt), (int)(idx % nt) * TT);
     return;
   }
-  idx -= n_dbias;
-  const long long half = (n_total - n_dbias) / 2;
-  const int nt = (a.R + TT - 1) / TT;
-  if (idx < half) dkdv_role<T, DP>(a, vec, sm, (int)(idx / nt), (int)(idx % nt) * TT);
-  else dq_role<T, DP>(a, vec, sm, (int)((idx - half) / nt), (int)((idx - half) % nt) * TT);
+  const int run = (int)(idx / nt % runs.n), bh = (int)(idx / nt / runs.n);
+  float* mine = nullptr;
+  const int ld = runs.n == 1 ? a.dbias_ld : a.R;
+  if (a.dbias) mine = (runs.n == 1 ? a.dbias : part + (long long)run * a.B * a.H * a.R * ld) + (long long)bh * a.R * ld;
+  dq_role<T, DP>(a, vec, sm, bh, run * runs.rows, min(a.S, (run + 1) * runs.rows), i0, mine, ld);
 }
 
-template <int DP> constexpr int fwd_smem() { return (3 * TT * (DP + 4) + TT * PLD) * 4; }
-template <int DP> constexpr int bwd_smem() {
-  constexpr int tiles = (4 * TT * (DP + 4) + 2 * TT * PLD) * 4, groups = kGroups<DP> * 4 * TB * (DP + 4) * 4;
-  return tiles > groups ? tiles : groups;
+// d(pair_bias) = the partial sums, added in order.
+__global__ void __launch_bounds__(256) generic_dbias_sum_kernel(const float* __restrict__ part, int n, long long rows, int R, float* __restrict__ dst,
+                                                                int ld) {
+  const long long total = rows * R;
+  for (long long e = (long long)blockIdx.x * 256 + threadIdx.x; e < total; e += (long long)gridDim.x * 256) {
+    float t = part[e];
+    for (int k = 1; k < n; ++k) t += part[k * total + e];
+    dst[ld == R ? e : e / R * ld + e % R] = t;
+  }
 }
+
+template <int DP> constexpr int fwd_smem() { return ((kAhead<DP> ? 5 : 3) * TT * (DP + 4) + TT * PLD) * 4; }
+template <int DP> constexpr int bwd_smem() { return ((kAhead<DP> ? 6 : 4) * TT * (DP + 4) + 2 * TT * PLD) * 4; }
 
 template <class T>
 bool vec_ok(const void* p, const Str4& s) {
@@ -553,6 +613,8 @@ cudaError_t launch_fwd_t(const Args& a, cudaStream_t st, int* launches) {
   return cudaGetLastError();
 }
 
+size_t delta_bytes(const Args& a) { return ((size_t)a.B * a.H * a.S * a.delta_ld * sizeof(float) + 255) / 256 * 256; }
+
 template <class T, int DP>
 cudaError_t launch_bwd_t(Args a, cudaStream_t st, int* launches) {
   const long long rows = (long long)a.B * a.H * a.S * a.R;
@@ -564,12 +626,18 @@ cudaError_t launch_bwd_t(Args a, cudaStream_t st, int* launches) {
   }
   auto kern = generic_bwd_kernel<T, DP>;
   if (!kernel_ready(reinterpret_cast<const void*>(kern), bwd_smem<DP>(), nullptr)) return cudaErrorUnknown;
-  const long long nt = (a.R + TT - 1) / TT, nb = (a.R + TB - 1) / TB;
-  const long long n_dbias = a.dbias ? (long long)a.B * a.H * nb * nb : 0;
-  const long long n_total = n_dbias + 2 * (long long)a.B * a.H * a.S * nt;
+  const Runs runs = plan_runs(a);
+  float* part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(a.delta) + delta_bytes(a));
+  const long long nt = (a.R + TT - 1) / TT;
+  const long long n_dq = (long long)a.B * a.H * runs.n * nt, n_total = n_dq + (long long)a.B * a.H * a.S * nt;
   const long long gx = n_total < (1 << 30) ? n_total : (1 << 30);
-  kern<<<dim3((unsigned)gx, (unsigned)((n_total + gx - 1) / gx)), NTH, bwd_smem<DP>(), st>>>(a, vec_flags<T>(a, true), n_dbias, n_total);
+  kern<<<dim3((unsigned)gx, (unsigned)((n_total + gx - 1) / gx)), NTH, bwd_smem<DP>(), st>>>(a, vec_flags<T>(a, true), runs, part, n_dq, n_total);
   *launches += 2;
+  if (a.dbias && runs.n > 1) {
+    const long long drows = (long long)a.B * a.H * a.R, blocks = (drows * a.R + 1023) / 1024;
+    generic_dbias_sum_kernel<<<(unsigned)(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(part, runs.n, drows, a.R, a.dbias, a.dbias_ld);
+    *launches += 1;
+  }
   return cudaGetLastError();
 }
 
@@ -589,6 +657,11 @@ cudaError_t launch_bwd_d(const Args& a, cudaStream_t st, int* launches) {
 }
 
 }  // namespace
+
+size_t generic_bwd_workspace_bytes(const Args& a) {
+  const Runs runs = plan_runs(a);
+  return delta_bytes(a) + (a.dbias && runs.n > 1 ? (size_t)runs.n * a.B * a.H * a.R * a.R * sizeof(float) : 0);
+}
 
 cudaError_t launch_generic_fwd(int dtype, const Args& a, cudaStream_t st, int* launches) {
   switch (dtype) {

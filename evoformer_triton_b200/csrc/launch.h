@@ -39,7 +39,9 @@ inline bool kernel_ready(const void* kern, int smem_bytes, int* num_regs) {
   return true;
 }
 
-// CUDA-core kernels (generic_kernels.cu).  Backward needs a.delta = [B,H,S,R] fp32 scratch.
+// CUDA-core kernels (generic_kernels.cu).  Backward needs generic_bwd_workspace_bytes() of scratch at a.delta
+// (asked for with a.dbias set if and only if d(pair_bias) is wanted).
+size_t generic_bwd_workspace_bytes(const Args& a);
 cudaError_t launch_generic_fwd(int dtype, const Args& a, cudaStream_t st, int* launches);
 cudaError_t launch_generic_bwd(int dtype, const Args& a, cudaStream_t st, int* launches);
 
