@@ -44,6 +44,7 @@ constexpr int BN = 64;   // keys per tile
 constexpr int kThreads = 384;
 constexpr int kTmemCols = 512;
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kGrow = 8.f / kLog2e;  // how far a tile's maximum may exceed the running one
 constexpr int MASK_MIN = 0;  // boolean keep-mask (or none): score = min(score, m), m = +-FLT_MAX
 constexpr int MASK_ADD = 1;  // additive mask
 
@@ -63,12 +64,12 @@ struct Cfg {
   static constexpr int offV = offK + KVW * NKV * kKV;
   static constexpr int offB = offV + KVW * NKV * kKV;
   static constexpr int offMask = offB + BST * BTL * kBias;
-  static constexpr int kNumBars = 2 * (2 * QST + 4 * NKV + 2 + 1 + 2 + 4) + 2 * BST;
+  static constexpr int kNumBars = 2 * (2 * QST + 4 * NKV + 2 + 1 + 1 + 4) + 2 * BST;
   static size_t bytes(int r_pad) {
     return (size_t)offMask + (size_t)4 * r_pad * 4 + 4 * 32 * 4 + kNumBars * 8 + 64 + 1024;
   }
-  // TMEM columns of warpgroup w: S double buffer, then PV double buffer
-  static constexpr int tmemWg = 2 * BN + 2 * DP;
+  // TMEM columns of warpgroup w: S double buffer, then O
+  static constexpr int tmemWg = 2 * BN + DP;
 };
 
 // A work item: warpgroup w works on query tile qt[w] of MSA row s[w] of (b, h).  Row-pair mode: rows
@@ -113,7 +114,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   uint32_t* sDirty = reinterpret_cast<uint32_t*>(sMask + 4 * r_pad);  // [warpgroup][stage][32]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDirty + 4 * 32);
   // barrier layout: per warpgroup w a block of PER, then the shared bias barriers
-  constexpr int PER = 2 * QST + 4 * NKV + 2 + 1 + 2 + 4;
+  constexpr int PER = 2 * QST + 4 * NKV + 2 + 1 + 1 + 4;
   auto q_full = [&](int w, int st) { return bars + w * PER + st; };
   auto q_empty = [&](int w, int st) { return bars + w * PER + QST + st; };
   auto k_full = [&](int w, int st) { return bars + w * PER + 2 * QST + st; };
@@ -122,9 +123,9 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   auto v_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 3 * NKV + st; };
   auto s_full = [&](int w, int i) { return bars + w * PER + 2 * QST + 4 * NKV + i; };
   auto p_full = [&](int w) { return bars + w * PER + 2 * QST + 4 * NKV + 2; };
-  auto o_full = [&](int w, int i) { return bars + w * PER + 2 * QST + 4 * NKV + 3 + i; };
-  auto m_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 5 + st; };
-  auto m_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 7 + st; };
+  auto o_full = [&](int w) { return bars + w * PER + 2 * QST + 4 * NKV + 3; };
+  auto m_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 4 + st; };
+  auto m_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 6 + st; };
   auto b_full = [&](int st) { return bars + 2 * PER + st; };
   auto b_empty = [&](int st) { return bars + 2 * PER + BST + st; };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kNumBars);
@@ -152,7 +153,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       }
       mbar_init(s_full(w, 0), 1); mbar_init(s_full(w, 1), 1);
       mbar_init(p_full(w), 4);  // one arrival per softmax warp
-      mbar_init(o_full(w, 0), 1); mbar_init(o_full(w, 1), 1);
+      mbar_init(o_full(w), 1);
       for (int st = 0; st < 2; ++st) { mbar_init(m_full(w, st), 1); mbar_init(m_empty(w, st), 4); }
     }
     for (int st = 0; st < BST; ++st) { mbar_init(b_full(st), 1); mbar_init(b_empty(st), 8); }
@@ -243,7 +244,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         mma_commit(k_empty(kw, st));
         mma_commit(s_full(w, g & 1));
       };
-      auto issue_pv = [&](uint32_t g) {
+      auto issue_pv = [&](uint32_t g, bool first) {  // O += P V; the first of an item overwrites
         const int st = g % NKV;
         mbar_wait(v_full(kw, st), (g / NKV) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
         mbar_wait(p_full(w), g & 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
@@ -251,16 +252,15 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         const uint32_t va = v_lo0 + st * (C::kKV >> 4);
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // 16 keys = 8 packed columns of P per step
-          mma_ts(tO + (g & 1) * DP, tS + (g & 1) * BN + kk * 8, pack_desc(va + kk * RB, kHiOp), kIdescO,
-                 kk > 0 ? 1u : 0u);
+          mma_ts(tO, tS + (g & 1) * BN + kk * 8, pack_desc(va + kk * RB, kHiOp), kIdescO, (kk > 0 || !first) ? 1u : 0u);
         mma_commit(v_empty(kw, st));
-        mma_commit(o_full(w, g & 1));
+        mma_commit(o_full(w));
       };
       for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
         mbar_wait(q_full(w, qn % QST), (qn / QST) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
         for (int t = 0; t < 2 && t < T_TILES; ++t) issue_s(base + t);
         for (int t = 0; t < T_TILES; ++t) {
-          issue_pv(base + t);
+          issue_pv(base + t, t == 0);
           if (t + 2 < T_TILES) issue_s(base + t + 2);  // S buffer (t&1) was read before P_t was signalled
         }
         mma_commit(q_empty(w, qn % QST));
@@ -355,10 +355,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const float* mrow_base = sMask + (w * 2 + mst) * r_pad;
       const uint32_t* dirty_row = sDirty + (w * 2 + mst) * 32;
 
-      float m_run = -FLT_MAX, l_run = 0.f, alpha_pending = 1.f;
-      float acc[DP];
-#pragma unroll
-      for (int d = 0; d < DP; ++d) acc[d] = 0.f;
+      float m_run = -FLT_MAX, l_run = 0.f;
 
       for (int t = 0; t < T_TILES; ++t, ++g) {
         mbar_wait(s_full(w, g & 1), (g >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
@@ -439,13 +436,36 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           if (lane == 0) mbar_arrive(b_empty(g % BST));  // one arrival per warp
         }
 
-        const float m_new = fmaxf(m_run, mx);
-        const float alpha = ex2((m_run - m_new) * kLog2e);
+        // The running maximum follows a tile's maximum only when that has grown by more than 2^8: the row
+        // sum and O carry the same factor, so their quotient does not change and nothing overflows.  Then,
+        // and only then, O is rescaled in tensor memory (P V of the tile before has to be complete).
+        if (t == 0) {
+          m_run = mx;
+        } else {
+          const bool grow = mx > m_run + kGrow;
+          if (__any_sync(0xffffffffu, grow)) {
+            const float m_up = grow ? mx : m_run;
+            const float alpha = ex2((m_run - m_up) * kLog2e);
+            m_run = m_up;
+            l_run *= alpha;
+            mbar_wait(o_full(w), (g - 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
+            tc_fence_after();
+#pragma unroll
+            for (int d0 = 0; d0 < DP; d0 += 16) {
+              uint32_t o[16];
+              tmem_ld16(t_base + 2 * BN + d0, o);
+              tmem_wait_ld();
+#pragma unroll
+              for (int u = 0; u < 16; ++u) o[u] = __float_as_uint(__uint_as_float(o[u]) * alpha);
+              tmem_st16(t_base + 2 * BN + d0, o);
+            }
+          }
+        }
         float lsum = 0.f;
         uint32_t pk[BN / 2];
         named_bar_sync(1 + w, 256);  // my turn on the exponential unit
-        if (m_new != -FLT_MAX) {
-          const float nm2 = -m_new * kLog2e;
+        if (m_run != -FLT_MAX) {
+          const float nm2 = -m_run * kLog2e;
           const F2 l2e2 = f2_make(kLog2e, kLog2e), nm22 = f2_make(nm2, nm2);
           F2 ls4[4];
 #pragma unroll
@@ -497,24 +517,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           }
         }
         named_bar_arrive(2 - w, 256);  // hand the turn to the other warpgroup
-        l_run = l_run * alpha + lsum;
-        m_run = m_new;
-
-        // fold the previous tile's P V into the accumulator (its MMA ran while we did the exps)
-        if (t > 0) {
-          mbar_wait(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
-          tc_fence_after();
-          uint32_t orr[DP];
-          tmem_ld<(DP >= 32 ? 32 : 16)>(t_base + 2 * BN + ((g - 1) & 1) * DP, *reinterpret_cast<uint32_t(*)[DP >= 32 ? 32 : 16]>(&orr[0]));
-          if constexpr (DP == 64)
-            tmem_ld32(t_base + 2 * BN + ((g - 1) & 1) * DP + 32, *reinterpret_cast<uint32_t(*)[32]>(&orr[32]));
-          tmem_wait_ld();
-          const F2 ap2 = f2_make(alpha_pending, alpha_pending);
-#pragma unroll
-          for (int d = 0; d < DP; d += 2)
-            f2_get(f2_fma(f2_make(acc[d], acc[d + 1]), ap2, f2_from_bits(orr[d], orr[d + 1])), acc[d], acc[d + 1]);
-        }
-        alpha_pending = alpha;
+        l_run += lsum;
 
         // P_n -> TMEM, packed two 16-bit values per column, over the first half of the S_n
         // columns this thread has just consumed (lane = row, column j = keys 2j, 2j+1): the
@@ -525,18 +528,14 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full(w));
       }
-      // last tile's P V
-      {
-        mbar_wait(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
-        tc_fence_after();
-        uint32_t orr[DP];
-        tmem_ld<(DP >= 32 ? 32 : 16)>(t_base + 2 * BN + ((g - 1) & 1) * DP, *reinterpret_cast<uint32_t(*)[DP >= 32 ? 32 : 16]>(&orr[0]));
-        if constexpr (DP == 64)
-          tmem_ld32(t_base + 2 * BN + ((g - 1) & 1) * DP + 32, *reinterpret_cast<uint32_t(*)[32]>(&orr[32]));
-        tmem_wait_ld();
+      // O of the item, complete with its last P V
+      mbar_wait(o_full(w), (g - 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
+      tc_fence_after();
+      float acc[DP];
 #pragma unroll
-        for (int d = 0; d < DP; ++d) acc[d] = fmaf(acc[d], alpha_pending, __uint_as_float(orr[d]));
-      }
+      for (int d0 = 0; d0 < DP; d0 += 16) tmem_ld16(t_base + 2 * BN + d0, *reinterpret_cast<uint32_t(*)[16]>(&acc[d0]));
+      tmem_wait_ld();
+      tc_fence_before();  // (the next item's first P V, which overwrites O, is released by a later arrival)
       if (active && i < a.R) {
         const float inv = 1.f / l_run;
         T* orow = reinterpret_cast<T*>(a.o) + off4(a.so, it.b, it.h, s, i);
