@@ -24,9 +24,8 @@
 // Per warpgroup and key tile n:  S_n = Q K_n^T lands in TMEM (double buffered); the
 // warpgroup turns it into P_n (rounded to the storage type as evoformer.py:84 does) and
 // writes it back over S_n in TMEM, from where it feeds the P V MMA as the A operand;
-// P_n V_n lands in a second TMEM double buffer and is folded into the
-// fp32 output accumulator in registers one tile later, scaled by the softmax correction
-// of that tile.  The MMA warp runs S_{n+1} while the warpgroup is busy with tile n.
+// O accumulates in TMEM over the item.  The MMA warp runs S_{n+1} while the warpgroup is busy with
+// tile n.
 #include <type_traits>
 
 #include "common.cuh"
@@ -109,8 +108,8 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   const int T_TILES = (a.R + BN - 1) / BN;
   const int r_pad = T_TILES * BN;
   float* sMask = reinterpret_cast<float*>(smem + C::offMask);  // [warpgroup][stage][r_pad]
-  // one word per key tile of a staged mask row: non-zero if the tile has a dropped key (a key tile
-  // without one skips the mask arithmetic and the mask loads in the boolean form); R <= 2048
+  // one word per key tile of a staged mask row: non-zero if the tile has a key that the mask changes;
+  // R <= 2048
   uint32_t* sDirty = reinterpret_cast<uint32_t*>(sMask + 4 * r_pad);  // [warpgroup][stage][32]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDirty + 4 * 32);
   // barrier layout: per warpgroup w a block of PER, then the shared bias barriers
@@ -313,7 +312,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
                 else unpack2<T>(raw[u], v, m[u]);
               }
               m[u] = j + u < a.R ? v : -FLT_MAX;
-              any |= m[u] < 0.f;
+              any |= kMin ? m[u] < 0.f : m[u] != 0.f;
             }
             if (j < r_pad) {
               *reinterpret_cast<float4*>(dst + j) = make_float4(m[0], m[1], m[2], m[3]);
@@ -375,8 +374,8 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tmem_ld32(t_base + (g & 1) * BN, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
         tmem_ld32(t_base + (g & 1) * BN + 32, *reinterpret_cast<uint32_t(*)[32]>(&sr[32]));
         tmem_wait_ld();
-        // A key tile of a boolean mask without a dropped key needs neither the mask values nor
-        // the `min` (most tiles: masks are mostly trailing padding); the flag is warp-uniform.
+        // A key tile whose mask drops no key (boolean) or adds only zeros needs neither the mask values
+        // nor the arithmetic (most tiles: masks are mostly trailing padding); the flag is warp-uniform.
         auto scores = [&](auto with_mask) {
           constexpr bool kMask = decltype(with_mask)::value;
 #pragma unroll
@@ -418,9 +417,10 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
             }
           }
         };
-        // (only where it measured faster: at D = 64 and D <= 16 the second copy of the loop costs
-        // more than the skipped instructions save)
-        if constexpr (DP == 32 && MASKMODE == MASK_MIN) {
+        // ([4,1,2048,32,64] with an additive mask 333 -> 312 us, [2,64,768,8,64] boolean 398 -> 378.  At
+        // D <= 16 the second copy of the loop costs more than the skipped instructions save: 741 -> 800 us
+        // on [1,1024,384,8,8], where a random mask leaves no tile without a dropped key.)
+        if constexpr (DP >= 32) {
           if (dirty_row[t] != 0u) scores(std::true_type{});
           else scores(std::false_type{});
         } else {
