@@ -1,0 +1,80 @@
+"""GPU: the places where the kernels' tiling, splitting and dispatch can go wrong, against the oracle:
+edges of the CUDA-core tiles and of the runs of MSA rows that share a partial d(pair_bias), the forward's
+rescaling of an output that is accumulated in tensor memory, key tiles that skip the mask arithmetic, and
+d(pair_bias) leaving in each type and layout."""
+import pytest
+import torch
+
+from oracle import evo_oracle as oc
+from test_parity_gpu import DEV, _lib, check, rand_inputs, run_op
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cfg", [
+    (1, 1, 1, 1, 8), (2, 3, 63, 2, 16), (1, 2, 64, 2, 32), (1, 37, 65, 2, 32), (1, 5, 129, 1, 64),
+    (1, 3, 130, 2, 100), (1, 2, 70, 1, 128), (1, 700, 40, 1, 7)], ids=lambda c: "B%dS%dR%dH%dD%d" % c)
+@pytest.mark.parametrize("mask,bias", [("bool", True), ("add32", True), ("none", False)])
+def test_cuda_core_tiles_fp32(cfg, mask, bias):
+    B, S, R, H, D = cfg
+    x = rand_inputs(B, S, R, H, D, torch.float32, seed=R + D, mask=mask, bias=bias)
+    got, paths = run_op(x)
+    assert paths == (_lib().PATH_GENERIC, _lib().PATH_GENERIC)
+    if R == 1:  # one key: P = 1, every score gradient is rounding noise around 0
+        assert torch.equal(got[0], x["V"]) or not x["res_mask"].any()
+        return
+    check(got, x, label=f"{cfg} {mask} ")
+
+
+def test_cuda_core_backward_is_reproducible_over_runs_of_rows():
+    x = rand_inputs(1, 90, 72, 2, 24, torch.float32, seed=2)
+    a, b = run_op(x)[0], run_op(x)[0]
+    assert all(torch.equal(u, v) for u, v in zip(a, b))
+
+
+@pytest.mark.parametrize("D,dtype,S", [(8, torch.float16, 3), (32, torch.bfloat16, 2), (64, torch.bfloat16, 1)])
+def test_running_maximum_that_keeps_growing(D, dtype, S):
+    """Scores that rise from key tile to key tile by far more than the forward lets the running maximum lag,
+    by less than that, and that fall again; the rows start with a tile whose keys are all dropped."""
+    R = 448
+    x = rand_inputs(1, S, R, 2, D, dtype, seed=D, keep_p=0.9)
+    ramp = torch.cat([torch.full((64,), float(v)) for v in (0, 3, 7, 30, 31, 60, 10)])
+    x["pair_bias"] = x["pair_bias"] * 0.5 + ramp
+    x["res_mask"][..., :64] = False
+    got, _ = run_op(x, want_path=_lib().PATH_TCGEN05)
+    check(got, x, label=f"ramp D={D} ")
+
+
+@pytest.mark.parametrize("mask", ["bool", "add32", "addsame"])
+@pytest.mark.parametrize("D", [16, 32, 64])
+def test_mask_that_touches_some_key_tiles(mask, D):
+    x = rand_inputs(1, 3, 328, 2, D, torch.bfloat16, seed=D, mask=mask, keep_p=1.1)
+    drop = torch.tensor([70, 71, 319])
+    if mask == "bool":
+        x["res_mask"][..., drop] = False
+    else:
+        x["res_mask"][..., drop] = torch.tensor([-1e9, 1.5, -2.0]).to(x["res_mask"].dtype)
+    got, _ = run_op(x, want_path=_lib().PATH_TCGEN05)
+    check(got, x, label=f"{mask} D={D} ")
+
+
+@pytest.mark.parametrize("layout", ["b1hrr", "brrh"])
+@pytest.mark.parametrize("bias_dtype", [torch.float32, torch.bfloat16, torch.float64])
+@pytest.mark.parametrize("R", [96, 130])
+def test_pair_bias_gradient_in_its_type_and_layout(layout, bias_dtype, R):
+    import evoformer_triton_b200 as evo
+    B, S, H, D = 2, 4, 3, 32
+    x = rand_inputs(B, S, R, H, D, torch.bfloat16, seed=R)
+    x["pair_bias"] = x["pair_bias"].bfloat16().float()
+    want = oc.attention_fwd_bwd(x["Q"], x["K"], x["V"], x["res_mask"], x["pair_bias"], x["dO"], upcast=torch.float32)[4]
+    bias = x["pair_bias"].to(bias_dtype)
+    if layout == "brrh":
+        bias = bias.reshape(B, H, R, R).permute(0, 2, 3, 1).contiguous()
+    q, k, v, b = (t.to(DEV).requires_grad_() for t in (x["Q"], x["K"], x["V"], bias))
+    out = evo.evoformer_attention(q, k, v, [x["res_mask"].to(DEV), b], layout="reinterpret", pair_bias_layout=layout)
+    out.backward(x["dO"].to(DEV))
+    torch.cuda.synchronize()
+    evo.check_device_status()
+    assert b.grad.dtype == bias_dtype and b.grad.shape == bias.shape
+    got = b.grad if layout == "b1hrr" else b.grad.permute(0, 3, 1, 2).reshape(B, 1, H, R, R)
+    assert oc.rel_err(got, want) < 1e-2
