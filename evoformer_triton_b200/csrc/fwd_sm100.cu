@@ -65,10 +65,12 @@ struct Cfg {
   static constexpr int offMask = offB + BST * BTL * kBias;
   static constexpr int kNumBars = 2 * (2 * QST + 4 * NKV + 2 + 1 + 1 + 4) + 2 * BST;
   static size_t bytes(int r_pad) {
-    return (size_t)offMask + (size_t)4 * r_pad * 4 + 4 * 32 * 4 + kNumBars * 8 + 64 + 1024;
+    return (size_t)offMask + (size_t)4 * r_pad * 4 + 4 * 32 * 4 + kOnes + kNumBars * 8 + 64 + 1024;
   }
-  // TMEM columns of warpgroup w: S double buffer, then O
-  static constexpr int tmemWg = 2 * BN + DP;
+  static constexpr int kOnes = 512;  // a 16 x 16 operand of ones
+  // TMEM columns of warpgroup w: S double buffer, then O, then the row sum of P (16 equal columns)
+  static constexpr int colL = 2 * BN + DP, tmemWg = colL + 16;
+  static_assert(2 * tmemWg <= kTmemCols, "TMEM budget");
 };
 
 // A work item: warpgroup w works on query tile qt[w] of MSA row s[w] of (b, h).  Row-pair mode: rows
@@ -111,7 +113,8 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   // one word per key tile of a staged mask row: non-zero if the tile has a key that the mask changes;
   // R <= 2048
   uint32_t* sDirty = reinterpret_cast<uint32_t*>(sMask + 4 * r_pad);  // [warpgroup][stage][32]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDirty + 4 * 32);
+  uint32_t* sOnes = sDirty + 4 * 32;  // 16 x 16 ones of the storage type
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOnes + C::kOnes / 4);
   // barrier layout: per warpgroup w a block of PER, then the shared bias barriers
   constexpr int PER = 2 * QST + 4 * NKV + 2 + 1 + 1 + 4;
   auto q_full = [&](int w, int st) { return bars + w * PER + st; };
@@ -159,6 +162,10 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     fence_mbar_init();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV);
     if (has_bias) prefetch_tmap(&tmB);
+  }
+  if (tid < C::kOnes / 4) {
+    sOnes[tid] = Pack2<T>::pack(1.f, 1.f);
+    fence_async_shared();
   }
   if (warp == 0) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -220,6 +227,8 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const int w = warp - 1;
       constexpr uint32_t kIdescS = make_idesc(kBf16, false, false, BM, BN);
       constexpr uint32_t kIdescO = make_idesc(kBf16, false, true, BM, DP);
+      constexpr uint32_t kIdescL = make_idesc(kBf16, false, false, BM, 16);
+      const uint64_t ones = make_sdesc_const(128, 256, 0) | (smem_u32(sOnes) >> 4);  // unswizzled 8 x 16-byte core matrices
       // Descriptor halves that never change: the high word holds the stride offset, version and
       // swizzle; the low word is (address >> 4) plus the leading-offset field.
       constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
@@ -252,6 +261,10 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // 16 keys = 8 packed columns of P per step
           mma_ts(tO, tS + (g & 1) * BN + kk * 8, pack_desc(va + kk * RB, kHiOp), kIdescO, (kk > 0 || !first) ? 1u : 0u);
+        // the row sums of P as it was rounded: O is divided by these (see the epilogue)
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk)
+          mma_ts(tS + C::colL, tS + (g & 1) * BN + kk * 8, ones, kIdescL, (kk > 0 || !first) ? 1u : 0u);
         mma_commit(v_empty(kw, st));
         mma_commit(o_full(w));
       };
@@ -451,7 +464,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
             mbar_wait(o_full(w), (g - 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
             tc_fence_after();
 #pragma unroll
-            for (int d0 = 0; d0 < DP; d0 += 16) {
+            for (int d0 = 0; d0 < DP + 16; d0 += 16) {  // O and the row sum behind it
               uint32_t o[16];
               tmem_ld16(t_base + 2 * BN + d0, o);
               tmem_wait_ld();
@@ -534,10 +547,16 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       float acc[DP];
 #pragma unroll
       for (int d0 = 0; d0 < DP; d0 += 16) tmem_ld16(t_base + 2 * BN + d0, *reinterpret_cast<uint32_t(*)[16]>(&acc[d0]));
+      // O is divided by the sum of the P it was made of, rounded to the storage type.  The running maximum
+      // may lag, so the largest P of a row is not exactly 1; with the sum of the unrounded values its
+      // rounding would go into O in full (an fp16 O was off by 5.4e-4 instead of 2.7e-4).  The log-sum-exp
+      // is that of the unrounded values.
+      uint32_t lr[4];
+      tmem_ld4(t_base + C::colL, lr);
       tmem_wait_ld();
       tc_fence_before();  // (the next item's first P V, which overwrites O, is released by a later arrival)
       if (active && i < a.R) {
-        const float inv = 1.f / l_run;
+        const float inv = 1.f / __uint_as_float(lr[0]);
         T* orow = reinterpret_cast<T*>(a.o) + off4(a.so, it.b, it.h, s, i);
         const T* grow = a.gate ? reinterpret_cast<const T*>(a.gate) + off4(a.sgate, it.b, it.h, s, i) : nullptr;
 #pragma unroll

@@ -265,13 +265,17 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
                : "r"(taddr)
                : "memory");
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : EVO_R4(r, 0) : "r"(taddr) : "memory");
+}
 #undef EVO_R4
 template <int N>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[N]) {
-  static_assert(N == 8 || N == 16 || N == 32, "unsupported TMEM load width");
+  static_assert(N == 4 || N == 8 || N == 16 || N == 32, "unsupported TMEM load width");
   if constexpr (N == 32) tmem_ld32(taddr, r);
   else if constexpr (N == 16) tmem_ld16(taddr, r);
-  else tmem_ld8(taddr, r);
+  else if constexpr (N == 8) tmem_ld8(taddr, r);
+  else tmem_ld4(taddr, r);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -491,6 +495,20 @@ __device__ __forceinline__ void mma_ts_x2(uint32_t d_tmem, uint32_t a_tmem, uint
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d0, %5, p;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], d1, %5, t;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(b_step), "r"(idesc), "r"(acc_first)
+      : "memory");
+}
+// One D[tmem] = A[smem] * B[smem] over one K slice, then a commit to `bar` (and to `bar2` if non-zero).
+__device__ __forceinline__ void mma_ss_x1_commit(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                 uint32_t bar, uint32_t bar2) {
+  asm volatile(
+      "{\n\t.reg .pred f, c;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 f, 0, 0;\n\t"
+      "setp.ne.b32 c, %6, 0;\n\t"
+      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, f;\n\t"
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t"
+      "@c tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t}"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(bar), "r"(bar2)
       : "memory");
 }
 // Two D[tmem] = A[smem] * B[smem] over two K slices (descriptors advance by `k_step` units), then a
