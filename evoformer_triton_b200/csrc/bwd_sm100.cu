@@ -46,7 +46,7 @@ constexpr int QT = 32;    // queries per quarter of a step
 constexpr int kSub = 1;
 // MSA rows per work item: each keeps a dK and a dV accumulator of DP columns in tensor memory for the
 // whole item, next to 256 columns of score buffers and two dQ partials
-template <int DP> struct RowsPerItem { static constexpr int G = (DP == 64) ? 1 : 3; };
+template <int DP> struct RowsPerItem { static constexpr int G = (DP == 64) ? 1 : (DP == 32) ? 3 : 7; };
 constexpr int kCW = 16;   // compute warps
 constexpr int kThreadsT = 640;  // 16 compute + 4 service warps, five warps per scheduler
 constexpr int kComputeRegs = 112, kServiceRegs = 32;  // after setmaxnreg; the launch-time pool must hold their sum
@@ -211,7 +211,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   constexpr int RB = L::RB;
   constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-  static_assert(DP == 32 || DP == 64, "padded head dimension");
+  static_assert(DP == 16 || DP == 32 || DP == 64, "padded head dimension");
   constexpr int G = RowsPerItem<DP>::G;
   constexpr int kTmemCols = 512;
   // TMEM: two (S^T, dP^T) half-tile buffers, the per-row dV and dK accumulators, two dQ partials
@@ -233,7 +233,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBars);
   const uint32_t bars_s = smem_u32(bars);
   const Bar kv_full{bars_s + 8 * 0};     // [G] K and V of row g of the current item landed
-  const Bar kv_empty{bars_s + 8 * 3};    // [G] ... and every MMA that reads them has completed
+  const Bar kv_empty{bars_s + 8 * 7};    // [G] ... and every MMA that reads them has completed
   const Bar st_full{bars_s + 8 * 32};     // [2] Q, dO and the statistics vectors of a step landed
   const Bar st_empty{bars_s + 8 * 40};    // [2] ... the step's last dV/dK MMAs have completed
   const Bar sd_full{bars_s + 8 * 48};    // [2][kSub] S^T and dP^T of score buffer (h, sub) of a step are in TMEM
@@ -287,7 +287,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   if (*abort_flag) return;
 
   if (tid == 0) {
-    for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 3 + i, 3); }  // kv_full; kv_empty: three MMA warps read K/V
+    for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); }  // kv_full; kv_empty: three MMA warps read K/V
     for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
     for (int i = 0; i < 2; ++i) {
       for (int q = 0; q < 2; ++q) { mbar_init(bars + 48 + 2 * i + q, 2); mbar_init(bars + 52 + 2 * i + q, kCW / (2 * kSub)); }  // sd_full, cdone
@@ -354,7 +354,9 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         // (the second commit: the item's last read of this warp's K or V tile of row g)
         const uint32_t bar2 = (h == 1 && sub == kSub - 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
         const uint32_t tD = tmem + (h ? col_in1 : col_in0) + sub * QB, qa = qb + (h * HT + sub * QB) * (RB >> 4);
-        if constexpr (DP == 32) {  // two K slices of 16
+        if constexpr (DP == 16) {  // one K slice of 16
+          mma_ss_x1_commit(tD, ka, qa, kHiOp, kIdescSD, (sd_full + (2 * h + sub)).a, bar2);
+        } else if constexpr (DP == 32) {  // two
           mma_ss_x2_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + (2 * h + sub)).a, bar2);
         } else {                   // four
           mma_ss_x4_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + (2 * h + sub)).a, bar2);
@@ -536,18 +538,19 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     // whose arrival lets the next item's first MMAs overwrite the slot.
     auto drain_dkdv = [&](int b, int h, int s, int j0, int g) {
       const int j = j0 + jrow;
+      constexpr int W = DP == 16 ? 8 : 16;  // columns at a time
 #pragma unroll
-      for (int part = 0; part < DP / 32; ++part) {
-        const int c0 = cb2 * (DP / 2) + part * 16;
-        uint32_t kr[16], vr[16];
-        tmem_ld16(t_lane + colDK + g * DP + c0, kr);
-        tmem_ld16(t_lane + colDV + g * DP + c0, vr);
+      for (int part = 0; part < DP / 2 / W; ++part) {
+        const int c0 = cb2 * (DP / 2) + part * W;
+        uint32_t kr[W], vr[W];
+        tmem_ld<W>(t_lane + colDK + g * DP + c0, kr);
+        tmem_ld<W>(t_lane + colDV + g * DP + c0, vr);
         tmem_wait_ld();
         if (j < a.R && s < a.S) {
           T* kd = reinterpret_cast<T*>(a.dk) + off4(a.sdk, b, h, s, j) + c0;
           T* vd = reinterpret_cast<T*>(a.dv) + off4(a.sdv, b, h, s, j) + c0;
 #pragma unroll
-          for (int d8 = 0; d8 < 2; ++d8) {
+          for (int d8 = 0; d8 < W / 8; ++d8) {
             if (c0 + d8 * 8 < a.D) {
               uint4 pk, pv;
               pk.x = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 0]) * scale, __uint_as_float(kr[d8 * 8 + 1]) * scale);
@@ -569,7 +572,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     // query rows go through its staging area ([32 rows][DP/4 floats]) into the fp32 accumulator in global
     // memory, as one small bulk tensor reduction that the warp issues itself.  It happens after the
     // warp's arrival, underneath the tensor core's turnaround for its half.
-    constexpr int QC = DP / 4;       // dQ columns per warp (8 or 16)
+    constexpr int QC = DP / 4;       // dQ columns per warp (4, 8 or 16)
     const int colblk = 2 * H + cb2;  // which of the four column blocks this warp drains
     auto send_dq = [&](int m, const StepT& d) {
       mbar_wait(dq_full + (m & 1), (m >> 1) & 1, abort_s, a.status, DEV_TIMEOUT_MMA);
@@ -824,8 +827,18 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }
 
-}  // namespace
+// Head dimensions up to 16: items of seven rows (padded to 16) flush d(pair_bias) and reload the bias tile
+// every seventh step instead of every third, but there are fewer of them and the last group of rows is
+// padded further.  They are taken where the CTA with the most steps gets no more than a tenth more.
+bool seven_rows_pay(const Args& a) {
+  const auto steps = [&](int G) {
+    const long long items = (long long)a.B * a.H * ((a.R + BT - 1) / BT) * ((a.S + G - 1) / G);
+    return (items + 147) / 148 * G;
+  };
+  return 10 * steps(7) <= 11 * steps(3);
+}
 
+}  // namespace
 
 bool sm100_bwd_supported(int dtype, const Args& a) {
   if (!sm100_fwd_supported(dtype, a)) return false;
@@ -841,6 +854,10 @@ size_t sm100_bwd_workspace_bytes(int, const Args& a) {
 
 int launch_sm100_bwd(int dtype, const Args& a, void* workspace, size_t workspace_bytes, cudaStream_t st,
                      int* launches) {
+  if (a.D <= 16 && seven_rows_pay(a)) {
+    if (dtype == EVOATTN_BF16) return launch_t<__nv_bfloat16, 16>(a, workspace, workspace_bytes, st, launches);
+    return launch_t<__half, 16>(a, workspace, workspace_bytes, st, launches);
+  }
   if (a.D <= 32) {
     if (dtype == EVOATTN_BF16) return launch_t<__nv_bfloat16, 32>(a, workspace, workspace_bytes, st, launches);
     return launch_t<__half, 32>(a, workspace, workspace_bytes, st, launches);
