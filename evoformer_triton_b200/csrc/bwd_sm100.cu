@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const Args a, float* __restri
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
           const float G = to_float<T>(gp[2 * u + w]), go = G * to_float<T>(op[2 * u + w]);
-          const float sg = sigmoidf_fast(to_float<T>(tp[2 * u + w]));
+          const float sg = sigmoid16(to_float<T>(tp[2 * u + w]));
           acc += go;
           x[w] = G * sg;
           y[w] = go * (1.f - sg);

@@ -367,6 +367,10 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const float* mrow_base = sMask + (w * 2 + mst) * r_pad;
       const uint32_t* dirty_row = sDirty + (w * 2 + mst) * 32;
 
+      // The gate's row is wanted in the epilogue, where every cycle of its latency would be waited for.
+      const T* grow = a.gate ? reinterpret_cast<const T*>(a.gate) + off4(a.sgate, it.b, it.h, s, i < a.R ? i : 0) : nullptr;
+      if (grow != nullptr) prefetch_l2(grow);
+
       float m_run = -FLT_MAX, l_run = 0.f;
 
       for (int t = 0; t < T_TILES; ++t, ++g) {
@@ -541,6 +545,11 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full(w));
       }
+      uint4 gw[DP / 8];
+      if (grow != nullptr) {
+#pragma unroll
+        for (int d8 = 0; d8 < DP / 8; ++d8) gw[d8] = d8 * 8 < a.D ? *reinterpret_cast<const uint4*>(grow + d8 * 8) : make_uint4(0, 0, 0, 0);
+      }
       // O of the item, complete with its last P V
       mbar_wait(o_full(w), (g - 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
       tc_fence_after();
@@ -558,7 +567,6 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       if (active && i < a.R) {
         const float inv = 1.f / __uint_as_float(lr[0]);
         T* orow = reinterpret_cast<T*>(a.o) + off4(a.so, it.b, it.h, s, i);
-        const T* grow = a.gate ? reinterpret_cast<const T*>(a.gate) + off4(a.sgate, it.b, it.h, s, i) : nullptr;
 #pragma unroll
         for (int d8 = 0; d8 < DP / 8; ++d8) {
           if (d8 * 8 < a.D) {
@@ -566,10 +574,14 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 #pragma unroll
             for (int u = 0; u < 8; ++u) f[u] = acc[d8 * 8 + u] * inv;
             if (grow != nullptr) {  // gated output: O * sigmoid(gate), in the epilogue
-              const uint4 gw = *reinterpret_cast<const uint4*>(grow + d8 * 8);
-              const T* gv = reinterpret_cast<const T*>(&gw);
+              const uint32_t w4[4] = {gw[d8].x, gw[d8].y, gw[d8].z, gw[d8].w};
 #pragma unroll
-              for (int u = 0; u < 8; ++u) f[u] *= sigmoidf_fast(to_float<T>(gv[u]));
+              for (int u = 0; u < 4; ++u) {
+                float g0, g1;
+                unpack2<T>(w4[u], g0, g1);
+                f[2 * u] *= sigmoid16(g0);
+                f[2 * u + 1] *= sigmoid16(g1);
+              }
             }
             uint4 v4;
             v4.x = Pack2<T>::pack(f[0], f[1]);

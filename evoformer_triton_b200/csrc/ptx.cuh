@@ -328,6 +328,8 @@ __device__ __forceinline__ uint32_t ldg_u8_if(const void* p, bool pred) {
   return v;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // ---------------------------------------------------------------- shared-memory access by 32-bit address
 // A load through a generic pointer that happens to point into shared memory is a generic load: it
 // pays the address-space check and 64-bit address arithmetic, and the hardware tracks it like a
@@ -358,6 +360,13 @@ __device__ __forceinline__ void sts_v4(uint32_t saddr, uint32_t x, uint32_t y, u
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 1 / (1 + e^-x) to a few units in the last place of fp32, for results that are rounded to 16 bits: an
+// exponential and a reciprocal, without the division's correction steps.
+__device__ __forceinline__ float sigmoid16(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(1.f + ex2(x * -1.4426950408889634f)));
   return y;
 }
 // Packed fp32x2 arithmetic (sm_100): one instruction works on two floats held in a 64-bit
