@@ -63,7 +63,7 @@ struct Cfg {
   static constexpr int offV = offK + KVW * NKV * kKV;
   static constexpr int offB = offV + KVW * NKV * kKV;
   static constexpr int offMask = offB + BST * BTL * kBias;
-  static constexpr int kNumBars = 2 * (2 * QST + 4 * NKV + 2 + 1 + 1 + 4) + 2 * BST;
+  static constexpr int kNumBars = 2 * (2 * QST + 4 * NKV + 2 + 2 + 2 + 4) + 2 * BST;
   static size_t bytes(int r_pad) {
     return (size_t)offMask + (size_t)4 * r_pad * 4 + 4 * 32 * 4 + kOnes + kNumBars * 8 + 64 + 1024;
   }
@@ -116,7 +116,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   uint32_t* sOnes = sDirty + 4 * 32;  // 16 x 16 ones of the storage type
   uint64_t* bars = reinterpret_cast<uint64_t*>(sOnes + C::kOnes / 4);
   // barrier layout: per warpgroup w a block of PER, then the shared bias barriers
-  constexpr int PER = 2 * QST + 4 * NKV + 2 + 1 + 1 + 4;
+  constexpr int PER = 2 * QST + 4 * NKV + 2 + 2 + 2 + 4;
   auto q_full = [&](int w, int st) { return bars + w * PER + st; };
   auto q_empty = [&](int w, int st) { return bars + w * PER + QST + st; };
   auto k_full = [&](int w, int st) { return bars + w * PER + 2 * QST + st; };
@@ -124,10 +124,13 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   auto v_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 2 * NKV + st; };
   auto v_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 3 * NKV + st; };
   auto s_full = [&](int w, int i) { return bars + w * PER + 2 * QST + 4 * NKV + i; };
-  auto p_full = [&](int w) { return bars + w * PER + 2 * QST + 4 * NKV + 2; };
-  auto o_full = [&](int w) { return bars + w * PER + 2 * QST + 4 * NKV + 3; };
-  auto m_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 4 + st; };
-  auto m_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 6 + st; };
+  // Two of each for tiles in turn: the softmax warps may finish a tile while the issuer still waits for the
+  // V of the one before, and a single barrier that is two phases on looks the same as one that has not
+  // moved (a parity wait cannot tell).
+  auto p_full = [&](int w, uint32_t i) { return bars + w * PER + 2 * QST + 4 * NKV + 2 + i; };
+  auto o_full = [&](int w, uint32_t i) { return bars + w * PER + 2 * QST + 4 * NKV + 4 + i; };
+  auto m_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 6 + st; };
+  auto m_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 8 + st; };
   auto b_full = [&](int st) { return bars + 2 * PER + st; };
   auto b_empty = [&](int st) { return bars + 2 * PER + BST + st; };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kNumBars);
@@ -154,8 +157,8 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         mbar_init(v_full(w, st), 1); mbar_init(v_empty(w, st), QP ? 2 : 1);
       }
       mbar_init(s_full(w, 0), 1); mbar_init(s_full(w, 1), 1);
-      mbar_init(p_full(w), 4);  // one arrival per softmax warp
-      mbar_init(o_full(w), 1);
+      mbar_init(p_full(w, 0), 4); mbar_init(p_full(w, 1), 4);  // one arrival per softmax warp
+      mbar_init(o_full(w, 0), 1); mbar_init(o_full(w, 1), 1);
       for (int st = 0; st < 2; ++st) { mbar_init(m_full(w, st), 1); mbar_init(m_empty(w, st), 4); }
     }
     for (int st = 0; st < BST; ++st) { mbar_init(b_full(st), 1); mbar_init(b_empty(st), 8); }
@@ -255,7 +258,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       auto issue_pv = [&](uint32_t g, bool first) {  // O += P V; the first of an item overwrites
         const int st = g % NKV;
         mbar_wait(v_full(kw, st), (g / NKV) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
-        mbar_wait(p_full(w), g & 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
+        mbar_wait(p_full(w, g & 1), (g >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
         tc_fence_after();
         const uint32_t va = v_lo0 + st * (C::kKV >> 4);
 #pragma unroll
@@ -266,7 +269,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         for (int kk = 0; kk < BN / 16; ++kk)
           mma_ts(tS + C::colL, tS + (g & 1) * BN + kk * 8, ones, kIdescL, (kk > 0 || !first) ? 1u : 0u);
         mma_commit(v_empty(kw, st));
-        mma_commit(o_full(w));
+        mma_commit(o_full(w, g & 1));
       };
       for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
         mbar_wait(q_full(w, qn % QST), (qn / QST) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
@@ -465,7 +468,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
             const float alpha = ex2((m_run - m_up) * kLog2e);
             m_run = m_up;
             l_run *= alpha;
-            mbar_wait(o_full(w), (g - 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
+            mbar_wait(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
             tc_fence_after();
 #pragma unroll
             for (int d0 = 0; d0 < DP + 16; d0 += 16) {  // O and the row sum behind it
@@ -543,7 +546,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full(w));
+        if (lane == 0) mbar_arrive(p_full(w, g & 1));
       }
       uint4 gw[DP / 8];
       if (grow != nullptr) {
@@ -551,7 +554,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         for (int d8 = 0; d8 < DP / 8; ++d8) gw[d8] = d8 * 8 < a.D ? *reinterpret_cast<const uint4*>(grow + d8 * 8) : make_uint4(0, 0, 0, 0);
       }
       // O of the item, complete with its last P V
-      mbar_wait(o_full(w), (g - 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
+      mbar_wait(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
       tc_fence_after();
       float acc[DP];
 #pragma unroll
