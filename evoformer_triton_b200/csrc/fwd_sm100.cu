@@ -46,6 +46,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kGrow = 8.f / kLog2e;  // how far a tile's maximum may exceed the running one
 constexpr int MASK_MIN = 0;  // boolean keep-mask (or none): score = min(score, m), m = +-FLT_MAX
 constexpr int MASK_ADD = 1;  // additive mask
+constexpr int BIAS_NONE = 0, BIAS_F32 = 1, BIAS_16 = 2;
 
 template <int DP, bool QP>
 struct Cfg {
@@ -95,7 +96,7 @@ __device__ __forceinline__ Item decode_item(int idx, int n_inner, int n_outer, i
   return it;
 }
 
-template <class T, int DP, int MASKMODE, bool BIAS16, bool QP>
+template <class T, int DP, int MASKMODE, int BIAS, bool QP>
 __global__ void __launch_bounds__(kThreads, 1)
 evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -142,7 +143,7 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   // items: (b, h, outer, inner) with inner fastest
   const int n_inner = QP ? a.S : (a.S + 1) / 2;
   const int n_outer = QP ? (NQT + 1) / 2 : NQT;
-  const bool has_bias = a.bias != nullptr;
+  constexpr bool has_bias = BIAS != BIAS_NONE, BIAS16 = BIAS == BIAS_16;
 
   // A launch that follows a failed one returns at once (one reader, so the CTA agrees).
   if (tid == 0) *abort_flag = (a.status && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
@@ -647,8 +648,9 @@ int launch_t(const Args& a, cudaStream_t st, int* launches) {
                              : (long long)a.B * a.H * NQT * ((a.S + 1) / 2);
   const int grid = (int)(items < g_num_sms ? items : g_num_sms);
   const bool add = a.mask_kind == EVOATTN_MASK_ADD_F32 || a.mask_kind == EVOATTN_MASK_ADD_SAME;
-  auto kern = a.bias16 ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, true, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, true, QP>)
-                       : (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, false, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, false, QP>);
+  auto kern = !a.bias ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_NONE, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_NONE, QP>)
+              : a.bias16 ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_16, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_16, QP>)
+                         : (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_F32, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_F32, QP>);
   if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)smem, nullptr)) return EVOATTN_ERR_CUDA;
   kern<<<grid, kThreads, smem, st>>>(a, (int)items, tq, tk, tv, tb);
   *launches += 1;
