@@ -1,5 +1,6 @@
-// Small device passes around the attention kernels: the conversion of a pair bias (and its gradient) between the layout a linear layer emits,
-// [B, R, R, H], and the [B, H, R, R] the kernels (and dsevoformer-triton/evoformer.py:638,652) use.
+// Small device passes around the attention kernels: the conversion of a pair bias (and its gradient)
+// between the layout a linear layer emits, [B, R, R, H], and the [B, H, R, R] the kernels (and
+// dsevoformer-triton/evoformer.py:638,652) use, and between dense and padded rows.
 // None of this exists in the reference: it takes the bias heads-first.
 #include <string.h>
 
@@ -45,17 +46,32 @@ __global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict
 }
 
 // A pair bias with arbitrary (b, h, i) strides -> rows of R values with a row stride of `ld`, the form
-// the tensor maps can read (whole 16-byte pieces).  One read and one write of the bias, no more: at
-// [4, 32, 300, 300] bf16 it moves 46 MB.  The last ld - R columns are never read and stay unwritten.
-template <class E>
-__global__ void __launch_bounds__(256) pad_rows_kernel(const E* __restrict__ src, Str3 st, E* __restrict__ dst, int H,
-                                                       int R, int ld) {
+// the tensor maps can read (whole 16-byte pieces).  All sizes in words of type W: the widest that divides
+// rows, strides and addresses.  Bound by memory; a warp per row, four loads in flight per lane.  The last
+// ld - R columns are never read and stay unwritten.
+template <class W>
+__global__ void __launch_bounds__(256) pad_rows_kernel(const W* __restrict__ src, Str3 st, W* __restrict__ dst, int H, int rows,
+                                                       int cols, int ld) {
   const int h = blockIdx.y % H, b = blockIdx.y / H;
-  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < R; i += gridDim.x * 8) {  // a warp per row
-    const E* in = src + (long long)b * st.a + (long long)h * st.b + (long long)i * st.c;
-    E* out = dst + ((long long)blockIdx.y * R + i) * ld;
-    for (int j = threadIdx.x & 31; j < R; j += 32) out[j] = in[j];
+  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= rows) return;
+  const W* in = src + (long long)b * st.a + (long long)h * st.b + (long long)i * st.c;
+  W* out = dst + ((long long)blockIdx.y * rows + i) * ld;
+  for (int j = threadIdx.x & 31; j < cols; j += 128) {
+    W v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (j + 32 * u < cols) v[u] = in[j + 32 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (j + 32 * u < cols) out[j + 32 * u] = v[u];
   }
+}
+template <class W>
+void pad_rows_t(const void* src, const int64_t* stride, void* dst, int es, int B, int H, int R, int ld, cudaStream_t st) {
+  const int n = (int)sizeof(W) / es;  // elements per word
+  const Str3 s{stride[0] / n, stride[1] / n, stride[2] / n};
+  pad_rows_kernel<W><<<dim3((R + 7) / 8, B * H), 256, 0, st>>>(static_cast<const W*>(src), s, static_cast<W*>(dst), H, R, R / n, ld / n);
 }
 
 template <class E>
@@ -103,14 +119,16 @@ int evoattn_bias_pad_rows(const void* src, const int64_t* stride, void* dst, int
   if (!src || !dst || !stride) return EVOATTN_ERR_NULL;
   if (B <= 0 || H <= 0 || R <= 0 || ld < R || (long long)B * H > 65535) return EVOATTN_ERR_SHAPE;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
-  const evo::Str3 s{stride[0], stride[1], stride[2]};
-  dim3 grid((R + 7) / 8, B * H);
-  if (dtype == EVOATTN_FP32)
-    evo::pad_rows_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(src), s, static_cast<float*>(dst), H, R, ld);
-  else if (dtype == EVOATTN_BF16 || dtype == EVOATTN_FP16)
-    evo::pad_rows_kernel<uint16_t><<<grid, 256, 0, st>>>(static_cast<const uint16_t*>(src), s, static_cast<uint16_t*>(dst), H, R, ld);
-  else
-    return EVOATTN_ERR_DTYPE;
+  if (dtype != EVOATTN_FP32 && dtype != EVOATTN_BF16 && dtype != EVOATTN_FP16) return EVOATTN_ERR_DTYPE;
+  const int es = dtype == EVOATTN_FP32 ? 4 : 2;
+  const auto fits = [&](int bytes) {
+    const uint64_t all = (uint64_t)(uintptr_t)src | (uintptr_t)dst | (uint64_t)(stride[0] * es) | (uint64_t)(stride[1] * es) |
+                         (uint64_t)(stride[2] * es) | (uint64_t)(R * es) | (uint64_t)(ld * es);
+    return all % bytes == 0;
+  };
+  if (fits(8)) evo::pad_rows_t<uint2>(src, stride, dst, es, B, H, R, ld, st);
+  else if (fits(4)) evo::pad_rows_t<uint32_t>(src, stride, dst, es, B, H, R, ld, st);
+  else evo::pad_rows_t<uint16_t>(src, stride, dst, es, B, H, R, ld, st);
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }
 
