@@ -108,6 +108,8 @@ __device__ __forceinline__ void mma_commit_if(uint32_t leader, Bar b) { mma_comm
 template <class T, int LG, bool GATE>
 __global__ void __launch_bounds__(256) prep_kernel(const Args a, float* __restrict__ nl, float* __restrict__ dq_acc,
                                                    const uint32_t dbias_f4) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const uint32_t gid = blockIdx.x * 256 + threadIdx.x;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   for (uint32_t e = gid; e < dbias_f4; e += gridDim.x * 256) reinterpret_cast<float4*>(a.dbias)[e] = zero;
@@ -169,16 +171,18 @@ void launch_prep(const Args& a, float* nl, float* dq_acc, cudaStream_t st) {
   const uint32_t f4 = a.dbias ? (uint32_t)((size_t)a.B * a.H * a.R * a.dbias_ld / 4) : 0u;
   const unsigned grid = (unsigned)((threads + 255) / 256);
   switch (lg) {
-    case 3: prep_kernel<T, 3, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
-    case 2: prep_kernel<T, 2, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
-    case 1: prep_kernel<T, 1, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
-    default: prep_kernel<T, 0, GATE><<<grid, 256, 0, st>>>(a, nl, dq_acc, f4); break;
+    case 3: launch_dependent(prep_kernel<T, 3, GATE>, grid, 256, 0, st, a, nl, dq_acc, f4); break;
+    case 2: launch_dependent(prep_kernel<T, 2, GATE>, grid, 256, 0, st, a, nl, dq_acc, f4); break;
+    case 1: launch_dependent(prep_kernel<T, 1, GATE>, grid, 256, 0, st, a, nl, dq_acc, f4); break;
+    default: launch_dependent(prep_kernel<T, 0, GATE>, grid, 256, 0, st, a, nl, dq_acc, f4); break;
   }
 }
 
 // dq = scale * dq_acc, cast to the storage type (dq_acc: contiguous fp32 [B,H,S,R,D]).
 template <class T>
 __global__ void __launch_bounds__(256) dq_store_kernel(Args a, const float* __restrict__ acc) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int d8n = a.D / 8;
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
   const long long total = (long long)a.B * a.H * a.S * a.R * d8n;
@@ -282,6 +286,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     return d;
   };
 
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (tid == 0) *abort_flag = (a.status && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
   __syncthreads();
   if (*abort_flag) return;
@@ -803,7 +809,7 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   int num_regs = 0;
   if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)L::bytes, &num_regs)) return EVOATTN_ERR_CUDA;
   if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
-  kern<<<(unsigned)ctas, kThreadsT, L::bytes, st>>>(a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
+  launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, L::bytes, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
   if (a.dbias_out) {
     const int rc = launch_dbias_out(a, st, launches);
     if (rc) return rc;
@@ -821,7 +827,9 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
     *launches += 1;
   }
   const long long n8 = (long long)rows * (a.D / 8);
-  dq_store_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(a, dq_acc);
+  const dim3 store_grid((unsigned)((n8 + 255) / 256));
+  if (a.exchange || a.dbias_out) dq_store_kernel<T><<<store_grid, 256, 0, st>>>(a, dq_acc);  // (another launch lies between)
+  else launch_dependent(dq_store_kernel<T>, store_grid, 256, 0, st, a, static_cast<const float*>(dq_acc));
   if (a.exchange && cudaStreamWaitEvent(st, join, 0) != cudaSuccess) return EVOATTN_ERR_CUDA;
   *launches += 3;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;

@@ -146,6 +146,8 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   constexpr bool has_bias = BIAS != BIAS_NONE, BIAS16 = BIAS == BIAS_16;
 
   // A launch that follows a failed one returns at once (one reader, so the CTA agrees).
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (tid == 0) *abort_flag = (a.status && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
   __syncthreads();
   if (*abort_flag) return;
@@ -629,7 +631,7 @@ int launch_t(const Args& a, cudaStream_t st, int* launches) {
               : a.bias16 ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_16, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_16, QP>)
                          : (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_F32, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_F32, QP>);
   if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)smem, nullptr)) return EVOATTN_ERR_CUDA;
-  kern<<<grid, kThreads, smem, st>>>(a, (int)items, tq, tk, tv, tb);
+  launch_dependent(kern, dim3((unsigned)grid), kThreads, smem, st, a, (int)items, tq, tk, tv, tb);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }

@@ -39,6 +39,25 @@ inline bool kernel_ready(const void* kern, int smem_bytes, int* num_regs) {
   return true;
 }
 
+// Launches a kernel that may be scheduled while the one before it on the stream is still draining
+// (programmatic dependent launch).  The kernel calls ptx::grid_dependency_wait() before it touches
+// global memory, which waits for that one to have completed, and ptx::grid_launch_dependents() to let the
+// next one in.  Saves the gap between the kernels of a call, about a microsecond each.
+template <class K, class... A>
+inline cudaError_t launch_dependent(K kern, dim3 grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // CUDA-core kernels (generic_kernels.cu).  Backward needs generic_bwd_workspace_bytes() of scratch at a.delta
 // (asked for with a.dbias set if and only if d(pair_bias) is wanted).
 size_t generic_bwd_workspace_bytes(const Args& a);
