@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "launch.h"
+#include "ptx.cuh"
 
 namespace evo {
 namespace {
@@ -15,6 +16,8 @@ namespace {
 template <class E>
 __global__ void __launch_bounds__(256) heads_first_kernel(const E* __restrict__ src, E* __restrict__ dst, int H, int R,
                                                           int ld) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   extern __shared__ unsigned char sm_raw[];
   E* sm = reinterpret_cast<E*>(sm_raw);
   const int j0 = blockIdx.x * 128, i = blockIdx.y, b = blockIdx.z;
@@ -32,6 +35,8 @@ __global__ void __launch_bounds__(256) heads_first_kernel(const E* __restrict__ 
 template <class E>
 __global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict__ src, int ld, E* __restrict__ dst, int H,
                                                          int R) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   extern __shared__ unsigned char sm_raw[];
   float* sm = reinterpret_cast<float*>(sm_raw);
   const int j0 = blockIdx.x * 128, i = blockIdx.y, b = blockIdx.z;
@@ -52,6 +57,8 @@ __global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict
 template <class W>
 __global__ void __launch_bounds__(256) pad_rows_kernel(const W* __restrict__ src, Str3 st, W* __restrict__ dst, int H, int rows,
                                                        int cols, int ld) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const int h = blockIdx.y % H, b = blockIdx.y / H;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i >= rows) return;
@@ -71,12 +78,14 @@ template <class W>
 void pad_rows_t(const void* src, const int64_t* stride, void* dst, int es, int B, int H, int R, int ld, cudaStream_t st) {
   const int n = (int)sizeof(W) / es;  // elements per word
   const Str3 s{stride[0] / n, stride[1] / n, stride[2] / n};
-  pad_rows_kernel<W><<<dim3((R + 7) / 8, B * H), 256, 0, st>>>(static_cast<const W*>(src), s, static_cast<W*>(dst), H, R, R / n, ld / n);
+  launch_dependent(pad_rows_kernel<W>, dim3((R + 7) / 8, B * H), 256, 0, st, static_cast<const W*>(src), s, static_cast<W*>(dst), H, R, R / n, ld / n);
 }
 
 template <class E>
 __global__ void __launch_bounds__(256) dbias_dense_kernel(const float* __restrict__ src, int ld, E* __restrict__ dst,
                                                           long long rows, int cols) {
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
   const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // a warp per row
   if (row >= rows) return;
   for (int j = threadIdx.x & 31; j < cols; j += 32) dst[row * cols + j] = from_float<E>(src[row * ld + j]);
@@ -87,10 +96,10 @@ void dbias_out_t(const Args& a, cudaStream_t st) {
   E* dst = reinterpret_cast<E*>(a.dbias_out);
   if (a.dbias_out_last) {
     dim3 grid((a.R + 127) / 128, a.R, a.B);
-    heads_last_kernel<E><<<grid, 256, (size_t)128 * a.H * 4, st>>>(a.dbias, a.dbias_ld, dst, a.H, a.R);
+    launch_dependent(heads_last_kernel<E>, grid, 256, (size_t)128 * a.H * 4, st, static_cast<const float*>(a.dbias), a.dbias_ld, dst, a.H, a.R);
   } else {
     const long long rows = (long long)a.B * a.H * a.R;
-    dbias_dense_kernel<E><<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(a.dbias, a.dbias_ld, dst, rows, a.R);
+    launch_dependent(dbias_dense_kernel<E>, dim3((unsigned)((rows + 7) / 8)), 256, 0, st, static_cast<const float*>(a.dbias), a.dbias_ld, dst, rows, a.R);
   }
 }
 
@@ -139,9 +148,9 @@ int evoattn_bias_to_heads_first_ld(const void* src, void* dst, int dtype, int B,
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   dim3 grid((R + 127) / 128, R, B);
   if (dtype == EVOATTN_FP32)
-    evo::heads_first_kernel<float><<<grid, 256, (size_t)128 * H * 4, st>>>(static_cast<const float*>(src), static_cast<float*>(dst), H, R, ld);
+    evo::launch_dependent(evo::heads_first_kernel<float>, grid, 256, (size_t)128 * H * 4, st, static_cast<const float*>(src), static_cast<float*>(dst), H, R, ld);
   else if (dtype == EVOATTN_BF16 || dtype == EVOATTN_FP16)
-    evo::heads_first_kernel<uint16_t><<<grid, 256, (size_t)128 * H * 2, st>>>(static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), H, R, ld);
+    evo::launch_dependent(evo::heads_first_kernel<uint16_t>, grid, 256, (size_t)128 * H * 2, st, static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), H, R, ld);
   else
     return EVOATTN_ERR_DTYPE;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
@@ -153,9 +162,9 @@ int evoattn_dbias_to_heads_last(const float* src, void* dst, int dtype, int B, i
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   dim3 grid((R + 127) / 128, R, B);
   const size_t smem = (size_t)128 * H * 4;
-  if (dtype == EVOATTN_FP32) evo::heads_last_kernel<float><<<grid, 256, smem, st>>>(src, R, static_cast<float*>(dst), H, R);
-  else if (dtype == EVOATTN_BF16) evo::heads_last_kernel<__nv_bfloat16><<<grid, 256, smem, st>>>(src, R, static_cast<__nv_bfloat16*>(dst), H, R);
-  else if (dtype == EVOATTN_FP16) evo::heads_last_kernel<__half><<<grid, 256, smem, st>>>(src, R, static_cast<__half*>(dst), H, R);
+  if (dtype == EVOATTN_FP32) evo::launch_dependent(evo::heads_last_kernel<float>, grid, 256, smem, st, src, R, static_cast<float*>(dst), H, R);
+  else if (dtype == EVOATTN_BF16) evo::launch_dependent(evo::heads_last_kernel<__nv_bfloat16>, grid, 256, smem, st, src, R, static_cast<__nv_bfloat16*>(dst), H, R);
+  else if (dtype == EVOATTN_FP16) evo::launch_dependent(evo::heads_last_kernel<__half>, grid, 256, smem, st, src, R, static_cast<__half*>(dst), H, R);
   else return EVOATTN_ERR_DTYPE;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }
