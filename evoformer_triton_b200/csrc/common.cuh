@@ -110,22 +110,6 @@ __device__ __forceinline__ long long off4(const Str4& s, int b, int h, int ss, i
   return (long long)b * s.b + (long long)h * s.h + (long long)ss * s.s + (long long)r * s.r;
 }
 
-// Residue mask applied to one score.  BOOL replaces (evoformer.py:69), the others add.
-template <class T>
-__device__ __forceinline__ float apply_mask(float x, const void* mask, int kind, long long idx, bool& replaced) {
-  replaced = false;
-  if (kind == EVOATTN_MASK_BOOL) {
-    if (reinterpret_cast<const unsigned char*>(mask)[idx] == 0) {
-      replaced = true;
-      return -FLT_MAX;
-    }
-    return x;
-  }
-  if (kind == EVOATTN_MASK_ADD_F32) return x + reinterpret_cast<const float*>(mask)[idx];
-  if (kind == EVOATTN_MASK_ADD_SAME) return x + to_float<T>(reinterpret_cast<const T*>(mask)[idx]);
-  return x;
-}
-
 // Pair-bias element (b, h, i, j) in either storage type.
 template <class T>
 __device__ __forceinline__ float load_bias(const Args& a, int b, int h, int i, int j) {
@@ -140,11 +124,6 @@ __device__ __forceinline__ float load_bias<float>(const Args& a, int b, int h, i
 
 __device__ __forceinline__ float sigmoidf_fast(float x) { return 1.f / (1.f + __expf(-x)); }
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
