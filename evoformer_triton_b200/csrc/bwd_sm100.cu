@@ -108,12 +108,13 @@ __device__ __forceinline__ void mma_commit_if(uint32_t leader, Bar b) { mma_comm
 // thread per row and a memset), gated [1,384,384,4,32] 54 us (273 + 26 us in two passes before).
 template <class T, int LG, bool GATE>
 __global__ void __launch_bounds__(256) prep_kernel(const Args a, float* __restrict__ nl, float* __restrict__ dq_acc,
-                                                   const uint32_t dbias_f4) {
+                                                   const size_t dbias_f4) {
   grid_dependency_wait();
   grid_launch_dependents();
   const uint32_t gid = blockIdx.x * 256 + threadIdx.x;
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (uint32_t e = gid; e < dbias_f4; e += gridDim.x * 256) reinterpret_cast<float4*>(a.dbias)[e] = zero;
+  // (64-bit count and position: 2^32 of these pieces are 64 GiB, which fits the device)
+  for (size_t e = gid; e < dbias_f4; e += (size_t)gridDim.x * 256) reinterpret_cast<float4*>(a.dbias)[e] = zero;
   const uint32_t row = gid >> LG, c = gid & ((1u << LG) - 1u);
   const uint32_t slab = row / (uint32_t)a.R, i = row - slab * (uint32_t)a.R;
   const uint32_t bh = slab / (uint32_t)a.S, s = slab - bh * (uint32_t)a.S;
@@ -169,7 +170,7 @@ void launch_prep(const Args& a, float* nl, float* dq_acc, cudaStream_t st) {
   const int chunks = a.D / 8;
   const int lg = chunks > 4 ? 3 : chunks > 2 ? 2 : chunks > 1 ? 1 : 0;
   const size_t threads = ((size_t)a.B * a.H * a.S * a.R) << lg;
-  const uint32_t f4 = a.dbias ? (uint32_t)((size_t)a.B * a.H * a.R * a.dbias_ld / 4) : 0u;
+  const size_t f4 = a.dbias ? (size_t)a.B * a.H * a.R * a.dbias_ld / 4 : 0;
   const unsigned grid = (unsigned)((threads + 255) / 256);
   switch (lg) {
     case 3: launch_dependent(prep_kernel<T, 3, GATE>, grid, 256, 0, st, a, nl, dq_acc, f4); break;

@@ -78,3 +78,31 @@ def test_pair_bias_gradient_in_its_type_and_layout(layout, bias_dtype, R):
     assert b.grad.dtype == bias_dtype and b.grad.shape == bias.shape
     got = b.grad if layout == "b1hrr" else b.grad.permute(0, 3, 1, 2).reshape(B, 1, H, R, R)
     assert oc.rel_err(got, want) < 1e-2
+
+
+def test_pair_bias_gradient_of_64_gib():
+    """d(pair_bias) of 2^34 values: its clearing in the backward's first pass counts beyond 32 bits.  The buffer
+    holds a marker before the call; a (b, h) slab that was not cleared would keep it."""
+    from evoformer_triton_b200 import attention, check_device_status
+    B, H, S, R, D = 512, 8, 1, 2048, 8
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 110 << 30:
+        pytest.skip("needs 64 GiB for the gradient and 32 GiB for the bias")
+    g = torch.Generator(device=DEV).manual_seed(8)
+    q, k, v, d_o = (torch.randn((B, H, S, R, D), generator=g, device=DEV).bfloat16() for _ in range(4))
+    q *= 0.25  # (no probability comes near 1, so no score gradient comes near the marker)
+    bias = torch.zeros((B, H, R, R), dtype=torch.bfloat16, device=DEV)
+    dbias = torch.full((B, H, R, R), 7.0, device=DEV)
+    o, lse = attention.attention_forward(q, k, v, None, bias, D ** -0.5)
+    attention.attention_backward(q, k, v, o, lse, None, bias, D ** -0.5, d_o, dbias_out=dbias)
+    torch.cuda.synchronize()
+    check_device_status()
+    assert attention.last_path["bwd"] == _lib().PATH_TCGEN05
+    for b, h in ((0, 0), (171, 3), (B - 1, H - 1)):
+        one = [t[b:b + 1, h:h + 1].contiguous() for t in (q, k, v, o, lse, bias, d_o)]
+        want = attention.attention_backward(*one[:5], None, one[5], D ** -0.5, one[6])[3]
+        assert torch.equal(dbias[b, h], want[0, 0]), (b, h)  # (one row: one addition to each element)
+    low, high = torch.aminmax(dbias)
+    assert -3.5 < low.item() and high.item() < 3.5  # no marker left anywhere
+    del bias, dbias
+    torch.cuda.empty_cache()
