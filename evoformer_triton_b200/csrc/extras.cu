@@ -55,15 +55,15 @@ __global__ void __launch_bounds__(256) heads_last_kernel(const float* __restrict
 // rows, strides and addresses.  Bound by memory; a warp per row, four loads in flight per lane.  The last
 // ld - R columns are never read and stay unwritten.
 template <class W>
-__global__ void __launch_bounds__(256) pad_rows_kernel(const W* __restrict__ src, Str3 st, W* __restrict__ dst, int H, int rows,
-                                                       int cols, int ld) {
+__global__ void __launch_bounds__(256) pad_rows_kernel(const W* __restrict__ src, Str3 st, W* __restrict__ dst, long long n_rows, int H,
+                                                       int rows, int cols, int ld) {
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
-  const int h = blockIdx.y % H, b = blockIdx.y / H;
-  const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (i >= rows) return;
-  const W* in = src + (long long)b * st.a + (long long)h * st.b + (long long)i * st.c;
-  W* out = dst + ((long long)blockIdx.y * rows + i) * ld;
+  const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // (b, h, i): any number of (b, h)
+  if (row >= n_rows) return;
+  const int bh = (int)(row / rows), i = (int)(row - (long long)bh * rows);
+  const W* in = src + (long long)(bh / H) * st.a + (long long)(bh % H) * st.b + (long long)i * st.c;
+  W* out = dst + row * ld;
   for (int j = threadIdx.x & 31; j < cols; j += 128) {
     W v[4];
 #pragma unroll
@@ -78,7 +78,8 @@ template <class W>
 void pad_rows_t(const void* src, const int64_t* stride, void* dst, int es, int B, int H, int R, int ld, cudaStream_t st) {
   const int n = (int)sizeof(W) / es;  // elements per word
   const Str3 s{stride[0] / n, stride[1] / n, stride[2] / n};
-  launch_dependent(pad_rows_kernel<W>, dim3((R + 7) / 8, B * H), 256, 0, st, static_cast<const W*>(src), s, static_cast<W*>(dst), H, R, R / n, ld / n);
+  const long long rows = (long long)B * H * R;
+  launch_dependent(pad_rows_kernel<W>, dim3((unsigned)((rows + 7) / 8)), 256, 0, st, static_cast<const W*>(src), s, static_cast<W*>(dst), rows, H, R, R / n, ld / n);
 }
 
 template <class E>
@@ -126,7 +127,8 @@ int evoattn_bias_to_heads_first(const void* src, void* dst, int dtype, int B, in
 int evoattn_bias_pad_rows(const void* src, const int64_t* stride, void* dst, int dtype, int B, int H, int R, int ld,
                           void* cuda_stream) {
   if (!src || !dst || !stride) return EVOATTN_ERR_NULL;
-  if (B <= 0 || H <= 0 || R <= 0 || ld < R || (long long)B * H > 65535) return EVOATTN_ERR_SHAPE;
+  if (B <= 0 || H <= 0 || R <= 0 || ld < R || (long long)B * H > 0x7fffffffLL) return EVOATTN_ERR_SHAPE;
+  if (((long long)B * H * R + 7) / 8 > 0x7fffffffLL) return EVOATTN_ERR_SHAPE;  // (blocks of eight rows)
   cudaStream_t st = reinterpret_cast<cudaStream_t>(cuda_stream);
   if (dtype != EVOATTN_FP32 && dtype != EVOATTN_BF16 && dtype != EVOATTN_FP16) return EVOATTN_ERR_DTYPE;
   const int es = dtype == EVOATTN_FP32 ? 4 : 2;

@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("cfg", [
     (2, 5, 127, 2, 32, torch.bfloat16, "bool"), (1, 7, 129, 3, 32, torch.float16, "add32"),
     (1, 4, 203, 2, 32, torch.bfloat16, "bool"), (1, 3, 257, 1, 64, torch.bfloat16, "addsame"),
-    (2, 1, 302, 4, 64, torch.bfloat16, "none"), (1, 9, 70, 4, 8, torch.float16, "bool")],
+    (2, 1, 302, 4, 64, torch.bfloat16, "none"), (1, 9, 70, 4, 8, torch.float16, "bool"),
+    (8192, 1, 5, 9, 8, torch.bfloat16, "none")],  # more (b, h) than a grid has rows
     ids=lambda c: "B%dS%dR%dH%dD%d-%s-%s" % (*c[:5], str(c[5]).split(".")[-1], c[6]))
 def test_any_number_of_residues(cfg, bias_dtype):
     B, S, R, H, D, dtype, mask = cfg
