@@ -198,6 +198,18 @@ Scratch plan_scratch(const evoattn_bwd_params* p, evo::Args* a, bool fast) {
   return s;
 }
 
+// The same for scratch that cannot grow.  The CUDA-core kernels speed up with partial sums of
+// d(pair_bias), one for each run of MSA rows; they take as many as there is room for, and need none.
+Scratch plan_scratch_within(size_t limit, const evoattn_bwd_params* p, evo::Args* a, bool fast) {
+  const Scratch all = plan_scratch(p, a, fast);
+  if (fast || all.total() <= limit || !(a->dbias || a->dbias_out)) return all;
+  a->max_runs = 1;
+  const size_t least = plan_scratch(p, a, fast).total();  // (sizes and limit are multiples of 256)
+  const size_t partial = (size_t)a->B * a->H * a->R * a->R * sizeof(float);
+  if (least < limit && (limit - least) / partial > 1) a->max_runs = (int)((limit - least) / partial);
+  return plan_scratch(p, a, fast);
+}
+
 // The backward with its scratch at `scratch` (caller-provided or the static array).
 int run_bwd(const evoattn_bwd_params* p, evo::Args& a, const Scratch& plan, bool fast, void* scratch, cudaStream_t st) {
   unsigned char* base = reinterpret_cast<unsigned char*>(scratch);
@@ -294,7 +306,7 @@ int evoattn_bwd_static_scratch(const evoattn_bwd_params* p, void* cuda_stream) {
   evo::Args a;
   fill_bwd_args(p, &a);
   const bool fast = use_sm100_bwd(p, a);
-  const Scratch plan = plan_scratch(p, &a, fast);
+  const Scratch plan = plan_scratch_within(EVOATTN_STATIC_SCRATCH_BYTES, p, &a, fast);
   if (plan.total() > EVOATTN_STATIC_SCRATCH_BYTES) return EVOATTN_ERR_WORKSPACE;
   // Looking the symbol up (done on every call) also makes the device's primary context current
   // on this thread, which the tensor-map encoder needs; nothing here allocates.

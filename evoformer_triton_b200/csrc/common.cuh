@@ -66,6 +66,7 @@ struct Args {
   Str4 sdgate;
   void* d_o_eff;
   const void* exchange;  // backward: evoattn_peer_allreduce_params of the d(pair_bias) exchange, or null
+  int max_runs;     // backward (CUDA-core kernels only): at most this many partial sums of d(pair_bias); 0: no limit
   float* dmask;     // backward (CUDA-core kernels only): gradient of an additive mask, [B,S,R] fp32
 };
 

@@ -553,14 +553,16 @@ __device__ __forceinline__ void dkdv_role(const Args& a, int vec, float* sm, int
 
 // How the MSA rows are dealt out to the blocks that compute dQ and d(pair_bias): runs of `rows`, each run
 // with a partial d(pair_bias) of its own unless there is only one.  Long enough that the partial sums
-// stay few, short enough for some four blocks per SM.
+// stay few (600 tiles' worth, 150 KB times R, at most), short enough for some four blocks per SM; fewer
+// where the scratch has no room for them.
 struct Runs {
   int rows, n;
 };
 Runs plan_runs(const Args& a) {
   if (!a.dbias) return Runs{1, a.S};
   const long long tiles = (long long)a.B * a.H * ((a.R + TT - 1) / TT);
-  const int want = (int)min((long long)a.S, (600 + tiles - 1) / tiles);
+  int want = (int)min((long long)a.S, (600 + tiles - 1) / tiles);
+  if (a.max_runs > 0) want = min(want, a.max_runs);
   const int rows = (a.S + want - 1) / want;
   return Runs{rows, (a.S + rows - 1) / rows};
 }

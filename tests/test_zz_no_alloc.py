@@ -128,6 +128,32 @@ def test_static_scratch_from_a_fresh_host_thread_and_near_the_limit():
         assert _rel(a, b) < 4e-3, (name, _rel(a, b))
 
 
+@pytest.mark.parametrize("cfg", [(1, 8, 32, 512, 32, torch.float32), (1, 8, 4, 1024, 8, torch.float32)],
+                         ids=["room_for_some_partial_sums", "room_for_none"])
+def test_static_scratch_makes_do_with_fewer_partial_sums(cfg):
+    """fp32 calls whose partial sums of d(pair_bias) (8 of 8 MiB, 4 of 32 MiB) do not fit the array."""
+    from evoformer_triton_b200 import _lib, attention
+    lib = _lib.load()
+    B, H, S, R, D, dtype = cfg
+    q, k, v, d_o, mask, bias = _make(B, H, S, R, D, dtype, seed=R + S)
+    o, lse = attention.attention_forward(q, k, v, mask, bias, D ** -0.5)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    ref = _fresh_outs(q, bias)
+    p = _bwd_params(q, k, v, o, lse, mask, bias, d_o, ref)
+    need = lib.evoattn_bwd_workspace_bytes(C.byref(p))
+    assert need > _lib.STATIC_SCRATCH_BYTES
+    ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+    p.workspace, p.workspace_bytes = ws.data_ptr(), need
+    assert lib.evoattn_bwd(C.byref(p), stream) == 0
+    got = _fresh_outs(q, bias)
+    p = _bwd_params(q, k, v, o, lse, mask, bias, d_o, got)
+    assert lib.evoattn_bwd_static_scratch(C.byref(p), stream) == 0
+    torch.cuda.synchronize()
+    for name, a, b in zip(("dq", "dk", "dv"), got, ref):
+        assert torch.equal(a, b), name  # nothing in their sums depends on the runs
+    assert _rel(got[3], ref[3]) < 1e-5  # the rows of a run are added in another grouping: 32 fp32 roundings at most
+
+
 def test_static_scratch_rejects_requests_beyond_its_array():
     from evoformer_triton_b200 import _lib, attention
     lib = _lib.load()
