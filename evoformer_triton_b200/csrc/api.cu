@@ -210,6 +210,14 @@ Scratch plan_scratch_within(size_t limit, const evoattn_bwd_params* p, evo::Args
   return plan_scratch(p, a, fast);
 }
 
+// Whether a tensor map could take a call only because something was padded for it: rows of the bias, or
+// of the d(pair_bias) that is wanted, that are not whole 16-byte pieces.
+bool has_padded_rows(const evoattn_bwd_params* p, const evo::Args& a) {
+  if (!a.bias) return false;
+  if (a.R * (a.bias16 ? 2 : 4) % 16 != 0) return true;
+  return (p->dbias || p->dbias_cast) && (a.R % 4 != 0 || ((uintptr_t)p->dbias & 15) != 0);
+}
+
 // The backward with its scratch at `scratch` (caller-provided or the static array).
 int run_bwd(const evoattn_bwd_params* p, evo::Args& a, const Scratch& plan, bool fast, void* scratch, cudaStream_t st) {
   unsigned char* base = reinterpret_cast<unsigned char*>(scratch);
@@ -305,8 +313,17 @@ int evoattn_bwd_static_scratch(const evoattn_bwd_params* p, void* cuda_stream) {
   if (rc) return rc;
   evo::Args a;
   fill_bwd_args(p, &a);
-  const bool fast = use_sm100_bwd(p, a);
-  const Scratch plan = plan_scratch_within(EVOATTN_STATIC_SCRATCH_BYTES, p, &a, fast);
+  bool fast = use_sm100_bwd(p, a);
+  Scratch plan = plan_scratch_within(EVOATTN_STATIC_SCRATCH_BYTES, p, &a, fast);
+  // The tensor-core kernels need an fp32 dQ accumulator and, for the lengths below, a padded d(pair_bias)
+  // (66 MiB at [1,128,501,8,32]); the CUDA-core kernels need one float per score row (2 MiB).  The lengths
+  // that reach the tensor cores by padding have always been served from this array and still are; the
+  // others have always been refused, and the caller chooses: a workspace, or EVOATTN_FLAG_FORCE_GENERIC.
+  if (fast && plan.total() > EVOATTN_STATIC_SCRATCH_BYTES && has_padded_rows(p, a)) {
+    fast = false;
+    fill_bwd_args(p, &a);
+    plan = plan_scratch_within(EVOATTN_STATIC_SCRATCH_BYTES, p, &a, fast);
+  }
   if (plan.total() > EVOATTN_STATIC_SCRATCH_BYTES) return EVOATTN_ERR_WORKSPACE;
   // Looking the symbol up (done on every call) also makes the device's primary context current
   // on this thread, which the tensor-map encoder needs; nothing here allocates.

@@ -172,7 +172,9 @@ int evoattn_bwd(const evoattn_bwd_params* p, void* cuda_stream);
  *  - A request that needs more than EVOATTN_STATIC_SCRATCH_BYTES of scratch (see
  *    evoattn_bwd_workspace_bytes) returns EVOATTN_ERR_WORKSPACE and launches nothing.  The one
  *    part of those bytes a call can do without is the partial sums of d(pair_bias) of the
- *    CUDA-core kernels (fp32 inputs, for one): it then takes as many as there is room for.
+ *    CUDA-core kernels (fp32 inputs, for one): it then takes as many as there is room for.  And a
+ *    16-bit call whose bias or d(pair_bias) has rows that are not whole 16-byte pieces runs on the
+ *    CUDA-core kernels where only their scratch fits.
  *  - The function calls no cudaMalloc, cudaFree or any other allocating routine.
  *  - The first call on each device looks up the array's device address (with that device
  *    current); make that first call before you start capturing a stream.

@@ -154,6 +154,33 @@ def test_static_scratch_makes_do_with_fewer_partial_sums(cfg):
     assert _rel(got[3], ref[3]) < 1e-5  # the rows of a run are added in another grouping: 32 fp32 roundings at most
 
 
+@pytest.mark.parametrize("R,rc", [(501, 0), (512, 7)])
+def test_static_scratch_beyond_the_array_on_tensor_cores(R, rc):
+    """16-bit calls whose tensor-core scratch does not fit the array: an odd length is served by the CUDA-core
+    kernels, as it was when those had all odd lengths; a length that never was is refused."""
+    from evoformer_triton_b200 import _lib, attention
+    lib = _lib.load()
+    B, H, S, D, dtype = 1, 8, 128, 32, torch.bfloat16
+    q, k, v, d_o, mask, bias = _make(B, H, S, R, D, dtype, seed=R)
+    rows = attention.pad_bias_rows(bias)
+    o, lse = attention.attention_forward(q, k, v, mask, rows, D ** -0.5)
+    assert attention.last_path["fwd"] == _lib.PATH_TCGEN05
+    got = _fresh_outs(q, bias)
+    p = _bwd_params(q, k, v, o, lse, mask, rows, d_o, got)
+    assert lib.evoattn_bwd_workspace_bytes(C.byref(p)) > _lib.STATIC_SCRATCH_BYTES
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.evoattn_bwd_static_scratch(C.byref(p), stream) == rc
+    torch.cuda.synchronize()
+    if rc != 0:  # nothing was launched
+        assert all((t == 7.0).all() for t in got)
+        return
+    assert lib.evoattn_last_path() == _lib.PATH_GENERIC
+    want = attention.attention_backward(q, k, v, o, lse, mask, rows, D ** -0.5, d_o)
+    assert attention.last_path["bwd"] == _lib.PATH_TCGEN05
+    for name, a, b in zip(("dq", "dk", "dv", "dbias"), got, want):
+        assert _rel(a, b) < 1e-2, (name, _rel(a, b))  # the tensor cores round P and dS to bf16 (2^-9)
+
+
 def test_static_scratch_rejects_requests_beyond_its_array():
     from evoformer_triton_b200 import _lib, attention
     lib = _lib.load()
