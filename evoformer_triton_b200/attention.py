@@ -287,7 +287,11 @@ class _EvoformerAttentionBase(torch.autograd.Function):
     bias_layout = "b1hrr"
 
     @classmethod
-    def apply(cls, Q, K, V, res_mask=None, pair_bias=None, *gate):
+    def apply(cls, Q, K, V, res_mask=None, pair_bias=None):
+        return cls._call(Q, K, V, res_mask, pair_bias)
+
+    @classmethod
+    def _call(cls, Q, K, V, res_mask, pair_bias, *gate):
         if getattr(_pending, "group", None) is not None:
             return super().apply(Q, K, V, res_mask, pair_bias, *gate)
         return _lib.host().attention(Q, K, V, res_mask, pair_bias, gate[0] if gate else None,
@@ -423,6 +427,10 @@ class GatedEvoformerAttention(_EvoformerAttentionBase):
 
     layout = "reinterpret"
 
+    @classmethod
+    def apply(cls, Q, K, V, res_mask, pair_bias, gate):
+        return cls._call(Q, K, V, res_mask, pair_bias, gate)
+
     @staticmethod
     def forward(ctx, Q, K, V, res_mask, pair_bias, gate):
         return GatedEvoformerAttention._forward(ctx, Q, K, V, res_mask, pair_bias, gate)
@@ -474,4 +482,4 @@ def evoformer_attention(Q, K, V, biases: Optional[Sequence[Optional[torch.Tensor
     if getattr(_pending, "group", None) is None:
         return _lib.host().attention(Q, K, V, biases[0], biases[1], gate, layout == "true", pair_bias_layout == "brrh")
     fn = _variant("true" if layout == "true" else "reinterpret", pair_bias_layout, gate is not None)
-    return fn.apply(Q, K, V, biases[0], biases[1], gate)
+    return fn._call(Q, K, V, biases[0], biases[1], gate)

@@ -37,6 +37,16 @@ def test_op_refuses_cpu_tensors():
         evo.EvoformerAttention.apply(x, x, x, None, None)
 
 
+@pytest.mark.parametrize("name,args", [("EvoformerAttention", 6), ("EvoformerAttentionTrueLayout", 6), ("EvoformerAttention", 2),
+                                       ("GatedEvoformerAttention", 5), ("GatedEvoformerAttention", 7)])
+def test_apply_takes_the_arguments_of_its_forward(name, args):
+    """As autograd.Function.apply does: one argument too many is not a gate, and a gated call needs its gate."""
+    import evoformer_triton_b200 as evo
+    x = torch.zeros(1, 1, 8, 1, 8, dtype=torch.bfloat16)
+    with pytest.raises(TypeError):
+        getattr(evo, name).apply(*(x, x, x, None, None, x, x)[:args])
+
+
 @pytest.mark.gpu
 def test_ds4sci_style_call_matches_oracle():
     """``evoformer_attention(Q, K, V, [mask_bias, pair_bias])`` and the compat DS4Sci shim: true
