@@ -299,42 +299,15 @@ class _EvoformerAttentionBase(torch.autograd.Function):
 
     @classmethod
     def _forward(cls, ctx, Q, K, V, res_mask, pair_bias, gate=None):
-        for t in (Q, K, V):
-            if not t.is_cuda:
-                raise RuntimeError("EvoformerAttention runs on CUDA tensors only; there is no CPU fallback")
-        if not (Q.shape[-1] == K.shape[-1] == V.shape[-1]):
-            raise AssertionError("Q, K, V must share the head dimension")  # evoformer.py:642-643
-        if Q.dtype not in _DTYPES or K.dtype != Q.dtype or V.dtype != Q.dtype:
-            raise TypeError("Q, K, V must share one dtype out of bfloat16, float16, float32")
+        q, k, v, mask, bias, g = _lib.host().prepare_call(Q, K, V, res_mask, pair_bias, gate, cls.layout == "true",
+                                                          cls.bias_layout == "brrh")
         B, S, R, H, D = Q.shape
         scale = D ** -0.5  # evoformer.py:646
-        if cls.layout == "reinterpret":
-            Q, K, V = Q.contiguous(), K.contiguous(), V.contiguous()
-        q, k, v = (_prep_operand(_view_dims(t, cls.layout)) for t in (Q, K, V))
-        g = None
-        if gate is not None:
-            if gate.shape != Q.shape or gate.dtype != Q.dtype:
-                raise TypeError("gate must have the shape and dtype of Q")
-            g = _prep_operand(_view_dims(gate.contiguous() if cls.layout == "reinterpret" else gate, cls.layout))
-        mask = None
-        if res_mask is not None:
-            mask = res_mask.reshape(B, S, R)  # [B,S,1,1,R] in the reference (evoformer.py:651)
-            if mask.dtype not in (torch.bool, torch.float32, Q.dtype):
-                mask = mask.to(torch.float32)
-        bias = None
-        if pair_bias is not None:
-            if cls.bias_layout == "brrh":
-                bias = bias_to_heads_first(pair_bias if pair_bias.dtype in (torch.float32, Q.dtype) else pair_bias.float())
-            else:
-                bias = pair_bias.reshape(B, H, R, R)  # [B,1,H,R,R] (evoformer.py:652)
-            # fp32 (test.py:36-42) and the q/k/v type (memory_benchmark.py:20, speed_benchmark.py:83) are
-            # read by the kernels as they are; anything else is widened once
-            if bias.dtype != torch.float32 and bias.dtype != Q.dtype:
-                bias = bias.float()
-            if bias.stride(-1) != 1:
-                bias = bias.contiguous()
-            if Q.dtype != torch.float32 and D <= 64 and D % 8 == 0 and R <= 2048:  # what the tensor-core kernels cover
-                bias = pad_bias_rows(bias)
+        q, k, v = (_view_dims(t, cls.layout) for t in (q, k, v))
+        g = None if g is None else _view_dims(g, cls.layout)
+        mask = None if mask is None else mask.view(B, S, R)  # [B,S,1,1,R] in the reference (evoformer.py:651)
+        if bias is not None:  # [B,1,H,R,R] (evoformer.py:652), or [B,H,R,>=R] where the rows had to be padded
+            bias = (bias.squeeze(1) if bias.dim() == 5 else bias)[..., :R]
         o, lse = attention_forward(q, k, v, mask, bias, scale, g)
         ctx.save_for_backward(q, k, v, mask, bias, o, lse, g)  # evoformer.py:729
         ctx.softmax_scale = scale

@@ -7,7 +7,8 @@
 //
 // Same semantics as the Python boundary (dsevoformer-triton/evoformer.py:633-862): the reinterpreting
 // head layout or the true one, None for mask and bias, additive or boolean masks, gating, both bias
-// layouts.  The N_seq-sharded op, which exchanges d(pair_bias) in its backward, stays in Python.
+// layouts.  The N_seq-sharded op, which exchanges d(pair_bias) in its backward, stays in Python and takes
+// its checks and the preparation of its inputs from here.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -149,8 +150,49 @@ Tensor kernel_bias(const Tensor& pb, const Dims& d, at::ScalarType qt, bool head
   return r;
 }
 
+using Maybe = c10::optional<Tensor>;
+
+[[noreturn]] void raise(PyObject* type, const char* text) {
+  PyErr_SetString(type, text);
+  throw py::error_already_set();
+}
+
+// Everything a kernel is given an address of is checked here: on Q's device, of a size that its strides
+// are read for.
+void check_call(const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask, const Maybe& bias, const Maybe& gate) {
+  const auto beside_q = [&](const Tensor& t, const char* name) {
+    if (t.device() != Q.device())
+      raise(PyExc_RuntimeError, (std::string(name) + " is on " + t.device().str() + ", Q on " + Q.device().str()).c_str());
+  };
+  if (mask) beside_q(*mask, "res_mask");
+  if (bias) beside_q(*bias, "pair_bias");
+  if (gate) beside_q(*gate, "gate");
+  for (const Tensor* t : {&Q, &K, &V})
+    if (!t->is_cuda()) raise(PyExc_RuntimeError, "EvoformerAttention runs on CUDA tensors only; there is no CPU fallback");
+  beside_q(K, "K");
+  beside_q(V, "V");
+  if (Q.dim() != 5) raise(PyExc_ValueError, "Q must have the shape [B, N_seq, N_res, H, D]");
+  if (K.size(-1) != Q.size(-1) || V.size(-1) != Q.size(-1))
+    raise(PyExc_AssertionError, "Q, K, V must share the head dimension");  // evoformer.py:642-643
+  if (!known(Q.scalar_type()) || K.scalar_type() != Q.scalar_type() || V.scalar_type() != Q.scalar_type())
+    raise(PyExc_TypeError, "Q, K, V must share one dtype out of bfloat16, float16, float32");
+  if (K.sizes() != Q.sizes() || V.sizes() != Q.sizes()) raise(PyExc_RuntimeError, "Q, K, V must have one shape");
+  if (gate && (gate->sizes() != Q.sizes() || gate->scalar_type() != Q.scalar_type()))
+    raise(PyExc_TypeError, "gate must have the shape and dtype of Q");
+}
+
+// The inputs of a call as the kernels take them.
+struct Operands {
+  Tensor q, k, v, mask, bias, gate;
+  Operands(const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask_in, const Maybe& bias_in, const Maybe& gate_in,
+           bool true_layout, bool heads_last, cudaStream_t st)
+      : q(operand(Q, true_layout)), k(operand(K, true_layout)), v(operand(V, true_layout)),
+        mask(kernel_mask(mask_in.value_or(Tensor()), Dims(Q), Q.scalar_type())),
+        bias(kernel_bias(bias_in.value_or(Tensor()), Dims(Q), Q.scalar_type(), heads_last, st)),
+        gate(gate_in ? operand(*gate_in, true_layout) : Tensor()) {}
+};
+
 struct Attention : public torch::autograd::Function<Attention> {
-  using Maybe = c10::optional<Tensor>;
 
   static Tensor forward(AutogradContext* ctx, const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask_in,
                         const Maybe& bias_in, const Maybe& gate_in, bool true_layout, bool heads_last) {
@@ -158,10 +200,8 @@ struct Attention : public torch::autograd::Function<Attention> {
     const Tensor res_mask = mask_in.value_or(Tensor()), pair_bias = bias_in.value_or(Tensor());
     const c10::cuda::CUDAGuard guard(Q.device());
     const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
-    const Tensor q = operand(Q, true_layout), k = operand(K, true_layout), v = operand(V, true_layout);
-    const Tensor gate = gate_in ? operand(*gate_in, true_layout) : Tensor();
-    const Tensor mask = kernel_mask(res_mask, d, Q.scalar_type());
-    const Tensor bias = kernel_bias(pair_bias, d, Q.scalar_type(), heads_last, st);
+    const Operands x(Q, K, V, mask_in, bias_in, gate_in, true_layout, heads_last, st);
+    const Tensor &q = x.q, &k = x.k, &v = x.v, &mask = x.mask, &bias = x.bias, &gate = x.gate;
     Tensor o = at::empty({d.B, d.S, d.R, d.H, d.D}, q.options());
     Tensor lse = at::empty({d.B, d.H, d.S, d.R}, q.options().dtype(at::kFloat));
     evoattn_fwd_params p{};
@@ -242,30 +282,26 @@ struct Attention : public torch::autograd::Function<Attention> {
   }
 };
 
-[[noreturn]] void raise(PyObject* type, const char* text) {
-  PyErr_SetString(type, text);
-  throw py::error_already_set();
+Tensor attention(const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask, const Maybe& bias, const Maybe& gate,
+                 bool true_layout, bool heads_last) {
+  check_call(Q, K, V, mask, bias, gate);
+  return Attention::apply(Q, K, V, mask, bias, gate, true_layout, heads_last);
 }
 
-Tensor attention(const Tensor& Q, const Tensor& K, const Tensor& V, const c10::optional<Tensor>& mask,
-                 const c10::optional<Tensor>& bias, const c10::optional<Tensor>& gate, bool true_layout, bool heads_last) {
-  for (const Tensor* t : {&Q, &K, &V})
-    if (!t->is_cuda()) raise(PyExc_RuntimeError, "EvoformerAttention runs on CUDA tensors only; there is no CPU fallback");
-  if (Q.dim() != 5) raise(PyExc_ValueError, "Q must have the shape [B, N_seq, N_res, H, D]");
-  if (K.size(-1) != Q.size(-1) || V.size(-1) != Q.size(-1))
-    raise(PyExc_AssertionError, "Q, K, V must share the head dimension");  // evoformer.py:642-643
-  if (!known(Q.scalar_type()) || K.scalar_type() != Q.scalar_type() || V.scalar_type() != Q.scalar_type())
-    raise(PyExc_TypeError, "Q, K, V must share one dtype out of bfloat16, float16, float32");
-  if (K.sizes() != Q.sizes() || V.sizes() != Q.sizes()) raise(PyExc_RuntimeError, "Q, K, V must have one shape");
-  if (gate && (gate->sizes() != Q.sizes() || gate->scalar_type() != Q.scalar_type()))
-    raise(PyExc_TypeError, "gate must have the shape and dtype of Q");
-  return Attention::apply(Q, K, V, mask, bias, gate, true_layout, heads_last);
+// What the Python boundary of the N_seq-sharded op hands to the C ABI: the checks and the preparation are these.
+std::vector<Tensor> prepare_call(const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask, const Maybe& bias,
+                                 const Maybe& gate, bool true_layout, bool heads_last) {
+  check_call(Q, K, V, mask, bias, gate);
+  const c10::cuda::CUDAGuard guard(Q.device());
+  const Operands x(Q, K, V, mask, bias, gate, true_layout, heads_last, at::cuda::getCurrentCUDAStream().stream());
+  return {x.q, x.k, x.v, x.mask, x.bias, x.gate};
 }
 
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention", &attention);
+  m.def("prepare_call", &prepare_call);
   m.def("status_word", &status_word);
   m.def("status_words", [] {
     std::lock_guard<std::mutex> lock(g_status_mutex);

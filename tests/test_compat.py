@@ -47,6 +47,21 @@ def test_apply_takes_the_arguments_of_its_forward(name, args):
         getattr(evo, name).apply(*(x, x, x, None, None, x, x)[:args])
 
 
+@pytest.mark.parametrize("sharded", [False, True], ids=["native", "python"])
+@pytest.mark.parametrize("name", ["res_mask", "pair_bias", "gate"])
+def test_every_operand_has_to_be_where_q_is(name, sharded):
+    """On either boundary: the address of a tensor elsewhere must not reach a kernel."""
+    import contextlib
+    import evoformer_triton_b200 as evo
+    from evoformer_triton_b200.attention import pair_bias_grad_summed_over
+    x = torch.zeros(1, 1, 8, 1, 8, dtype=torch.bfloat16)
+    args = {"res_mask": torch.ones(1, 1, 1, 1, 8, dtype=torch.bool), "pair_bias": torch.zeros(1, 1, 1, 8, 8), "gate": x}
+    args[name] = args[name].to("meta")
+    with pair_bias_grad_summed_over(None) if sharded else contextlib.nullcontext():
+        with pytest.raises(RuntimeError, match=f"{name} is on meta, Q on cpu"):
+            evo.evoformer_attention(x, x, x, [args["res_mask"], args["pair_bias"]], gate=args["gate"])
+
+
 @pytest.mark.gpu
 def test_ds4sci_style_call_matches_oracle():
     """``evoformer_attention(Q, K, V, [mask_bias, pair_bias])`` and the compat DS4Sci shim: true

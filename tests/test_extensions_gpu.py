@@ -88,3 +88,52 @@ def test_additive_mask_gets_a_gradient(D, dtype):
     evo.check_device_status()
     assert m.grad is not None and m.grad.shape == x["res_mask"].shape
     _check((out, t["Q"].grad, t["K"].grad, t["V"].grad, t["pair_bias"].grad, None, m.grad), want)
+
+
+@pytest.fixture
+def group_of_one():
+    import torch.distributed as dist
+    dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1, device_id=torch.device(DEV))
+    yield
+    dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("cfg", [("reinterpret", "b1hrr", False, 136), ("true", "brrh", True, 136), ("reinterpret", "brrh", True, 77),
+                                 ("true", "b1hrr", False, 77)], ids=lambda c: "-".join(map(str, c)))
+def test_sharded_boundary_matches_the_native_one(cfg, group_of_one):
+    """The Python boundary (the one whose backward sums d(pair_bias) over ranks, here one) gives what the native
+    boundary does, and refuses the same inputs before their addresses reach a kernel."""
+    import evoformer_triton_b200 as evo
+    from evoformer_triton_b200.attention import pair_bias_grad_summed_over
+    layout, bias_layout, gated, R = cfg
+    B, S, H, D = 2, 5, 4, 32
+    x = _inputs(B, S, R, H, D, torch.bfloat16, seed=R)
+    bias = x["pair_bias"].bfloat16()
+    if bias_layout == "brrh":
+        bias = bias.reshape(B, H, R, R).permute(0, 2, 3, 1).contiguous()
+
+    def call(**other):
+        t = {n: x[n].to(DEV).requires_grad_() for n in ("Q", "K", "V", "gate")}
+        t["bias"], t["mask"] = bias.to(DEV).requires_grad_(), x["res_mask"].to(DEV)
+        t.update(other)
+        out = evo.evoformer_attention(t["Q"], t["K"], t["V"], [t["mask"], t["bias"]], layout=layout, pair_bias_layout=bias_layout,
+                                      gate=t["gate"] if gated else None)
+        out.backward(x["dO"].to(DEV))
+        return [out.detach()] + [t[n].grad for n in ("Q", "K", "V", "bias")] + ([t["gate"].grad] if gated else [])
+
+    want = call()
+    with pair_bias_grad_summed_over(None):
+        got = call()
+        for bad in ({"K": x["K"][:, :-1].contiguous().to(DEV)}, {"mask": x["res_mask"]}, {"bias": bias}):
+            with pytest.raises(RuntimeError):
+                call(**bad)
+    for bad in ({"K": x["K"][:, :-1].contiguous().to(DEV)}, {"mask": x["res_mask"]}, {"bias": bias}):
+        with pytest.raises(RuntimeError):
+            call(**bad)
+    torch.cuda.synchronize()
+    evo.check_device_status()
+    for i, (a, b) in enumerate(zip(got, want)):
+        if i in (1, 4):  # dQ and d(pair_bias) are summed across blocks in no fixed order
+            assert a.shape == b.shape and oc.rel_err(a, b) < 4e-3, i
+        else:
+            assert torch.equal(a, b), i
