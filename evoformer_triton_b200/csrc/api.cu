@@ -127,8 +127,12 @@ bool use_sm100_bwd(const evoattn_bwd_params* p, const evo::Args& a) {
       !stride_ok16(p->dv_stride, es))
     return false;
   if (p->fwd.gate && ((((uintptr_t)p->dgate) & 15) || !stride_ok16(p->dgate_stride, es))) return false;
-  // A dense d(pair_bias) whose rows are not whole 16-byte pieces costs the tensor-core path a padded
-  // buffer and one more pass; a handful of score rows is done sooner on the CUDA cores.
+  // Of the odd lengths with a d(pair_bias), the smallest calls keep the dispatch that all of them once had:
+  // the CUDA cores, with P and dS in fp32.  The line does not separate the faster kernels.  Backward calls in
+  // us, tensor / CUDA cores, [B,S,R,H]: D = 8: [1,1,33,1] 15.7 / 9.6, [1,5,51,2] 16.5 / 12.8, [1,1,511,1]
+  // 47.0 / 50.9; D = 32: 15.5 / 12.7, 16.8 / 16.2, 40.9 / 75.4; D = 64: 12.2 / 17.4, 13.0 / 21.8,
+  // 27.1 / 107.2.  So it gains a few us at one tile of residues and D <= 32 and loses elsewhere; moving a
+  // call across it would take its P and dS to 16 bits (errors 1.4 times as large).
   if (p->fwd.bias && (p->dbias || p->dbias_cast) && p->fwd.R % 4 != 0 && (long long)a.B * a.H * a.S * a.R <= 512) return false;
   return evo::sm100_bwd_supported(p->fwd.dtype, a);
 }

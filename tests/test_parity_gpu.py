@@ -145,7 +145,7 @@ SHAPES = [
     (1, 2, 260, 2, 32, torch.bfloat16, "bool", False),     # no pair bias
     (1, 1, 640, 1, 64, torch.bfloat16, "none", False),
     (1, 2, 96, 2, 24, torch.bfloat16, "bool", True),       # D not a power of two
-    (1, 2, 50, 2, 32, torch.bfloat16, "bool", True),       # R % 4 != 0: CUDA-core path
+    (1, 2, 50, 2, 32, torch.bfloat16, "bool", True),       # R % 4 != 0 and few rows: backward on the CUDA cores
     (1, 4, 200, 2, 32, torch.bfloat16, "add32", True),     # additive masks at D=32
     (1, 5, 136, 2, 32, torch.float16, "addsame", True),
     (1, 7, 384, 3, 24, torch.bfloat16, "add32", False),    # D < 32 padded, no pair bias, ragged row group
@@ -325,8 +325,8 @@ def test_fully_masked_row_ragged_tile(D, dtype):
 
 def test_padded_bias_rows_with_odd_n_res():
     """A pair bias whose rows are padded to a 16-byte multiple while N_res itself is not a
-    multiple of 4: the forward can take it through a tensor map, the dense d(pair_bias) cannot
-    leave through one, so the backward has to fall back to the CUDA-core kernels, not fail."""
+    multiple of 4: the forward takes it through a tensor map; a backward this small, whose dense
+    d(pair_bias) cannot leave through one, runs on the CUDA-core kernels in fp32 arithmetic."""
     import evoformer_triton_b200 as evo
     from evoformer_triton_b200 import attention
     x = rand_inputs(1, 3, 50, 2, 32, torch.bfloat16, seed=29)
