@@ -799,10 +799,8 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   const int NT = (a.R + BT - 1) / BT;
   const long long items = (long long)a.B * a.H * NT * ((a.S + G - 1) / G);
   if (items > 0x7fffffffLL / (G * NT)) return EVOATTN_ERR_SHAPE;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return EVOATTN_ERR_CUDA;
+  const int sms = sm_count();
+  if (sms <= 0) return EVOATTN_ERR_CUDA;
   const long long ctas = items < sms ? items : sms;
   auto kern = !a.bias ? evo_bwd_sm100_kernel<T, DP, false, false>
                       : (a.bias16 ? evo_bwd_sm100_kernel<T, DP, true, true> : evo_bwd_sm100_kernel<T, DP, true, false>);
@@ -837,15 +835,20 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }
 
-// Head dimensions up to 16: items of seven rows (padded to 16) flush d(pair_bias) and reload the bias tile
-// every seventh step instead of every third, but there are fewer of them and the last group of rows is
-// padded further.  They are taken where the CTA with the most steps gets no more than a tenth more.
-bool seven_rows_pay(const Args& a) {
+// Head dimensions up to 16: items of seven rows (padded to 16 columns) flush d(pair_bias) and reload the bias
+// tile every seventh step instead of every third, but there are fewer of them and the last group of rows is
+// padded further.  They are taken where the CTA with the most steps gets no more than a tenth more of them,
+// or, without a d(pair_bias), a twenty-fifth.  Time of the backward call, seven rows over three, by how many more
+// steps that CTA gets (N_res 128 to 1000, D = 8 and 16):
+//   with d(pair_bias):     0.90-0.94 at as many steps, 0.95 at 4 % more, 0.97 at 8 %, 1.05 at 17 %
+//   with a bias alone:     0.95-0.98                   0.98              1.02-1.03    1.08
+//   without a bias:        0.97                        1.00              1.04         1.07
+bool seven_rows_pay(const Args& a, int sms) {
   const auto steps = [&](int G) {
     const long long items = (long long)a.B * a.H * ((a.R + BT - 1) / BT) * ((a.S + G - 1) / G);
-    return (items + 147) / 148 * G;
+    return (items + sms - 1) / sms * G;
   };
-  return 10 * steps(7) <= 11 * steps(3);
+  return a.bias && a.dbias ? 10 * steps(7) <= 11 * steps(3) : 25 * steps(7) <= 26 * steps(3);
 }
 
 }  // namespace
@@ -864,7 +867,9 @@ size_t sm100_bwd_workspace_bytes(int, const Args& a) {
 
 int launch_sm100_bwd(int dtype, const Args& a, void* workspace, size_t workspace_bytes, cudaStream_t st,
                      int* launches) {
-  if (a.D <= 16 && seven_rows_pay(a)) {
+  const int sms = sm_count();
+  if (sms <= 0) return EVOATTN_ERR_CUDA;
+  if (a.D <= 16 && seven_rows_pay(a, sms)) {
     if (dtype == EVOATTN_BF16) return launch_t<__nv_bfloat16, 16>(a, workspace, workspace_bytes, st, launches);
     return launch_t<__half, 16>(a, workspace, workspace_bytes, st, launches);
   }

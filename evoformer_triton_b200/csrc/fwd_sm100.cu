@@ -593,17 +593,6 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
-// SM count of the current device (looked up once per device).
-int num_sms_of_current_device() {
-  static int table[64] = {};
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (table[dev] > 0) return table[dev];
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 0;
-  table[dev] = n;
-  return n;
-}
-
 template <class T, int DP, bool QP>
 int launch_t(const Args& a, cudaStream_t st, int* launches) {
   using C = Cfg<DP, QP>;
@@ -618,14 +607,14 @@ int launch_t(const Args& a, cudaStream_t st, int* launches) {
   } else {
     tb = tq;
   }
-  const int g_num_sms = num_sms_of_current_device();
-  if (g_num_sms <= 0) return EVOATTN_ERR_CUDA;
+  const int sms = sm_count();
+  if (sms <= 0) return EVOATTN_ERR_CUDA;
   const int T_TILES = (a.R + BN - 1) / BN;
   const int NQT = (a.R + BM - 1) / BM;
   const size_t smem = C::bytes(T_TILES * BN);
   const long long items = QP ? (long long)a.B * a.H * ((NQT + 1) / 2) * a.S
                              : (long long)a.B * a.H * NQT * ((a.S + 1) / 2);
-  const int grid = (int)(items < g_num_sms ? items : g_num_sms);
+  const int grid = (int)(items < sms ? items : sms);
   const bool add = a.mask_kind == EVOATTN_MASK_ADD_F32 || a.mask_kind == EVOATTN_MASK_ADD_SAME;
   auto kern = !a.bias ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_NONE, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_NONE, QP>)
               : a.bias16 ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_16, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_16, QP>)

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <atomic>
 #include <mutex>
 #include <unordered_map>
 #include <utility>
@@ -37,6 +38,17 @@ inline bool kernel_ready(const void* kern, int smem_bytes, int* num_regs) {
   }
   if (num_regs) *num_regs = f.num_regs;
   return true;
+}
+
+// SM count of the current device, or 0 (asked of the driver once per device).
+inline int sm_count() {
+  static std::atomic<int> table[64];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if ((n = table[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 0;
+  table[dev].store(n, std::memory_order_relaxed);
+  return n;
 }
 
 // Launches a kernel that may be scheduled while the one before it on the stream is still draining

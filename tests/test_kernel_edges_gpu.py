@@ -80,6 +80,38 @@ def test_pair_bias_gradient_in_its_type_and_layout(layout, bias_dtype, R):
     assert oc.rel_err(got, want) < 1e-2
 
 
+@pytest.mark.parametrize("cfg", [
+    (1, 63, 200, 8, 8, torch.bfloat16, "bool", "fp32", False), (1, 60, 200, 8, 16, torch.float16, "add32", "same", False),
+    (2, 14, 400, 8, 8, torch.bfloat16, "addsame", "none", False), (2, 13, 397, 8, 16, torch.bfloat16, "bool", "same", True),
+    (1, 120, 130, 8, 16, torch.float16, "none", "fp32", False)],
+    ids=lambda c: "B%dS%dR%dH%dD%d-%s-%s-%s%s" % (*c[:5], str(c[5]).split(".")[-1], c[6], c[7], "-gate" if c[8] else ""))
+def test_items_of_seven_rows(cfg):
+    """Head dimensions up to 16 with enough MSA rows for work items of seven: types, masks, biases, a gate, row groups
+    that are not full, residues that do not fill a tile, one and two items to a block."""
+    import evoformer_triton_b200 as evo
+    from evoformer_triton_b200 import attention
+    B, S, R, H, D, dtype, mask, bias, gated = cfg
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    steps = lambda G: -(-B * H * -(-R // 128) * -(-S // G) // sms) * G  # noqa: E731
+    assert 25 * steps(7) <= 26 * steps(3)  # the launcher's condition: these sizes do take seven rows
+    x = rand_inputs(B, S, R, H, D, dtype, seed=S + R, mask=mask, bias=bias != "none", keep_p=0.85)
+    if bias == "same":
+        x["pair_bias"] = x["pair_bias"].to(dtype)
+    gate = torch.randn(x["Q"].shape, generator=torch.Generator().manual_seed(1)).to(dtype) if gated else None
+    want = oc.extended_attention_fwd_bwd(x["Q"], x["K"], x["V"], x["res_mask"], x["pair_bias"], x["dO"], gate=gate,
+                                         upcast=torch.float32)
+    t = {n: None if v is None else v.to(DEV) for n, v in dict(x, gate=gate).items()}
+    wrt = [t[n].requires_grad_() for n in ("Q", "K", "V", "pair_bias", "gate") if t[n] is not None]
+    out = evo.evoformer_attention(t["Q"], t["K"], t["V"], [t["res_mask"], t["pair_bias"]], layout="reinterpret", gate=t["gate"])
+    grads = torch.autograd.grad(out, wrt, t["dO"])
+    torch.cuda.synchronize()
+    evo.check_device_status()
+    assert attention.last_path["bwd"] == _lib().PATH_TCGEN05
+    want = [w for w, n in zip(want[1:6], ("Q", "K", "V", "pair_bias", "gate")) if t[n] is not None]
+    for g, w in zip(grads, want):
+        assert oc.rel_err(g, w) < 1e-2
+
+
 def test_pair_bias_gradient_of_64_gib():
     """d(pair_bias) of 2^34 values: its clearing in the backward's first pass counts beyond 32 bits.  The buffer
     holds a marker before the call; a (b, h) slab that was not cleared would keep it."""
