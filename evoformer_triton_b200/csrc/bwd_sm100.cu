@@ -40,10 +40,6 @@ using namespace ptx;
 constexpr int BT = 128;   // tile edge (queries and keys)
 constexpr int HT = 64;    // queries per half of a step (one warp group)
 constexpr int QT = 32;    // queries per quarter of a step
-// S^T / dP^T buffers per half: 1 = one of 64 queries shared by the half's eight warps; 2 = one of 32
-// queries per group of four warps (four groups that hand over to the tensor core independently;
-// measured 2 % slower on the 384-residue workloads: forty smaller MMAs per step instead of thirty-two)
-constexpr int kSub = 1;
 // MSA rows per work item: each keeps a dK and a dV accumulator of DP columns in tensor memory for the
 // whole item, next to 256 columns of score buffers and two dQ partials
 template <int DP> struct RowsPerItem { static constexpr int G = (DP == 64) ? 1 : (DP == 32) ? 3 : 7; };
@@ -242,8 +238,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   const Bar kv_empty{bars_s + 8 * 7};    // [G] ... and every MMA that reads them has completed
   const Bar st_full{bars_s + 8 * 32};     // [2] Q, dO and the statistics vectors of a step landed
   const Bar st_empty{bars_s + 8 * 40};    // [2] ... the step's last dV/dK MMAs have completed
-  const Bar sd_full{bars_s + 8 * 48};    // [2][kSub] S^T and dP^T of score buffer (h, sub) of a step are in TMEM
-  const Bar cdone{bars_s + 8 * 52};      // [2][kSub] the warps of that buffer have its P^T and dS^T in TMEM (for the dV/dK MMAs)
+  const Bar sd_full{bars_s + 8 * 48};    // [2], two apart: S^T and dP^T of half h of a step are in TMEM
+  const Bar cdone{bars_s + 8 * 52};      // [2], two apart: the warps of that half have its P^T and dS^T in TMEM (for the dV/dK MMAs)
   const Bar sdone{bars_s + 8 * 23};      // [2] ... and have stored their half of dS in shared memory (for the dQ MMAs)
   const Bar b_full{bars_s + 8 * 14};     // [2] half h (64 queries) of the pair-bias tile landed
   const Bar b_done{bars_s + 8 * 16};     // [2] ... has been read for the last time
@@ -298,7 +294,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); }  // kv_full; kv_empty: three MMA warps read K/V
     for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
     for (int i = 0; i < 2; ++i) {
-      for (int q = 0; q < 2; ++q) { mbar_init(bars + 48 + 2 * i + q, 2); mbar_init(bars + 52 + 2 * i + q, kCW / (2 * kSub)); }  // sd_full, cdone
+      mbar_init(bars + 48 + 2 * i, 2); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full, cdone
       mbar_init(bars + 14 + i, 1); mbar_init(bars + 16 + i, kCW / 2);  // b_full, b_done
       mbar_init(bars + 19 + i, 1);                                     // dq_full
       mbar_init(bars + 23 + i, kCW / 2);                               // sdone
@@ -334,7 +330,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       // leader lane in a converged warp).
       const bool isA = (warp == kCW);
       if (lane == 0) {
-      constexpr uint32_t kIdescSD = make_idesc(kBf16, false, false, BT, HT / kSub);   // S^T, dP^T: K-major operands, N = 64 or 32
+      constexpr uint32_t kIdescSD = make_idesc(kBf16, false, false, BT, HT);   // S^T, dP^T: K-major operands, N = 64
       constexpr uint32_t kIdescOut = make_idesc(kBf16, false, true, BT, DP);   // dV, dK: A from TMEM, B MN-major
       constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
       constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
@@ -354,20 +350,19 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         if (++p.stg == (uint32_t)kStages) { p.stg = 0; p.ring_par ^= 1u; }
         return p;
       };
-      constexpr int QB = HT / kSub;  // queries per S^T / dP^T buffer
       // Everything an MMA group needs is computed before the wait it follows: this thread shares its
       // scheduler with four arithmetic warps, so every instruction between the wake-up and the MMA is
       // paid several times over, and it sits on the critical path of the half that waits for it.
-      auto issue_in = [&](const Pos& p, uint32_t ka, uint32_t qb, int h, int sub) {
+      auto issue_in = [&](const Pos& p, uint32_t ka, uint32_t qb, int h) {
         // (the second commit: the item's last read of this warp's K or V tile of row g)
-        const uint32_t bar2 = (h == 1 && sub == kSub - 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
-        const uint32_t tD = tmem + (h ? col_in1 : col_in0) + sub * QB, qa = qb + (h * HT + sub * QB) * (RB >> 4);
+        const uint32_t bar2 = (h == 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
+        const uint32_t tD = tmem + (h ? col_in1 : col_in0), qa = qb + h * HT * (RB >> 4);
         if constexpr (DP == 16) {  // one K slice of 16
-          mma_ss_x1_commit(tD, ka, qa, kHiOp, kIdescSD, (sd_full + (2 * h + sub)).a, bar2);
+          mma_ss_x1_commit(tD, ka, qa, kHiOp, kIdescSD, (sd_full + 2 * h).a, bar2);
         } else if constexpr (DP == 32) {  // two
-          mma_ss_x2_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + (2 * h + sub)).a, bar2);
+          mma_ss_x2_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + 2 * h).a, bar2);
         } else {                   // four
-          mma_ss_x4_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + (2 * h + sub)).a, bar2);
+          mma_ss_x4_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + 2 * h).a, bar2);
         }
       };
       Pos cur{0, 0, 0u, 0u, 0u};
@@ -376,8 +371,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         mbar_wait(kv_full + 0, 0, abort_s, a.status, DEV_TIMEOUT_TMA);
         tc_fence_after();
         const uint32_t ka = (kv_lo + 0) | kLoLbo, qb = in_lo | kLoLbo;
-#pragma unroll
-        for (int sub = 0; sub < kSub; ++sub) { issue_in(cur, ka, qb, 0, sub); issue_in(cur, ka, qb, 1, sub); }
+        issue_in(cur, ka, qb, 0);
+        issue_in(cur, ka, qb, 1);
       }
       for (int n = 0; n < total_steps; ++n) {
         const Pos nxt = after(cur);
@@ -393,27 +388,19 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         const uint32_t qb = (in_lo + nxt.stg * (L::kStage >> 4)) | kLoLbo;
         const uint32_t st_full_bar = (st_full + (int)nxt.stg).a, kv_full_bar = (kv_full + nxt.g).a;
 #pragma unroll
-        for (int sub = 0; sub < kSub; ++sub) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            mbar_wait(cdone + (2 * h + sub), n & 1, abort_s, a.status, DEV_TIMEOUT_SYNC);
-            // (an item's first MMA of row g overwrites an accumulator that all warps of half 0 drain first)
-            if (kSub == 2 && h == 0 && sub == 0 && cur.it == 0) mbar_wait(cdone + 1, n & 1, abort_s, a.status, DEV_TIMEOUT_SYNC);
-            tc_fence_after();
-            const uint32_t tA = tmem + (h ? col_in1 : col_in0) + sub * QB;
-            const uint32_t ba = ob + (4 * h + (4 / kSub) * sub) * kRowBlk;
-            const uint32_t first = (h == 0 && sub == 0) ? first0 : 1u;
-            if constexpr (kSub == 1) mma_ts_x4(acc, tA, ba, kHiOp, kRowBlk, kIdescOut, first);
-            else mma_ts_x2(acc, tA, ba, kHiOp, kRowBlk, kIdescOut, first);
-            if (h == 1 && sub == kSub - 1) mma_commit_if_s(1u, st_empty_bar);
-            if (more) {
-              if (h == 0 && sub == 0) {
-                mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, a.status, DEV_TIMEOUT_TMA);
-                if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, a.status, DEV_TIMEOUT_TMA);
-                tc_fence_after();
-              }
-              issue_in(nxt, ka, qb, h, sub);
+        for (int h = 0; h < 2; ++h) {
+          mbar_wait(cdone + 2 * h, n & 1, abort_s, a.status, DEV_TIMEOUT_SYNC);
+          tc_fence_after();
+          const uint32_t tA = tmem + (h ? col_in1 : col_in0);
+          mma_ts_x4(acc, tA, ob + 4 * h * kRowBlk, kHiOp, kRowBlk, kIdescOut, h == 0 ? first0 : 1u);
+          if (h == 1) mma_commit_if_s(1u, st_empty_bar);
+          if (more) {
+            if (h == 0) {
+              mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, a.status, DEV_TIMEOUT_TMA);
+              if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, a.status, DEV_TIMEOUT_TMA);
+              tc_fence_after();
             }
+            issue_in(nxt, ka, qb, h);
           }
         }
         cur = nxt;
@@ -629,7 +616,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       for (int sub = 0; sub < 2; ++sub) {
         // this warp's queries of the half: 32*cb2 + 16*sub .. +16
         if (sub == 0) {
-          mbar_wait(sd_full + (2 * H + (kSub == 2 ? cb2 : 0)), n & 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+          mbar_wait(sd_full + 2 * H, n & 1, abort_s, a.status, DEV_TIMEOUT_MMA);
           tc_fence_after();
         }
         uint32_t sr[16], dr[16];
@@ -693,7 +680,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(cdone + (2 * H + (kSub == 2 ? cb2 : 0)));
+          if (lane == 0) mbar_arrive(cdone + 2 * H);
         }
         if (flush_dbias && last_of_group) {
           // The group's last row: this thread's 16 d_bias values of the chunk (one key, 16 queries) go
