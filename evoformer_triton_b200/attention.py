@@ -279,7 +279,7 @@ def pair_bias_grad_summed_over(group, peer_reducer=None):
 class _EvoformerAttentionBase(torch.autograd.Function):
     """What the public classes share.  A call goes to the native boundary (csrc/host.cpp); inside
     :func:`pair_bias_grad_summed_over` it is this Function itself, whose backward sums d(pair_bias)
-    over the ranks.  ``layout`` (how heads are found in Q/K/V) and ``bias_layout``
+    over the ranks, and so it is where a tracer wants one node (:func:`_python_boundary`).  ``layout`` (how heads are found in Q/K/V) and ``bias_layout``
     (``"b1hrr"``: the reference's ``[B, 1, H, R, R]``; ``"brrh"``: ``[B, R, R, H]`` as a linear
     layer emits it) are fixed by the public subclasses."""
 
@@ -293,9 +293,13 @@ class _EvoformerAttentionBase(torch.autograd.Function):
     @classmethod
     def _call(cls, Q, K, V, res_mask, pair_bias, *gate):
         if getattr(_pending, "group", None) is not None:
-            return super().apply(Q, K, V, res_mask, pair_bias, *gate)
+            return cls._function(Q, K, V, res_mask, pair_bias, *gate)
         return _lib.host().attention(Q, K, V, res_mask, pair_bias, gate[0] if gate else None,
                                      cls.layout == "true", cls.bias_layout == "brrh")
+
+    @classmethod
+    def _function(cls, *args):
+        return super().apply(*args)
 
     @classmethod
     def _forward(cls, ctx, Q, K, V, res_mask, pair_bias, gate=None):
@@ -312,7 +316,8 @@ class _EvoformerAttentionBase(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, mask, bias, o, lse, g)  # evoformer.py:729
         ctx.softmax_scale = scale
         ctx.bias_meta = None if pair_bias is None else (pair_bias.dtype, tuple(pair_bias.shape))
-        ctx.reduce_group = _pending.group
+        ctx.mask_meta = None if res_mask is None else (res_mask.dtype, tuple(res_mask.shape))
+        ctx.reduce_group = getattr(_pending, "group", None)
         return _unview(o, cls.layout)
 
     @classmethod
@@ -324,22 +329,25 @@ class _EvoformerAttentionBase(torch.autograd.Function):
         if d_o.dtype != q.dtype:
             d_o = d_o.to(q.dtype)
         want_dbias = bias is not None and ctx.needs_input_grad[4]
-        if mask is not None and mask.is_floating_point() and ctx.needs_input_grad[3]:
+        want_dmask = mask is not None and mask.is_floating_point() and ctx.needs_input_grad[3]
+        if want_dmask and ctx.reduce_group is not None:
             raise RuntimeError("a mask gradient is not available in the N_seq-sharded op (the mask rows are sharded)")
-        reducer = ctx.reduce_group[1] if want_dbias else None
+        reducer = ctx.reduce_group[1] if want_dbias and ctx.reduce_group is not None else None
         dbias_out = reducer.buffer(bias.numel()) if reducer is not None else None
         # (with a peer reducer the call sums d(pair_bias) over the ranks itself, next to its last kernel)
         res = attention_backward(q, k, v, o, lse, mask, bias, ctx.softmax_scale, d_o, want_dbias=want_dbias,
-                                 dbias_out=dbias_out, gate=g,
+                                 dbias_out=dbias_out, gate=g, want_dmask=want_dmask,
                                  exchange=None if reducer is None else reducer.exchange_params(bias.numel()))
         dq, dk, dv, dbias = res[:4]
-        dgate = res[4] if len(res) > 4 else None
+        dgate, dmask = res[4:] if len(res) > 4 else (None, None)
+        if dmask is not None:
+            dtype, shape = ctx.mask_meta
+            dmask = dmask.reshape(shape).to(dtype)
         d_pair_bias = None
         if dbias is not None:
             dtype, shape = ctx.bias_meta
-            if reducer is not None:  # N_seq is sharded: the other ranks' rows belong to the sum
-                pass                 # (summed inside the backward call)
-            else:
+            # N_seq is sharded: the other ranks' rows belong to the sum (with a reducer it was taken in the call)
+            if ctx.reduce_group is not None and reducer is None:
                 import torch.distributed as dist
                 dist.all_reduce(dbias, op=dist.ReduceOp.SUM, group=ctx.reduce_group[0])
             # the sum over N_seq stays in fp32 until this single cast (evoformer.py:860 casts to dO's dtype)
@@ -349,7 +357,7 @@ class _EvoformerAttentionBase(torch.autograd.Function):
                 d_pair_bias = dbias.reshape(shape).to(dtype)
                 if reducer is not None and d_pair_bias.data_ptr() == dbias.data_ptr():
                     d_pair_bias = d_pair_bias.clone()  # the exchange buffer is reused by the next call
-        grads = (_unview(dq, cls.layout), _unview(dk, cls.layout), _unview(dv, cls.layout), None, d_pair_bias)
+        grads = (_unview(dq, cls.layout), _unview(dk, cls.layout), _unview(dv, cls.layout), dmask, d_pair_bias)
         if g is not None:
             grads = grads + (_unview(dgate, cls.layout),)
         return grads
@@ -418,6 +426,9 @@ def _variant(layout: str, bias_layout: str, gated: bool):
     key = (layout, bias_layout, gated)
     fn = _VARIANTS.get(key)
     if fn is None:
+        def apply(cls, Q, K, V, res_mask=None, pair_bias=None, gate=None):  # (what a traced node calls)
+            return cls._call(Q, K, V, res_mask, pair_bias, gate)
+
         def forward(ctx, Q, K, V, res_mask=None, pair_bias=None, gate=None):
             return fn._forward(ctx, Q, K, V, res_mask, pair_bias, gate)
 
@@ -426,13 +437,19 @@ def _variant(layout: str, bias_layout: str, gated: bool):
             return grads if len(grads) == 6 else grads + (None,)
 
         fn = type(f"EvoformerAttention_{layout}_{bias_layout}{'_gated' if gated else ''}", (_EvoformerAttentionBase,),
-                  {"layout": layout, "bias_layout": bias_layout,
+                  {"layout": layout, "bias_layout": bias_layout, "apply": classmethod(apply),
                    "forward": staticmethod(forward), "backward": staticmethod(backward)})
         _VARIANTS[key] = fn
     return fn
 
 
 _VARIANTS = {}
+
+
+def _python_boundary(Q, K, V, res_mask, pair_bias, gate, true_layout, heads_last):
+    """A call as a Python autograd.Function: what ``torch.jit.trace`` records as one node that runs the op."""
+    fn = _variant("true" if true_layout else "reinterpret", "brrh" if heads_last else "b1hrr", gate is not None)
+    return fn._function(Q, K, V, res_mask, pair_bias, gate)
 
 
 def evoformer_attention(Q, K, V, biases: Optional[Sequence[Optional[torch.Tensor]]] = None, *, layout="true",

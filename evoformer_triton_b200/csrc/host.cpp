@@ -7,10 +7,11 @@
 //
 // Same semantics as the Python boundary (dsevoformer-triton/evoformer.py:633-862): the reinterpreting
 // head layout or the true one, None for mask and bias, additive or boolean masks, gating, both bias
-// layouts.  The N_seq-sharded op, which exchanges d(pair_bias) in its backward, stays in Python and takes
-// its checks and the preparation of its inputs from here.
+// layouts.  The N_seq-sharded op, which exchanges d(pair_bias) in its backward, and a call that is being
+// traced stay in Python and take their checks and the preparation of their inputs from here.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -284,11 +285,14 @@ struct Attention : public torch::autograd::Function<Attention> {
 
 Tensor attention(const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask, const Maybe& bias, const Maybe& gate,
                  bool true_layout, bool heads_last) {
+  // A tracer would record this call as the allocation of its result; it takes the Python Function as one node.
+  if (torch::jit::tracer::isTracing())
+    return py::module_::import("evoformer_triton_b200.attention").attr("_python_boundary")(Q, K, V, mask, bias, gate, true_layout, heads_last).cast<Tensor>();
   check_call(Q, K, V, mask, bias, gate);
   return Attention::apply(Q, K, V, mask, bias, gate, true_layout, heads_last);
 }
 
-// What the Python boundary of the N_seq-sharded op hands to the C ABI: the checks and the preparation are these.
+// What the Python boundary hands to the C ABI: the checks and the preparation are these.
 std::vector<Tensor> prepare_call(const Tensor& Q, const Tensor& K, const Tensor& V, const Maybe& mask, const Maybe& bias,
                                  const Maybe& gate, bool true_layout, bool heads_last) {
   check_call(Q, K, V, mask, bias, gate);

@@ -137,3 +137,31 @@ def test_sharded_boundary_matches_the_native_one(cfg, group_of_one):
             assert a.shape == b.shape and oc.rel_err(a, b) < 4e-3, i
         else:
             assert torch.equal(a, b), i
+
+
+@pytest.mark.parametrize("entry", ["apply", "list"])
+def test_traced_call_runs_the_op(entry):
+    """torch.jit.trace records the op itself, not the allocation of its result: the traced call on other inputs
+    gives what the op gives, and its gradients (the additive mask's among them)."""
+    import evoformer_triton_b200 as evo
+    g = torch.Generator(device=DEV).manual_seed(4)
+    B, S, R, H, D = 1, 3, 77, 2, 32
+    draw = lambda *shape: torch.randn(shape, generator=g, device=DEV)  # noqa: E731
+
+    def inputs():
+        q, k, v, gate = (draw(B, S, R, H, D).bfloat16().requires_grad_() for _ in range(4))
+        mask, bias = draw(B, S, 1, 1, R).requires_grad_(), draw(B, 1, H, R, R).requires_grad_()
+        return (q, k, v, mask, bias) + ((gate,) if entry == "list" else ())
+
+    def op(q, k, v, mask, bias, gate=None):
+        if entry == "apply":
+            return evo.EvoformerAttention.apply(q, k, v, mask, bias)
+        return evo.evoformer_attention(q, k, v, [mask, bias], gate=gate)
+
+    x, y = inputs(), inputs()
+    traced = torch.jit.trace(op, x, check_trace=False)
+    d_o = draw(B, S, R, H, D).bfloat16()
+    got, want = traced(*y), op(*y)
+    assert torch.equal(got, want)
+    for a, b in zip(torch.autograd.grad(got, y, d_o), torch.autograd.grad(want, y, d_o)):
+        assert a.dtype == b.dtype and a.shape == b.shape and oc.rel_err(a, b) < 1e-3  # (sums in no fixed order)
