@@ -342,24 +342,40 @@ def main():
     op_peak_mem = torch.cuda.max_memory_allocated(dev) - mem_before
     zero_grads()
 
-    # ---- per-kernel split (forward kernel, backward call), same flush discipline
+    # ---- split of the step (forward kernel, backward call), same flush discipline; each is a graph of its
+    # own, because launched from Python a call this short takes the host longer than the device
     with torch.no_grad():
         qv, kv, vv, dov = (attention._view_dims(t.detach(), "reinterpret") for t in (Q, K, V, dO))
         mk = mask.reshape(w.B, w.S, w.R)
         bs = bias.detach().reshape(w.B, w.H, w.R, w.R)
+        o, lse = attention.attention_forward(qv, kv, vv, mk, bs, w.D ** -0.5)
+
+        def forward():
+            return attention.attention_forward(qv, kv, vv, mk, bs, w.D ** -0.5)
+
+        def backward():
+            return attention.attention_backward(qv, kv, vv, o, lse, mk, bs, w.D ** -0.5, dov)
+
+        forward_graph = backward_graph = None
+        if graph is not None:
+            forward_graph, backward_graph = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+            with torch.cuda.graph(forward_graph):
+                forward()
+            with torch.cuda.graph(backward_graph):
+                backward()
+            forward, backward = forward_graph.replay, backward_graph.replay
         f_ms, b_ms = [], []
         for i in range(3 + 10):
-            flush.zero_()
-            e0, e1, e2 = ev(), ev(), ev()
-            e0.record()
-            o, lse = attention.attention_forward(qv, kv, vv, mk, bs, w.D ** -0.5)
-            e1.record()
-            attention.attention_backward(qv, kv, vv, o, lse, mk, bs, w.D ** -0.5, dov)
-            e2.record()
-            torch.cuda.synchronize()
-            if i >= 3:
-                f_ms.append(e0.elapsed_time(e1))
-                b_ms.append(e1.elapsed_time(e2))
+            for call, times in ((forward, f_ms), (backward, b_ms)):
+                flush.zero_()
+                e0, e1 = ev(), ev()
+                e0.record()
+                call()
+                e1.record()
+                torch.cuda.synchronize()
+                if i >= 3:
+                    times.append(e0.elapsed_time(e1))
+        forward = backward = forward_graph = backward_graph = None
         fwd_ms, bwd_ms = statistics.mean(f_ms), statistics.mean(b_ms)
         bwd_launches = attention.launches["bwd"]
     peaks = measured_peaks()
