@@ -50,7 +50,8 @@ _force_generic = False
 
 
 def force_generic(on: bool) -> None:
-    """Route every call to the CUDA-core kernels (used by tests to cross-check)."""
+    """Route every call to the CUDA-core kernels: slower, with P and dS of 16-bit calls in fp32 where the tensor
+    cores take them in the storage type (errors about 1.4 times smaller)."""
     global _force_generic
     _force_generic = bool(on)
     _lib.host().force_generic(_force_generic)

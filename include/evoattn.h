@@ -62,7 +62,8 @@ enum {
 
 /* flags */
 enum {
-  EVOATTN_FLAG_FORCE_GENERIC = 1 /* use the CUDA-core kernels even where a tcgen05 kernel exists */
+  EVOATTN_FLAG_FORCE_GENERIC = 1 /* use the CUDA-core kernels even where a tcgen05 kernel exists: slower, with
+                                    P and dS of 16-bit calls in fp32 instead of their storage type */
 };
 
 /* Which kernel family served the last call on this thread (for tests and logs). */
