@@ -84,8 +84,8 @@ struct Bar {
   uint32_t a;
 };
 __device__ __forceinline__ Bar operator+(Bar b, int i) { return Bar{b.a + 8u * static_cast<uint32_t>(i)}; }
-__device__ __forceinline__ bool mbar_wait(Bar b, uint32_t parity, uint32_t abort_s, int* status, int code) {
-  return mbar_wait_s(b.a, parity, abort_s, status, code);
+__device__ __forceinline__ void mbar_wait(Bar b, uint32_t parity, uint32_t abort_s, int code) {
+  mbar_wait_s(b.a, parity, abort_s, code);
 }
 __device__ __forceinline__ void mbar_arrive(Bar b) { mbar_arrive_s(b.a); }
 __device__ __forceinline__ void mbar_expect_tx(Bar b, uint32_t bytes) { mbar_expect_tx_s(b.a, bytes); }
@@ -367,13 +367,14 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       };
       Pos cur{0, 0, 0u, 0u, 0u};
       if (total_steps > 0) {
-        mbar_wait(st_full + 0, 0, abort_s, a.status, DEV_TIMEOUT_TMA);
-        mbar_wait(kv_full + 0, 0, abort_s, a.status, DEV_TIMEOUT_TMA);
+        mbar_wait(st_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
+        mbar_wait(kv_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
         tc_fence_after();
         const uint32_t ka = (kv_lo + 0) | kLoLbo, qb = in_lo | kLoLbo;
         issue_in(cur, ka, qb, 0);
         issue_in(cur, ka, qb, 1);
       }
+#pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const Pos nxt = after(cur);
         const bool more = n + 1 < total_steps;
@@ -389,15 +390,15 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         const uint32_t st_full_bar = (st_full + (int)nxt.stg).a, kv_full_bar = (kv_full + nxt.g).a;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          mbar_wait(cdone + 2 * h, n & 1, abort_s, a.status, DEV_TIMEOUT_SYNC);
+          mbar_wait(cdone + 2 * h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
           tc_fence_after();
           const uint32_t tA = tmem + (h ? col_in1 : col_in0);
           mma_ts_x4(acc, tA, ob + 4 * h * kRowBlk, kHiOp, kRowBlk, kIdescOut, h == 0 ? first0 : 1u);
           if (h == 1) mma_commit_if_s(1u, st_empty_bar);
           if (more) {
             if (h == 0) {
-              mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, a.status, DEV_TIMEOUT_TMA);
-              if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, a.status, DEV_TIMEOUT_TMA);
+              mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
+              if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, DEV_TIMEOUT_TMA);
               tc_fence_after();
             }
             issue_in(nxt, ka, qb, h);
@@ -427,15 +428,16 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const int tiles = my_items * NT;
       if (has_bias && tiles > 0) { const StepT d0 = decode(0); load_bias(d0, 0); load_bias(d0, 1); }
       int g = 0, it = 0, t = 0;  // row of the group, query tile, running (item, query tile) index
+#pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const bool turn = has_bias && g == G - 1 && t + 1 < tiles;  // the group's last step: the halves come back
         StepT nb = StepT{0, 0, 0, 0, 0, 0};
         if (turn) nb = decode((t + 1) * G);  // (divisions: before the waits, not between them)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          mbar_wait(sdone + h, n & 1, abort_s, a.status, DEV_TIMEOUT_SYNC);
+          mbar_wait(sdone + h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
           if (turn) {
-            mbar_wait(b_done + h, t & 1, abort_s, a.status, DEV_TIMEOUT_SYNC);
+            mbar_wait(b_done + h, t & 1, abort_s, DEV_TIMEOUT_SYNC);
             load_bias(nb, h);
           }
         }
@@ -455,11 +457,12 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       // have completed; Q, dO and the two statistics vectors of a step ride a two-deep ring.
       const uint32_t sKV_s = smem_u32(sKV), sStage_s = smem_u32(sStage);
       StepT d = decode(0);
+#pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const int stg = n % kStages;
         if (d.it == 0) {
           const int k = n / SPI;
-          mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+          mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
           if (lane == 0) {
             const uint32_t dst = sKV_s + (2 * d.g) * L::kTile;
             mbar_expect_tx(kv_full + d.g, 2 * L::kTile);
@@ -468,7 +471,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           }
           __syncwarp();
         }
-        mbar_wait(st_empty + stg, ((n / kStages) & 1) ^ 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+        mbar_wait(st_empty + stg, ((n / kStages) & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
         if (lane == 0) {
           const uint32_t dst = sStage_s + stg * L::kStage;
           const uint32_t bar = (st_full + stg).a;
@@ -570,7 +573,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     constexpr int QC = DP / 4;       // dQ columns per warp (4, 8 or 16)
     const int colblk = 2 * H + cb2;  // which of the four column blocks this warp drains
     auto send_dq = [&](int m, const StepT& d) {
-      mbar_wait(dq_full + (m & 1), (m >> 1) & 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+      mbar_wait(dq_full + (m & 1), (m >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
       uint32_t qr[QC];
       tmem_ld<QC>(t_lane + colDQ + (m & 1) * DP + colblk * QC, qr);
@@ -595,6 +598,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 #pragma unroll
     for (int e = 0; e < 16; ++e) bacc[e] = f2_make(0.f, 0.f);
 
+#pragma unroll 1
     for (int n = 0; n < total_steps; ++n) {
       const StepT nxt = advance(cur, n + 1);
       const bool more = n + 1 < total_steps;
@@ -606,8 +610,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const uint32_t vec_s = sStage_s + stg * L::kStage + 2 * L::kTile;
       const bool last_of_group = (g == G - 1);
       // the statistics vectors of this step are read with ordinary loads: observe their arrival here
-      mbar_wait(st_full + stg, (n / kStages) & 1, abort_s, a.status, DEV_TIMEOUT_TMA);
-      if (has_bias && g == 0) mbar_wait(b_full + H, (n / G) & 1, abort_s, a.status, DEV_TIMEOUT_TMA);
+      mbar_wait(st_full + stg, (n / kStages) & 1, abort_s, DEV_TIMEOUT_TMA);
+      if (has_bias && g == 0) mbar_wait(b_full + H, (n / G) & 1, abort_s, DEV_TIMEOUT_TMA);
       // a row whose keys are all dropped has nl = +inf for every query (the mask row is shared by
       // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
       const bool deadstep = (lds_f32(vec_s) == kInf);
@@ -616,7 +620,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       for (int sub = 0; sub < 2; ++sub) {
         // this warp's queries of the half: 32*cb2 + 16*sub .. +16
         if (sub == 0) {
-          mbar_wait(sd_full + 2 * H, n & 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+          mbar_wait(sd_full + 2 * H, n & 1, abort_s, DEV_TIMEOUT_MMA);
           tc_fence_after();
         }
         uint32_t sr[16], dr[16];
@@ -705,7 +709,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       }
       // dS^T -> shared memory, [key][query] rows of 128 bytes per half, 128-byte swizzle; the tile is
       // free once the dQ MMAs of the previous step have read it
-      mbar_wait(ds_empty, (n & 1) ^ 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+      mbar_wait(ds_empty, (n & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
 #pragma unroll
       for (int c = 0; c < 4; ++c)  // dk[4 * c ..]: queries 32 * cb2 + 8 * c .. of this half
         sts_v4(drow + (((4 * cb2 + c) ^ (jrow & 7)) << 4), dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
@@ -726,7 +730,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       if (H == 0) {
         // every dV / dK MMA of this CTA has completed once the last step's tile stage has been released
         const int last = total_steps - 1;
-        mbar_wait(st_empty + (last % kStages), (last / kStages) & 1, abort_s, a.status, DEV_TIMEOUT_MMA);
+        mbar_wait(st_empty + (last % kStages), (last / kStages) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
         for (int g = 0; g < G; ++g) drain_dkdv(pb, ph, ps0 + g, pj0, g);
       }
@@ -734,10 +738,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     if (lane == 0) tma_wait_group0();  // this warp's reductions have completed before the CTA may exit
   }
 
-  if (*abort_flag) {
-    const long long t0 = clock64();
-    while (clock64() - t0 < 200000) {}
-  }
+  if (*abort_flag) report_abort(*abort_flag, a.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);

@@ -5,27 +5,36 @@
 // (_attn_fwd) compute:  O = softmax(scale*Q K^T + bias, masked) V  and the row
 // log-sum-exp, without ever writing the R x R scores to memory.
 //
-// Persistent, warp-specialised kernel, one CTA per SM, 384 threads:
+// Persistent, warp-specialised kernel, one CTA per SM, NW = 2, 3 or 4 softmax warpgroups:
 //   warp 0      TMA producer: Q tiles, K/V tiles (64 keys each) and pair-bias tiles
-//   warp 1, 2   issue the tcgen05.mma of warpgroup A, B
+//   warp 1, 2   issue the tcgen05.mma of half of the warpgroups each
 //   warp 3      stages the residue-mask rows of the next item in shared memory
-//   warps 4-7   softmax warpgroup A        warps 8-11   softmax warpgroup B
-// A work item is one 128-row query tile of TWO consecutive MSA rows s of one (b,h):
-// warpgroup A takes row 2p, B takes row 2p+1.  Both rows use the same pair-bias tile, so
-// it is staged in shared memory once per item pair.  Inside a warpgroup thread t owns
-// score row t (= TMEM lane t) and all 64 columns of the current key tile, so the row
-// maximum and sum need no exchange between threads.
+//   warps 4..   softmax warpgroups
+// A work item is one 128-row query tile of NW consecutive MSA rows s of one (b,h), one row for each
+// warpgroup.  All of them use the same pair-bias tile, which is staged in shared memory once.  Inside a
+// warpgroup thread t owns score row t (= TMEM lane t) and all 64 columns of the current key tile, so the row
+// sum needs no exchange between threads.
 //
 // With a single MSA row (N_seq = 1, the shape of the reference's own benchmark sweep) there is no
 // second row to pair: the kernel is then instantiated in query-pair mode, where an item is two
-// consecutive query tiles of the same row, the warpgroups share one K/V ring and each has its own
+// consecutive query tiles of the same row, the warpgroups share the K/V tiles and each has its own
 // pair-bias tile in a stage.
 //
-// Per warpgroup and key tile n:  S_n = Q K_n^T lands in TMEM (double buffered); the
-// warpgroup turns it into P_n (rounded to the storage type as evoformer.py:84 does) and
-// writes it back over S_n in TMEM, from where it feeds the P V MMA as the A operand;
-// O accumulates in TMEM over the item.  The MMA warp runs S_{n+1} while the warpgroup is busy with
-// tile n.
+// Per warpgroup and key tile n:  S_n = Q K_n^T lands in TMEM; the warpgroup turns it into P_n (rounded to
+// the storage type as evoformer.py:84 does) and writes it back over S_n in TMEM, from where it feeds the P V
+// MMA as the A operand; O accumulates in TMEM over the item.  With two warpgroups S is double buffered; with
+// three or four (168 to 112 registers a thread) it is not, and the other warpgroups hide the hand-over.
+//
+// The exponentials of a tile do not wait for its maximum: they are taken against the running maximum m of the
+// tiles before (of the first tile, its own), straight from the scores: load, two FMAs, ex2, row sum, pack.  Only
+// if a row's sum of the tile shows that some exp2(x - m) may exceed 2^8 (its sum does) is the tile's maximum
+// taken, m and O follow it where it has grown by more than that, and the tile is done again.  So the maximum
+// pass costs one tile in T_TILES instead of every one, and no score is held in a register.
+//
+// Bound by the issue slots and hand-overs around the exponentials (16 a cycle and SM: [1,256,1024,4,32] would
+// take 236 us).  That shape takes 379 us with four warpgroups, and 540 with the form before, which had the
+// maximum in line, two warpgroups taking turns, one TMA copy per row and MMAs issued from a single-lane branch;
+// [1,128,384,8,32] 97 -> 77, [1,1024,384,8,8] fp16 703 -> 507, [1,128,768,8,64] 349 -> 309 us.
 #include <type_traits>
 
 #include "common.cuh"
@@ -40,109 +49,126 @@ using namespace ptx;
 
 constexpr int BM = 128;  // query rows per warpgroup tile
 constexpr int BN = 64;   // keys per tile
-constexpr int kThreads = 384;
 constexpr int kTmemCols = 512;
+constexpr size_t kMaxSmem = 232448;  // of one CTA
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kMaxSum = 256.f;       // sum of a tile's exponentials above which one of them may exceed 2^8
 constexpr float kGrow = 8.f / kLog2e;  // how far a tile's maximum may exceed the running one
 constexpr int MASK_MIN = 0;  // boolean keep-mask (or none): score = min(score, m), m = +-FLT_MAX
 constexpr int MASK_ADD = 1;  // additive mask
 constexpr int BIAS_NONE = 0, BIAS_F32 = 1, BIAS_16 = 2;
 
-template <int DP, bool QP>
+// NW softmax warpgroups per CTA, each with a query tile of one MSA row at a time.  QP: query-pair mode.
+template <int DP, int NW, bool QP, int BIAS>
 struct Cfg {
+  static_assert(!QP || NW == 2, "query-pair mode has two warpgroups");
   static constexpr int RB = DP * 2;                    // bytes per staged row
-  static constexpr int QST = (DP == 64) ? 1 : 2;       // Q stages per warpgroup
-  static constexpr int NKV = (DP == 64) ? 2 : 4;       // K and V ring depth per warpgroup
-  static constexpr int BST = 2;                        // pair-bias stages (shared by both warpgroups)
-  static constexpr int KVW = QP ? 1 : 2;               // K/V rings: one per warpgroup, or one shared (query-pair mode)
-  static constexpr int BTL = QP ? 2 : 1;               // pair-bias tiles per stage: one shared, or one per warpgroup
+  static constexpr int QST = (DP == 64 || NW > 2) ? 1 : 2;  // Q stages
+  static constexpr int SB = NW > 2 ? 1 : 2;            // score buffers per warpgroup
+  static constexpr int NK = DP == 64 && NW > 2 ? 1 : SB + 1;  // K stages (S is through with one early in a tile)
+  static constexpr int NV = (DP == 64 || NW > 2) ? 2 : 3;  // stages of V and the pair bias
+  static constexpr int KVR = QP ? 1 : NW;              // rows of K and V in a stage: one per warpgroup, or one shared
+  static constexpr int BTL = QP ? 2 : 1;               // pair-bias tiles in a stage: one shared, or one per warpgroup
+  static constexpr int kThreads = 128 + 128 * NW;
+  static constexpr int kServiceRegs = NW == 2 ? 40 : NW == 3 ? 56 : 32, kSoftmaxRegs = NW == 2 ? 232 : NW == 3 ? 152 : 112;
   static constexpr int kQ = BM * RB;
   static constexpr int kKV = BN * RB;
-  static constexpr int kBias = BM * BN * 4;            // 32 KB = two 128x32 fp32 boxes
+  static constexpr int kBias = BIAS == BIAS_NONE ? 0 : BM * BN * (BIAS == BIAS_16 ? 2 : 4);  // one tile; fp32: two 128x32 boxes
+  static constexpr int kVB = KVR * kKV + BTL * kBias;  // a stage: V, then the bias
+  static constexpr int kOnes = 16 * RB;                // 16 keys by DP columns of ones
   static constexpr int offQ = 0;
-  static constexpr int offK = offQ + 2 * QST * kQ;
-  static constexpr int offV = offK + KVW * NKV * kKV;
-  static constexpr int offB = offV + KVW * NKV * kKV;
-  static constexpr int offMask = offB + BST * BTL * kBias;
-  static constexpr int kNumBars = 2 * (2 * QST + 4 * NKV + 2 + 2 + 2 + 4) + 2 * BST;
+  static constexpr int offK = offQ + NW * QST * kQ;
+  static constexpr int offV = offK + NK * KVR * kKV;
+  static constexpr int offOnes = offV + NV * kVB;
+  static constexpr int offMask = offOnes + (kOnes < 1024 ? 1024 : kOnes);
+  static constexpr int PER = 3 * SB + 4;               // barriers of a warpgroup
+  static constexpr int kNumBars = NW * PER + 2 * (QST + NK + NV);
   static size_t bytes(int r_pad) {
-    return (size_t)offMask + (size_t)4 * r_pad * 4 + 4 * 32 * 4 + kOnes + kNumBars * 8 + 64 + 1024;
+    return (size_t)offMask + (size_t)2 * NW * (r_pad * 4 + 4) + kNumBars * 8 + 64 + 1024;
   }
-  static constexpr int kOnes = 512;  // a 16 x 16 operand of ones
-  // TMEM columns of warpgroup w: S double buffer, then O, then the row sum of P (16 equal columns)
-  static constexpr int colL = 2 * BN + DP, tmemWg = colL + 16;
-  static_assert(2 * tmemWg <= kTmemCols, "TMEM budget");
+  // TMEM columns of a warpgroup: S buffers, then O, then the row sum of P (16 equal columns)
+  static constexpr int colO = SB * BN, colL = colO + DP, tmemWg = colL + 16;
+  static_assert(NW * tmemWg <= kTmemCols, "TMEM budget");
+  static_assert(offK % 1024 == 0 && offV % 1024 == 0 && kVB % 1024 == 0 && offOnes % 1024 == 0, "swizzled tiles");
 };
 
-// A work item: warpgroup w works on query tile qt[w] of MSA row s[w] of (b, h).  Row-pair mode: rows
-// 2p and 2p+1, the same query tile; query-pair mode: one row, query tiles 2p and 2p+1.
-struct Item {
-  int b, h, qt[2], s[2];
+// n / d by a multiplication, exact for n < 2^31: m = ceil(2^(31 + s) / d), s = ceil(log2 d).
+struct FastDiv {
+  uint32_t m, s, d;
 };
-template <bool QP>
-__device__ __forceinline__ Item decode_item(int idx, int n_inner, int n_outer, int H) {
+FastDiv fast_div(uint32_t d) {
+  uint32_t s = 0;
+  while ((1ull << s) < d) ++s;
+  return FastDiv{static_cast<uint32_t>(((1ull << (31 + s)) + d - 1) / d), 31 + s, d};
+}
+__device__ __forceinline__ uint32_t div_mod(uint32_t n, const FastDiv& f, uint32_t& rem) {
+  const uint32_t q = static_cast<uint32_t>((static_cast<unsigned long long>(n) * f.m) >> f.s);
+  rem = n - q * f.d;
+  return q;
+}
+// Work items (b, h, outer, inner), inner fastest.  Row mode: warpgroup w works on MSA row NW * inner + w,
+// query tile `outer`.  Query-pair mode: on row `inner`, query tile 2 * outer + w.
+struct Walk {
+  int n_items;
+  FastDiv inner, outer, heads;
+};
+struct Item {
+  uint32_t b, h, outer, inner;
+};
+__device__ __forceinline__ Item decode_item(int idx, const Walk& wk) {
   Item it;
-  const int inner = idx % n_inner; idx /= n_inner;   // row pair (row-pair mode) or row (query-pair mode)
-  const int outer = idx % n_outer; idx /= n_outer;   // query tile, or pair of query tiles
-  it.h = idx % H;
-  it.b = idx / H;
-  if (QP) {
-    it.s[0] = it.s[1] = inner;
-    it.qt[0] = 2 * outer; it.qt[1] = 2 * outer + 1;
-  } else {
-    it.s[0] = 2 * inner; it.s[1] = 2 * inner + 1;
-    it.qt[0] = it.qt[1] = outer;
-  }
+  uint32_t n = div_mod(static_cast<uint32_t>(idx), wk.inner, it.inner);
+  n = div_mod(n, wk.outer, it.outer);
+  it.b = div_mod(n, wk.heads, it.h);
   return it;
 }
 
-template <class T, int DP, int MASKMODE, int BIAS, bool QP>
-__global__ void __launch_bounds__(kThreads, 1)
-evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CUtensorMap tmQ,
+template <class T, int DP, int MASKMODE, int BIAS, int NW, bool QP>
+__global__ void __launch_bounds__(Cfg<DP, NW, QP, BIAS>::kThreads, 1)
+evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtensorMap tmQ,
                      const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                      const __grid_constant__ CUtensorMap tmB) {
-  using C = Cfg<DP, QP>;
-  constexpr int RB = C::RB, QST = C::QST, NKV = C::NKV, BST = C::BST;
+  using C = Cfg<DP, NW, QP, BIAS>;
+  constexpr int RB = C::RB, QST = C::QST, NK = C::NK, NV = C::NV, SB = C::SB;
   constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t smem_s = smem_u32(smem);
   const int T_TILES = (a.R + BN - 1) / BN;
   const int r_pad = T_TILES * BN;
   float* sMask = reinterpret_cast<float*>(smem + C::offMask);  // [warpgroup][stage][r_pad]
-  // one word per key tile of a staged mask row: non-zero if the tile has a key that the mask changes;
-  // R <= 2048
-  uint32_t* sDirty = reinterpret_cast<uint32_t*>(sMask + 4 * r_pad);  // [warpgroup][stage][32]
-  uint32_t* sOnes = sDirty + 4 * 32;  // 16 x 16 ones of the storage type
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sOnes + C::kOnes / 4);
-  // barrier layout: per warpgroup w a block of PER, then the shared bias barriers
-  constexpr int PER = 2 * QST + 4 * NKV + 2 + 2 + 2 + 4;
-  auto q_full = [&](int w, int st) { return bars + w * PER + st; };
-  auto q_empty = [&](int w, int st) { return bars + w * PER + QST + st; };
-  auto k_full = [&](int w, int st) { return bars + w * PER + 2 * QST + st; };
-  auto k_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + NKV + st; };
-  auto v_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 2 * NKV + st; };
-  auto v_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 3 * NKV + st; };
-  auto s_full = [&](int w, int i) { return bars + w * PER + 2 * QST + 4 * NKV + i; };
-  // Two of each for tiles in turn: the softmax warps may finish a tile while the issuer still waits for the
-  // V of the one before, and a single barrier that is two phases on looks the same as one that has not
-  // moved (a parity wait cannot tell).
-  auto p_full = [&](int w, uint32_t i) { return bars + w * PER + 2 * QST + 4 * NKV + 2 + i; };
-  auto o_full = [&](int w, uint32_t i) { return bars + w * PER + 2 * QST + 4 * NKV + 4 + i; };
-  auto m_full = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 6 + st; };
-  auto m_empty = [&](int w, int st) { return bars + w * PER + 2 * QST + 4 * NKV + 8 + st; };
-  auto b_full = [&](int st) { return bars + 2 * PER + st; };
-  auto b_empty = [&](int st) { return bars + 2 * PER + BST + st; };
+  // one bit per key tile of a staged mask row (R <= 2048): the tile has a key that the mask changes
+  uint32_t* sDirty = reinterpret_cast<uint32_t*>(sMask + 2 * NW * r_pad);  // [warpgroup][stage]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sDirty + 2 * NW);
+  const uint32_t bars_s = smem_u32(bars);
+  // barriers: a block of PER for each warpgroup, then those of the rings
+  // With two score buffers there are two of each of these for tiles in turn: the softmax warps may finish a
+  // tile while the issuer still waits for the V of the one before, and a single barrier that is two phases on
+  // looks the same as one that has not moved (a parity wait cannot tell).
+  auto s_full = [&](int w, uint32_t i) { return bars_s + 8 * (w * C::PER + i); };
+  auto p_full = [&](int w, uint32_t i) { return bars_s + 8 * (w * C::PER + SB + i); };
+  auto o_full = [&](int w, uint32_t i) { return bars_s + 8 * (w * C::PER + 2 * SB + i); };
+  auto m_full = [&](int w, int st) { return bars_s + 8 * (w * C::PER + 3 * SB + st); };
+  auto m_empty = [&](int w, int st) { return bars_s + 8 * (w * C::PER + 3 * SB + 2 + st); };
+  const uint32_t rings = bars_s + 8 * (NW * C::PER);
+  auto q_full = [&](uint32_t st) { return rings + 8 * st; };
+  auto q_empty = [&](uint32_t st) { return rings + 8 * (QST + st); };
+  auto k_full = [&](uint32_t st) { return rings + 8 * (2 * QST + st); };
+  auto k_empty = [&](uint32_t st) { return rings + 8 * (2 * QST + NK + st); };
+  auto v_full = [&](uint32_t st) { return rings + 8 * (2 * (QST + NK) + st); };  // V and the pair bias
+  auto v_empty = [&](uint32_t st) { return rings + 8 * (2 * (QST + NK) + NV + st); };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + C::kNumBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + C::kNumBars + 1);
-  volatile uint32_t* scratch = reinterpret_cast<volatile uint32_t*>(bars + C::kNumBars + 2);  // written, never read
+  const uint32_t abort_s = smem_u32(const_cast<int*>(abort_flag));
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
   const int NQT = (a.R + BM - 1) / BM;
-  // items: (b, h, outer, inner) with inner fastest
-  const int n_inner = QP ? a.S : (a.S + 1) / 2;
-  const int n_outer = QP ? (NQT + 1) / 2 : NQT;
+  // MSA row and query tile of warpgroup w (either may lie beyond the last one)
+  auto row_of = [&](const Item& it, int w) { return (int)it.inner * (QP ? 1 : NW) + (QP ? 0 : w); };
+  auto tile_of = [&](const Item& it, int w) { return (int)it.outer * (QP ? NW : 1) + (QP ? w : 0); };
   constexpr bool has_bias = BIAS != BIAS_NONE, BIAS16 = BIAS == BIAS_16;
 
   // A launch that follows a failed one returns at once (one reader, so the CTA agrees).
@@ -153,26 +179,27 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   if (*abort_flag) return;
 
   if (tid == 0) {
-    for (int w = 0; w < 2; ++w) {
-      for (int st = 0; st < QST; ++st) { mbar_init(q_full(w, st), 1); mbar_init(q_empty(w, st), 1); }
-      for (int st = 0; st < NKV; ++st) {  // (query-pair mode: both issuers release the one shared ring)
-        mbar_init(k_full(w, st), 1); mbar_init(k_empty(w, st), QP ? 2 : 1);
-        mbar_init(v_full(w, st), 1); mbar_init(v_empty(w, st), QP ? 2 : 1);
+#pragma unroll 1
+    for (int w = 0; w < NW; ++w) {
+      for (int i = 0; i < SB; ++i) {
+        mbar_init_s(s_full(w, i), has_bias && SB == 1 ? 2 : 1);  // the MMA, and the bias tile (below)
+        mbar_init_s(p_full(w, i), 4);  // one arrival per softmax warp
+        mbar_init_s(o_full(w, i), 1);
       }
-      mbar_init(s_full(w, 0), 1); mbar_init(s_full(w, 1), 1);
-      mbar_init(p_full(w, 0), 4); mbar_init(p_full(w, 1), 4);  // one arrival per softmax warp
-      mbar_init(o_full(w, 0), 1); mbar_init(o_full(w, 1), 1);
-      for (int st = 0; st < 2; ++st) { mbar_init(m_full(w, st), 1); mbar_init(m_empty(w, st), 4); }
+      for (int st = 0; st < 2; ++st) { mbar_init_s(m_full(w, st), 1); mbar_init_s(m_empty(w, st), 4); }
     }
-    for (int st = 0; st < BST; ++st) { mbar_init(b_full(st), 1); mbar_init(b_empty(st), 8); }
+    // (every warpgroup's issuer releases the stages that they share)
+    for (int st = 0; st < QST; ++st) { mbar_init_s(q_full(st), 1); mbar_init_s(q_empty(st), NW); }
+    for (int st = 0; st < NK; ++st) { mbar_init_s(k_full(st), 1); mbar_init_s(k_empty(st), NW); }
+    for (int st = 0; st < NV; ++st) { mbar_init_s(v_full(st), 1); mbar_init_s(v_empty(st), NW); }
     fence_mbar_init();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV);
     if (has_bias) prefetch_tmap(&tmB);
   }
-  if (tid < C::kOnes / 4) {
-    sOnes[tid] = Pack2<T>::pack(1.f, 1.f);
-    fence_async_shared();
-  }
+  if (tid < C::kOnes / 4) reinterpret_cast<uint32_t*>(smem + C::offOnes)[tid] = Pack2<T>::pack(1.f, 1.f);
+  if (C::kOnes / 4 > C::kThreads && tid + C::kThreads < C::kOnes / 4)
+    reinterpret_cast<uint32_t*>(smem + C::offOnes)[tid + C::kThreads] = Pack2<T>::pack(1.f, 1.f);
+  fence_async_shared();
   if (warp == 0) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -180,110 +207,141 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp < 4) {
-    setmaxnreg_dec<40>();
-    if (warp == 0 && lane == 0) {
+    setmaxnreg_dec<C::kServiceRegs>();
+    if (warp == 0) {
       // =============================== TMA producer ===============================
-      uint32_t qn[2] = {0, 0}, gt = 0;
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-        const Item it = decode_item<QP>(item, n_inner, n_outer, a.H);
-        int srow[2];
-        srow[0] = min(it.s[0], a.S - 1);
-        srow[1] = min(it.s[1], a.S - 1);
-        for (int w = 0; w < 2; ++w) {  // (a query tile beyond the last one loads as zeros)
-          const int st = qn[w] % QST;
-          mbar_wait(q_empty(w, st), ((qn[w] / QST) & 1) ^ 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
-          mbar_expect_tx(q_full(w, st), C::kQ);
-          tma_load_5d(smem + C::offQ + (w * QST + st) * C::kQ, &tmQ, q_full(w, st), 0, it.qt[w] * BM, srow[w], it.h, it.b);
-          ++qn[w];
+      // Few copies per tile (K, V of all rows and the bias: three or four), since issuing one, with its wait,
+      // costs hundreds of cycles: with a copy per row this warp set the pace of the kernel.
+      uint32_t n_item = 0, kt = 0, kp = 1, vt = 0, vp = 1;  // items; stage and parity of the rings
+#pragma unroll 1
+      for (int item = blockIdx.x; item < wk.n_items; item += gridDim.x, ++n_item) {
+        const Item it = decode_item(item, wk);
+        const int s0 = row_of(it, 0), i0 = tile_of(it, 0) * BM;  // (rows and query tiles beyond the last load as zeros)
+        const uint32_t qs = n_item % QST;
+        mbar_wait_s(q_empty(qs), ((n_item / QST) & 1) ^ 1, abort_s, DEV_TIMEOUT_SYNC);
+        if (elect_one()) {
+          mbar_expect_tx_s(q_full(qs), NW * C::kQ);
+          tma_load_5d_s(smem_s + C::offQ + qs * (NW * C::kQ), &tmQ, q_full(qs), 0, i0, s0, it.h, it.b);
         }
-        for (int t = 0; t < T_TILES; ++t, ++gt) {
-          const int st = gt % NKV;
-          const uint32_t par = ((gt / NKV) & 1) ^ 1;
-          for (int w = 0; w < C::KVW; ++w) {
-            mbar_wait(k_empty(w, st), par, abort_flag, a.status, DEV_TIMEOUT_SYNC);
-            mbar_expect_tx(k_full(w, st), C::kKV);
-            tma_load_5d(smem + C::offK + (w * NKV + st) * C::kKV, &tmK, k_full(w, st), 0, t * BN, srow[w], it.h, it.b);
+        __syncwarp();
+#pragma unroll 1
+        for (int j0 = 0; j0 < r_pad; j0 += BN) {
+          mbar_wait_s(k_empty(kt), kp, abort_s, DEV_TIMEOUT_SYNC);
+          if (elect_one()) {
+            mbar_expect_tx_s(k_full(kt), C::KVR * C::kKV);
+            tma_load_5d_s(smem_s + C::offK + kt * (C::KVR * C::kKV), &tmK, k_full(kt), 0, j0, s0, it.h, it.b);
           }
-          if (has_bias) {
-            const int bs = gt % BST;
-            mbar_wait(b_empty(bs), ((gt / BST) & 1) ^ 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
-            mbar_expect_tx(b_full(bs), C::BTL * (BIAS16 ? C::kBias / 2 : C::kBias));
-            for (int u = 0; u < C::BTL; ++u) {  // one tile for both warpgroups, or one each
-              uint8_t* dst = smem + C::offB + (bs * C::BTL + u) * C::kBias;
-              if constexpr (BIAS16) {  // one box of 128 rows x 64 16-bit values (rows of 128 bytes)
-                tma_load_4d(dst, &tmB, b_full(bs), t * BN, it.qt[u] * BM, it.h, it.b);
-              } else {                 // two boxes of 128 rows x 32 floats
-                tma_load_4d(dst, &tmB, b_full(bs), t * BN, it.qt[u] * BM, it.h, it.b);
-                tma_load_4d(dst + C::kBias / 2, &tmB, b_full(bs), t * BN + 32, it.qt[u] * BM, it.h, it.b);
-              }
+          __syncwarp();
+          mbar_wait_s(v_empty(vt), vp, abort_s, DEV_TIMEOUT_SYNC);
+          if (elect_one()) {
+            const uint32_t dst = smem_s + C::offV + vt * C::kVB;
+            mbar_expect_tx_s(v_full(vt), C::kVB);
+            if constexpr (has_bias) {  // rows of 64 16-bit values, or twice rows of 32 floats
+              tma_load_4d_s(dst + C::KVR * C::kKV, &tmB, v_full(vt), j0, i0, it.h, it.b);
+              if constexpr (!BIAS16)
+                tma_load_4d_s(dst + C::KVR * C::kKV + C::BTL * (C::kBias / 2), &tmB, v_full(vt), j0 + 32, i0, it.h, it.b);
             }
+            tma_load_5d_s(dst, &tmV, v_full(vt), 0, j0, s0, it.h, it.b);
           }
-          for (int w = 0; w < C::KVW; ++w) {
-            mbar_wait(v_empty(w, st), par, abort_flag, a.status, DEV_TIMEOUT_SYNC);
-            mbar_expect_tx(v_full(w, st), C::kKV);
-            tma_load_5d(smem + C::offV + (w * NKV + st) * C::kKV, &tmV, v_full(w, st), 0, t * BN, srow[w], it.h, it.b);
-          }
+          __syncwarp();
+          if (++kt == NK) { kt = 0; kp ^= 1; }
+          if (++vt == NV) { vt = 0; vp ^= 1; }
         }
       }
-    } else if ((warp == 1 || warp == 2) && lane == 0) {
-      // =============================== MMA issuer of warpgroup w ===============================
-      const int w = warp - 1;
+    } else if (warp == 1 || warp == 2) {
+      // =============================== MMA issuers: half of the warpgroups each ===============================
+      constexpr int HALF = (NW + 1) / 2;
+      const int w0 = (warp - 1) * HALF, w1 = warp == 1 ? HALF : NW;
       constexpr uint32_t kIdescS = make_idesc(kBf16, false, false, BM, BN);
-      constexpr uint32_t kIdescO = make_idesc(kBf16, false, true, BM, DP);
-      constexpr uint32_t kIdescL = make_idesc(kBf16, false, false, BM, 16);
-      const uint64_t ones = make_sdesc_const(128, 256, 0) | (smem_u32(sOnes) >> 4);  // unswizzled 8 x 16-byte core matrices
+      constexpr uint32_t kIdescO = make_idesc(kBf16, false, true, BM, DP + 16);
       // Descriptor halves that never change: the high word holds the stride offset, version and
       // swizzle; the low word is (address >> 4) plus the leading-offset field.
       constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
       constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
-      const uint32_t q_lo0 = (smem_u32(smem + C::offQ + w * QST * C::kQ) >> 4) | kLoLbo;
-      const int kw = QP ? 0 : w;  // the K/V ring this warpgroup reads
-      const uint32_t k_lo0 = (smem_u32(smem + C::offK + kw * NKV * C::kKV) >> 4) | kLoLbo;
-      const uint32_t v_lo0 = (smem_u32(smem + C::offV + kw * NKV * C::kKV) >> 4) | kLoLbo;
-      const uint32_t tS = tmem + w * C::tmemWg, tO = tS + 2 * BN;
-      uint32_t qn = 0, base = 0;  // items done, key tiles done
-      auto issue_s = [&](uint32_t g) {  // g: running key-tile index
-        const int st = g % NKV;
-        mbar_wait(k_full(kw, st), (g / NKV) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
+      const uint32_t q_lo0 = ((smem_s + C::offQ) >> 4) | kLoLbo, k_lo0 = ((smem_s + C::offK) >> 4) | kLoLbo;
+      const uint32_t v_lo0 = (smem_s + C::offV) >> 4, ones = (smem_s + C::offOnes) >> 4;
+      uint32_t n_item = 0;
+      uint32_t gs = 0, kt = 0, kp = 0;  // next S: key tile, K stage and its parity
+      uint32_t go = 0, vt = 0, vp = 0;  // next P V: key tile, V stage and its parity
+      // S of the next key tile for the warpgroups of this warp.  With one score buffer the softmax warps wait
+      // for S and the bias tile at once: this warp sees the tile land and arrives on their barrier too.
+      auto issue_s = [&](int w, bool last) {
+        const uint32_t qa = q_lo0 + (n_item % QST * NW + w) * (C::kQ >> 4);
+        const uint32_t ka = k_lo0 + (kt * C::KVR + (QP ? 0 : w)) * (C::kKV >> 4);
+        const uint32_t tS = tmem + w * C::tmemWg + (gs % SB) * BN, bar = s_full(w, gs % SB);
+        mbar_wait_s(k_full(kt), kp, abort_s, DEV_TIMEOUT_TMA);
         tc_fence_after();
-        const uint32_t qa = q_lo0 + (qn % QST) * (C::kQ >> 4);
-        const uint32_t ka = k_lo0 + st * (C::kKV >> 4);
+        const uint32_t el = elect_one();
 #pragma unroll
         for (int kk = 0; kk < DP / 16; ++kk)
-          mma_ss(tS + (g & 1) * BN, pack_desc(qa + kk * 2, kHiOp), pack_desc(ka + kk * 2, kHiOp), kIdescS,
-                 kk > 0 ? 1u : 0u);
-        mma_commit(k_empty(kw, st));
-        mma_commit(s_full(w, g & 1));
+          mma_ss_e(el, tS, pack_desc(qa + kk * 2, kHiOp), pack_desc(ka + kk * 2, kHiOp), kIdescS, kk > 0 ? 1u : 0u);
+        mma_commit_if_s(el, bar);
+        mma_commit_if_s(el, k_empty(kt));
+        if (last) mma_commit_if_s(el, q_empty(n_item % QST));
       };
-      auto issue_pv = [&](uint32_t g, bool first) {  // O += P V; the first of an item overwrites
-        const int st = g % NKV;
-        mbar_wait(v_full(kw, st), (g / NKV) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
-        mbar_wait(p_full(w, g & 1), (g >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
+      auto next_s = [&]() {
+        ++gs;
+        if (++kt == NK) { kt = 0; kp ^= 1; }
+      };
+      auto bias_landed = [&](int w, uint32_t st, uint32_t par) {
+        if constexpr (has_bias && SB == 1) {
+          mbar_wait_s(v_full(st), par, abort_s, DEV_TIMEOUT_TMA);
+          if (elect_one()) mbar_arrive_s(s_full(w, 0));
+          __syncwarp();
+        }
+      };
+      // O += P V, and the row sums of P as it was rounded, by which O is divided (see the epilogue): the B
+      // operand is DP columns of V followed by 16 of ones, which are simply its next block along N (the leading
+      // offset leads from the V tile to them).
+      auto issue_pv = [&](int w, bool first, bool last) {  // (the first of an item overwrites)
+        const uint32_t va = v_lo0 + vt * (C::kVB >> 4) + (QP ? 0 : w) * (C::kKV >> 4);
+        const uint32_t tW = tmem + w * C::tmemWg, tP = tW + (go % SB) * BN;
+        const uint32_t d0 = va | ((ones - va) << 16);
+        mbar_wait_s(v_full(vt), vp, abort_s, DEV_TIMEOUT_TMA);
+        mbar_wait_s(p_full(w, go % SB), (go / SB) & 1, abort_s, DEV_TIMEOUT_SYNC);
         tc_fence_after();
-        const uint32_t va = v_lo0 + st * (C::kKV >> 4);
+        const uint32_t el = elect_one();
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)  // 16 keys = 8 packed columns of P per step
-          mma_ts(tO, tS + (g & 1) * BN + kk * 8, pack_desc(va + kk * RB, kHiOp), kIdescO, (kk > 0 || !first) ? 1u : 0u);
-        // the row sums of P as it was rounded: O is divided by these (see the epilogue)
-#pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk)
-          mma_ts(tS + C::colL, tS + (g & 1) * BN + kk * 8, ones, kIdescL, (kk > 0 || !first) ? 1u : 0u);
-        mma_commit(v_empty(kw, st));
-        mma_commit(o_full(w, g & 1));
+          mma_ts_e(el, tW + C::colO, tP + kk * 8, pack_desc(d0 + kk * (RB - (RB << 16)), kHiOp), kIdescO, (kk > 0 || !first) ? 1u : 0u);
+        if (SB == 2 || last) mma_commit_if_s(el, o_full(w, go % SB));
+        mma_commit_if_s(el, v_empty(vt));  // (P has arrived, so the bias tile has been read)
       };
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-        mbar_wait(q_full(w, qn % QST), (qn / QST) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
-        for (int t = 0; t < 2 && t < T_TILES; ++t) issue_s(base + t);
-        for (int t = 0; t < T_TILES; ++t) {
-          issue_pv(base + t, t == 0);
-          if (t + 2 < T_TILES) issue_s(base + t + 2);  // S buffer (t&1) was read before P_t was signalled
+#pragma unroll 1
+      for (int item = blockIdx.x; item < wk.n_items; item += gridDim.x) {
+        mbar_wait_s(q_full(n_item % QST), (n_item / QST) & 1, abort_s, DEV_TIMEOUT_TMA);
+#pragma unroll 1
+        for (int t = 0; t < SB && t < T_TILES; ++t) {
+#pragma unroll 1
+          for (int w = w0; w < w1; ++w) {
+            issue_s(w, t == T_TILES - 1);
+            bias_landed(w, vt, vp);
+          }
+          next_s();
         }
-        mma_commit(q_empty(w, qn % QST));
-        ++qn;
-        base += T_TILES;
+#pragma unroll 1
+        for (int t = 0; t < T_TILES; ++t) {
+          const bool more = t + SB < T_TILES;
+          const uint32_t vt1 = vt + 1 == NV ? 0 : vt + 1, vp1 = vp ^ (vt + 1 == NV ? 1u : 0u);
+#pragma unroll 1
+          for (int w = w0; w < w1; ++w) {
+            issue_pv(w, t == 0, t == T_TILES - 1);
+            // (the score buffer was read before P was signalled, and P is read before it is overwritten: the MMAs
+            // of one thread execute in order)
+            if (more) {
+              issue_s(w, t + SB == T_TILES - 1);
+              bias_landed(w, vt1, vp1);
+            }
+          }
+          vt = vt1;
+          vp = vp1;
+          ++go;
+          if (more) next_s();
+        }
+        ++n_item;
       }
     } else if (warp == 3) {
       // =============================== residue-mask stager ===============================
@@ -296,15 +354,18 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const int es = kind == EVOATTN_MASK_BOOL ? 1 : kind == EVOATTN_MASK_ADD_F32 ? 4 : 2;
       const long long step = a.smask.c * es;  // bytes from key to key
       uint32_t n = 0;
-      for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n) {
-        const Item it = decode_item<QP>(item, n_inner, n_outer, a.H);
+#pragma unroll 1
+      for (int item = blockIdx.x; item < wk.n_items; item += gridDim.x, ++n) {
+        const Item it = decode_item(item, wk);
         const int st = n & 1;
-        for (int w = 0; w < 2; ++w) {
+#pragma unroll 1
+        for (int w = 0; w < NW; ++w) {
           const unsigned char* ptr = reinterpret_cast<const unsigned char*>(a.mask) +
-                                     ((long long)it.b * a.smask.a + (long long)min(it.s[w], a.S - 1) * a.smask.b) * es;
-          mbar_wait(m_empty(w, st), ((n >> 1) & 1) ^ 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
+                                     ((long long)it.b * a.smask.a + (long long)min(row_of(it, w), a.S - 1) * a.smask.b) * es;
+          mbar_wait_s(m_empty(w, st), ((n >> 1) & 1) ^ 1, abort_s, DEV_TIMEOUT_SYNC);
           float* dst = sMask + (w * 2 + st) * r_pad;
-          uint32_t* dirty = sDirty + (w * 2 + st) * 32;
+          uint32_t dirty = 0;
+#pragma unroll 1
           for (int j0 = 0; j0 < r_pad; j0 += 256) {
             const int j = j0 + lane * 8;
             const unsigned char* q = ptr + j * step;
@@ -338,195 +399,187 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
               *reinterpret_cast<float4*>(dst + j + 4) = make_float4(m[4], m[5], m[6], m[7]);
             }
             const uint32_t lanes_any = __ballot_sync(0xffffffffu, any);  // eight lanes to a key tile
-            if (lane < 4) dirty[j0 / BN + lane] = (lanes_any >> (8 * lane)) & 0xffu;
+            for (int k = 0; k < 4; ++k)
+              if ((lanes_any >> (8 * k)) & 0xffu) dirty |= 1u << (j0 / BN + k);
           }
+          if (lane == 0) sDirty[w * 2 + st] = dirty;
           __syncwarp();
-          if (lane == 0) mbar_arrive(m_full(w, st));
+          if (lane == 0) mbar_arrive_s(m_full(w, st));
         }
       }
     }
   } else {
     // =============================== softmax warpgroups ===============================
-    setmaxnreg_inc<232>();
+    setmaxnreg_inc<C::kSoftmaxRegs>();
     const int w = (warp >> 2) - 1;
     const int row = (warp & 3) * 32 + lane;
     const uint32_t t_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + w * C::tmemWg;
     const float scale = a.scale;
     const F2 scale2 = f2_make(scale, scale);
+    // this thread's row of a bias tile (in query-pair mode the two tiles of a box follow one another)
+    constexpr int kBoxBias = BIAS16 ? C::kBias : C::kBias / 2;
+    const uint32_t brow0_s = smem_s + C::offV + C::KVR * C::kKV + (QP ? w : 0) * kBoxBias + row * 128;
+    uint32_t vt = 0, vp = 0;     // stage of the bias ring and its parity
     uint32_t g = 0, n_item = 0;  // running key-tile and item index
-    // The two warpgroups take turns in the exponential phase (named barriers 1 and 2 pass a
-    // token back and forth): while one keeps the MUFU busy, the other runs its load / bias /
-    // mask / max phase on the FMA, ALU and shared-memory pipes instead of both queueing on
-    // the same unit.
-    if (w == 1) named_bar_arrive(1, 256);
-
-    for (int item = blockIdx.x; item < n_items; item += gridDim.x, ++n_item) {
-      const Item it = decode_item<QP>(item, n_inner, n_outer, a.H);
-      const int s_raw = it.s[w];
-      const bool active = s_raw < a.S && it.qt[w] < NQT;
-      const int s = s_raw < a.S ? s_raw : a.S - 1;
-      const int i = it.qt[w] * BM + row;
+#pragma unroll 1
+    for (int item = blockIdx.x; item < wk.n_items; item += gridDim.x, ++n_item) {
+      const Item it = decode_item(item, wk);
+      const bool active = row_of(it, w) < a.S && tile_of(it, w) < NQT;
+      const int s = min(row_of(it, w), a.S - 1);
+      const int i = tile_of(it, w) * BM + row;
 
       // residue-mask row of (b, s), staged by warp 3
       const uint32_t mst = n_item & 1;
-      mbar_wait(m_full(w, mst), (n_item >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_SYNC);
-      const float* mrow_base = sMask + (w * 2 + mst) * r_pad;
-      const uint32_t* dirty_row = sDirty + (w * 2 + mst) * 32;
+      mbar_wait_s(m_full(w, mst), (n_item >> 1) & 1, abort_s, DEV_TIMEOUT_SYNC);
+      const uint32_t mrow_s = smem_u32(sMask) + (w * 2 + mst) * r_pad * 4;
+      const uint32_t dirty = lds_u32(smem_u32(sDirty) + (w * 2 + mst) * 4);
 
       // The gate's row is wanted in the epilogue, where every cycle of its latency would be waited for.
       const T* grow = a.gate ? reinterpret_cast<const T*>(a.gate) + off4(a.sgate, it.b, it.h, s, i < a.R ? i : 0) : nullptr;
       if (grow != nullptr) prefetch_l2(grow);
 
       float m_run = -FLT_MAX, l_run = 0.f;
+      bool alive = false;  // every row of this warp has a running maximum
 
+#pragma unroll 1
       for (int t = 0; t < T_TILES; ++t, ++g) {
-        mbar_wait(s_full(w, g & 1), (g >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
+        const uint32_t tS = t_base + (g % SB) * BN;
+        const uint32_t brow_s = brow0_s + vt * C::kVB;
+        const uint32_t mtile_s = mrow_s + t * (BN * 4);
+        mbar_wait_s(s_full(w, g % SB), (g / SB) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
-        if (has_bias) mbar_wait(b_full(g % BST), (g / BST) & 1, abort_flag, a.status, DEV_TIMEOUT_TMA);
-        const uint8_t* bstage = smem + C::offB + ((g % BST) * C::BTL + (QP ? w : 0)) * C::kBias + row * 128;
-        const float* mrow = mrow_base + t * BN;
+        if (has_bias && SB == 2) mbar_wait_s(v_full(vt), vp, abort_s, DEV_TIMEOUT_TMA);
 
-        // scores of my row: x = scale*S + bias, then the mask.  Written in groups of eight
-        // independent elements (loads, FMAs, mins, then eight separate max chains) so that the
-        // in-order issue never waits on the previous instruction's result.
-        float x[BN];
-        float mx8[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) mx8[u] = -FLT_MAX;
-        uint32_t sr[BN];
-        tmem_ld32(t_base + (g & 1) * BN, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
-        tmem_ld32(t_base + (g & 1) * BN + 32, *reinterpret_cast<uint32_t(*)[32]>(&sr[32]));
-        tmem_wait_ld();
-        // A key tile whose mask drops no key (boolean) or adds only zeros needs neither the mask values
-        // nor the arithmetic (most tiles: masks are mostly trailing padding); the flag is warp-uniform.
-        auto scores = [&](auto with_mask) {
-          constexpr bool kMask = decltype(with_mask)::value;
-#pragma unroll
-          for (int g8 = 0; g8 < BN / 8; ++g8) {
+        // Scores of my row, eight at a time: x = scale*S + bias, then the mask.
+        auto scores8 = [&](const uint32_t* s8, int g8, auto with_mask, float (&v)[8]) {
+          float bvv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          if constexpr (BIAS16) {
+            // eight 16-bit values of my row (rows of 128 bytes, 128-byte swizzle), widened here
+            const uint4 wv = lds_v4(brow_s + ((g8 ^ (row & 7)) << 4));
+            unpack2<T>(wv.x, bvv[0], bvv[1]); unpack2<T>(wv.y, bvv[2], bvv[3]);
+            unpack2<T>(wv.z, bvv[4], bvv[5]); unpack2<T>(wv.w, bvv[6], bvv[7]);
+          } else if constexpr (has_bias) {
             const int c = g8 >> 2, q4 = (g8 & 3) * 2;
-            float bvv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (has_bias) {
-              if constexpr (BIAS16) {
-                // eight 16-bit values of my row (rows of 128 bytes, 128-byte swizzle), widened here
-                const uint4 w = *reinterpret_cast<const uint4*>(bstage + ((g8 ^ (row & 7)) << 4));
-                const T* hv = reinterpret_cast<const T*>(&w);
+            const float4 b0 = lds_v4f(brow_s + c * (C::BTL * kBoxBias) + ((q4 ^ (row & 7)) << 4));
+            const float4 b1 = lds_v4f(brow_s + c * (C::BTL * kBoxBias) + (((q4 + 1) ^ (row & 7)) << 4));
+            bvv[0] = b0.x; bvv[1] = b0.y; bvv[2] = b0.z; bvv[3] = b0.w;
+            bvv[4] = b1.x; bvv[5] = b1.y; bvv[6] = b1.z; bvv[7] = b1.w;
+          }
 #pragma unroll
-                for (int u = 0; u < 8; ++u) bvv[u] = to_float<T>(hv[u]);
-              } else {
-                const float4 b0 = *reinterpret_cast<const float4*>(bstage + c * (C::kBias / 2) + ((q4 ^ (row & 7)) << 4));
-                const float4 b1 = *reinterpret_cast<const float4*>(bstage + c * (C::kBias / 2) + (((q4 + 1) ^ (row & 7)) << 4));
-                bvv[0] = b0.x; bvv[1] = b0.y; bvv[2] = b0.z; bvv[3] = b0.w;
-                bvv[4] = b1.x; bvv[5] = b1.y; bvv[6] = b1.z; bvv[7] = b1.w;
-              }
-            }
-            float v[8];
+          for (int u = 0; u < 8; u += 2)  // x = scale*S + bias, two elements per instruction
+            f2_get(f2_fma(f2_from_bits(s8[u], s8[u + 1]), scale2, f2_make(bvv[u], bvv[u + 1])), v[u], v[u + 1]);
+          if constexpr (decltype(with_mask)::value) {
+            const float4 k0 = lds_v4f(mtile_s + g8 * 32);
+            const float4 k1 = lds_v4f(mtile_s + g8 * 32 + 16);
+            const float mkv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
 #pragma unroll
-            for (int u = 0; u < 8; u += 2) {  // x = scale*S + bias, two elements per instruction
-              const F2 t = f2_fma(f2_from_bits(sr[g8 * 8 + u], sr[g8 * 8 + u + 1]), scale2, f2_make(bvv[u], bvv[u + 1]));
-              f2_get(t, v[u], v[u + 1]);
-            }
-            if constexpr (kMask) {
-              const float4 k0 = *reinterpret_cast<const float4*>(mrow + g8 * 8);
-              const float4 k1 = *reinterpret_cast<const float4*>(mrow + g8 * 8 + 4);
-              const float mkv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-#pragma unroll
-              for (int u = 0; u < 8; ++u) v[u] = (MASKMODE == MASK_MIN) ? fminf(v[u], mkv[u]) : (v[u] + mkv[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u += 2) {
-              x[g8 * 8 + u] = v[u];
-              x[g8 * 8 + u + 1] = v[u + 1];
-              mx8[u >> 1] = max3(mx8[u >> 1], v[u], v[u + 1]);
-            }
+            for (int u = 0; u < 8; ++u) v[u] = (MASKMODE == MASK_MIN) ? fminf(v[u], mkv[u]) : (v[u] + mkv[u]);
           }
         };
-        // ([4,1,2048,32,64] with an additive mask 333 -> 312 us, [2,64,768,8,64] boolean 398 -> 378.  At
-        // D <= 16 the second copy of the loop costs more than the skipped instructions save: 741 -> 800 us
-        // on [1,1024,384,8,8], where a random mask leaves no tile without a dropped key.)
-        if constexpr (DP >= 32) {
-          if (dirty_row[t] != 0u) scores(std::true_type{});
-          else scores(std::false_type{});
-        } else {
-          scores(std::true_type{});
-        }
-        const float mx = fmaxf(fmaxf(mx8[0], mx8[1]), fmaxf(mx8[2], mx8[3]));
-        if (has_bias) {
-          // The stage is handed back only after the bias loads above have returned: the store needs
-          // the row maximum, which needs every one of them (an mbarrier arrival by itself does not
-          // wait for shared loads that are still queued).
-          *scratch = __float_as_uint(mx);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(b_empty(g % BST));  // one arrival per warp
-        }
 
-        // The running maximum follows a tile's maximum only when that has grown by more than 2^8: the row
-        // sum and O carry the same factor, so their quotient does not change and nothing overflows.  Then,
-        // and only then, O is rescaled in tensor memory (P V of the tile before has to be complete).
-        if (t == 0) {
-          m_run = mx;
-        } else {
-          const bool grow = mx > m_run + kGrow;
-          if (__any_sync(0xffffffffu, grow)) {
-            const float m_up = grow ? mx : m_run;
-            const float alpha = ex2((m_run - m_up) * kLog2e);
-            m_run = m_up;
-            l_run *= alpha;
-            mbar_wait(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
-            tc_fence_after();
-#pragma unroll
-            for (int d0 = 0; d0 < DP + 16; d0 += 16) {  // O and the row sum behind it
-              uint32_t o[16];
-              tmem_ld16(t_base + 2 * BN + d0, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int u = 0; u < 16; ++u) o[u] = __float_as_uint(__uint_as_float(o[u]) * alpha);
-              tmem_st16(t_base + 2 * BN + d0, o);
-            }
-          }
-        }
         float lsum = 0.f;
         uint32_t pk[BN / 2];
-        named_bar_sync(1 + w, 256);  // my turn on the exponential unit
-        if (m_run != -FLT_MAX) {
-          const float nm2 = -m_run * kLog2e;
-          const F2 l2e2 = f2_make(kLog2e, kLog2e), nm22 = f2_make(nm2, nm2);
-          F2 ls4[4];
+        bool go = alive, settled = false;
+#pragma unroll 1
+        for (;;) {
+          bool bad = true;
+          if (go) {
+            const float nm2 = -m_run * kLog2e;
+            const F2 l2e2 = f2_make(kLog2e, kLog2e), nm22 = f2_make(nm2, nm2);
+            F2 ls4[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) ls4[u] = f2_make(0.f, 0.f);
+            for (int u = 0; u < 4; ++u) ls4[u] = f2_make(0.f, 0.f);
+            auto exps = [&](auto with_mask) {
+              uint32_t sr[2][16];  // S, sixteen columns ahead of the arithmetic
+              tmem_ld16(tS, sr[0]);
 #pragma unroll
-          for (int e = 0; e < BN; e += 2) {
-            float y0, y1;
-            f2_get(f2_fma(f2_make(x[e], x[e + 1]), l2e2, nm22), y0, y1);
-            const float p0 = ex2(y0), p1 = ex2(y1);
-            ls4[(e >> 1) & 3] = f2_add(ls4[(e >> 1) & 3], f2_make(p0, p1));
-            pk[e / 2] = Pack2<T>::pack(p0, p1);
+              for (int g8 = 0; g8 < BN / 8; ++g8) {
+                if (g8 % 2 == 0) {
+                  tmem_wait_ld();
+                  if (g8 + 2 < BN / 8) tmem_ld16(tS + 8 * g8 + 16, sr[(g8 / 2 + 1) & 1]);
+                }
+                float v[8];
+                scores8(sr[(g8 / 2) & 1] + 8 * (g8 & 1), g8, with_mask, v);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  float y0, y1;
+                  f2_get(f2_fma(f2_make(v[2 * u], v[2 * u + 1]), l2e2, nm22), y0, y1);
+                  const float p0 = ex2(y0), p1 = ex2(y1);
+                  ls4[u] = f2_add(ls4[u], f2_make(p0, p1));
+                  pk[g8 * 4 + u] = Pack2<T>::pack(p0, p1);
+                }
+              }
+            };
+            if (__builtin_expect((dirty >> t) & 1u, 0)) exps(std::true_type{});
+            else exps(std::false_type{});
+            float lsa[8];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) f2_get(ls4[u], lsa[2 * u], lsa[2 * u + 1]);
+            lsum = ((lsa[0] + lsa[1]) + (lsa[2] + lsa[3])) + ((lsa[4] + lsa[5]) + (lsa[6] + lsa[7]));
+            bad = __any_sync(0xffffffffu, !(lsum <= kMaxSum));
           }
-          float lsa[8];
+          if (__builtin_expect(!bad || settled, 1)) break;
+          // The tile's own maximum, and the running one follows it.
+          float mx = -FLT_MAX;
+#pragma unroll 1
+          for (int h = 0; h < BN / 16; ++h) {
+            uint32_t s16[16];
+            tmem_ld16(tS + 16 * h, s16);
+            tmem_wait_ld();
 #pragma unroll
-          for (int u = 0; u < 4; ++u) f2_get(ls4[u], lsa[2 * u], lsa[2 * u + 1]);
-          lsum = ((lsa[0] + lsa[1]) + (lsa[2] + lsa[3])) + ((lsa[4] + lsa[5]) + (lsa[6] + lsa[7]));
-        } else {
+            for (int k = 0; k < 2; ++k) {
+              float v[8];
+              scores8(s16 + 8 * k, 2 * h + k, std::true_type{}, v);
+#pragma unroll
+              for (int u = 0; u < 8; u += 2) mx = max3(mx, v[u], v[u + 1]);
+            }
+          }
+          if (t == 0) {
+            m_run = mx;
+          } else {
+            const bool grow = mx > m_run + kGrow;
+            if (__any_sync(0xffffffffu, grow)) {
+              const float m_up = grow ? mx : m_run;
+              const float alpha = ex2((m_run - m_up) * kLog2e);
+              m_run = m_up;
+              l_run *= alpha;
+              // (P V of the tile before has to be complete: with one score buffer, S of this tile came after it)
+              if constexpr (SB == 2) mbar_wait_s(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+              tc_fence_after();
+#pragma unroll 1
+              for (int d0 = 0; d0 < DP + 16; d0 += 16) {  // O and the row sum behind it
+                uint32_t o[16];
+                tmem_ld16(t_base + C::colO + d0, o);
+                tmem_wait_ld();
+#pragma unroll
+                for (int u = 0; u < 16; ++u) o[u] = __float_as_uint(__uint_as_float(o[u]) * alpha);
+                tmem_st16(t_base + C::colO + d0, o);
+              }
+            }
+          }
+          alive = !__any_sync(0xffffffffu, m_run == -FLT_MAX);
+          go = __any_sync(0xffffffffu, m_run != -FLT_MAX);
+          settled = true;
+        }
+        if (!alive && m_run == -FLT_MAX) {
           // every key seen so far was dropped: the scores are all -FLT_MAX and the softmax is
           // uniform over the real keys (test.py:54-55 semantics)
+          const int real = min(BN, a.R - t * BN);
+          lsum = (float)real;
 #pragma unroll
-          for (int e = 0; e < BN; e += 2) {
-            const float p0 = (t * BN + e < a.R) ? 1.f : 0.f;
-            const float p1 = (t * BN + e + 1 < a.R) ? 1.f : 0.f;
-            lsum += p0 + p1;
-            pk[e / 2] = Pack2<T>::pack(p0, p1);
-          }
+          for (int e = 0; e < BN; e += 2) pk[e / 2] = Pack2<T>::pack(e < real ? 1.f : 0.f, e + 1 < real ? 1.f : 0.f);
         }
-        named_bar_arrive(2 - w, 256);  // hand the turn to the other warpgroup
         l_run += lsum;
+        if (++vt == NV) { vt = 0; vp ^= 1; }
 
         // P_n -> TMEM, packed two 16-bit values per column, over the first half of the S_n
         // columns this thread has just consumed (lane = row, column j = keys 2j, 2j+1): the
         // A operand of P V comes straight from tensor memory.
-        tmem_st32(t_base + (g & 1) * BN, pk);
+        tmem_st32(tS, pk);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full(w, g & 1));
+        if (lane == 0) mbar_arrive_s(p_full(w, g % SB));
       }
       uint4 gw[DP / 8];
       if (grow != nullptr) {
@@ -534,11 +587,12 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         for (int d8 = 0; d8 < DP / 8; ++d8) gw[d8] = d8 * 8 < a.D ? *reinterpret_cast<const uint4*>(grow + d8 * 8) : make_uint4(0, 0, 0, 0);
       }
       // O of the item, complete with its last P V
-      mbar_wait(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_flag, a.status, DEV_TIMEOUT_MMA);
+      if constexpr (SB == 2) mbar_wait_s(o_full(w, (g - 1) & 1), ((g - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+      else mbar_wait_s(o_full(w, 0), n_item & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
       float acc[DP];
 #pragma unroll
-      for (int d0 = 0; d0 < DP; d0 += 16) tmem_ld16(t_base + 2 * BN + d0, *reinterpret_cast<uint32_t(*)[16]>(&acc[d0]));
+      for (int d0 = 0; d0 < DP; d0 += 16) tmem_ld16(t_base + C::colO + d0, *reinterpret_cast<uint32_t(*)[16]>(&acc[d0]));
       // O is divided by the sum of the P it was made of, rounded to the storage type.  The running maximum
       // may lag, so the largest P of a row is not exactly 1; with the sum of the unrounded values its
       // rounding would go into O in full (an fp16 O was off by 5.4e-4 instead of 2.7e-4).  The log-sum-exp
@@ -578,31 +632,26 @@ evo_fwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         a.lse[li] = (m_run == -FLT_MAX) ? -FLT_MAX : (m_run + logf(l_run));
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(m_empty(w, mst));
+      if (lane == 0) mbar_arrive_s(m_empty(w, mst));
     }
-    if (w == 0) named_bar_sync(1, 256);  // consume the last token so no arrival is left pending
   }
 
-  if (*abort_flag) {
-    // give copies that may still be in flight time to land before the CTA retires
-    const long long t0 = clock64();
-    while (clock64() - t0 < 200000) {}
-  }
+  if (*abort_flag) report_abort(*abort_flag, a.status);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
-template <class T, int DP, bool QP>
+template <class T, int DP, int BIAS, int NW, bool QP>
 int launch_t(const Args& a, cudaStream_t st, int* launches) {
-  using C = Cfg<DP, QP>;
+  using C = Cfg<DP, NW, QP, BIAS>;
   CUtensorMap tq, tk, tv, tb;
-  if (!make_qkv_map(&tq, a.q, a.sq, a.B, a.H, a.S, a.R, a.D, DP, BM)) return EVOATTN_ERR_CUDA;
-  if (!make_qkv_map(&tk, a.k, a.sk, a.B, a.H, a.S, a.R, a.D, DP, BN)) return EVOATTN_ERR_CUDA;
-  if (!make_qkv_map(&tv, a.v, a.sv, a.B, a.H, a.S, a.R, a.D, DP, BN)) return EVOATTN_ERR_CUDA;
+  if (!make_qkv_map(&tq, a.q, a.sq, a.B, a.H, a.S, a.R, a.D, DP, QP ? NW * BM : BM, C::KVR)) return EVOATTN_ERR_CUDA;
+  if (!make_qkv_map(&tk, a.k, a.sk, a.B, a.H, a.S, a.R, a.D, DP, BN, C::KVR)) return EVOATTN_ERR_CUDA;
+  if (!make_qkv_map(&tv, a.v, a.sv, a.B, a.H, a.S, a.R, a.D, DP, BN, C::KVR)) return EVOATTN_ERR_CUDA;
   if (a.bias) {
-    const bool ok = a.bias16 ? make_bias16_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, BM, BN)
-                             : make_bias_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, BM, 32);
+    const bool ok = a.bias16 ? make_bias16_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, C::BTL * BM, BN)
+                             : make_bias_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, C::BTL * BM, 32);
     if (!ok) return EVOATTN_ERR_CUDA;
   } else {
     tb = tq;
@@ -612,33 +661,66 @@ int launch_t(const Args& a, cudaStream_t st, int* launches) {
   const int T_TILES = (a.R + BN - 1) / BN;
   const int NQT = (a.R + BM - 1) / BM;
   const size_t smem = C::bytes(T_TILES * BN);
-  const long long items = QP ? (long long)a.B * a.H * ((NQT + 1) / 2) * a.S
-                             : (long long)a.B * a.H * NQT * ((a.S + 1) / 2);
+  const int inner = QP ? a.S : (a.S + NW - 1) / NW, outer = QP ? (NQT + NW - 1) / NW : NQT;
+  const long long items = (long long)a.B * a.H * outer * inner;
+  const Walk wk{(int)items, fast_div((uint32_t)inner), fast_div((uint32_t)outer), fast_div((uint32_t)a.H)};
   const int grid = (int)(items < sms ? items : sms);
   const bool add = a.mask_kind == EVOATTN_MASK_ADD_F32 || a.mask_kind == EVOATTN_MASK_ADD_SAME;
-  auto kern = !a.bias ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_NONE, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_NONE, QP>)
-              : a.bias16 ? (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_16, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_16, QP>)
-                         : (add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS_F32, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS_F32, QP>);
-  if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)smem, nullptr)) return EVOATTN_ERR_CUDA;
-  launch_dependent(kern, dim3((unsigned)grid), kThreads, smem, st, a, (int)items, tq, tk, tv, tb);
+  auto kern = add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS, NW, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS, NW, QP>;
+  // setmaxnreg.inc waits until the scheduler's register pool (1 + NW warps at the launch-time count) has what
+  // it asks for: never launch a build whose pool cannot hold the warps' requests.
+  int num_regs = 0;
+  if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)smem, &num_regs)) return EVOATTN_ERR_CUDA;
+  if ((1 + NW) * num_regs < NW * C::kSoftmaxRegs + C::kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
+  launch_dependent(kern, dim3((unsigned)grid), C::kThreads, smem, st, a, wk, tq, tk, tv, tb);
   *launches += 1;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
 }
 
-// A single MSA row with several query tiles runs in query-pair mode (both warpgroups get work);
-// everything else pairs MSA rows, which shares the larger tile (the pair bias) between them.
-template <class T, int DP>
+// A single MSA row with several query tiles runs in query-pair mode (both warpgroups get work).  Several rows
+// share the larger tile, the pair bias, two to four of them at a time.
+template <class T, int DP, int BIAS>
 int launch_mode(const Args& a, cudaStream_t st, int* launches) {
   const int r_pad = (a.R + BN - 1) / BN * BN;
-  if (a.S == 1 && a.R > BM && Cfg<DP, true>::bytes(r_pad) <= 232448) return launch_t<T, DP, true>(a, st, launches);
-  return launch_t<T, DP, false>(a, st, launches);
+  if (a.S == 1 && a.R > BM && Cfg<DP, 2, true, BIAS>::bytes(r_pad) <= kMaxSmem) return launch_t<T, DP, BIAS, 2, true>(a, st, launches);
+  const int sms = sm_count();
+  if (sms <= 0) return EVOATTN_ERR_CUDA;
+  // Time of the busiest CTA: the items it walks, times what an item of two, three or four rows costs (each
+  // measured with the CTAs evenly loaded, [1,148,1024,4,32] 17.6, 22.3 and 27.7 us, [1,64,768,8,64] 16.0 and 21.4).
+  // What the rounding to whole items does to it: [1,128,384,8,32] 89.1, 76.9 and 78.1 us, [1,64,500,4,16] 41.1,
+  // 41.0 and 37.3, [1,4,384,8,32] 12.4, 15.0 and 18.5, [1,96,384,8,64] 76.8 and 80.3.
+  const auto cost = [&](int nw, long long item) {
+    const long long items = (long long)a.B * a.H * ((a.R + BM - 1) / BM) * ((a.S + nw - 1) / nw);
+    return (items + sms - 1) / sms * item;
+  };
+  int nw = 2;
+  long long best = cost(2, 100);
+  const long long three = cost(3, DP == 64 ? 137 : 130);
+  if (Cfg<DP, 3, false, BIAS>::bytes(r_pad) <= kMaxSmem && three < best) {
+    nw = 3;
+    best = three;
+  }
+  if constexpr (DP <= 32) {
+    if (Cfg<DP, 4, false, BIAS>::bytes(r_pad) <= kMaxSmem && cost(4, 158) < best) nw = 4;
+  }
+  if constexpr (DP <= 32) {
+    if (nw == 4) return launch_t<T, DP, BIAS, 4, false>(a, st, launches);
+  }
+  if (nw == 3) return launch_t<T, DP, BIAS, 3, false>(a, st, launches);
+  return launch_t<T, DP, BIAS, 2, false>(a, st, launches);
+}
+template <class T, int DP>
+int launch_bias(const Args& a, cudaStream_t st, int* launches) {
+  if (!a.bias) return launch_mode<T, DP, BIAS_NONE>(a, st, launches);
+  if (a.bias16) return launch_mode<T, DP, BIAS_16>(a, st, launches);
+  return launch_mode<T, DP, BIAS_F32>(a, st, launches);
 }
 
 template <class T>
 int launch_d(const Args& a, cudaStream_t st, int* launches) {
-  if (a.D <= 16) return launch_mode<T, 16>(a, st, launches);
-  if (a.D <= 32) return launch_mode<T, 32>(a, st, launches);
-  return launch_mode<T, 64>(a, st, launches);
+  if (a.D <= 16) return launch_bias<T, 16>(a, st, launches);
+  if (a.D <= 32) return launch_bias<T, 32>(a, st, launches);
+  return launch_bias<T, 64>(a, st, launches);
 }
 
 }  // namespace

@@ -22,119 +22,51 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+// The primitives on 32-bit shared-window addresses (smem_u32 of the barrier, computed once): no
+// generic-pointer arithmetic or address-space conversion per call.
+__device__ __forceinline__ void mbar_init_s(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// The same test with a suspend-time hint: the hardware parks the thread until the phase completes
-// or the hint (nanoseconds, capped by the system) runs out, so a waiting warp does not compete
-// for issue slots with the warps that do the arithmetic.
-__device__ __forceinline__ bool mbar_try_wait_parked(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(1000000u)
-      : "memory");
-  return ok != 0;
-}
-
-// About one second at B200 clocks.
-constexpr long long kWaitLimitCycles = 2000000000LL;
-
-// Bounded wait.  `abort_flag` lives in shared memory and is shared by the CTA: once any
-// wait has failed, all later waits fall through at once.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                          int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (;;) {
-    if (mbar_try_wait_parked(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitLimitCycles) {
-      *abort_flag = 1;
-      if (status) atomicCAS(status, 0, code);
-      return false;
-    }
-  }
-}
-
-// The same primitives on 32-bit shared-window addresses (smem_u32 of the barrier, computed once):
-// no generic-pointer arithmetic or address-space conversion per call, and a wait loop that looks
-// at the clock and the abort flag only after every 1024 unsuccessful tries.
 __device__ __forceinline__ void mbar_arrive_s(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_s(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
+// Bounded wait on an mbarrier (32-bit shared-window addresses; about one second at B200 clocks).  `abort_flag_s`
+// is a word of shared memory that belongs to the CTA: once any wait has run out it holds that wait's code, all
+// later waits fall through, and the end of the kernel reports it (report_abort).  The retries carry a
+// suspend-time hint: the hardware parks the thread until the phase completes, so a waiting warp does not
+// compete for issue slots with the warps that do the arithmetic.  All of it is one short sequence on purpose: a
+// kernel has some thirty waits, and the code of its loops has to fit the instruction caches.
+constexpr uint32_t kWaitLimitCycles = 2000000000u;
+__device__ __forceinline__ void mbar_wait_s(uint32_t bar, uint32_t parity, uint32_t abort_flag_s, int code) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Up to 1024 suspended tries in one tight loop (a waiting warp shares its scheduler with warps that
-// have arithmetic to issue: every instruction of the polling loop takes an issue slot from them).
-__device__ __forceinline__ bool mbar_try_wait_burst_s(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .u32 c;\n\t"
-      "mov.u32 c, 0;\n"
-      "EVO_W_AGAIN:\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "{\n\t.reg .pred p;\n\t.reg .u32 t0, t1;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n\t"
       "@p bra EVO_W_DONE;\n\t"
-      "add.u32 c, c, 1;\n\t"
-      "setp.lt.u32 p, c, 1024;\n\t"
+      "mov.u32 t0, %%clock;\n"
+      "EVO_W_AGAIN:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1, 1000000;\n\t"
+      "@p bra EVO_W_DONE;\n\t"
+      "ld.volatile.shared.u32 t1, [%2];\n\t"
+      "setp.ne.u32 p, t1, 0;\n\t"
+      "@p bra EVO_W_DONE;\n\t"
+      "mov.u32 t1, %%clock;\n\t"
+      "sub.u32 t1, t1, t0;\n\t"
+      "setp.lt.u32 p, t1, %4;\n\t"
       "@p bra EVO_W_AGAIN;\n\t"
-      "setp.ne.u32 p, 0, 0;\n"
-      "EVO_W_DONE:\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(1000000u)
+      "st.volatile.shared.u32 [%2], %3;\n"
+      "EVO_W_DONE:\n\t}"
+      ::"r"(bar), "r"(parity), "r"(abort_flag_s), "r"(code), "n"(kWaitLimitCycles)
       : "memory");
-  return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait_slow_s(uint32_t bar, uint32_t parity, uint32_t abort_flag_s, int* status, int code) {
-  long long t0 = 0;
-  for (uint32_t round = 0;; ++round) {
-    if (mbar_try_wait_burst_s(bar, parity)) return true;
-    uint32_t ab;
-    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(ab) : "r"(abort_flag_s));
-    if (ab) return false;
-    if (round == 0) {
-      t0 = clock64();
-    } else if (clock64() - t0 > kWaitLimitCycles) {
-      asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_flag_s), "r"(1u) : "memory");
-      if (status) atomicCAS(status, 0, code);
-      return false;
-    }
-  }
-}
-__device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, uint32_t abort_flag_s, int* status, int code) {
-  if (mbar_try_wait_s(bar, parity)) return true;
-  return mbar_wait_slow_s(bar, parity, abort_flag_s, status, code);
+// What every thread of a CTA does at the end if a wait has run out: the status word gets the code of that wait,
+// and copies that may still be in flight get time to land before the CTA retires.
+static __device__ __noinline__ void report_abort(int code, int* status) {
+  if (threadIdx.x == 0 && status) atomicCAS(status, 0, code);
+  const long long t0 = clock64();
+  while (clock64() - t0 < 200000) {}
 }
 
 // Generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05.mma).
@@ -143,20 +75,6 @@ __device__ __forceinline__ void fence_async_shared() {
 }
 
 // ---------------------------------------------------------------- TMA (tiled, no multicast)
-__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
-                                            int c3, int c4) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
-                                            int c3) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-      : "memory");
-}
 __device__ __forceinline__ void tma_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Wait until the bulk groups of this thread have finished READING their shared-memory source.
 __device__ __forceinline__ void tma_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -183,30 +101,32 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // ---------------------------------------------------------------- tcgen05: MMA
-// D[tmem] (+)= A[smem] * B[smem];  issued by ONE thread.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
+// One lane of a converged warp.  Every operand of a tcgen05.mma lives in a uniform register: in a branch that one
+// lane takes (lane == 0) the compiler has to move each of them there, and the waits of that branch are slow too.
+// With the whole warp walking the issue loop on warp-uniform values and only the instruction itself under this
+// predicate, a hand-over of four MMAs with A in tensor memory, two with A in shared memory, three commits and
+// the wait for them took 376 cycles next to 16 busy warps, against 830 from a single-lane branch.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e;
+}
+// The MMAs of a converged warp, issued by its elected lane.
+__device__ __forceinline__ void mma_ss_e(uint32_t elected, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                         uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
+__device__ __forceinline__ void mma_ts_e(uint32_t elected, uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                         uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
-}
-// Arrive on an mbarrier once every tcgen05 op this thread issued so far has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
 }
 
 // Instruction descriptor for kind::f16 (bf16 or fp16 operands, fp32 accumulate).
@@ -339,6 +259,16 @@ __device__ __forceinline__ float lds_f32(uint32_t saddr) {
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(saddr));
   return v;
 }
+__device__ __forceinline__ uint32_t lds_u32(uint32_t saddr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr));
+  return v;
+}
+__device__ __forceinline__ uint4 lds_v4(uint32_t saddr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr));
+  return v;
+}
 __device__ __forceinline__ uint16_t lds_u16(uint32_t saddr) {
   uint16_t v;
   asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr));
@@ -422,10 +352,6 @@ template <int N> __device__ __forceinline__ void setmaxnreg_dec() {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Named barrier among `nthreads` threads (ids 1..15; id 0 is __syncthreads).
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 
 // ---------------------------------------------------------------- leader-predicated commit
 // For a warp that runs with all 32 lanes converged and predicates only the instruction that must be
@@ -579,10 +505,6 @@ __device__ __forceinline__ void mma_ss_x8(uint32_t d_tmem, uint32_t a_lo, uint32
       : "memory");
 }
 
-// Non-blocking arrival on a named barrier that other threads wait on with named_bar_sync.
-__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
 
 }  // namespace ptx
 }  // namespace evo

@@ -28,14 +28,14 @@ uint64_t fix_stride(long long stride_elems, int esize, uint64_t fallback_bytes, 
 }  // namespace
 
 bool make_qkv_map(CUtensorMap* out, const void* base, const Str4& st, int B, int H, int S, int R, int D, int box_d,
-                  int box_r) {
+                  int box_r, int box_s) {
   std::call_once(g_once, resolve);
   if (!g_encode) return false;
   const uint64_t row = static_cast<uint64_t>(D) * 2;
   cuuint64_t dims[5] = {(cuuint64_t)D, (cuuint64_t)R, (cuuint64_t)S, (cuuint64_t)H, (cuuint64_t)B};
   cuuint64_t strides[4] = {fix_stride(st.r, 2, row, R), fix_stride(st.s, 2, row, S), fix_stride(st.h, 2, row, H),
                            fix_stride(st.b, 2, row, B)};
-  cuuint32_t box[5] = {(cuuint32_t)box_d, (cuuint32_t)box_r, 1, 1, 1};
+  cuuint32_t box[5] = {(cuuint32_t)box_d, (cuuint32_t)box_r, (cuuint32_t)box_s, 1, 1};
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   const int row_bytes = box_d * 2;
   CUtensorMapSwizzle swz = row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B

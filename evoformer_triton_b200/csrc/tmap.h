@@ -9,10 +9,10 @@
 namespace evo {
 
 // 16-bit [B,H,S,R,D] attention-view tensor -> 5-D map with dims (D, R, S, H, B).
-// Box = (box_d, box_r, 1, 1, 1); rows of box_d*2 bytes are swizzled with the matching
-// 32/64/128-byte pattern.  Elements beyond D or R read as zero.
+// Box = (box_d, box_r, box_s, 1, 1): the tiles of box_s consecutive MSA rows, back to back; rows of
+// box_d*2 bytes are swizzled with the matching 32/64/128-byte pattern.  Elements beyond D, R or S read as zero.
 bool make_qkv_map(CUtensorMap* out, const void* base, const Str4& stride_elems, int B, int H, int S, int R, int D,
-                  int box_d, int box_r);
+                  int box_d, int box_r, int box_s = 1);
 
 // fp32 [B,H,R,R] pair bias -> 4-D map with dims (R_j, R_i, H, B); box = (box_j, box_i, 1, 1)
 // with box_j = 32 (rows of 128 bytes, 128-byte swizzle) or 16 (rows of 64 bytes, 64-byte swizzle).

@@ -138,3 +138,50 @@ def test_pair_bias_gradient_of_64_gib():
     assert -3.5 < low.item() and high.item() < 3.5  # no marker left anywhere
     del bias, dbias
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("cfg", [
+    # rows in an item (0: query pairs), B, S, R, H, D, dtype, mask, bias
+    (4, 1, 594, 72, 8, 32, torch.bfloat16, "bool", "fp32"), (4, 1, 595, 40, 8, 8, torch.float16, "add32", "same"),
+    (4, 2, 296, 65, 8, 16, torch.bfloat16, "none", "none"), (3, 1, 100, 136, 4, 32, torch.float16, "addsame", "same"),
+    (3, 1, 592, 64, 8, 64, torch.bfloat16, "bool", "fp32"), (3, 1, 590, 40, 8, 48, torch.bfloat16, "add32", "same"),
+    (2, 1, 5, 200, 3, 32, torch.bfloat16, "bool", "same"), (2, 3, 1, 100, 2, 64, torch.float16, "none", "fp32"),
+    (0, 2, 1, 272, 3, 32, torch.bfloat16, "addsame", "fp32"), (0, 2, 1, 520, 2, 64, torch.float16, "bool", "same")],
+    ids=lambda c: "rows%d-B%dS%dR%dH%dD%d-%s-%s-%s" % (*c[:6], str(c[6]).split(".")[-1], c[7], c[8]))
+def test_forward_items_of_each_size(cfg):
+    """Forward items of two, three and four MSA rows and of two query tiles: row groups and query pairs that are not
+    full, one and several items to a block, scores whose maximum lies beyond the first key tile, a row whose keys
+    are all dropped.  Against float64; the bound is what rounding P and O to the storage type gives (twice eps / 2),
+    and the log-sum-exp has fp32's."""
+    from evoformer_triton_b200 import attention, check_device_status
+    rows, B, S, R, H, D, dtype, mask, bias = cfg
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148 and rows:  # the launcher's rule: these sizes do take items of `rows` rows
+        cost = {2: 100, 3: 137 if D > 32 else 130, 4: 158}
+        busiest = {n: -(-B * H * -(-R // 128) * -(-S // n) // sms) * c for n, c in cost.items() if n < 4 or D <= 32}
+        assert min(busiest, key=lambda n: (busiest[n], n)) == rows
+    x = rand_inputs(B, S, R, H, D, dtype, seed=S + R, mask=mask, bias=bias != "none", keep_p=0.8)
+    x["Q"][..., R // 2:, :, :] *= 6  # (some rows' scores spread far enough for the running maximum to move)
+    if mask == "bool":
+        x["res_mask"][0, 0] = False
+    q, k, v = (x[n].to(DEV).reshape(B, H, S, R, D) for n in ("Q", "K", "V"))
+    b = None if bias == "none" else x["pair_bias"].reshape(B, H, R, R).to(DEV).to(torch.float32 if bias == "fp32" else dtype)
+    m = None if mask == "none" else x["res_mask"].reshape(B, S, R).to(DEV)
+    o, lse = attention.attention_forward(q, k, v, m, b, D ** -0.5)
+    torch.cuda.synchronize()
+    check_device_status()
+    assert attention.last_path["fwd"] == _lib().PATH_TCGEN05
+    p = (q.double() @ k.double().transpose(-1, -2)) * D ** -0.5
+    if b is not None:
+        p += b.double()[:, :, None]
+    if mask == "bool":
+        p.masked_fill_(~m[:, None, :, None, :], -1e300)
+    elif m is not None:
+        p += m.double()[:, None, :, None, :]
+    want_lse = p.logsumexp(-1)
+    want = p.softmax(-1) @ v.double()
+    assert (o.double() - want).norm() <= torch.finfo(dtype).eps * want.norm()
+    live = want_lse > -1e30
+    assert (lse.double() - want_lse)[live].abs().max().item() < 2e-5
+    if mask == "bool":
+        assert (lse[~live] == torch.finfo(torch.float32).min).all()
