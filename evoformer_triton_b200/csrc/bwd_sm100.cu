@@ -64,12 +64,13 @@ struct SmemT {
   static constexpr int offDS = offStage + kStages * kStage;
   static constexpr int offBias = offDS + kDS;
   static constexpr int offOut = offBias + kBias;
-  static constexpr int offBars = offOut + kCW * kOutWarp;
+  static constexpr int offMask = offOut + kCW * kOutWarp;    // [G][128 keys]: what the mask adds to a score
+  static constexpr int offBars = offMask + G * BT * 4;
   // 64 barrier slots (see the kernel) and the slack for aligning the tiles to 1024 bytes.  At DP = 64
-  // only 512 bytes of slack fit: the kernel checks what the base address needs and gives up with a
-  // status code if it is more (the dynamic shared memory of a kernel without static shared memory
-  // starts on a 1024-byte boundary on this architecture, so it needs none).
-  static constexpr int kSlack = (DP == 64) ? 512 : 1024;
+  // none fits: the kernel checks what the base address needs and gives up with a status code if that is
+  // anything (the dynamic shared memory of a kernel without static shared memory starts on a 1024-byte
+  // boundary on this architecture, so it needs none).
+  static constexpr int kSlack = (DP == 64) ? 0 : 1024;
   static constexpr size_t bytes = offBars + 512 + kSlack;
   static_assert(offDS % 1024 == 0 && kStage % 1024 == 0 && offStage % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static_assert(bytes <= 232448, "shared memory budget of one CTA");
@@ -89,8 +90,6 @@ __device__ __forceinline__ void mbar_wait(Bar b, uint32_t parity, uint32_t abort
 }
 __device__ __forceinline__ void mbar_arrive(Bar b) { mbar_arrive_s(b.a); }
 __device__ __forceinline__ void mbar_expect_tx(Bar b, uint32_t bytes) { mbar_expect_tx_s(b.a, bytes); }
-__device__ __forceinline__ void mma_commit_if(uint32_t leader, Bar b) { mma_commit_if_s(leader, b.a); }
-
 
 // The first pass of a backward call: delta[b,h,s,i] = <dO_i, O_i> (evoformer.py:299-326), nl = -lse*log2e,
 // and zeros in the buffers that the fused kernel adds to (the fp32 dQ accumulator, d(pair_bias)).
@@ -214,6 +213,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
   constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
   static_assert(DP == 16 || DP == 32 || DP == 64, "padded head dimension");
+  static_assert(kStages == 2, "steps alternate between two stages");
   constexpr int G = RowsPerItem<DP>::G;
   constexpr int kTmemCols = 512;
   // TMEM: two (S^T, dP^T) half-tile buffers, the per-row dV and dK accumulators, two dQ partials
@@ -245,11 +245,13 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   const Bar b_done{bars_s + 8 * 16};     // [2] ... has been read for the last time
   const Bar ds_empty{bars_s + 8 * 18};   // the dQ MMAs of a step have read the dS tile
   const Bar dq_full{bars_s + 8 * 19};    // [2] the dQ partial of a step is complete in TMEM
+  const Bar mk_full{bars_s + 8 * 25};    // [G] the mask of row g of the current item is in shared memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 22);  // (bars 23, 24: sdone)
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 22);  // (bars 23, 24: sdone; 25..31: mk_full)
   const uint32_t abort_s = smem_u32(const_cast<int*>(abort_flag));
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
   const int NT = (a.R + BT - 1) / BT;
   const int NC = (a.S + G - 1) / G;
   constexpr bool has_bias = kHasBias;
@@ -291,7 +293,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   if (*abort_flag) return;
 
   if (tid == 0) {
-    for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); }  // kv_full; kv_empty: three MMA warps read K/V
+    for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); mbar_init(bars + 25 + i, 1); }  // kv_full; kv_empty: three MMA warps read K/V
     for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + 48 + 2 * i, 2); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full, cdone
@@ -313,7 +315,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   if (warp >= kCW) {
     setmaxnreg_dec<kServiceRegs>();
@@ -325,11 +327,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       // S^T columns of both buffers (S^T = K_j Q_i^T in, dV_j += P^T dO_i out), warp 17 the dP^T columns
       // (dP^T = V_j dO_i^T in, dK_j += dS^T Q_i out): the MMA that overwrites a buffer is always issued
       // by the thread that issued the MMAs reading it.  Warp 18 issues dQ_i = dS K_j, which depends on
-      // neither.  One lane of each warp runs the whole issue loop (measured: a tcgen05.mma issued from a
-      // single-thread branch costs the warp a quarter less than the same instruction predicated on a
-      // leader lane in a converged warp).
+      // neither.  The warps walk their loops converged (see elect_one).
       const bool isA = (warp == kCW);
-      if (lane == 0) {
       constexpr uint32_t kIdescSD = make_idesc(kBf16, false, false, BT, HT);   // S^T, dP^T: K-major operands, N = 64
       constexpr uint32_t kIdescOut = make_idesc(kBf16, false, true, BT, DP);   // dV, dK: A from TMEM, B MN-major
       constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
@@ -357,13 +356,12 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         // (the second commit: the item's last read of this warp's K or V tile of row g)
         const uint32_t bar2 = (h == 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
         const uint32_t tD = tmem + (h ? col_in1 : col_in0), qa = qb + h * HT * (RB >> 4);
-        if constexpr (DP == 16) {  // one K slice of 16
-          mma_ss_x1_commit(tD, ka, qa, kHiOp, kIdescSD, (sd_full + 2 * h).a, bar2);
-        } else if constexpr (DP == 32) {  // two
-          mma_ss_x2_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + 2 * h).a, bar2);
-        } else {                   // four
-          mma_ss_x4_commit(tD, ka, qa, kHiOp, 2, kIdescSD, (sd_full + 2 * h).a, bar2);
-        }
+        const uint32_t el = elect_one();
+#pragma unroll
+        for (int kk = 0; kk < DP / 16; ++kk)
+          mma_ss_e(el, tD, pack_desc(ka + 2 * kk, kHiOp), pack_desc(qa + 2 * kk, kHiOp), kIdescSD, kk > 0 ? 1u : 0u);
+        mma_commit_if_s(el, (sd_full + 2 * h).a);
+        if (bar2) mma_commit_if_s(el, bar2);
       };
       Pos cur{0, 0, 0u, 0u, 0u};
       if (total_steps > 0) {
@@ -393,8 +391,11 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           mbar_wait(cdone + 2 * h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
           tc_fence_after();
           const uint32_t tA = tmem + (h ? col_in1 : col_in0);
-          mma_ts_x4(acc, tA, ob + 4 * h * kRowBlk, kHiOp, kRowBlk, kIdescOut, h == 0 ? first0 : 1u);
-          if (h == 1) mma_commit_if_s(1u, st_empty_bar);
+          const uint32_t el = elect_one();
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ts_e(el, acc, tA + 16 * kk, pack_desc(ob + (4 * h + kk) * kRowBlk, kHiOp), kIdescOut, h == 0 && kk == 0 ? first0 : 1u);
+          if (h == 1) mma_commit_if_s(el, st_empty_bar);
           if (more) {
             if (h == 0) {
               mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
@@ -406,10 +407,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         }
         cur = nxt;
       }
-      }  // lane 0
     } else if (warp == kCW + 2) {
       // =============================== tensor-core issuer of dQ; pair-bias loads ===============================
-      if (lane == 0) {
       constexpr uint32_t kIdescDQ = make_idesc(kBf16, true, true, BT, DP);     // A = dS^T read MN-major, B = K MN-major
       constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
       constexpr uint32_t kHiDS = static_cast<uint32_t>(make_sdesc_const(16, 1024, SWZ_128B) >> 32);
@@ -422,8 +421,11 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       // for the group's first step and replaced as soon as the warps of that half have read it for
       // the last time.
       auto load_bias = [&](const StepT& d, int h) {
-        mbar_expect_tx(b_full + h, HT * kBRow);
-        tma_load_4d_s(sBias_s + h * (HT * kBRow), &tmB, (b_full + h).a, d.j0, d.it * BT + h * HT, d.h, d.b);
+        if (elect_one()) {
+          mbar_expect_tx(b_full + h, HT * kBRow);
+          tma_load_4d_s(sBias_s + h * (HT * kBRow), &tmB, (b_full + h).a, d.j0, d.it * BT + h * HT, d.h, d.b);
+        }
+        __syncwarp();
       };
       const int tiles = my_items * NT;
       if (has_bias && tiles > 0) { const StepT d0 = decode(0); load_bias(d0, 0); load_bias(d0, 1); }
@@ -444,26 +446,47 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tc_fence_after();
         const uint32_t ka = (kv_lo + (2 * g) * (L::kTile >> 4)) | kLoLbo;
         // dQ_i partial = dS K_j : A = dS^T tile [key][query] read MN-major (M = query), K runs over the keys
-        mma_ss_x8(tmem + colDQ + (n & 1) * DP, ds_lo | kLoLboDS, kHiDS, 128, ka, kHiOp, kRowBlk, kIdescDQ);
-        mma_commit_if(1u, dq_full + (n & 1));
-        mma_commit_if(1u, ds_empty);
-        if (it == NT - 1) mma_commit_if(1u, kv_empty + g);
+        const uint32_t el = elect_one();
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          mma_ss_e(el, tmem + colDQ + (n & 1) * DP, pack_desc((ds_lo | kLoLboDS) + 128 * kk, kHiDS), pack_desc(ka + kk * kRowBlk, kHiOp), kIdescDQ, kk > 0 ? 1u : 0u);
+        mma_commit_if_s(el, (dq_full + (n & 1)).a);
+        mma_commit_if_s(el, ds_empty.a);
+        if (it == NT - 1) mma_commit_if_s(el, (kv_empty + g).a);
         if (++g == G) { g = 0; ++t; if (++it == NT) it = 0; }
       }
-      }  // lane 0
     } else {
       // =============================== tile loader ===============================
       // K/V of row g stay for the whole item and are replaced when the item's last MMAs that read them
       // have completed; Q, dO and the two statistics vectors of a step ride a two-deep ring.
-      const uint32_t sKV_s = smem_u32(sKV), sStage_s = smem_u32(sStage);
+      const uint32_t sKV_s = smem_u32(sKV), sStage_s = smem_u32(sStage), sMask_s = smem_u32(smem + L::offMask);
+      auto mask_of = [&](int b, int s, int j) -> float {
+        if (s >= a.S || j >= a.R) return -__int_as_float(0x7f800000);
+        if (a.mask_kind == EVOATTN_MASK_NONE) return 0.f;
+        const long long mi = (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c;
+        if (a.mask_kind == EVOATTN_MASK_BOOL) return reinterpret_cast<const unsigned char*>(a.mask)[mi] ? 0.f : -__int_as_float(0x7f800000);
+        if (a.mask_kind == EVOATTN_MASK_ADD_F32) return reinterpret_cast<const float*>(a.mask)[mi] * kLog2e;
+        return to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]) * kLog2e;
+      };
       StepT d = decode(0);
 #pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const int stg = n % kStages;
         if (d.it == 0) {
           const int k = n / SPI;
+          // The mask of the row: four keys a lane, loaded before the wait.  In the log2 domain it is added to a
+          // score: 0 keeps it, -inf drops it (a dropped score gives P = 0 exactly, as exp(-FLT_MAX - lse)
+          // does in evoformer.py:69,600).  (The last dQ MMA of the row is behind kv_empty, so its last
+          // step has read the mask before.)
+          float mk[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mk[u] = mask_of(d.b, d.s, d.j0 + lane + 32 * u);
           mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
-          if (lane == 0) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) sts_f32(sMask_s + (d.g * BT + lane + 32 * u) * 4, mk[u]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(mk_full + d.g);
+          if (elect_one()) {
             const uint32_t dst = sKV_s + (2 * d.g) * L::kTile;
             mbar_expect_tx(kv_full + d.g, 2 * L::kTile);
             tma_load_5d_s(dst, &tmK, (kv_full + d.g).a, 0, d.j0, d.s, d.h, d.b);
@@ -472,7 +495,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           __syncwarp();
         }
         mbar_wait(st_empty + stg, ((n / kStages) & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t dst = sStage_s + stg * L::kStage;
           const uint32_t bar = (st_full + stg).a;
           mbar_expect_tx(st_full + stg, L::kStage);
@@ -490,7 +513,11 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     // Warps 0-7 work on half 0 (queries 0..63 of the tile) of every step, warps 8-15 on half 1: two
     // groups that run half a step apart, so that while one waits (for its S^T/dP^T, for tensor
     // memory, for its MMAs) the other has arithmetic to issue.  Warp w: keys 32*(w%4).. (its TMEM
-    // lanes), queries 32*((w/4)%2).. of its half, in two chunks of 16.
+    // lanes), queries 32*((w/4)%2).. of its half, in two chunks of 16.  Their instructions set the pace (five warps
+    // a scheduler, no wait of any length): positions are loop counters and the mask of a key comes staged.
+    // Backward calls with that, the issue loops walked by converged warps and the waits in one short sequence,
+    // before and after, us: [1,128,384,8,32] 211 -> 195, [1,384,384,4,32] 348 -> 306, [1,1024,384,8,8] fp16
+    // 1251 -> 1083, [1,128,768,8,64] 1195 -> 1148, [4,1,2048,32,64] without d(pair_bias) 819 -> 742.
     setmaxnreg_inc<kComputeRegs>();
     const int q4 = warp & 3, cb2 = (warp >> 2) & 1, H = warp >> 3;
     const int jrow = q4 * 32 + lane;
@@ -506,25 +533,6 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     const uint32_t brow0 = smem_u32(sBias) + (H * HT + QT * cb2) * kBRow + jrow * (kBias16 ? 2 : 4);
     const uint32_t drow = sDS_s + H * (L::kDS / 2) + jrow * 128;
 
-    // The residue mask of (b, s, key) in two halves, so that the load can be issued a step before
-    // its value is needed: the raw element ...
-    auto mask_fetch = [&](int b, int s, int j, bool wanted) -> uint32_t {
-      const bool ok = wanted && s < a.S && j < a.R && a.mask_kind != EVOATTN_MASK_NONE;
-      const long long mi = (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c;
-      if (a.mask_kind == EVOATTN_MASK_BOOL) return ldg_u8_if(reinterpret_cast<const unsigned char*>(a.mask) + mi, ok);
-      if (a.mask_kind == EVOATTN_MASK_ADD_F32) return ldg_u32_if(reinterpret_cast<const uint32_t*>(a.mask) + mi, ok);
-      return ldg_u16_if(reinterpret_cast<const uint16_t*>(a.mask) + mi, ok);
-    };
-    // ... and the float that is added to a score in the log2 domain: 0 keeps it, -inf drops it (a
-    // dropped score gives P = 0 exactly, as exp(-FLT_MAX - lse) does in evoformer.py:69,600)
-    auto mask_decode = [&](uint32_t raw, int s, int j) -> float {
-      if (s >= a.S || j >= a.R) return -kInf;
-      if (a.mask_kind == EVOATTN_MASK_NONE) return 0.f;
-      if (a.mask_kind == EVOATTN_MASK_BOOL) return raw ? 0.f : -kInf;
-      if (a.mask_kind == EVOATTN_MASK_ADD_F32) return __uint_as_float(raw) * kLog2e;
-      const uint16_t h16 = (uint16_t)raw;
-      return to_float<T>(*reinterpret_cast<const T*>(&h16)) * kLog2e;
-    };
     // This warp's staging area is free again once its previous bulk reduction has read it.
     auto staging_free = [&]() {
       if (lane == 0) tma_wait_group_read0();
@@ -572,7 +580,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     // warp's arrival, underneath the tensor core's turnaround for its half.
     constexpr int QC = DP / 4;       // dQ columns per warp (4, 8 or 16)
     const int colblk = 2 * H + cb2;  // which of the four column blocks this warp drains
-    auto send_dq = [&](int m, const StepT& d) {
+    // (row0: the first of the 32 query rows; slab: (b,h,s), negative for a padded row)
+    auto send_dq = [&](int m, int row0, int slab) {
       mbar_wait(dq_full + (m & 1), (m >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
       uint32_t qr[QC];
@@ -584,37 +593,40 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         sts_v4(out_s + lane * (QC * 4) + 16 * c, qr[4 * c], qr[4 * c + 1], qr[4 * c + 2], qr[4 * c + 3]);
       fence_async_shared();
       __syncwarp();
-      if (lane == 0 && d.s < a.S && colblk * QC < a.D) {
-        tma_reduce_add_3d_s(&tmDQ, out_s, colblk * QC, d.it * BT + q4 * 32, (d.b * a.H + d.h) * a.S + d.s);
+      if (lane == 0 && slab >= 0 && colblk * QC < a.D) {
+        tma_reduce_add_3d_s(&tmDQ, out_s, colblk * QC, row0, slab);
         tma_commit_group();
       }
     };
 
-    StepT cur = decode(0), prv = cur;
-    uint32_t mraw = mask_fetch(cur.b, cur.s, cur.j0 + jrow, total_steps > 0);
+    int p_row0 = 0, p_slab = -1;           // the step whose dQ partial has not left yet
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
+    const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
     const F2 l2e2 = f2_make(kLog2e, kLog2e), c12 = f2_make(c1, c1), neg1 = f2_make(-1.f, -1.f);
     F2 bacc[16];  // d(pair_bias) of this thread's key and its 32 queries, summed over the rows of a group
 #pragma unroll
     for (int e = 0; e < 16; ++e) bacc[e] = f2_make(0.f, 0.f);
 
+    int n = 0;          // running step
+    uint32_t tile = 0;  // running (item, query tile)
 #pragma unroll 1
-    for (int n = 0; n < total_steps; ++n) {
-      const StepT nxt = advance(cur, n + 1);
-      const bool more = n + 1 < total_steps;
-      const int g = cur.g;
-      const float mj = mask_decode(mraw, cur.s, cur.j0 + jrow);
-      const F2 mj2 = f2_make(mj, mj);
-      mraw = mask_fetch(nxt.b, nxt.s, nxt.j0 + jrow, more);  // in flight during this step
-      const int stg = n % kStages;
-      const uint32_t vec_s = sStage_s + stg * L::kStage + 2 * L::kTile;
+    for (int k = 0; k < my_items; ++k) {
+    const StepT cur = decode(n);
+#pragma unroll 1
+    for (int it = 0; it < NT; ++it, ++tile)
+#pragma unroll 1
+    for (int g = 0; g < G; ++g, ++n) {
+      const uint32_t vec_s = sStage_s + (n & 1) * L::kStage + 2 * L::kTile;
       const bool last_of_group = (g == G - 1);
+      if (it == 0) mbar_wait(mk_full + g, k & 1, abort_s, DEV_TIMEOUT_TMA);
+      const float mj = lds_f32(mask_s + g * (BT * 4));
       // the statistics vectors of this step are read with ordinary loads: observe their arrival here
-      mbar_wait(st_full + stg, (n / kStages) & 1, abort_s, DEV_TIMEOUT_TMA);
-      if (has_bias && g == 0) mbar_wait(b_full + H, (n / G) & 1, abort_s, DEV_TIMEOUT_TMA);
+      mbar_wait(st_full + (n & 1), (n >> 1) & 1, abort_s, DEV_TIMEOUT_TMA);
+      if (has_bias && g == 0) mbar_wait(b_full + H, tile & 1, abort_s, DEV_TIMEOUT_TMA);
       // a row whose keys are all dropped has nl = +inf for every query (the mask row is shared by
       // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
       const bool deadstep = (lds_f32(vec_s) == kInf);
+      const F2 mj2 = f2_make(mj, mj);
       uint32_t dk[16];
 #pragma unroll
       for (int sub = 0; sub < 2; ++sub) {
@@ -679,7 +691,15 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tmem_st8(cS + 16 * sub, pk);
         tmem_st8(cP + 16 * sub, *reinterpret_cast<uint32_t(*)[8]>(&dk[sub * 8]));
         // P^T and dS^T of this warp's score buffer are in tensor memory: its dV / dK MMAs may go
-        if (sub == 1 && H == 0 && cur.it == 0 && n >= SPI) drain_dkdv(pb, ph, ps0 + g, pj0, g);  // before those MMAs overwrite it
+        if (sub == 1 && H == 0 && it == 0 && k > 0) {  // before those MMAs overwrite it
+          // With one row per item the other half's MMAs of the step before belong to this slot too: wait until they
+          // are through.  With more rows, all of theirs were issued before the S^T and dP^T of this step.
+          if constexpr (G == 1) {
+            mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+            tc_fence_after();
+          }
+          drain_dkdv(pb, ph, ps0 + g, pj0, g);
+        }
         if (sub == 1) {
           tmem_wait_st();
           tc_fence_before();
@@ -702,7 +722,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           fence_async_shared();
           __syncwarp();
           if (lane == 0) {
-            tma_reduce_add_4d_s(&tmDB, out_s, cur.j0 + q4 * 32, cur.it * BT + H * HT + QT * cb2 + 16 * sub, cur.h, cur.b);
+            tma_reduce_add_4d_s(&tmDB, out_s, cur.j0 + q4 * 32, it * BT + H * HT + QT * cb2 + 16 * sub, cur.h, cur.b);
             tma_commit_group();
           }
         }
@@ -719,18 +739,19 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         mbar_arrive(sdone + H);
         if (has_bias && last_of_group) mbar_arrive(b_done + H);
       }
-      if (n > 0) send_dq(n - 1, prv);  // its MMAs ran underneath this step
-      if (cur.it == NT - 1 && last_of_group) { pb = cur.b; ph = cur.h; ps0 = cur.s - g; pj0 = cur.j0; }
-      prv = cur;
-      cur = nxt;
+      if (n > 0) send_dq(n - 1, p_row0, p_slab);  // its MMAs ran underneath this step
+      p_row0 = it * BT + q4 * 32;
+      p_slab = cur.s + g < a.S ? (cur.b * a.H + cur.h) * a.S + cur.s + g : -1;
+    }
+    pb = cur.b; ph = cur.h; ps0 = cur.s; pj0 = cur.j0;
     }
 
     if (total_steps > 0) {
-      send_dq(total_steps - 1, prv);
+      send_dq(total_steps - 1, p_row0, p_slab);
       if (H == 0) {
         // every dV / dK MMA of this CTA has completed once the last step's tile stage has been released
         const int last = total_steps - 1;
-        mbar_wait(st_empty + (last % kStages), (last / kStages) & 1, abort_s, DEV_TIMEOUT_MMA);
+        mbar_wait(st_empty + (last & 1), (last >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
         for (int g = 0; g < G; ++g) drain_dkdv(pb, ph, ps0 + g, pj0, g);
       }
