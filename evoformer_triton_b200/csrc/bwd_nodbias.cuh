@@ -1,0 +1,641 @@
+// The fused backward kernel for calls that want no d(pair_bias) (inference-like fine tuning, a frozen bias, no
+// bias at all): the same items, steps and halves as evo_bwd_sm100_kernel, whose file this one is part of.  What the
+// missing gradient makes room for in shared memory changes how dQ leaves: a step's partial is one swizzled tile
+// that the loader adds to global memory by one bulk reduction, where every compute warp had to wait for its own
+// staging area and issue a reduction of its own; and the bias has a third half tile.  The compute warps wait three
+// times a step (S^T and dP^T with the statistics; the bias; dQ of the step before with the place for it) instead of
+// five.  Bound, as the other form, by the instructions and hand-overs of the compute warps.  Backward calls, us,
+// against that form: [4,1,2048,32,64] 742 -> 570, [4,1,300,32,64] 46 -> 42, [1,128,384,8,32] without a bias 148 -> 139.
+// With a d(pair_bias) it is the slower of the two: the bulk reductions of both leave at some 16 bytes a cycle and SM
+// one after another ([1,128,384,8,32] 195 and 199, [1,128,768,8,64] 1 148 and 1 182).
+#pragma once
+
+constexpr int BIAS_NONE = 0, BIAS_F32 = 1, BIAS_16 = 2;
+
+template <int DP, int BIAS>
+struct SmemN {
+  static constexpr int G = RowsPerItem<DP>::G;
+  static constexpr int RB = DP * 2;                          // bytes per staged row
+  static constexpr int kTile = BT * RB;                      // one Q, dO, K or V tile
+  static constexpr int kVec = BT * 4;                        // one vector of row statistics
+  static constexpr int kStage = 2 * kTile + 2 * kVec;        // Q, dO, -lse*log2e, delta of one step
+  static constexpr int kDS = BT * BT * 2;                    // dS^T: two halves of [128 keys][64 queries]
+  // The pair bias: half tiles [64 i][128 j], unswizzled; one more than is read at a time where it fits
+  static constexpr int kHalfF32 = HT * BT * 4, kHalf = BIAS == BIAS_16 ? kHalfF32 / 2 : kHalfF32;
+  static constexpr int kBufs = BIAS == BIAS_NONE ? 0 : DP == 64 && BIAS == BIAS_F32 ? 2 : 3;
+  static constexpr int kOut = BT * DP * 4;                   // a step's dQ partial
+  static constexpr int kMaskRows = DP == 32 && BIAS == BIAS_F32 ? 0 : G;  // (in registers where a kilobyte is missing)
+  static constexpr int offKV = 0;                            // [g][K, V], resident for the whole item
+  static constexpr int offStage = offKV + 2 * G * kTile;
+  static constexpr int offDS = offStage + kStages * kStage;
+  static constexpr int offBias = offDS + kDS;
+  static constexpr int offOut = offBias + kBufs * kHalf;
+  static constexpr int offMask = offOut + kOut;              // [kMaskRows][128 keys]: what the mask adds to a score
+  static constexpr int offBars = offMask + kMaskRows * BT * 4;
+  // 64 barrier slots (see the kernel) and the slack for aligning the tiles to 1024 bytes, as much of it as
+  // fits: the kernel checks what the base address needs and gives up with a status code if it is more (the
+  // dynamic shared memory of a kernel without static shared memory starts on a 1024-byte boundary on this
+  // architecture, so it needs none).
+  static constexpr int kSlack = offBars + 512 + 1024 <= 232448 ? 1024 : 0;
+  static constexpr size_t bytes = offBars + 512 + kSlack;
+  static_assert(offDS % 1024 == 0 && kStage % 1024 == 0 && offStage % 1024 == 0 && offOut % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+  static_assert(bytes <= 232448, "shared memory budget of one CTA");
+};
+
+template <class T, int DP, int BIAS>
+__global__ void __launch_bounds__(kThreadsT, 1)
+evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CUtensorMap tmQ,
+                const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmB,
+                const __grid_constant__ CUtensorMap tmDQ,
+                const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL) {
+  using L = SmemN<DP, BIAS>;
+  constexpr int RB = L::RB;
+  constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
+  constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+  static_assert(DP == 16 || DP == 32 || DP == 64, "padded head dimension");
+  static_assert(kStages == 2, "steps alternate between two stages");
+  constexpr int G = RowsPerItem<DP>::G;
+  constexpr int kTmemCols = 512;
+  // TMEM: two (S^T, dP^T) half-tile buffers, the per-row dV and dK accumulators, two dQ partials
+  constexpr int colS0 = 0, colDP0 = HT, colS1 = 2 * HT, colDP1 = 3 * HT;
+  constexpr int colDV = 4 * HT, colDK = colDV + G * DP, colDQ = colDK + G * DP;
+  static_assert(colDQ + 2 * DP <= kTmemCols, "TMEM budget");
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if (static_cast<int>(smem - smem_raw) > L::kSlack) {  // the same for every thread of every CTA
+    if (threadIdx.x == 0 && a.status) atomicCAS(a.status, 0, DEV_TIMEOUT_SYNC);
+    return;
+  }
+  uint8_t* sKV = smem + L::offKV;
+  uint8_t* sStage = smem + L::offStage;
+  uint8_t* sDS = smem + L::offDS;
+  uint8_t* sBias = smem + L::offBias;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBars);
+  const uint32_t bars_s = smem_u32(bars);
+  const Bar kv_full{bars_s + 8 * 0};     // [G] K and V of row g of the current item landed
+  const Bar kv_empty{bars_s + 8 * 7};    // [G] ... and every MMA that reads them has completed
+  const Bar st_full{bars_s + 8 * 32};     // [2] Q, dO and the statistics vectors of a step landed
+  const Bar st_empty{bars_s + 8 * 40};    // [2] ... the step's last dV/dK MMAs have completed
+  const Bar sd_full{bars_s + 8 * 48};    // [2], two apart: S^T and dP^T of half h of a step are in TMEM, its statistics landed
+  const Bar cdone{bars_s + 8 * 52};      // [2], two apart: the warps of that half have its P^T and dS^T in TMEM (for the dV/dK MMAs)
+  const Bar sdone{bars_s + 8 * 23};      // [2] ... and dS in shared memory (for the dQ MMAs), with the dQ partial of the step before
+  const Bar b_full{bars_s + 8 * 56};     // [kBufs] a half (64 queries) of a pair-bias tile landed
+  const Bar b_done{bars_s + 8 * 60};     // [kBufs] ... has been read for the last time
+  const Bar dq_full{bars_s + 8 * 19};    // [2] the dQ partial of a step is complete in TMEM, the dS tile read, and the place for it free
+  const Bar mk_full{bars_s + 8 * 25};    // [G] the mask of row g of the current item is in shared memory
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 22);  // (bars 23, 24: sdone; 25..31: mk_full)
+  const uint32_t abort_s = smem_u32(const_cast<int*>(abort_flag));
+
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
+  const int NT = (a.R + BT - 1) / BT;
+  const int NC = (a.S + G - 1) / G;
+  constexpr bool has_bias = BIAS != BIAS_NONE, kBias16 = BIAS == BIAS_16;
+  // Whether the dV / dK MMAs of a half may go before its dS is stored, or all go at once ([4,1,2048,32,64] 597 us
+  // and 570; [1,128,384,8,32] without a bias 139 and 150).
+  constexpr bool EARLY = DP < 64;
+  constexpr int kBufs = has_bias ? L::kBufs : 1, kHalf = L::kHalf;
+  constexpr int kBRow = kBias16 ? BT * 2 : BT * 4;  // bytes per row (one query, 128 keys) of the staged bias tile
+  // Persistent CTAs: CTA c owns the items c, c + gridDim.x, ..., SPI steps per item.  A short last
+  // row group (S % G != 0) is padded with rows >= S: their tiles and statistics arrive as zeros and
+  // their mask is -inf, so P = dS = 0, and nothing of them is stored.
+  const int SPI = NT * G;
+  const int my_items = (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int total_steps = my_items * SPI;
+  auto decode = [&](int N) {
+    StepT d;
+    const int k = N / SPI, n = N - k * SPI;
+    d.it = n / G;
+    d.g = n - d.it * G;
+    int idx = (int)blockIdx.x + k * (int)gridDim.x;
+    const int chunk = idx % NC; idx /= NC;
+    d.j0 = (idx % NT) * BT; idx /= NT;
+    d.h = idx % a.H;
+    d.b = idx / a.H;
+    d.s = chunk * G + d.g;
+    return d;
+  };
+  auto advance = [&](const StepT& c, int n) {  // position of step n = the one after c (no divisions inside an item)
+    StepT d = c;
+    if (++d.g == G) {
+      d.g = 0;
+      if (++d.it == NT) return decode(n);
+    }
+    d.s = c.s - c.g + d.g;
+    return d;
+  };
+
+  // What the mask adds to a score of (b, s, key) in the log2 domain: 0 keeps it, -inf drops it (a dropped score
+  // gives P = 0 exactly, as exp(-FLT_MAX - lse) does in evoformer.py:69,600).
+  auto mask_of = [&](int b, int s, int j) -> float {
+    if (s >= a.S || j >= a.R) return -__int_as_float(0x7f800000);
+    if (a.mask_kind == EVOATTN_MASK_NONE) return 0.f;
+    const long long mi = (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c;
+    if (a.mask_kind == EVOATTN_MASK_BOOL) return reinterpret_cast<const unsigned char*>(a.mask)[mi] ? 0.f : -__int_as_float(0x7f800000);
+    if (a.mask_kind == EVOATTN_MASK_ADD_F32) return reinterpret_cast<const float*>(a.mask)[mi] * kLog2e;
+    return to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]) * kLog2e;
+  };
+
+  grid_dependency_wait();
+  grid_launch_dependents();
+  if (tid == 0) *abort_flag = (a.status && *reinterpret_cast<volatile int*>(a.status) != 0) ? 1 : 0;
+  __syncthreads();
+  if (*abort_flag) return;
+
+  if (tid == 0) {
+    for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); mbar_init(bars + 25 + i, 1); }  // kv_full; kv_empty: three MMA warps read K/V
+    for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bars + 48 + 2 * i, 3); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full: two commits, one warp; cdone
+      mbar_init(bars + 19 + i, 2);                                     // dq_full: the commit, and the loader
+    }
+    for (int i = 0; i < kBufs; ++i) { mbar_init(bars + 56 + i, 1); mbar_init(bars + 60 + i, kCW / 2); }  // b_full, b_done
+    for (int i = 0; i < 2; ++i) mbar_init(bars + 23 + i, kCW / 2);  // sdone
+    fence_mbar_init();
+    prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmDO);
+    prefetch_tmap(&tmNL); prefetch_tmap(&tmDL);
+    prefetch_tmap(&tmDQ);
+    if (has_bias) prefetch_tmap(&tmB);
+  }
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+  if (warp >= kCW) {
+    setmaxnreg_dec<kServiceRegs>();
+    if (warp <= kCW + 1) {
+      // =============================== tensor-core issuers: warp 16 (S^T, dV), warp 17 (dP^T, dK) ==========
+      // Issuing a tcgen05.mma costs the issuing warp fifty cycles and more, so the 32 MMAs of a step
+      // are spread over three warps on three schedulers.  A thread's MMAs run in issue order, MMAs of
+      // different threads in no particular order, so the split follows the data: warp 16 owns the
+      // S^T columns of both buffers (S^T = K_j Q_i^T in, dV_j += P^T dO_i out), warp 17 the dP^T columns
+      // (dP^T = V_j dO_i^T in, dK_j += dS^T Q_i out): the MMA that overwrites a buffer is always issued
+      // by the thread that issued the MMAs reading it.  Warp 18 issues dQ_i = dS K_j, which depends on
+      // neither.  The warps walk their loops converged (see elect_one).
+      const bool isA = (warp == kCW);
+      constexpr uint32_t kIdescSD = make_idesc(kBf16, false, false, BT, HT);   // S^T, dP^T: K-major operands, N = 64
+      constexpr uint32_t kIdescOut = make_idesc(kBf16, false, true, BT, DP);   // dV, dK: A from TMEM, B MN-major
+      constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
+      constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
+      constexpr uint32_t kRowBlk = (16 * RB) >> 4;  // 16 tile rows, in descriptor address units
+      // warp 16 reads K (A operand) and Q (B), then dO (B of dV); warp 17 reads V and dO, then Q (B of dK)
+      const uint32_t kv_lo = (smem_u32(sKV) >> 4) + (isA ? 0 : (L::kTile >> 4));
+      const uint32_t in_lo = (smem_u32(sStage) >> 4) + (isA ? 0 : (L::kTile >> 4));
+      const uint32_t out_lo = (smem_u32(sStage) >> 4) + (isA ? (L::kTile >> 4) : 0);
+      const uint32_t col_in0 = isA ? colS0 : colDP0, col_in1 = isA ? colS1 : colDP1;
+      const uint32_t col_acc = isA ? colDV : colDK;
+
+      // Position of a step inside this CTA's list, advanced without divisions: row g of the group,
+      // query tile it, ring stage and the parities of the stage ring and of the item.
+      struct Pos { int g, it; uint32_t stg, ring_par, item_par; };
+      auto after = [&](Pos p) {
+        if (++p.g == G) { p.g = 0; if (++p.it == NT) { p.it = 0; p.item_par ^= 1u; } }
+        if (++p.stg == (uint32_t)kStages) { p.stg = 0; p.ring_par ^= 1u; }
+        return p;
+      };
+      // Everything an MMA group needs is computed before the wait it follows: this thread shares its
+      // scheduler with four arithmetic warps, so every instruction between the wake-up and the MMA is
+      // paid several times over, and it sits on the critical path of the half that waits for it.
+      auto issue_in = [&](const Pos& p, uint32_t ka, uint32_t qb, int h) {
+        // (the second commit: the item's last read of this warp's K or V tile of row g)
+        const uint32_t bar2 = (h == 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
+        const uint32_t tD = tmem + (h ? col_in1 : col_in0), qa = qb + h * HT * (RB >> 4);
+        const uint32_t el = elect_one();
+#pragma unroll
+        for (int kk = 0; kk < DP / 16; ++kk)
+          mma_ss_e(el, tD, pack_desc(ka + 2 * kk, kHiOp), pack_desc(qa + 2 * kk, kHiOp), kIdescSD, kk > 0 ? 1u : 0u);
+        mma_commit_if_s(el, (sd_full + 2 * h).a);
+        if (bar2) mma_commit_if_s(el, bar2);
+        // The compute warps wait for S^T, dP^T and the statistics at once: this warp has seen these land.
+        if (isA) {
+          if (el) mbar_arrive(sd_full + 2 * h);
+          __syncwarp();
+        }
+      };
+      Pos cur{0, 0, 0u, 0u, 0u};
+      if (total_steps > 0) {
+        mbar_wait(st_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
+        mbar_wait(kv_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
+        tc_fence_after();
+        const uint32_t ka = (kv_lo + 0) | kLoLbo, qb = in_lo | kLoLbo;
+        issue_in(cur, ka, qb, 0);
+        issue_in(cur, ka, qb, 1);
+      }
+#pragma unroll 1
+      for (int n = 0; n < total_steps; ++n) {
+        const Pos nxt = after(cur);
+        const bool more = n + 1 < total_steps;
+        // this step: dV_j[g] += P^T dO_i (warp 16) or dK_j[g] += dS^T Q_i (warp 17);
+        // A = 16 queries of P^T / dS^T (8 packed TMEM columns), B = their dO / Q rows
+        const uint32_t acc = tmem + col_acc + cur.g * DP;
+        const uint32_t ob = (out_lo + cur.stg * (L::kStage >> 4)) | kLoLbo;
+        const uint32_t first0 = (cur.it == 0) ? 0u : 1u;  // the item's first MMA of row g overwrites
+        const uint32_t st_empty_bar = (st_empty + (int)cur.stg).a;
+        // next step: S^T = K_j Q_i^T (warp 16) or dP^T = V_j dO_i^T (warp 17) into the buffer just read
+        const uint32_t ka = (kv_lo + (2 * nxt.g) * (L::kTile >> 4)) | kLoLbo;
+        const uint32_t qb = (in_lo + nxt.stg * (L::kStage >> 4)) | kLoLbo;
+        const uint32_t st_full_bar = (st_full + (int)nxt.stg).a, kv_full_bar = (kv_full + nxt.g).a;
+        auto issue_out = [&](int h) {
+          mbar_wait(cdone + 2 * h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+          tc_fence_after();
+          const uint32_t tA = tmem + (h ? col_in1 : col_in0);
+          const uint32_t el = elect_one();
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            mma_ts_e(el, acc, tA + 16 * kk, pack_desc(ob + (4 * h + kk) * kRowBlk, kHiOp), kIdescOut, h == 0 && kk == 0 ? first0 : 1u);
+          if (h == 1) mma_commit_if_s(el, st_empty_bar);
+        };
+        issue_out(0);
+        if (more) {
+          mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
+          if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, DEV_TIMEOUT_TMA);
+          tc_fence_after();
+          issue_in(nxt, ka, qb, 0);
+        }
+        issue_out(1);
+        if (more) issue_in(nxt, ka, qb, 1);
+        cur = nxt;
+      }
+    } else if (warp == kCW + 2) {
+      // =============================== tensor-core issuer of dQ; pair-bias loads ===============================
+      constexpr uint32_t kIdescDQ = make_idesc(kBf16, true, true, BT, DP);     // A = dS^T read MN-major, B = K MN-major
+      constexpr uint32_t kHiDS = static_cast<uint32_t>(make_sdesc_const(16, 1024, SWZ_128B) >> 32);
+      constexpr uint32_t kLoLboDS = static_cast<uint32_t>(make_sdesc_const(BT * 128, 0, 0) & 0xffffffffu);
+      const uint32_t kv_lo0 = smem_u32(sKV) >> 4, ds_lo = smem_u32(sDS) >> 4;
+      constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
+      constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
+      constexpr uint32_t kRowBlk = (16 * RB) >> 4;  // 16 tile rows, in descriptor address units
+      const uint32_t sBias_s = smem_u32(sBias);
+      // The bias tile (i, j) is the same for the G rows of a group.  Its halves (64 queries) go round the
+      // buffers: half q = 2 * tile + h is loaded into buffer q % kBufs when the warps that read half q - kBufs
+      // there have done so for the last time.
+      auto load_bias = [&](uint32_t q) {
+        const StepT d = decode((int)(q >> 1) * G);
+        const uint32_t buf = q % kBufs;
+        if (elect_one()) {
+          mbar_expect_tx(b_full + (int)buf, kHalf);
+          tma_load_4d_s(sBias_s + buf * kHalf, &tmB, (b_full + (int)buf).a, d.j0, d.it * BT + (int)(q & 1) * HT, d.h, d.b);
+        }
+        __syncwarp();
+      };
+      const uint32_t halves = has_bias ? 2u * my_items * NT : 0u;
+#pragma unroll 1
+      for (uint32_t q = 0; q < kBufs && q < halves; ++q) load_bias(q);
+      int g = 0, it = 0;  // row of the group, query tile
+      uint32_t q = 0;     // half tile that is read next for the last time
+#pragma unroll 1
+      for (int n = 0; n < total_steps; ++n) {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          mbar_wait(sdone + h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+          if (has_bias && g == G - 1) {  // the group's last step
+            if (q + kBufs < halves) {
+              mbar_wait(b_done + (int)(q % kBufs), (q / kBufs) & 1, abort_s, DEV_TIMEOUT_SYNC);
+              load_bias(q + kBufs);
+            }
+            ++q;
+          }
+        }
+        tc_fence_after();
+        // dQ_i partial = dS K_j : A = dS^T tile [key][query] read MN-major (M = query), K runs over the keys
+        const uint32_t kq = (kv_lo0 + (2 * g) * (L::kTile >> 4)) | kLoLbo;
+        const uint32_t el = elect_one();
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          mma_ss_e(el, tmem + colDQ + (n & 1) * DP, pack_desc((ds_lo | kLoLboDS) + 128 * kk, kHiDS), pack_desc(kq + kk * kRowBlk, kHiOp), kIdescDQ, kk > 0 ? 1u : 0u);
+        mma_commit_if_s(el, (dq_full + (n & 1)).a);
+        if (it == NT - 1) mma_commit_if_s(el, (kv_empty + g).a);
+        if (++g == G) { g = 0; if (++it == NT) it = 0; }
+      }
+    } else {
+      // =============================== tile loader ===============================
+      // K/V of row g stay for the whole item and are replaced when the item's last MMAs that read them
+      // have completed; Q, dO and the two statistics vectors of a step ride a two-deep ring.
+      const uint32_t sKV_s = smem_u32(sKV), sStage_s = smem_u32(sStage), sMask_s = smem_u32(smem + L::offMask);
+      // A step's dQ partial leaves from here too: it is in shared memory when the next step's dS is.  When the
+      // reduction has read the place, the next one may be stored there, for which the compute warps wait on
+      // dq_full (so sdone of a step cannot come before this warp has seen that of the step before).
+      const uint32_t sOut_s = smem_u32(smem + L::offOut);
+      auto send_dq = [&](int row0, int slab) {
+        if (elect_one()) {
+          if (slab >= 0) {
+            tma_reduce_add_3d_s(&tmDQ, sOut_s, 0, row0, slab);
+            if (DP == 64 && a.D > 32) tma_reduce_add_3d_s(&tmDQ, sOut_s + BT * 128, 32, row0, slab);
+          }
+          tma_commit_group();
+        }
+        __syncwarp();
+      };
+      auto dq_place_free = [&](int m) {  // for the partial of step m
+        if (elect_one()) {
+          tma_wait_group_read0();
+          mbar_arrive(dq_full + (m & 1));
+        }
+        __syncwarp();
+      };
+      StepT d = decode(0);
+      auto load_kv = [&](int n) {
+        const int k = n / SPI;
+        float mk[4];
+        if constexpr (L::kMaskRows > 0) {  // four keys of the row's mask a lane, loaded before the wait
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mk[u] = mask_of(d.b, d.s, d.j0 + lane + 32 * u);
+        }
+        mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
+        if constexpr (L::kMaskRows > 0) {
+          // (the last dQ MMA of the row is behind kv_empty, so its last step has read the mask before)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) sts_f32(sMask_s + (d.g * BT + lane + 32 * u) * 4, mk[u]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(mk_full + d.g);
+        }
+        if (elect_one()) {
+          const uint32_t dst = sKV_s + (2 * d.g) * L::kTile;
+          mbar_expect_tx(kv_full + d.g, 2 * L::kTile);
+          tma_load_5d_s(dst, &tmK, (kv_full + d.g).a, 0, d.j0, d.s, d.h, d.b);
+          tma_load_5d_s(dst + L::kTile, &tmV, (kv_full + d.g).a, 0, d.j0, d.s, d.h, d.b);
+        }
+        __syncwarp();
+      };
+      int row1 = 0, slab1 = -1, row2 = 0, slab2 = -1, row3 = 0, slab3 = -1;  // of one, two and three steps ago
+#pragma unroll 1
+      for (int n = 0; n < total_steps + 2; ++n) {
+        const int stg = n % kStages;
+        const bool load = n < total_steps;
+        // (with one row per item, kv_empty waits for the step before, which waits for dq_place_free)
+        if (G > 1 && load && d.it == 0) load_kv(n);
+        mbar_wait(st_empty + stg, ((n / kStages) & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);  // (of step n - 2)
+        if (load) {
+          if (elect_one()) {
+            const uint32_t dst = sStage_s + stg * L::kStage;
+            const uint32_t bar = (st_full + stg).a;
+            mbar_expect_tx(st_full + stg, L::kStage);
+            tma_load_5d_s(dst, &tmQ, bar, 0, d.it * BT, d.s, d.h, d.b);
+            tma_load_5d_s(dst + L::kTile, &tmDO, bar, 0, d.it * BT, d.s, d.h, d.b);
+            tma_load_3d_s(dst + 2 * L::kTile, &tmNL, bar, d.it * BT, d.s, d.b * a.H + d.h);
+            tma_load_3d_s(dst + 2 * L::kTile + L::kVec, &tmDL, bar, d.it * BT, d.s, d.b * a.H + d.h);
+          }
+          __syncwarp();
+        }
+        {
+          if (n >= 2) {
+            mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+            mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+            if (n >= 3) send_dq(row3, slab3);
+            dq_place_free(n - 2);
+          }
+          row3 = row2; slab3 = slab2;
+          row2 = row1; slab2 = slab1;
+          row1 = d.it * BT;
+          slab1 = d.s < a.S ? (d.b * a.H + d.h) * a.S + d.s : -1;
+        }
+        if (G == 1 && load && d.it == 0) load_kv(n);
+        if (load) d = advance(d, n + 1);
+      }
+      if (total_steps > 0) {  // the last step's partial: the compute warps arrive once more
+        mbar_wait(sdone + 0, total_steps & 1, abort_s, DEV_TIMEOUT_SYNC);
+        mbar_wait(sdone + 1, total_steps & 1, abort_s, DEV_TIMEOUT_SYNC);
+        send_dq(row3, slab3);
+        if (elect_one()) tma_wait_group0();
+        __syncwarp();
+      }
+    }
+  } else {
+    // =============================== compute warps ===============================
+    // Warps 0-7 work on half 0 (queries 0..63 of the tile) of every step, warps 8-15 on half 1: two
+    // groups that run half a step apart, so that while one waits (for its S^T/dP^T, for tensor
+    // memory, for its MMAs) the other has arithmetic to issue.  Warp w: keys 32*(w%4).. (its TMEM
+    // lanes), queries 32*((w/4)%2).. of its half, in two chunks of 16.
+    setmaxnreg_inc<kComputeRegs>();
+    const int q4 = warp & 3, cb2 = (warp >> 2) & 1, H = warp >> 3;
+    const int jrow = q4 * 32 + lane;
+    const uint32_t t_lane = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
+    const uint32_t cS = t_lane + (H ? colS1 : colS0) + QT * cb2, cP = t_lane + (H ? colDP1 : colDP0) + QT * cb2;
+    const float scale = a.scale;
+    const float inv_r = 1.f / (float)a.R;
+    const float kInf = __int_as_float(0x7f800000);
+    const float c1 = scale * kLog2e;
+    // 32-bit shared-window addresses: every access below stays a shared-memory instruction
+    const uint32_t sStage_s = smem_u32(sStage), sDS_s = smem_u32(sDS);
+    const uint32_t sBias_s = smem_u32(sBias);
+    const uint32_t drow = sDS_s + H * (L::kDS / 2) + jrow * 128;
+
+    // dK, dV of row-group slot g (MSA row s of (b,h), keys j0..): TMEM -> registers -> global.
+    // Done by the warps of half 0 (half of the DP columns each, 16 at a time): they are the ones
+    // whose arrival lets the next item's first MMAs overwrite the slot.
+    auto drain_dkdv = [&](int b, int h, int s, int j0, int g) {
+      const int j = j0 + jrow;
+      constexpr int W = DP == 16 ? 8 : 16;  // columns at a time
+#pragma unroll
+      for (int part = 0; part < DP / 2 / W; ++part) {
+        const int c0 = cb2 * (DP / 2) + part * W;
+        uint32_t kr[W], vr[W];
+        tmem_ld<W>(t_lane + colDK + g * DP + c0, kr);
+        tmem_ld<W>(t_lane + colDV + g * DP + c0, vr);
+        tmem_wait_ld();
+        if (j < a.R && s < a.S) {
+          T* kd = reinterpret_cast<T*>(a.dk) + off4(a.sdk, b, h, s, j) + c0;
+          T* vd = reinterpret_cast<T*>(a.dv) + off4(a.sdv, b, h, s, j) + c0;
+#pragma unroll
+          for (int d8 = 0; d8 < W / 8; ++d8) {
+            if (c0 + d8 * 8 < a.D) {
+              uint4 pk, pv;
+              pk.x = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 0]) * scale, __uint_as_float(kr[d8 * 8 + 1]) * scale);
+              pk.y = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 2]) * scale, __uint_as_float(kr[d8 * 8 + 3]) * scale);
+              pk.z = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 4]) * scale, __uint_as_float(kr[d8 * 8 + 5]) * scale);
+              pk.w = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 6]) * scale, __uint_as_float(kr[d8 * 8 + 7]) * scale);
+              pv.x = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 0]), __uint_as_float(vr[d8 * 8 + 1]));
+              pv.y = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 2]), __uint_as_float(vr[d8 * 8 + 3]));
+              pv.z = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 4]), __uint_as_float(vr[d8 * 8 + 5]));
+              pv.w = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 6]), __uint_as_float(vr[d8 * 8 + 7]));
+              *reinterpret_cast<uint4*>(kd + d8 * 8) = pk;
+              *reinterpret_cast<uint4*>(vd + d8 * 8) = pv;
+            }
+          }
+        }
+      }
+    };
+    // The dQ partial of step m (TMEM lanes = queries): a warp takes DP/4 columns of its 32 query rows.
+    constexpr int QC = DP / 4;
+    const int colblk = 2 * H + cb2;  // which of the four column blocks this warp takes
+    // ... into the swizzled tile (two of 32 columns at DP = 64) that leaves as a whole
+    auto store_dq = [&](int m) {
+      uint32_t qr[QC];
+      tmem_ld<QC>(t_lane + colDQ + (m & 1) * DP + colblk * QC, qr);
+      tmem_wait_ld();
+      const uint32_t out = smem_u32(smem + L::offOut);
+#pragma unroll
+      for (int c = 0; c < QC / 4; ++c) {
+        const int c16 = colblk * (QC / 4) + c;  // 16-byte piece of the row
+        const uint32_t at = DP == 16 ? jrow * 64 + ((c16 ^ ((jrow >> 1) & 3)) << 4)
+                                     : (c16 >> 3) * (BT * 128) + jrow * 128 + (((c16 & 7) ^ (jrow & 7)) << 4);
+        sts_v4(out + at, qr[4 * c], qr[4 * c + 1], qr[4 * c + 2], qr[4 * c + 3]);
+      }
+    };
+    int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
+    const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
+    float mreg[DP == 32 ? G : 1];
+    const F2 l2e2 = f2_make(kLog2e, kLog2e), c12 = f2_make(c1, c1), neg1 = f2_make(-1.f, -1.f);
+    int n = 0;            // running step
+    uint32_t tile = 0;    // running (item, query tile)
+    uint32_t bias_s = 0;  // the half bias tile that this warp reads
+    Bar bdone{0};
+#pragma unroll 1
+    for (int k = 0; k < my_items; ++k) {
+    const StepT cur = decode(n);
+    if constexpr (L::kMaskRows == 0) {
+#pragma unroll
+      for (int r = 0; r < G; ++r) mreg[r] = mask_of(cur.b, cur.s + r, cur.j0 + jrow);
+    }
+#pragma unroll 1
+    for (int it = 0; it < NT; ++it, ++tile)
+#pragma unroll 1
+    for (int g = 0; g < G; ++g, ++n) {
+      const uint32_t vec_s = sStage_s + (n & 1) * L::kStage + 2 * L::kTile;
+      const bool last_of_group = (g == G - 1);
+      float mj;
+      if constexpr (L::kMaskRows == 0) {
+        mj = g == 0 ? mreg[0] : g == 1 ? mreg[1] : mreg[2];
+      } else {
+        if (it == 0) mbar_wait(mk_full + g, k & 1, abort_s, DEV_TIMEOUT_TMA);
+        mj = lds_f32(mask_s + g * (BT * 4));
+      }
+      if (has_bias && g == 0) {
+        const uint32_t q = 2 * tile + H;
+        bias_s = sBias_s + (q % kBufs) * kHalf;
+        bdone = b_done + (int)(q % kBufs);
+        mbar_wait(b_full + (int)(q % kBufs), (q / kBufs) & 1, abort_s, DEV_TIMEOUT_TMA);
+      }
+      const uint32_t brow0 = bias_s + QT * cb2 * kBRow + jrow * (kBias16 ? 2 : 4);
+      mbar_wait(sd_full + 2 * H, n & 1, abort_s, DEV_TIMEOUT_MMA);  // S^T and dP^T, statistics
+      tc_fence_after();
+      // a row whose keys are all dropped has nl = +inf for every query (the mask row is shared by
+      // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
+      const bool deadstep = (lds_f32(vec_s) == kInf);
+      const F2 mj2 = f2_make(mj, mj);
+      uint32_t dk[16];
+#pragma unroll
+      for (int sub = 0; sub < 2; ++sub) {
+        // this warp's queries of the half: 32*cb2 + 16*sub .. +16
+        uint32_t sr[16], dr[16];
+        tmem_ld16(cS + 16 * sub, sr);
+        tmem_ld16(cP + 16 * sub, dr);
+        const uint32_t vnl = vec_s + (H * HT + QT * cb2 + 16 * sub) * 4, vdl = vnl + BT * 4;
+        const uint32_t brow = brow0 + (16 * sub) * kBRow;
+        tmem_wait_ld();
+        uint32_t pk[8];
+        if (!deadstep) {
+#pragma unroll
+          for (int c4 = 0; c4 < 4; ++c4) {
+            const float4 nl = lds_v4f(vnl + 16 * c4);
+            const float4 dl = lds_v4f(vdl + 16 * c4);
+            // two queries per instruction (the pairs lie side by side in every operand)
+            F2 t[2] = {f2_make(nl.x, nl.y), f2_make(nl.z, nl.w)};
+            const F2 de[2] = {f2_make(dl.x, dl.y), f2_make(dl.z, dl.w)};
+            if (has_bias) {
+              float bv[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                if constexpr (kBias16) {
+                  const uint16_t raw = lds_u16(brow + (4 * c4 + u) * kBRow);
+                  bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
+                } else {
+                  bv[u] = lds_f32(brow + (4 * c4 + u) * kBRow);
+                }
+              }
+              t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
+              t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int e = 4 * c4 + 2 * u;
+              // x = S*(scale*log2e) + (bias*log2e - lse*log2e) + mask
+              float x0, x1;
+              f2_get(f2_add(f2_fma(f2_from_bits(sr[e], sr[e + 1]), c12, t[u]), mj2), x0, x1);
+              const float p0 = ex2(x0), p1 = ex2(x1);
+              // dS = P (dP - delta)
+              const F2 ds = f2_mul(f2_make(p0, p1), f2_fma(de[u], neg1, f2_from_bits(dr[e], dr[e + 1])));
+              float d0, d1;
+              f2_get(ds, d0, d1);
+              pk[2 * c4 + u] = Pack2<T>::pack(p0, p1);
+              dk[sub * 8 + 2 * c4 + u] = Pack2<T>::pack(d0, d1);
+            }
+          }
+        } else {
+          const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
+          const uint32_t w = Pack2<T>::pack(pu, pu);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) { pk[e] = w; dk[sub * 8 + e] = 0u; }  // replaced scores are constants: dS = 0
+        }
+        // P^T and dS^T, two 16-bit values per column, over the columns this thread has just read:
+        // the A operands of the dV and dK MMAs (16 queries = 8 packed columns each)
+        tmem_st8(cS + 16 * sub, pk);
+        tmem_st8(cP + 16 * sub, *reinterpret_cast<uint32_t(*)[8]>(&dk[sub * 8]));
+      }
+      if (H == 0 && it == 0 && k > 0) {  // before this step's dV / dK MMAs overwrite them
+        // With one row per item the other half's MMAs of the step before belong to them too; with more rows, all of
+        // theirs were issued before the S^T and dP^T of this step.
+        if constexpr (G == 1) {
+          mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+          tc_fence_after();
+        }
+        drain_dkdv(pb, ph, ps0 + g, pj0, g);
+      }
+      // P^T and dS^T are in tensor memory: the dV / dK MMAs and the next S^T and dP^T may go, under what follows
+      if constexpr (EARLY) {
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(cdone + 2 * H);
+      }
+      // dQ of the previous step is complete, and the place it leaves from is free
+      if (n > 0) mbar_wait(dq_full + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+      tc_fence_after();
+      if (n > 0) store_dq(n - 1);
+      // dS^T -> shared memory, [key][query] rows of 128 bytes per half, 128-byte swizzle
+#pragma unroll
+      for (int c = 0; c < 4; ++c)  // dk[4 * c ..]: queries 32 * cb2 + 8 * c .. of this half
+        sts_v4(drow + (((4 * cb2 + c) ^ (jrow & 7)) << 4), dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
+      fence_async_shared();
+      if constexpr (!EARLY) tmem_wait_st();
+      tc_fence_before();  // (the next MMAs into the dQ columns just read follow from this arrival)
+      __syncwarp();
+      if (lane == 0) {
+        if constexpr (!EARLY) mbar_arrive(cdone + 2 * H);
+        mbar_arrive(sdone + H);
+        if (has_bias && last_of_group) mbar_arrive(bdone);
+      }
+    }
+    pb = cur.b; ph = cur.h; ps0 = cur.s; pj0 = cur.j0;
+    }
+
+    if (total_steps > 0) {
+      mbar_wait(dq_full + ((total_steps - 1) & 1), ((total_steps - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+      tc_fence_after();
+      store_dq(total_steps - 1);
+      fence_async_shared();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sdone + H);
+      if (H == 0) {
+        // every dV / dK MMA of this CTA has completed once the last step's tile stage has been released
+        const int last = total_steps - 1;
+        mbar_wait(st_empty + (last & 1), (last >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+        tc_fence_after();
+        for (int g = 0; g < G; ++g) drain_dkdv(pb, ph, ps0 + g, pj0, g);
+      }
+    }
+  }
+
+  if (*abort_flag) report_abort(*abort_flag, a.status);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+}

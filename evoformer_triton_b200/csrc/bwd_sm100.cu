@@ -765,6 +765,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
+#include "bwd_nodbias.cuh"
+
 size_t align_up(size_t x, size_t al) { return (x + al - 1) / al * al; }
 
 // One vector of row statistics: [B,H,S,delta_ld] fp32.
@@ -793,7 +795,11 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   if (!make_qkv_map(&tk, a.k, a.sk, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tv, a.v, a.sv, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tdo, a.d_o, a.sdo, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
-  if (!make_rows_f32_plain_map(&tdq, dq_acc, a.D, a.R, (long long)a.B * a.H * a.S, DP / 4, 32)) return EVOATTN_ERR_CUDA;
+  const bool nodbias = !a.dbias;
+  const long long slabs = (long long)a.B * a.H * a.S;
+  if (!(nodbias ? make_rows_f32_map(&tdq, dq_acc, a.D, a.R, slabs, DP < 32 ? DP : 32, BT, /*swizzle=*/true)
+                : make_rows_f32_map(&tdq, dq_acc, a.D, a.R, slabs, DP / 4, 32, /*swizzle=*/false)))
+    return EVOATTN_ERR_CUDA;
   if (!make_stats_map(&tnl, nl, a.B * a.H, a.S, a.R, a.delta_ld, BT)) return EVOATTN_ERR_CUDA;
   if (!make_stats_map(&tdl, a.delta, a.B * a.H, a.S, a.R, a.delta_ld, BT)) return EVOATTN_ERR_CUDA;
   tb = tq;
@@ -811,14 +817,18 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   const int sms = sm_count();
   if (sms <= 0) return EVOATTN_ERR_CUDA;
   const long long ctas = items < sms ? items : sms;
-  auto kern = !a.bias ? evo_bwd_sm100_kernel<T, DP, false, false>
-                      : (a.bias16 ? evo_bwd_sm100_kernel<T, DP, true, true> : evo_bwd_sm100_kernel<T, DP, true, false>);
+  const auto kern = a.bias16 ? evo_bwd_sm100_kernel<T, DP, true, true> : evo_bwd_sm100_kernel<T, DP, true, false>;
+  const auto kern_n = !a.bias ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_NONE>
+                      : (a.bias16 ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_16> : evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_F32>);
+  const void* entry = nodbias ? reinterpret_cast<const void*>(kern_n) : reinterpret_cast<const void*>(kern);
+  const size_t smem = !nodbias ? L::bytes : !a.bias ? SmemN<DP, BIAS_NONE>::bytes : a.bias16 ? SmemN<DP, BIAS_16>::bytes : SmemN<DP, BIAS_F32>::bytes;
   // setmaxnreg.inc waits until the scheduler's register pool (five warps at the launch-time count)
   // has what it asks for: never launch a build whose pool cannot hold the warps' requests.
   int num_regs = 0;
-  if (!kernel_ready(reinterpret_cast<const void*>(kern), (int)L::bytes, &num_regs)) return EVOATTN_ERR_CUDA;
+  if (!kernel_ready(entry, (int)smem, &num_regs)) return EVOATTN_ERR_CUDA;
   if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
-  launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, L::bytes, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
+  if (nodbias) launch_dependent(kern_n, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdq, tnl, tdl);
+  else launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
   if (a.dbias_out) {
     const int rc = launch_dbias_out(a, st, launches);
     if (rc) return rc;

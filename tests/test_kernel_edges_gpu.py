@@ -185,3 +185,42 @@ def test_forward_items_of_each_size(cfg):
     assert (lse.double() - want_lse)[live].abs().max().item() < 2e-5
     if mask == "bool":
         assert (lse[~live] == torch.finfo(torch.float32).min).all()
+
+
+@pytest.mark.parametrize("cfg", [
+    # B, S, R, H, D, dtype, mask, bias
+    (1, 5, 200, 2, 32, torch.bfloat16, "bool", "none"), (1, 70, 264, 8, 32, torch.float16, "addsame", "same"),
+    (2, 61, 132, 8, 24, torch.bfloat16, "bool", "fp32"), (1, 64, 130, 8, 8, torch.float16, "add32", "none"),
+    (1, 63, 200, 8, 16, torch.bfloat16, "bool", "same"), (1, 40, 300, 8, 64, torch.bfloat16, "bool", "none"),
+    (2, 1, 520, 4, 48, torch.float16, "addsame", "same"), (1, 3, 64, 1, 64, torch.bfloat16, "none", "fp32"),
+    (1, 1, 1, 1, 32, torch.bfloat16, "none", "none")],
+    ids=lambda c: "B%dS%dR%dH%dD%d-%s-%s-%s" % (*c[:5], str(c[5]).split(".")[-1], c[6], c[7]))
+def test_backward_without_pair_bias_gradient(cfg):
+    """The backward kernel that has no d(pair_bias) to sum, against float64: one and several items to a block, row
+    groups that are not full, one step in all, a row whose keys are all dropped.  P, dS and the results are rounded to
+    the storage type, eps / 2 each, and no more."""
+    from evoformer_triton_b200 import attention, check_device_status
+    B, S, R, H, D, dtype, mask, bias = cfg
+    x = rand_inputs(B, S, R, H, D, dtype, seed=S + R, mask=mask, bias=bias != "none", keep_p=0.8)
+    if mask == "bool":
+        x["res_mask"][0, 0] = False
+    q, k, v, d_o = (x[n].to(DEV).reshape(B, H, S, R, D) for n in ("Q", "K", "V", "dO"))
+    b = None if bias == "none" else x["pair_bias"].reshape(B, H, R, R).to(DEV).to(torch.float32 if bias == "fp32" else dtype)
+    m = None if mask == "none" else x["res_mask"].reshape(B, S, R).to(DEV)
+    o, lse = attention.attention_forward(q, k, v, m, b, D ** -0.5)
+    dq, dk, dv, none = attention.attention_backward(q, k, v, o, lse, m, b, D ** -0.5, d_o, want_dbias=False)
+    torch.cuda.synchronize()
+    check_device_status()
+    assert none is None and attention.last_path["bwd"] == _lib().PATH_TCGEN05
+    Q, K, V, G = (t.double().requires_grad_() for t in (q, k, v, d_o))
+    p = (Q @ K.transpose(-1, -2)) * D ** -0.5
+    if b is not None:
+        p = p + b.double()[:, :, None]
+    if mask == "bool":
+        p = p.masked_fill(~m[:, None, :, None, :], -1e300)
+    elif m is not None:
+        p = p + m.double()[:, None, :, None, :]
+    want = torch.autograd.grad(p.softmax(-1) @ V, (Q, K, V), G)
+    for name, got, w in zip(("dQ", "dK", "dV"), (dq, dk, dv), want):
+        scale = max(w.norm().item(), torch.finfo(dtype).eps * G.norm().item())  # (one key: no gradient but rounding)
+        assert (got.double() - w).norm().item() <= 1.5 * torch.finfo(dtype).eps * scale, name
