@@ -51,6 +51,7 @@ constexpr int BM = 128;  // query rows per warpgroup tile
 constexpr int BN = 64;   // keys per tile
 constexpr int kTmemCols = 512;
 constexpr size_t kMaxSmem = 232448;  // of one CTA
+constexpr int kMaxRes = 2048;        // longest N_res: two mask rows for each warpgroup are staged in shared memory
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMaxSum = 256.f;       // sum of a tile's exponentials above which one of them may exceed 2^8
 constexpr float kGrow = 8.f / kLog2e;  // how far a tile's maximum may exceed the running one
@@ -65,8 +66,14 @@ struct Cfg {
   static constexpr int RB = DP * 2;                    // bytes per staged row
   static constexpr int QST = (DP == 64 || NW > 2) ? 1 : 2;  // Q stages
   static constexpr int SB = NW > 2 ? 1 : 2;            // score buffers per warpgroup
-  static constexpr int NK = DP == 64 && NW > 2 ? 1 : SB + 1;  // K stages (S is through with one early in a tile)
-  static constexpr int NV = (DP == 64 || NW > 2) ? 2 : 3;  // stages of V and the pair bias
+  // Query pairs with an fp32 bias: a stage of V and the bias is 64 KB and more, so there are two of them, and at
+  // DP = 64 two of K, which leaves room for the masks of every length.  Bound by reading the bias (332 us of it at
+  // 2 048).  Forward of [4,1,R,32,D] bf16, us, as query pairs and as items of two rows, the second of which does not
+  // exist: R = 2048, D = 8 343 and 426, D = 32 354 and 447, D = 64 376 and 538; R = 300 18.5 and 22.6, 20.6 and 22.6,
+  // 24.1 (either way, a third K stage made no difference).
+  static constexpr bool kWide = QP && BIAS == BIAS_F32;
+  static constexpr int NK = DP == 64 && NW > 2 ? 1 : DP == 64 && kWide ? 2 : SB + 1;  // K stages (S is through with one early in a tile)
+  static constexpr int NV = (DP == 64 || NW > 2 || kWide) ? 2 : 3;  // stages of V and the pair bias
   static constexpr int KVR = QP ? 1 : NW;              // rows of K and V in a stage: one per warpgroup, or one shared
   static constexpr int BTL = QP ? 2 : 1;               // pair-bias tiles in a stage: one shared, or one per warpgroup
   static constexpr int kThreads = 128 + 128 * NW;
@@ -83,9 +90,14 @@ struct Cfg {
   static constexpr int offMask = offOnes + (kOnes < 1024 ? 1024 : kOnes);
   static constexpr int PER = 3 * SB + 4;               // barriers of a warpgroup
   static constexpr int kNumBars = NW * PER + 2 * (QST + NK + NV);
-  static size_t bytes(int r_pad) {
-    return (size_t)offMask + (size_t)2 * NW * (r_pad * 4 + 4) + kNumBars * 8 + 64 + 1024;
+  // Slack for aligning the tiles to 1024 bytes; where it does not fit the kernel checks that the base address
+  // needs none (the dynamic shared memory of a kernel without static shared memory starts on such a boundary on
+  // this architecture) and gives up with a status code otherwise.
+  static constexpr int kSlack = DP == 64 && kWide ? 0 : 1024;
+  static constexpr size_t bytes(int r_pad) {
+    return (size_t)offMask + (size_t)2 * NW * (r_pad * 4 + 4) + kNumBars * 8 + 64 + kSlack;
   }
+  static_assert(!QP || bytes(kMaxRes) <= kMaxSmem, "query-pair mode is there for every length");
   // TMEM columns of a warpgroup: S buffers, then O, then the row sum of P (16 equal columns)
   static constexpr int colO = SB * BN, colL = colO + DP, tmemWg = colL + 16;
   static_assert(NW * tmemWg <= kTmemCols, "TMEM budget");
@@ -135,6 +147,10 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if (static_cast<int>(smem - smem_raw) > C::kSlack) {  // the same for every thread of every CTA
+    if (threadIdx.x == 0 && a.status) atomicCAS(a.status, 0, DEV_TIMEOUT_SYNC);
+    return;
+  }
   const uint32_t smem_s = smem_u32(smem);
   const int T_TILES = (a.R + BN - 1) / BN;
   const int r_pad = T_TILES * BN;
@@ -682,7 +698,7 @@ int launch_t(const Args& a, cudaStream_t st, int* launches) {
 template <class T, int DP, int BIAS>
 int launch_mode(const Args& a, cudaStream_t st, int* launches) {
   const int r_pad = (a.R + BN - 1) / BN * BN;
-  if (a.S == 1 && a.R > BM && Cfg<DP, 2, true, BIAS>::bytes(r_pad) <= kMaxSmem) return launch_t<T, DP, BIAS, 2, true>(a, st, launches);
+  if (a.S == 1 && a.R > BM) return launch_t<T, DP, BIAS, 2, true>(a, st, launches);
   const int sms = sm_count();
   if (sms <= 0) return EVOATTN_ERR_CUDA;
   // Time of the busiest CTA: the items it walks, times what an item of two, three or four rows costs (each
@@ -728,7 +744,7 @@ int launch_d(const Args& a, cudaStream_t st, int* launches) {
 bool sm100_fwd_supported(int dtype, const Args& a) {
   if (dtype != EVOATTN_BF16 && dtype != EVOATTN_FP16) return false;
   if (a.D % 8 != 0 || a.D > 64) return false;
-  if (a.R > 2048) return false;  // two mask rows are staged in shared memory
+  if (a.R > kMaxRes) return false;
   if (a.bias) {
     const int es = a.bias16 ? 2 : 4;
     if ((reinterpret_cast<uintptr_t>(a.bias) & 15) != 0) return false;

@@ -146,7 +146,9 @@ def test_pair_bias_gradient_of_64_gib():
     (4, 2, 296, 65, 8, 16, torch.bfloat16, "none", "none"), (3, 1, 100, 136, 4, 32, torch.float16, "addsame", "same"),
     (3, 1, 592, 64, 8, 64, torch.bfloat16, "bool", "fp32"), (3, 1, 590, 40, 8, 48, torch.bfloat16, "add32", "same"),
     (2, 1, 5, 200, 3, 32, torch.bfloat16, "bool", "same"), (2, 3, 1, 100, 2, 64, torch.float16, "none", "fp32"),
-    (0, 2, 1, 272, 3, 32, torch.bfloat16, "addsame", "fp32"), (0, 2, 1, 520, 2, 64, torch.float16, "bool", "same")],
+    (0, 2, 1, 272, 3, 32, torch.bfloat16, "addsame", "fp32"), (0, 2, 1, 520, 2, 64, torch.float16, "bool", "same"),
+    (0, 2, 1, 264, 3, 16, torch.float16, "bool", "fp32"), (0, 1, 1, 2048, 3, 32, torch.bfloat16, "add32", "fp32"),
+    (0, 2, 1, 1476, 3, 64, torch.float16, "bool", "fp32"), (0, 1, 1, 2048, 80, 64, torch.bfloat16, "add32", "fp32")],
     ids=lambda c: "rows%d-B%dS%dR%dH%dD%d-%s-%s-%s" % (*c[:6], str(c[6]).split(".")[-1], c[7], c[8]))
 def test_forward_items_of_each_size(cfg):
     """Forward items of two, three and four MSA rows and of two query tiles: row groups and query pairs that are not
@@ -167,10 +169,14 @@ def test_forward_items_of_each_size(cfg):
     q, k, v = (x[n].to(DEV).reshape(B, H, S, R, D) for n in ("Q", "K", "V"))
     b = None if bias == "none" else x["pair_bias"].reshape(B, H, R, R).to(DEV).to(torch.float32 if bias == "fp32" else dtype)
     m = None if mask == "none" else x["res_mask"].reshape(B, S, R).to(DEV)
-    o, lse = attention.attention_forward(q, k, v, m, b, D ** -0.5)
-    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        o, lse = attention.attention_forward(q, k, v, m, b, D ** -0.5)
+        torch.cuda.synchronize()
     check_device_status()
     assert attention.last_path["fwd"] == _lib().PATH_TCGEN05
+    ran = [e.name for e in prof.events() if "evo_fwd_sm100_kernel" in e.name]
+    if sms == 148 or not rows:  # template arguments: type, padded head dimension, mask, bias, warpgroups, query pairs
+        assert len(ran) == 1 and ran[0].split(">")[0].endswith(f"{rows or 2}, {'false' if rows else 'true'}"), ran
     p = (q.double() @ k.double().transpose(-1, -2)) * D ** -0.5
     if b is not None:
         p += b.double()[:, :, None]
