@@ -634,8 +634,6 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     }
   }
 
-  if (*abort_flag) report_abort(*abort_flag, a.status);
-  tc_fence_before();
-  __syncthreads();
+  end_of_cta(abort_flag, a.status);
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }

@@ -759,9 +759,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     if (lane == 0) tma_wait_group0();  // this warp's reductions have completed before the CTA may exit
   }
 
-  if (*abort_flag) report_abort(*abort_flag, a.status);
-  tc_fence_before();
-  __syncthreads();
+  end_of_cta(abort_flag, a.status);
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 

@@ -652,9 +652,7 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
     }
   }
 
-  if (*abort_flag) report_abort(*abort_flag, a.status);
-  tc_fence_before();
-  __syncthreads();
+  end_of_cta(abort_flag, a.status);
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 

@@ -1,8 +1,8 @@
 // Inline-PTX wrappers for sm_100a: mbarrier, TMA tiled copies, tcgen05 (alloc, mma,
 // commit, ld/st), proxy fences, and the UMMA descriptor encodings.  Every wait is
-// bounded: when its limit runs out it records a code in the caller's status word,
-// raises the CTA-wide abort flag and returns, so a broken pipeline ends instead of
-// hanging the GPU.
+// bounded: when its limit runs out it raises the CTA-wide abort flag and returns, and the
+// end of the kernel records its code in the caller's status word, so a broken pipeline ends
+// instead of hanging the GPU.
 #pragma once
 
 #include <cuda.h>
@@ -35,7 +35,7 @@ __device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes) {
 }
 // Bounded wait on an mbarrier (32-bit shared-window addresses; about one second at B200 clocks).  `abort_flag_s`
 // is a word of shared memory that belongs to the CTA: once any wait has run out it holds that wait's code, all
-// later waits fall through, and the end of the kernel reports it (report_abort).  The retries carry a
+// later waits fall through, and the end of the kernel reports it (end_of_cta).  The retries carry a
 // suspend-time hint: the hardware parks the thread until the phase completes, so a waiting warp does not
 // compete for issue slots with the warps that do the arithmetic.  All of it is one short sequence on purpose: a
 // kernel has some thirty waits, and the code of its loops has to fit the instruction caches.
@@ -99,6 +99,15 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// The end of a CTA, for all of its threads; what it still owns (tensor memory) is freed after this.  The flag is
+// looked at behind the barrier, when every warp is through with its waits: the thread that reports belongs to a warp
+// that may be done long before the last of them, and a wait that ran out after that would go unreported.
+__device__ __forceinline__ void end_of_cta(volatile int* abort_flag, int* status) {
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) report_abort(*abort_flag, status);
+}
 
 // ---------------------------------------------------------------- tcgen05: MMA
 // One lane of a converged warp.  Every operand of a tcgen05.mma lives in a uniform register: in a branch that one
