@@ -55,6 +55,7 @@ constexpr int kMaxRes = 2048;        // longest N_res: two mask rows for each wa
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMaxSum = 256.f;       // sum of a tile's exponentials above which one of them may exceed 2^8
 constexpr float kGrow = 8.f / kLog2e;  // how far a tile's maximum may exceed the running one
+constexpr float kFar = 65536.f;        // running maximum up to which an exponent is formed in one FMA (see far_tile)
 constexpr int MASK_MIN = 0;  // boolean keep-mask (or none): score = min(score, m), m = +-FLT_MAX
 constexpr int MASK_ADD = 1;  // additive mask
 constexpr int BIAS_NONE = 0, BIAS_F32 = 1, BIAS_16 = 2;
@@ -133,6 +134,73 @@ __device__ __forceinline__ Item decode_item(int idx, const Walk& wk) {
   n = div_mod(n, wk.outer, it.outer);
   it.b = div_mod(n, wk.heads, it.h);
   return it;
+}
+
+// Eight scores of query row `row`, the g8-th eight of a key tile: x = scale*S + bias, then the mask.
+template <class T, int MASKMODE, int BIAS, int BOXES, bool MASKED>
+__device__ __forceinline__ void row_scores8(const uint32_t* s8, int g8, int row, F2 scale2, uint32_t brow_s, uint32_t mtile_s,
+                                            float (&v)[8]) {
+  float bvv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, mkv[8];
+  if constexpr (BIAS == BIAS_16) {
+    // eight 16-bit values of my row (rows of 128 bytes, 128-byte swizzle), widened here
+    const uint4 wv = lds_v4(brow_s + ((g8 ^ (row & 7)) << 4));
+    unpack2<T>(wv.x, bvv[0], bvv[1]); unpack2<T>(wv.y, bvv[2], bvv[3]);
+    unpack2<T>(wv.z, bvv[4], bvv[5]); unpack2<T>(wv.w, bvv[6], bvv[7]);
+  } else if constexpr (BIAS == BIAS_F32) {  // (two boxes of 32 columns, BOXES bytes apart)
+    const int c = g8 >> 2, q4 = (g8 & 3) * 2;
+    const float4 b0 = lds_v4f(brow_s + c * BOXES + ((q4 ^ (row & 7)) << 4));
+    const float4 b1 = lds_v4f(brow_s + c * BOXES + (((q4 + 1) ^ (row & 7)) << 4));
+    bvv[0] = b0.x; bvv[1] = b0.y; bvv[2] = b0.z; bvv[3] = b0.w;
+    bvv[4] = b1.x; bvv[5] = b1.y; bvv[6] = b1.z; bvv[7] = b1.w;
+  }
+  if constexpr (MASKED) {
+    const float4 k0 = lds_v4f(mtile_s + g8 * 32);
+    const float4 k1 = lds_v4f(mtile_s + g8 * 32 + 16);
+    mkv[0] = k0.x; mkv[1] = k0.y; mkv[2] = k0.z; mkv[3] = k0.w;
+    mkv[4] = k1.x; mkv[5] = k1.y; mkv[6] = k1.z; mkv[7] = k1.w;
+  }
+#pragma unroll
+  for (int u = 0; u < 8; u += 2) {  // two elements per instruction
+    F2 x = f2_fma(f2_from_bits(s8[u], s8[u + 1]), scale2, f2_make(bvv[u], bvv[u + 1]));
+    if constexpr (MASKED && MASKMODE == MASK_ADD) x = f2_add(x, f2_make(mkv[u], mkv[u + 1]));
+    f2_get(x, v[u], v[u + 1]);
+  }
+  if constexpr (MASKED && MASKMODE == MASK_MIN) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = fminf(v[u], mkv[u]);
+  }
+}
+
+// P of a key tile against a maximum m beyond kFar.  (x - m) log2 e in one FMA carries the rounding of m log2 e, half a
+// unit in its last place: 2^-8 at kFar, but 64 at 1e9, where all scores of a query lie whose bias drops it whole; its
+// probabilities came out at 2^18 (infinite in fp16) or at 0.  Here the difference is formed first.  (So it is in the
+// key tiles that an additive mask changes, where the packed instruction more is the one that a packed mask saves.)
+// Sixteen keys at a time and straight into place: P_n lies over columns of S_n that have been read.  Returns the row
+// sum.  Not inlined, which leaves the registers of the tile loop as they are; inlined, the forward of
+// [1,128,768,8,64] took 314 us instead of 306, of [1,128,384,8,32] without a bias 74 instead of 72.
+template <class T, int BIAS, int BOXES>
+__device__ __noinline__ float far_tile(uint32_t tS, float m, int row, float scale, uint32_t brow_s, uint32_t mtile_s) {
+  const F2 scale2 = f2_make(scale, scale);
+  float sum = 0.f;
+#pragma unroll 1
+  for (int h = 0; h < BN / 16; ++h) {
+    uint32_t s16[16], p8[8];
+    tmem_ld16(tS + 16 * h, s16);
+    tmem_wait_ld();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      float v[8];
+      row_scores8<T, MASK_MIN, BIAS, BOXES, true>(s16 + 8 * k, 2 * h + k, row, scale2, brow_s, mtile_s, v);
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        const float p0 = ex2((v[u] - m) * kLog2e), p1 = ex2((v[u + 1] - m) * kLog2e);
+        sum += p0 + p1;
+        p8[4 * k + u / 2] = Pack2<T>::pack(p0, p1);
+      }
+    }
+    tmem_st8(tS + 8 * h, p8);
+  }
+  return sum;
 }
 
 template <class T, int DP, int MASKMODE, int BIAS, int NW, bool QP>
@@ -448,14 +516,14 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
       const uint32_t mst = n_item & 1;
       mbar_wait_s(m_full(w, mst), (n_item >> 1) & 1, abort_s, DEV_TIMEOUT_SYNC);
       const uint32_t mrow_s = smem_u32(sMask) + (w * 2 + mst) * r_pad * 4;
-      const uint32_t dirty = lds_u32(smem_u32(sDirty) + (w * 2 + mst) * 4);
+      uint32_t dirty = lds_u32(smem_u32(sDirty) + (w * 2 + mst) * 4);
 
       // The gate's row is wanted in the epilogue, where every cycle of its latency would be waited for.
       const T* grow = a.gate ? reinterpret_cast<const T*>(a.gate) + off4(a.sgate, it.b, it.h, s, i < a.R ? i : 0) : nullptr;
       if (grow != nullptr) prefetch_l2(grow);
 
       float m_run = -FLT_MAX, l_run = 0.f;
-      bool alive = false;  // every row of this warp has a running maximum
+      bool alive = false;  // every row of this warp has a running maximum that the fast path below can take
 
 #pragma unroll 1
       for (int t = 0; t < T_TILES; ++t, ++g) {
@@ -466,31 +534,8 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
         tc_fence_after();
         if (has_bias && SB == 2) mbar_wait_s(v_full(vt), vp, abort_s, DEV_TIMEOUT_TMA);
 
-        // Scores of my row, eight at a time: x = scale*S + bias, then the mask.
         auto scores8 = [&](const uint32_t* s8, int g8, auto with_mask, float (&v)[8]) {
-          float bvv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          if constexpr (BIAS16) {
-            // eight 16-bit values of my row (rows of 128 bytes, 128-byte swizzle), widened here
-            const uint4 wv = lds_v4(brow_s + ((g8 ^ (row & 7)) << 4));
-            unpack2<T>(wv.x, bvv[0], bvv[1]); unpack2<T>(wv.y, bvv[2], bvv[3]);
-            unpack2<T>(wv.z, bvv[4], bvv[5]); unpack2<T>(wv.w, bvv[6], bvv[7]);
-          } else if constexpr (has_bias) {
-            const int c = g8 >> 2, q4 = (g8 & 3) * 2;
-            const float4 b0 = lds_v4f(brow_s + c * (C::BTL * kBoxBias) + ((q4 ^ (row & 7)) << 4));
-            const float4 b1 = lds_v4f(brow_s + c * (C::BTL * kBoxBias) + (((q4 + 1) ^ (row & 7)) << 4));
-            bvv[0] = b0.x; bvv[1] = b0.y; bvv[2] = b0.z; bvv[3] = b0.w;
-            bvv[4] = b1.x; bvv[5] = b1.y; bvv[6] = b1.z; bvv[7] = b1.w;
-          }
-#pragma unroll
-          for (int u = 0; u < 8; u += 2)  // x = scale*S + bias, two elements per instruction
-            f2_get(f2_fma(f2_from_bits(s8[u], s8[u + 1]), scale2, f2_make(bvv[u], bvv[u + 1])), v[u], v[u + 1]);
-          if constexpr (decltype(with_mask)::value) {
-            const float4 k0 = lds_v4f(mtile_s + g8 * 32);
-            const float4 k1 = lds_v4f(mtile_s + g8 * 32 + 16);
-            const float mkv[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = (MASKMODE == MASK_MIN) ? fminf(v[u], mkv[u]) : (v[u] + mkv[u]);
-          }
+          row_scores8<T, MASKMODE, BIAS, C::BTL * kBoxBias, decltype(with_mask)::value>(s8, g8, row, scale2, brow_s, mtile_s, v);
         };
 
         float lsum = 0.f;
@@ -518,8 +563,12 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
                 scores8(sr[(g8 / 2) & 1] + 8 * (g8 & 1), g8, with_mask, v);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
+                  const F2 x2 = f2_make(v[2 * u], v[2 * u + 1]);
                   float y0, y1;
-                  f2_get(f2_fma(f2_make(v[2 * u], v[2 * u + 1]), l2e2, nm22), y0, y1);
+                  if constexpr (decltype(with_mask)::value && MASKMODE == MASK_ADD)  // (see far_tile)
+                    f2_get(f2_mul(f2_add(x2, f2_make(-m_run, -m_run)), l2e2), y0, y1);
+                  else
+                    f2_get(f2_fma(x2, l2e2, nm22), y0, y1);
                   const float p0 = ex2(y0), p1 = ex2(y1);
                   ls4[u] = f2_add(ls4[u], f2_make(p0, p1));
                   pk[g8 * 4 + u] = Pack2<T>::pack(p0, p1);
@@ -576,14 +625,26 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
           alive = !__any_sync(0xffffffffu, m_run == -FLT_MAX);
           go = __any_sync(0xffffffffu, m_run != -FLT_MAX);
           settled = true;
+          if (__any_sync(0xffffffffu, m_run != -FLT_MAX && fabsf(m_run) > kFar)) {  // (see far_tile)
+            if constexpr (MASKMODE == MASK_ADD) dirty = ~0u;
+            else alive = go = false;
+          }
         }
-        if (!alive && m_run == -FLT_MAX) {
-          // every key seen so far was dropped: the scores are all -FLT_MAX and the softmax is
-          // uniform over the real keys (test.py:54-55 semantics)
-          const int real = min(BN, a.R - t * BN);
-          lsum = (float)real;
+        if (!alive) {
+          if (!go && __any_sync(0xffffffffu, m_run != -FLT_MAX)) {
+            lsum = far_tile<T, BIAS, C::BTL * kBoxBias>(tS, m_run, row, scale, brow_s, mtile_s);
+            tmem_wait_st();
+            tmem_ld32(tS, pk);
+            tmem_wait_ld();
+          }
+          if (m_run == -FLT_MAX) {
+            // every key seen so far was dropped: the scores are all -FLT_MAX and the softmax is
+            // uniform over the real keys (test.py:54-55 semantics)
+            const int real = min(BN, a.R - t * BN);
+            lsum = (float)real;
 #pragma unroll
-          for (int e = 0; e < BN; e += 2) pk[e / 2] = Pack2<T>::pack(e < real ? 1.f : 0.f, e + 1 < real ? 1.f : 0.f);
+            for (int e = 0; e < BN; e += 2) pk[e / 2] = Pack2<T>::pack(e < real ? 1.f : 0.f, e + 1 < real ? 1.f : 0.f);
+          }
         }
         l_run += lsum;
         if (++vt == NV) { vt = 0; vp ^= 1; }

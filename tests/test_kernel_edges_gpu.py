@@ -45,6 +45,69 @@ def test_running_maximum_that_keeps_growing(D, dtype, S):
     check(got, x, label=f"ramp D={D} ")
 
 
+@pytest.mark.parametrize("S", [1, 5])
+@pytest.mark.parametrize("D", [8, 32, 64])
+@pytest.mark.parametrize("dtype,drop", [(torch.float16, -1e9), (torch.float16, -6e4), (torch.float16, -3e38), (torch.bfloat16, -1e9),
+                                        (torch.bfloat16, -2e9), (torch.bfloat16, -1e30)])
+def test_rows_that_an_additive_mask_drops_whole(dtype, drop, D, S):
+    """Scores near the mask's value, where a float has no bits left for the rest: those that come out equal have equal
+    probabilities, as a softmax in fp32 gives them, and a row whose first keys are dropped so goes on to its others.
+    The bound is what rounding P and O to the storage type gives (twice eps / 2)."""
+    from evoformer_triton_b200 import attention, check_device_status
+    B, H, R = 2, 2, 200
+    g = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v = (torch.randn((B, H, S, R, D), generator=g, device=DEV).to(dtype) for _ in range(3))
+    bias = torch.randn((B, H, R, R), generator=g, device=DEV)
+    mask = torch.zeros((B, S, R), device=DEV)
+    mask[0, 0] = drop
+    mask[1, S - 1, :150] = drop
+    o, lse = attention.attention_forward(q, k, v, mask, bias, D ** -0.5)
+    torch.cuda.synchronize()
+    check_device_status()
+    assert attention.last_path["fwd"] == _lib().PATH_TCGEN05
+    x = (q.double() @ k.double().transpose(-1, -2)) * D ** -0.5 + bias.double()[:, :, None]
+    x = (x.float() + mask[:, None, :, None, :]).double()  # (the sum with the mask is rounded to a float, the rest is not)
+    want = x.softmax(-1) @ v.double()
+    for b, s in ((0, 0), (1, S - 1)):
+        w = want[b, :, s]
+        assert (o[b, :, s].double() - w).norm() <= torch.finfo(dtype).eps * w.norm(), (b, s)
+    assert (o.double() - want).norm() <= torch.finfo(dtype).eps * want.norm()
+
+
+@pytest.mark.parametrize("S", [1, 5])
+@pytest.mark.parametrize("D", [8, 32, 64])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("mask", ["none", "bool", "add32"])
+def test_queries_whose_bias_lies_far_out(mask, dtype, D, S):
+    """The same for a pair bias that drops (or lifts) all keys of some queries, next to ordinary ones, ones whose first
+    keys only are so, and ones at the lowest float, which count as dropped."""
+    from evoformer_triton_b200 import attention, check_device_status
+    B, H, R = 1, 2, 200
+    g = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v = (torch.randn((B, H, S, R, D), generator=g, device=DEV).to(dtype) for _ in range(3))
+    bias = torch.randn((B, H, R, R), generator=g, device=DEV)
+    lowest = torch.finfo(torch.float32).min
+    for i, far in ((3, -1e9), (4, lowest), (70, 1e9), (71, -2e9), (130, -1e30), (199, -1e9)):
+        bias[:, :, i] = far
+    bias[:, :, 140, :100] = -1e9
+    bias[:, :, 141, 64:] = 3e9
+    keep = torch.rand((B, S, R), generator=g, device=DEV) < 0.9
+    m = {"none": None, "bool": keep, "add32": torch.where(keep, 0.0, -1e9)}[mask]
+    o, lse = attention.attention_forward(q, k, v, m, bias, D ** -0.5)
+    torch.cuda.synchronize()
+    check_device_status()
+    assert attention.last_path["fwd"] == _lib().PATH_TCGEN05
+    x = ((q.double() @ k.double().transpose(-1, -2)) * D ** -0.5 + bias.double()[:, :, None]).float()
+    if mask == "bool":
+        x = torch.where(m[:, None, :, None, :], x, lowest)
+    elif mask == "add32":
+        x = x + m[:, None, :, None, :]
+    want = x.clamp(min=lowest).double().softmax(-1) @ v.double()
+    assert (o.double() - want).norm() <= torch.finfo(dtype).eps * want.norm()
+    for i in (3, 4, 70, 71, 130, 140, 141, 199):
+        assert (o[:, :, :, i].double() - want[:, :, :, i]).norm() <= torch.finfo(dtype).eps * want[:, :, :, i].norm(), i
+
+
 @pytest.mark.parametrize("mask", ["bool", "add32", "addsame"])
 @pytest.mark.parametrize("D", [16, 32, 64])
 def test_mask_that_touches_some_key_tiles(mask, D):
@@ -169,7 +232,7 @@ def test_forward_items_of_each_size(cfg):
     q, k, v = (x[n].to(DEV).reshape(B, H, S, R, D) for n in ("Q", "K", "V"))
     b = None if bias == "none" else x["pair_bias"].reshape(B, H, R, R).to(DEV).to(torch.float32 if bias == "fp32" else dtype)
     m = None if mask == "none" else x["res_mask"].reshape(B, S, R).to(DEV)
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA], acc_events=True) as prof:
         o, lse = attention.attention_forward(q, k, v, m, b, D ** -0.5)
         torch.cuda.synchronize()
     check_device_status()
