@@ -27,9 +27,10 @@
 //
 // The exponentials of a tile do not wait for its maximum: they are taken against the running maximum m of the
 // tiles before (of the first tile, its own), straight from the scores: load, two FMAs, ex2, row sum, pack.  Only
-// if a row's sum of the tile shows that some exp2(x - m) may exceed 2^8 (its sum does) is the tile's maximum
-// taken, m and O follow it where it has grown by more than that, and the tile is done again.  So the maximum
-// pass costs one tile in T_TILES instead of every one, and no score is held in a register.
+// if a row's sum of the tile shows that some exp2(x - m) may be too large (its sum is) is the tile's maximum
+// taken, m and O follow it, and the tile is done again.  So the maximum pass costs one tile in T_TILES instead of
+// every one, and no score is held in a register.  Where the scores rise from tile to tile by more than m may lag
+// (Lag), the next tile's maximum is taken first, and its exponentials only once.
 //
 // Bound by the issue slots and hand-overs around the exponentials (16 a cycle and SM: [1,256,1024,4,32] would
 // take 236 us).  That shape takes 379 us with four warpgroups, and 540 with the form before, which had the
@@ -53,8 +54,16 @@ constexpr int kTmemCols = 512;
 constexpr size_t kMaxSmem = 232448;  // of one CTA
 constexpr int kMaxRes = 2048;        // longest N_res: two mask rows for each warpgroup are staged in shared memory
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kMaxSum = 256.f;       // sum of a tile's exponentials above which one of them may exceed 2^8
-constexpr float kGrow = 8.f / kLog2e;  // how far a tile's maximum may exceed the running one
+// How far the running maximum may lag.  kMaxSum: sum of a tile's exponentials up to which they serve; kRise: rise of a
+// tile's maximum above the running one up to which the sum of its 64 cannot be more.  fp16 ends at 2^16; bf16 and the
+// fp32 sums do not care how large P is (2^84 is left for the values of V).  A line at 2^8, with a maximum that followed
+// only where it had grown by that much, made every tile after a moderate rise pay for both passes.  Forward, us, with
+// that, with the line here, and of the kernel that took every tile's maximum; a bias that rises along the keys by
+// 8 bits / by 64 bits / by 7 bits once: [1,128,768,8,32] bf16 373 / 469 / 467, 227 / 262 / 226, 317 / 345 / 343;
+// [1,64,768,8,64] bf16 265 / 330 / 325, 168 / 189 / 168, 193 / 208 / 208 (fp16, which may lag less: 260 at 64 bits).
+template <class T> struct Lag;
+template <> struct Lag<__half> { static constexpr float kMaxSum = 32768.f, kRise = 9.f / kLog2e; };
+template <> struct Lag<__nv_bfloat16> { static constexpr float kMaxSum = 4294967296.f, kRise = 26.f / kLog2e; };
 constexpr float kFar = 65536.f;        // running maximum up to which an exponent is formed in one FMA (see far_tile)
 constexpr int MASK_MIN = 0;  // boolean keep-mask (or none): score = min(score, m), m = +-FLT_MAX
 constexpr int MASK_ADD = 1;  // additive mask
@@ -581,30 +590,31 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
 #pragma unroll
             for (int u = 0; u < 4; ++u) f2_get(ls4[u], lsa[2 * u], lsa[2 * u + 1]);
             lsum = ((lsa[0] + lsa[1]) + (lsa[2] + lsa[3])) + ((lsa[4] + lsa[5]) + (lsa[6] + lsa[7]));
-            bad = __any_sync(0xffffffffu, !(lsum <= kMaxSum));
+            bad = __any_sync(0xffffffffu, !(lsum <= Lag<T>::kMaxSum));
           }
           if (__builtin_expect(!bad || settled, 1)) break;
           // The tile's own maximum, and the running one follows it.
           float mx = -FLT_MAX;
 #pragma unroll 1
-          for (int h = 0; h < BN / 16; ++h) {
-            uint32_t s16[16];
-            tmem_ld16(tS + 16 * h, s16);
+          for (int h = 0; h < BN / 32; ++h) {
+            uint32_t s32[32];
+            tmem_ld32(tS + 32 * h, s32);
             tmem_wait_ld();
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
+            for (int k = 0; k < 4; ++k) {
               float v[8];
-              scores8(s16 + 8 * k, 2 * h + k, std::true_type{}, v);
+              scores8(s32 + 8 * k, 4 * h + k, std::true_type{}, v);
 #pragma unroll
               for (int u = 0; u < 8; u += 2) mx = max3(mx, v[u], v[u + 1]);
             }
           }
+          bool steep = false;  // the next tile may well rise as much again
           if (t == 0) {
             m_run = mx;
           } else {
-            const bool grow = mx > m_run + kGrow;
-            if (__any_sync(0xffffffffu, grow)) {
-              const float m_up = grow ? mx : m_run;
+            steep = mx > m_run + Lag<T>::kRise;
+            if (__any_sync(0xffffffffu, mx > m_run)) {
+              const float m_up = fmaxf(mx, m_run);
               const float alpha = ex2((m_run - m_up) * kLog2e);
               m_run = m_up;
               l_run *= alpha;
@@ -622,7 +632,7 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
               }
             }
           }
-          alive = !__any_sync(0xffffffffu, m_run == -FLT_MAX);
+          alive = !__any_sync(0xffffffffu, m_run == -FLT_MAX || steep);
           go = __any_sync(0xffffffffu, m_run != -FLT_MAX);
           settled = true;
           if (__any_sync(0xffffffffu, m_run != -FLT_MAX && fabsf(m_run) > kFar)) {  // (see far_tile)

@@ -45,6 +45,68 @@ def test_running_maximum_that_keeps_growing(D, dtype, S):
     check(got, x, label=f"ramp D={D} ")
 
 
+@pytest.mark.parametrize("S", [1, 3])
+@pytest.mark.parametrize("D", [8, 32, 64])
+@pytest.mark.parametrize("dtype,bits", [(torch.float16, 8.5), (torch.float16, 9.5), (torch.float16, 14), (torch.float16, 17),
+                                        (torch.bfloat16, 25.5), (torch.bfloat16, 33), (torch.bfloat16, 140)])
+def test_maximum_that_lags_as_far_as_it_may(dtype, bits, D, S):
+    """Key tiles whose scores lie just below and just beyond what the exponentials against the maximum of the tiles
+    before can take (2^15 and 2^32 in a tile's sum), one such rise after another, then a level stretch; in one query of
+    32, and in all.  The bound is what rounding P and O to the storage type gives (twice eps / 2)."""
+    from evoformer_triton_b200 import attention, check_device_status
+    B, H, R = 1, 2, 640
+    g = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v = (torch.randn((B, H, S, R, D), generator=g, device=DEV).to(dtype) * 0.25 for _ in range(3))
+    steps = torch.tensor([0, 1, 2, 2, 2, 3, 1, 4, 4, 5.]) * bits * 0.6931472
+    bias = torch.randn((B, H, R, R), generator=g, device=DEV) * 0.1
+    bias[:, :, :256] += steps.repeat_interleave(64).to(DEV)
+    bias[:, :, 256::32] += steps.repeat_interleave(64).to(DEV)
+    o, lse = attention.attention_forward(q, k, v, None, bias, D ** -0.5)
+    torch.cuda.synchronize()
+    check_device_status()
+    assert attention.last_path["fwd"] == _lib().PATH_TCGEN05
+    x = (q.double() @ k.double().transpose(-1, -2)) * D ** -0.5 + bias.double()[:, :, None]
+    want = x.softmax(-1) @ v.double()
+    assert (o.double() - want).norm() <= torch.finfo(dtype).eps * want.norm()
+    want_lse = x.logsumexp(-1)  # (scores up to 490: half a unit in the last place of such a float is 1.5e-5)
+    assert ((lse.double() - want_lse).abs() <= 1e-5 + 2.0 ** -23 * want_lse.abs()).all()
+
+
+@pytest.mark.parametrize("S,D,dtype", [(64, 64, torch.bfloat16), (64, 64, torch.float16), (128, 32, torch.bfloat16)])
+@pytest.mark.parametrize("kind", ["rises", "jumps", "dropped rows"])
+def test_forward_takes_drifting_scores_in_its_stride(kind, S, D, dtype):
+    """A bias that rises along the keys by 8 bits, one that jumps by 7 once, and rows that the mask drops whole cost
+    what independent scores cost: 1.00 to 1.05 as measured, 1.5 to 2 where every tile pays for a second pass."""
+    from evoformer_triton_b200 import attention, check_device_status
+    B, H, R = 1, 8, 768
+    g = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v = (torch.randn((B, H, S, R, D), generator=g, device=DEV).to(dtype) * 0.5 for _ in range(3))
+    flat = torch.randn((B, H, R, R), generator=g, device=DEV)
+    j = torch.arange(R, device=DEV)
+    drift = {"rises": flat + j / R * 8 * 0.6931472, "jumps": flat + (j > 76) * 7 * 0.6931472, "dropped rows": flat}[kind]
+    mask = torch.zeros((B, S, R), device=DEV)
+    mask[:, :, 700:] = -1e9
+    other = mask.clone()
+    if kind == "dropped rows":
+        other[:, ::4] = -1e9
+
+    def time(bias, m):
+        best = float("inf")
+        for _ in range(9):
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record()
+            for _ in range(5):
+                attention.attention_forward(q, k, v, m, bias, D ** -0.5)
+            ev[1].record()
+            torch.cuda.synchronize()
+            best = min(best, ev[0].elapsed_time(ev[1]))
+        return best
+
+    base, got = time(flat, mask), time(drift, other)
+    check_device_status()
+    assert got < 1.25 * base, (base, got)
+
+
 @pytest.mark.parametrize("S", [1, 5])
 @pytest.mark.parametrize("D", [8, 32, 64])
 @pytest.mark.parametrize("dtype,drop", [(torch.float16, -1e9), (torch.float16, -6e4), (torch.float16, -3e38), (torch.bfloat16, -1e9),
