@@ -854,18 +854,21 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
 
 // Head dimensions up to 16: items of seven rows (padded to 16 columns) flush d(pair_bias) and reload the bias
 // tile every seventh step instead of every third, but there are fewer of them and the last group of rows is
-// padded further.  They are taken where the CTA with the most steps gets no more than a tenth more of them,
-// or, without a d(pair_bias), a twenty-fifth.  Time of the backward call, seven rows over three, by how many more
-// steps that CTA gets (N_res 128 to 1000, D = 8 and 16):
-//   with d(pair_bias):     0.90-0.94 at as many steps, 0.95 at 4 % more, 0.97 at 8 %, 1.05 at 17 %
-//   with a bias alone:     0.95-0.98                   0.98              1.02-1.03    1.08
-//   without a bias:        0.97                        1.00              1.04         1.07
+// padded further.  They are taken where the CTA with the most steps gets no more than 15 % more of them, or 5 % with
+// an fp32 bias that wants no gradient (whose third half tile then pays for itself at three rows already).  Time of
+// the backward call, seven rows over three, by how many more steps that CTA gets (D = 8 and 16, N_res 200 to 1000;
+// at 128 and 256 an fp32 bias without a gradient is 0.05 to 0.1 above):
+//                                as many    5 % more   10 %       17 %       27 %
+//   with d(pair_bias):           0.86-0.89  0.89-0.92  0.93-0.97  0.98-1.00  1.06-1.09
+//   with an fp32 bias alone:     0.89-0.91  0.94-0.96  0.95-0.99  1.03-1.05  1.08-1.14
+//   with a 16-bit bias alone:    0.85-0.90  0.89-0.92  0.93-0.95  1.00-1.01  1.05-1.10
+//   without a bias:              0.80-0.86  0.86-0.89  0.89-0.92  0.95-0.98  1.02-1.06
 bool seven_rows_pay(const Args& a, int sms) {
   const auto steps = [&](int G) {
     const long long items = (long long)a.B * a.H * ((a.R + BT - 1) / BT) * ((a.S + G - 1) / G);
     return (items + sms - 1) / sms * G;
   };
-  return a.bias && a.dbias ? 10 * steps(7) <= 11 * steps(3) : 25 * steps(7) <= 26 * steps(3);
+  return 100 * steps(7) <= (a.bias && !a.bias16 && !a.dbias ? 105 : 115) * steps(3);
 }
 
 }  // namespace
