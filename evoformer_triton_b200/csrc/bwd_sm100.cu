@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(256) dq_store_kernel(Args a, const float* __re
   *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.dq) + off4(a.sdq, b, h, s, i) + d8 * 8) = pk;
 }
 
-template <class T, int DP, bool kHasBias, bool kBias16>
+template <class T, int DP, bool kBias16>
 __global__ void __launch_bounds__(kThreadsT, 1)
 evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CUtensorMap tmQ,
                 const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -254,9 +254,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
   const int NT = (a.R + BT - 1) / BT;
   const int NC = (a.S + G - 1) / G;
-  constexpr bool has_bias = kHasBias;
   constexpr int kBRow = kBias16 ? BT * 2 : BT * 4;  // bytes per row (one query, 128 keys) of the staged bias tile
-  const bool flush_dbias = has_bias && a.dbias != nullptr;
   // Persistent CTAs: CTA c owns the items c, c + gridDim.x, ..., SPI steps per item.  A short last
   // row group (S % G != 0) is padded with rows >= S: their tiles and statistics arrive as zeros and
   // their mask is -inf, so P = dS = 0, and nothing of them is stored.
@@ -305,8 +303,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     fence_mbar_init();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmDO);
     prefetch_tmap(&tmNL); prefetch_tmap(&tmDL); prefetch_tmap(&tmDQ);
-    if (has_bias) prefetch_tmap(&tmB);
-    if (flush_dbias) prefetch_tmap(&tmDB);
+    prefetch_tmap(&tmB); prefetch_tmap(&tmDB);
   }
   if (warp == 0) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -428,11 +425,11 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         __syncwarp();
       };
       const int tiles = my_items * NT;
-      if (has_bias && tiles > 0) { const StepT d0 = decode(0); load_bias(d0, 0); load_bias(d0, 1); }
+      if (tiles > 0) { const StepT d0 = decode(0); load_bias(d0, 0); load_bias(d0, 1); }
       int g = 0, it = 0, t = 0;  // row of the group, query tile, running (item, query tile) index
 #pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
-        const bool turn = has_bias && g == G - 1 && t + 1 < tiles;  // the group's last step: the halves come back
+        const bool turn = g == G - 1 && t + 1 < tiles;  // the group's last step: the halves come back
         StepT nb = StepT{0, 0, 0, 0, 0, 0};
         if (turn) nb = decode((t + 1) * G);  // (divisions: before the waits, not between them)
 #pragma unroll
@@ -601,6 +598,11 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 
     int p_row0 = 0, p_slab = -1;           // the step whose dQ partial has not left yet
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
+    // Always true.  With more than one row it has to be looked at all the same, which the compiler cannot know: given
+    // last_of_group alone it makes two copies of a step, whose registers do not fit (8 to 24 bytes of spills; the
+    // backward of [1,128,384,8,32] took 210 us instead of 195, [1,1024,384,8,8] fp16 1177 instead of 1083).  With one
+    // row the unconditional form is the faster one ([1,128,768,8,64] 1 092 instead of 1 160).
+    const bool flush = G == 1 || a.dbias != nullptr;
     const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
     const F2 l2e2 = f2_make(kLog2e, kLog2e), c12 = f2_make(c1, c1), neg1 = f2_make(-1.f, -1.f);
     F2 bacc[16];  // d(pair_bias) of this thread's key and its 32 queries, summed over the rows of a group
@@ -622,7 +624,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       const float mj = lds_f32(mask_s + g * (BT * 4));
       // the statistics vectors of this step are read with ordinary loads: observe their arrival here
       mbar_wait(st_full + (n & 1), (n >> 1) & 1, abort_s, DEV_TIMEOUT_TMA);
-      if (has_bias && g == 0) mbar_wait(b_full + H, tile & 1, abort_s, DEV_TIMEOUT_TMA);
+      if (g == 0) mbar_wait(b_full + H, tile & 1, abort_s, DEV_TIMEOUT_TMA);
       // a row whose keys are all dropped has nl = +inf for every query (the mask row is shared by
       // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
       const bool deadstep = (lds_f32(vec_s) == kInf);
@@ -650,20 +652,18 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
             // two queries per instruction (the pairs lie side by side in every operand)
             F2 t[2] = {f2_make(nl.x, nl.y), f2_make(nl.z, nl.w)};
             const F2 de[2] = {f2_make(dl.x, dl.y), f2_make(dl.z, dl.w)};
-            if (has_bias) {
-              float bv[4];
+            float bv[4];
 #pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                if constexpr (kBias16) {
-                  const uint16_t raw = lds_u16(brow + (4 * c4 + u) * kBRow);
-                  bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
-                } else {
-                  bv[u] = lds_f32(brow + (4 * c4 + u) * kBRow);
-                }
+            for (int u = 0; u < 4; ++u) {
+              if constexpr (kBias16) {
+                const uint16_t raw = lds_u16(brow + (4 * c4 + u) * kBRow);
+                bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
+              } else {
+                bv[u] = lds_f32(brow + (4 * c4 + u) * kBRow);
               }
-              t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
-              t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
             }
+            t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
+            t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
               const int e = 4 * c4 + 2 * u;
@@ -706,7 +706,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           __syncwarp();
           if (lane == 0) mbar_arrive(cdone + 2 * H);
         }
-        if (flush_dbias && last_of_group) {
+        if (last_of_group && flush) {
           // The group's last row: this thread's 16 d_bias values of the chunk (one key, 16 queries) go
           // through the warp's staging area ([16 queries][32 keys]) and are added to d_bias in global
           // memory by a bulk tensor reduction that the warp issues itself.
@@ -737,7 +737,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(sdone + H);
-        if (has_bias && last_of_group) mbar_arrive(b_done + H);
+        if (last_of_group) mbar_arrive(b_done + H);
       }
       if (n > 0) send_dq(n - 1, p_row0, p_slab);  // its MMAs ran underneath this step
       p_row0 = it * BT + q4 * 32;
@@ -815,7 +815,7 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   const int sms = sm_count();
   if (sms <= 0) return EVOATTN_ERR_CUDA;
   const long long ctas = items < sms ? items : sms;
-  const auto kern = a.bias16 ? evo_bwd_sm100_kernel<T, DP, true, true> : evo_bwd_sm100_kernel<T, DP, true, false>;
+  const auto kern = a.bias16 ? evo_bwd_sm100_kernel<T, DP, true> : evo_bwd_sm100_kernel<T, DP, false>;
   const auto kern_n = !a.bias ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_NONE>
                       : (a.bias16 ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_16> : evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_F32>);
   const void* entry = nodbias ? reinterpret_cast<const void*>(kern_n) : reinterpret_cast<const void*>(kern);
