@@ -1,5 +1,5 @@
 // The fused backward kernel for calls that want no d(pair_bias) (inference-like fine tuning, a frozen bias, no
-// bias at all): the same items, steps and halves as evo_bwd_sm100_kernel, whose file this one is part of.  What the
+// bias at all): the same items, steps and halves as evo_bwd_sm100_kernel.  What the
 // missing gradient makes room for in shared memory changes how dQ leaves: a step's partial is one swizzled tile
 // that the loader adds to global memory by one bulk reduction, where every compute warp had to wait for its own
 // staging area and issue a reduction of its own; and the bias has a third half tile.  The compute warps wait three
@@ -10,16 +10,15 @@
 // one after another ([1,128,384,8,32] 195 and 199, [1,128,768,8,64] 1 148 and 1 182).
 #pragma once
 
-constexpr int BIAS_NONE = 0, BIAS_F32 = 1, BIAS_16 = 2;
+#include "bwd_common.cuh"
+
+namespace evo {
+namespace {
 
 template <int DP, int BIAS>
-struct SmemN {
-  static constexpr int G = RowsPerItem<DP>::G;
-  static constexpr int RB = DP * 2;                          // bytes per staged row
-  static constexpr int kTile = BT * RB;                      // one Q, dO, K or V tile
-  static constexpr int kVec = BT * 4;                        // one vector of row statistics
-  static constexpr int kStage = 2 * kTile + 2 * kVec;        // Q, dO, -lse*log2e, delta of one step
-  static constexpr int kDS = BT * BT * 2;                    // dS^T: two halves of [128 keys][64 queries]
+struct SmemN : TilesT<DP> {
+  using Tiles = TilesT<DP>;
+  using Tiles::G, Tiles::kTile, Tiles::kStage, Tiles::kDS;
   // The pair bias: half tiles [64 i][128 j], unswizzled; one more than is read at a time where it fits
   static constexpr int kHalfF32 = HT * BT * 4, kHalf = BIAS == BIAS_16 ? kHalfF32 / 2 : kHalfF32;
   static constexpr int kBufs = BIAS == BIAS_NONE ? 0 : DP == 64 && BIAS == BIAS_F32 ? 2 : 3;
@@ -50,17 +49,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
                 const __grid_constant__ CUtensorMap tmDQ,
                 const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL) {
   using L = SmemN<DP, BIAS>;
-  constexpr int RB = L::RB;
-  constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
-  constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-  static_assert(DP == 16 || DP == 32 || DP == 64, "padded head dimension");
-  static_assert(kStages == 2, "steps alternate between two stages");
-  constexpr int G = RowsPerItem<DP>::G;
-  constexpr int kTmemCols = 512;
-  // TMEM: two (S^T, dP^T) half-tile buffers, the per-row dV and dK accumulators, two dQ partials
-  constexpr int colS0 = 0, colDP0 = HT, colS1 = 2 * HT, colDP1 = 3 * HT;
-  constexpr int colDV = 4 * HT, colDK = colDV + G * DP, colDQ = colDK + G * DP;
-  static_assert(colDQ + 2 * DP <= kTmemCols, "TMEM budget");
+  constexpr int G = L::G;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -91,53 +80,14 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
-  const int NT = (a.R + BT - 1) / BT;
-  const int NC = (a.S + G - 1) / G;
   constexpr bool has_bias = BIAS != BIAS_NONE, kBias16 = BIAS == BIAS_16;
   // Whether the dV / dK MMAs of a half may go before its dS is stored, or all go at once ([4,1,2048,32,64] 597 us
   // and 570; [1,128,384,8,32] without a bias 139 and 150).
   constexpr bool EARLY = DP < 64;
   constexpr int kBufs = has_bias ? L::kBufs : 1, kHalf = L::kHalf;
   constexpr int kBRow = kBias16 ? BT * 2 : BT * 4;  // bytes per row (one query, 128 keys) of the staged bias tile
-  // Persistent CTAs: CTA c owns the items c, c + gridDim.x, ..., SPI steps per item.  A short last
-  // row group (S % G != 0) is padded with rows >= S: their tiles and statistics arrive as zeros and
-  // their mask is -inf, so P = dS = 0, and nothing of them is stored.
-  const int SPI = NT * G;
-  const int my_items = (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int total_steps = my_items * SPI;
-  auto decode = [&](int N) {
-    StepT d;
-    const int k = N / SPI, n = N - k * SPI;
-    d.it = n / G;
-    d.g = n - d.it * G;
-    int idx = (int)blockIdx.x + k * (int)gridDim.x;
-    const int chunk = idx % NC; idx /= NC;
-    d.j0 = (idx % NT) * BT; idx /= NT;
-    d.h = idx % a.H;
-    d.b = idx / a.H;
-    d.s = chunk * G + d.g;
-    return d;
-  };
-  auto advance = [&](const StepT& c, int n) {  // position of step n = the one after c (no divisions inside an item)
-    StepT d = c;
-    if (++d.g == G) {
-      d.g = 0;
-      if (++d.it == NT) return decode(n);
-    }
-    d.s = c.s - c.g + d.g;
-    return d;
-  };
-
-  // What the mask adds to a score of (b, s, key) in the log2 domain: 0 keeps it, -inf drops it (a dropped score
-  // gives P = 0 exactly, as exp(-FLT_MAX - lse) does in evoformer.py:69,600).
-  auto mask_of = [&](int b, int s, int j) -> float {
-    if (s >= a.S || j >= a.R) return -__int_as_float(0x7f800000);
-    if (a.mask_kind == EVOATTN_MASK_NONE) return 0.f;
-    const long long mi = (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c;
-    if (a.mask_kind == EVOATTN_MASK_BOOL) return reinterpret_cast<const unsigned char*>(a.mask)[mi] ? 0.f : -__int_as_float(0x7f800000);
-    if (a.mask_kind == EVOATTN_MASK_ADD_F32) return reinterpret_cast<const float*>(a.mask)[mi] * kLog2e;
-    return to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]) * kLog2e;
-  };
+  const Steps<G> steps(a, n_items);
+  const int NT = steps.NT, my_items = steps.items, total_steps = steps.total;
 
   grid_dependency_wait();
   grid_launch_dependents();
@@ -161,7 +111,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     if (has_bias) prefetch_tmap(&tmB);
   }
   if (warp == 0) {
-    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_alloc(tmem_slot, L::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -172,113 +122,18 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
   if (warp >= kCW) {
     setmaxnreg_dec<kServiceRegs>();
     if (warp <= kCW + 1) {
-      // =============================== tensor-core issuers: warp 16 (S^T, dV), warp 17 (dP^T, dK) ==========
-      // Issuing a tcgen05.mma costs the issuing warp fifty cycles and more, so the 32 MMAs of a step
-      // are spread over three warps on three schedulers.  A thread's MMAs run in issue order, MMAs of
-      // different threads in no particular order, so the split follows the data: warp 16 owns the
-      // S^T columns of both buffers (S^T = K_j Q_i^T in, dV_j += P^T dO_i out), warp 17 the dP^T columns
-      // (dP^T = V_j dO_i^T in, dK_j += dS^T Q_i out): the MMA that overwrites a buffer is always issued
-      // by the thread that issued the MMAs reading it.  Warp 18 issues dQ_i = dS K_j, which depends on
-      // neither.  The warps walk their loops converged (see elect_one).
-      const bool isA = (warp == kCW);
-      constexpr uint32_t kIdescSD = make_idesc(kBf16, false, false, BT, HT);   // S^T, dP^T: K-major operands, N = 64
-      constexpr uint32_t kIdescOut = make_idesc(kBf16, false, true, BT, DP);   // dV, dK: A from TMEM, B MN-major
-      constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
-      constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
-      constexpr uint32_t kRowBlk = (16 * RB) >> 4;  // 16 tile rows, in descriptor address units
-      // warp 16 reads K (A operand) and Q (B), then dO (B of dV); warp 17 reads V and dO, then Q (B of dK)
-      const uint32_t kv_lo = (smem_u32(sKV) >> 4) + (isA ? 0 : (L::kTile >> 4));
-      const uint32_t in_lo = (smem_u32(sStage) >> 4) + (isA ? 0 : (L::kTile >> 4));
-      const uint32_t out_lo = (smem_u32(sStage) >> 4) + (isA ? (L::kTile >> 4) : 0);
-      const uint32_t col_in0 = isA ? colS0 : colDP0, col_in1 = isA ? colS1 : colDP1;
-      const uint32_t col_acc = isA ? colDV : colDK;
-
-      // Position of a step inside this CTA's list, advanced without divisions: row g of the group,
-      // query tile it, ring stage and the parities of the stage ring and of the item.
-      struct Pos { int g, it; uint32_t stg, ring_par, item_par; };
-      auto after = [&](Pos p) {
-        if (++p.g == G) { p.g = 0; if (++p.it == NT) { p.it = 0; p.item_par ^= 1u; } }
-        if (++p.stg == (uint32_t)kStages) { p.stg = 0; p.ring_par ^= 1u; }
-        return p;
-      };
-      // Everything an MMA group needs is computed before the wait it follows: this thread shares its
-      // scheduler with four arithmetic warps, so every instruction between the wake-up and the MMA is
-      // paid several times over, and it sits on the critical path of the half that waits for it.
-      auto issue_in = [&](const Pos& p, uint32_t ka, uint32_t qb, int h) {
-        // (the second commit: the item's last read of this warp's K or V tile of row g)
-        const uint32_t bar2 = (h == 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
-        const uint32_t tD = tmem + (h ? col_in1 : col_in0), qa = qb + h * HT * (RB >> 4);
-        const uint32_t el = elect_one();
-#pragma unroll
-        for (int kk = 0; kk < DP / 16; ++kk)
-          mma_ss_e(el, tD, pack_desc(ka + 2 * kk, kHiOp), pack_desc(qa + 2 * kk, kHiOp), kIdescSD, kk > 0 ? 1u : 0u);
-        mma_commit_if_s(el, (sd_full + 2 * h).a);
-        if (bar2) mma_commit_if_s(el, bar2);
-        // The compute warps wait for S^T, dP^T and the statistics at once: this warp has seen these land.
-        if (isA) {
-          if (el) mbar_arrive(sd_full + 2 * h);
-          __syncwarp();
-        }
-      };
-      Pos cur{0, 0, 0u, 0u, 0u};
-      if (total_steps > 0) {
-        mbar_wait(st_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
-        mbar_wait(kv_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
-        tc_fence_after();
-        const uint32_t ka = (kv_lo + 0) | kLoLbo, qb = in_lo | kLoLbo;
-        issue_in(cur, ka, qb, 0);
-        issue_in(cur, ka, qb, 1);
-      }
-#pragma unroll 1
-      for (int n = 0; n < total_steps; ++n) {
-        const Pos nxt = after(cur);
-        const bool more = n + 1 < total_steps;
-        // this step: dV_j[g] += P^T dO_i (warp 16) or dK_j[g] += dS^T Q_i (warp 17);
-        // A = 16 queries of P^T / dS^T (8 packed TMEM columns), B = their dO / Q rows
-        const uint32_t acc = tmem + col_acc + cur.g * DP;
-        const uint32_t ob = (out_lo + cur.stg * (L::kStage >> 4)) | kLoLbo;
-        const uint32_t first0 = (cur.it == 0) ? 0u : 1u;  // the item's first MMA of row g overwrites
-        const uint32_t st_empty_bar = (st_empty + (int)cur.stg).a;
-        // next step: S^T = K_j Q_i^T (warp 16) or dP^T = V_j dO_i^T (warp 17) into the buffer just read
-        const uint32_t ka = (kv_lo + (2 * nxt.g) * (L::kTile >> 4)) | kLoLbo;
-        const uint32_t qb = (in_lo + nxt.stg * (L::kStage >> 4)) | kLoLbo;
-        const uint32_t st_full_bar = (st_full + (int)nxt.stg).a, kv_full_bar = (kv_full + nxt.g).a;
-        auto issue_out = [&](int h) {
-          mbar_wait(cdone + 2 * h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-          tc_fence_after();
-          const uint32_t tA = tmem + (h ? col_in1 : col_in0);
-          const uint32_t el = elect_one();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_ts_e(el, acc, tA + 16 * kk, pack_desc(ob + (4 * h + kk) * kRowBlk, kHiOp), kIdescOut, h == 0 && kk == 0 ? first0 : 1u);
-          if (h == 1) mma_commit_if_s(el, st_empty_bar);
-        };
-        issue_out(0);
-        if (more) {
-          mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
-          if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, DEV_TIMEOUT_TMA);
-          tc_fence_after();
-          issue_in(nxt, ka, qb, 0);
-        }
-        issue_out(1);
-        if (more) issue_in(nxt, ka, qb, 1);
-        cur = nxt;
-      }
+      // tensor-core issuers of S^T and dV (warp 16), dP^T and dK (warp 17)
+      issue_scores_and_outputs<T, DP, true>(warp == kCW, tmem, smem_u32(sKV), smem_u32(sStage), NT, total_steps,
+                                            IssueBars{kv_full, kv_empty, st_full, st_empty, sd_full, cdone}, abort_s);
     } else if (warp == kCW + 2) {
       // =============================== tensor-core issuer of dQ; pair-bias loads ===============================
-      constexpr uint32_t kIdescDQ = make_idesc(kBf16, true, true, BT, DP);     // A = dS^T read MN-major, B = K MN-major
-      constexpr uint32_t kHiDS = static_cast<uint32_t>(make_sdesc_const(16, 1024, SWZ_128B) >> 32);
-      constexpr uint32_t kLoLboDS = static_cast<uint32_t>(make_sdesc_const(BT * 128, 0, 0) & 0xffffffffu);
-      const uint32_t kv_lo0 = smem_u32(sKV) >> 4, ds_lo = smem_u32(sDS) >> 4;
-      constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
-      constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
-      constexpr uint32_t kRowBlk = (16 * RB) >> 4;  // 16 tile rows, in descriptor address units
+      const uint32_t sKV_s = smem_u32(sKV), sDS_s = smem_u32(sDS);
       const uint32_t sBias_s = smem_u32(sBias);
       // The bias tile (i, j) is the same for the G rows of a group.  Its halves (64 queries) go round the
       // buffers: half q = 2 * tile + h is loaded into buffer q % kBufs when the warps that read half q - kBufs
       // there have done so for the last time.
       auto load_bias = [&](uint32_t q) {
-        const StepT d = decode((int)(q >> 1) * G);
+        const StepT d = steps.decode((int)(q >> 1) * G);
         const uint32_t buf = q % kBufs;
         if (elect_one()) {
           mbar_expect_tx(b_full + (int)buf, kHalf);
@@ -305,12 +160,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
           }
         }
         tc_fence_after();
-        // dQ_i partial = dS K_j : A = dS^T tile [key][query] read MN-major (M = query), K runs over the keys
-        const uint32_t kq = (kv_lo0 + (2 * g) * (L::kTile >> 4)) | kLoLbo;
-        const uint32_t el = elect_one();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          mma_ss_e(el, tmem + colDQ + (n & 1) * DP, pack_desc((ds_lo | kLoLboDS) + 128 * kk, kHiDS), pack_desc(kq + kk * kRowBlk, kHiOp), kIdescDQ, kk > 0 ? 1u : 0u);
+        const uint32_t el = issue_dq<T, DP>(tmem + L::colDQ + (n & 1) * DP, sDS_s, sKV_s + 2 * g * L::kTile);
         mma_commit_if_s(el, (dq_full + (n & 1)).a);
         if (it == NT - 1) mma_commit_if_s(el, (kv_empty + g).a);
         if (++g == G) { g = 0; if (++it == NT) it = 0; }
@@ -341,13 +191,13 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         }
         __syncwarp();
       };
-      StepT d = decode(0);
+      StepT d = steps.decode(0);
       auto load_kv = [&](int n) {
-        const int k = n / SPI;
+        const int k = n / (NT * G);
         float mk[4];
         if constexpr (L::kMaskRows > 0) {  // four keys of the row's mask a lane, loaded before the wait
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mk[u] = mask_of(d.b, d.s, d.j0 + lane + 32 * u);
+          for (int u = 0; u < 4; ++u) mk[u] = mask_term<T>(a, d.b, d.s, d.j0 + lane + 32 * u);
         }
         mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
         if constexpr (L::kMaskRows > 0) {
@@ -398,7 +248,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
           slab1 = d.s < a.S ? (d.b * a.H + d.h) * a.S + d.s : -1;
         }
         if (G == 1 && load && d.it == 0) load_kv(n);
-        if (load) d = advance(d, n + 1);
+        if (load) d = steps.advance(d, n + 1);
       }
       if (total_steps > 0) {  // the last step's partial: the compute warps arrive once more
         mbar_wait(sdone + 0, total_steps & 1, abort_s, DEV_TIMEOUT_SYNC);
@@ -418,58 +268,22 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     const int q4 = warp & 3, cb2 = (warp >> 2) & 1, H = warp >> 3;
     const int jrow = q4 * 32 + lane;
     const uint32_t t_lane = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
-    const uint32_t cS = t_lane + (H ? colS1 : colS0) + QT * cb2, cP = t_lane + (H ? colDP1 : colDP0) + QT * cb2;
-    const float scale = a.scale;
+    const uint32_t cS = t_lane + (H ? L::colS1 : L::colS0) + QT * cb2, cP = t_lane + (H ? L::colDP1 : L::colDP0) + QT * cb2;
     const float inv_r = 1.f / (float)a.R;
     const float kInf = __int_as_float(0x7f800000);
-    const float c1 = scale * kLog2e;
+    const float c1 = a.scale * kLog2e;
     // 32-bit shared-window addresses: every access below stays a shared-memory instruction
     const uint32_t sStage_s = smem_u32(sStage), sDS_s = smem_u32(sDS);
     const uint32_t sBias_s = smem_u32(sBias);
     const uint32_t drow = sDS_s + H * (L::kDS / 2) + jrow * 128;
 
-    // dK, dV of row-group slot g (MSA row s of (b,h), keys j0..): TMEM -> registers -> global.
-    // Done by the warps of half 0 (half of the DP columns each, 16 at a time): they are the ones
-    // whose arrival lets the next item's first MMAs overwrite the slot.
-    auto drain_dkdv = [&](int b, int h, int s, int j0, int g) {
-      const int j = j0 + jrow;
-      constexpr int W = DP == 16 ? 8 : 16;  // columns at a time
-#pragma unroll
-      for (int part = 0; part < DP / 2 / W; ++part) {
-        const int c0 = cb2 * (DP / 2) + part * W;
-        uint32_t kr[W], vr[W];
-        tmem_ld<W>(t_lane + colDK + g * DP + c0, kr);
-        tmem_ld<W>(t_lane + colDV + g * DP + c0, vr);
-        tmem_wait_ld();
-        if (j < a.R && s < a.S) {
-          T* kd = reinterpret_cast<T*>(a.dk) + off4(a.sdk, b, h, s, j) + c0;
-          T* vd = reinterpret_cast<T*>(a.dv) + off4(a.sdv, b, h, s, j) + c0;
-#pragma unroll
-          for (int d8 = 0; d8 < W / 8; ++d8) {
-            if (c0 + d8 * 8 < a.D) {
-              uint4 pk, pv;
-              pk.x = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 0]) * scale, __uint_as_float(kr[d8 * 8 + 1]) * scale);
-              pk.y = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 2]) * scale, __uint_as_float(kr[d8 * 8 + 3]) * scale);
-              pk.z = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 4]) * scale, __uint_as_float(kr[d8 * 8 + 5]) * scale);
-              pk.w = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 6]) * scale, __uint_as_float(kr[d8 * 8 + 7]) * scale);
-              pv.x = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 0]), __uint_as_float(vr[d8 * 8 + 1]));
-              pv.y = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 2]), __uint_as_float(vr[d8 * 8 + 3]));
-              pv.z = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 4]), __uint_as_float(vr[d8 * 8 + 5]));
-              pv.w = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 6]), __uint_as_float(vr[d8 * 8 + 7]));
-              *reinterpret_cast<uint4*>(kd + d8 * 8) = pk;
-              *reinterpret_cast<uint4*>(vd + d8 * 8) = pv;
-            }
-          }
-        }
-      }
-    };
     // The dQ partial of step m (TMEM lanes = queries): a warp takes DP/4 columns of its 32 query rows.
     constexpr int QC = DP / 4;
     const int colblk = 2 * H + cb2;  // which of the four column blocks this warp takes
     // ... into the swizzled tile (two of 32 columns at DP = 64) that leaves as a whole
     auto store_dq = [&](int m) {
       uint32_t qr[QC];
-      tmem_ld<QC>(t_lane + colDQ + (m & 1) * DP + colblk * QC, qr);
+      tmem_ld<QC>(t_lane + L::colDQ + (m & 1) * DP + colblk * QC, qr);
       tmem_wait_ld();
       const uint32_t out = smem_u32(smem + L::offOut);
 #pragma unroll
@@ -483,17 +297,17 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
     const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
     float mreg[DP == 32 ? G : 1];
-    const F2 l2e2 = f2_make(kLog2e, kLog2e), c12 = f2_make(c1, c1), neg1 = f2_make(-1.f, -1.f);
+    const F2 c12 = f2_make(c1, c1);
     int n = 0;            // running step
     uint32_t tile = 0;    // running (item, query tile)
     uint32_t bias_s = 0;  // the half bias tile that this warp reads
     Bar bdone{0};
 #pragma unroll 1
     for (int k = 0; k < my_items; ++k) {
-    const StepT cur = decode(n);
+    const StepT cur = steps.decode(n);
     if constexpr (L::kMaskRows == 0) {
 #pragma unroll
-      for (int r = 0; r < G; ++r) mreg[r] = mask_of(cur.b, cur.s + r, cur.j0 + jrow);
+      for (int r = 0; r < G; ++r) mreg[r] = mask_term<T>(a, cur.b, cur.s + r, cur.j0 + jrow);
     }
 #pragma unroll 1
     for (int it = 0; it < NT; ++it, ++tile)
@@ -533,42 +347,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         tmem_wait_ld();
         uint32_t pk[8];
         if (!deadstep) {
-#pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {
-            const float4 nl = lds_v4f(vnl + 16 * c4);
-            const float4 dl = lds_v4f(vdl + 16 * c4);
-            // two queries per instruction (the pairs lie side by side in every operand)
-            F2 t[2] = {f2_make(nl.x, nl.y), f2_make(nl.z, nl.w)};
-            const F2 de[2] = {f2_make(dl.x, dl.y), f2_make(dl.z, dl.w)};
-            if (has_bias) {
-              float bv[4];
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                if constexpr (kBias16) {
-                  const uint16_t raw = lds_u16(brow + (4 * c4 + u) * kBRow);
-                  bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
-                } else {
-                  bv[u] = lds_f32(brow + (4 * c4 + u) * kBRow);
-                }
-              }
-              t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
-              t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
-            }
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int e = 4 * c4 + 2 * u;
-              // x = S*(scale*log2e) + (bias*log2e - lse*log2e) + mask
-              float x0, x1;
-              f2_get(f2_add(f2_fma(f2_from_bits(sr[e], sr[e + 1]), c12, t[u]), mj2), x0, x1);
-              const float p0 = ex2(x0), p1 = ex2(x1);
-              // dS = P (dP - delta)
-              const F2 ds = f2_mul(f2_make(p0, p1), f2_fma(de[u], neg1, f2_from_bits(dr[e], dr[e + 1])));
-              float d0, d1;
-              f2_get(ds, d0, d1);
-              pk[2 * c4 + u] = Pack2<T>::pack(p0, p1);
-              dk[sub * 8 + 2 * c4 + u] = Pack2<T>::pack(d0, d1);
-            }
-          }
+          score_chunk<T, BIAS, kBRow>(sr, dr, vnl, vdl, brow, c12, mj2, pk, dk + 8 * sub, [](int, F2) {});
         } else {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);
@@ -587,7 +366,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
           mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
           tc_fence_after();
         }
-        drain_dkdv(pb, ph, ps0 + g, pj0, g);
+        drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
       }
       // P^T and dS^T are in tensor memory: the dV / dK MMAs and the next S^T and dP^T may go, under what follows
       if constexpr (EARLY) {
@@ -629,11 +408,14 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         const int last = total_steps - 1;
         mbar_wait(st_empty + (last & 1), (last >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
-        for (int g = 0; g < G; ++g) drain_dkdv(pb, ph, ps0 + g, pj0, g);
+        for (int g = 0; g < G; ++g) drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
       }
     }
   }
 
   end_of_cta(abort_flag, a.status);
-  if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+  if (warp == 0) tmem_dealloc(tmem, L::kTmemCols);
 }
+
+}  // namespace
+}  // namespace evo

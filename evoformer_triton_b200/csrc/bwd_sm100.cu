@@ -25,8 +25,8 @@
 //
 // Warps: 0-15 compute (warp w: keys 32*(w%4).., queries 32*((w/4)%2).. of half w/8), 16-18 issue the
 // tcgen05.mma (18 also loads the pair-bias tiles), 19 loads the other tiles.
-#include <type_traits>
-
+#include "bwd_common.cuh"
+#include "bwd_nodbias.cuh"
 #include "common.cuh"
 #include "launch.h"
 #include "ptx.cuh"
@@ -35,28 +35,10 @@
 namespace evo {
 namespace {
 
-using namespace ptx;
-
-constexpr int BT = 128;   // tile edge (queries and keys)
-constexpr int HT = 64;    // queries per half of a step (one warp group)
-constexpr int QT = 32;    // queries per quarter of a step
-// MSA rows per work item: each keeps a dK and a dV accumulator of DP columns in tensor memory for the
-// whole item, next to 256 columns of score buffers and two dQ partials
-template <int DP> struct RowsPerItem { static constexpr int G = (DP == 64) ? 1 : (DP == 32) ? 3 : 7; };
-constexpr int kCW = 16;   // compute warps
-constexpr int kThreadsT = 640;  // 16 compute + 4 service warps, five warps per scheduler
-constexpr int kComputeRegs = 112, kServiceRegs = 32;  // after setmaxnreg; the launch-time pool must hold their sum
-constexpr int kStages = 2;  // (three or four stages measured no faster: the loads are not what a step waits for)
-constexpr float kLog2e = 1.4426950408889634f;
-
 template <int DP>
-struct SmemT {
-  static constexpr int G = RowsPerItem<DP>::G;
-  static constexpr int RB = DP * 2;                          // bytes per staged row
-  static constexpr int kTile = BT * RB;                      // one Q, dO, K or V tile
-  static constexpr int kVec = BT * 4;                        // one vector of row statistics
-  static constexpr int kStage = 2 * kTile + 2 * kVec;        // Q, dO, -lse*log2e, delta of one step
-  static constexpr int kDS = BT * BT * 2;                    // dS^T: two halves of [128 keys][64 queries]
+struct SmemT : TilesT<DP> {
+  using Tiles = TilesT<DP>;
+  using Tiles::G, Tiles::kTile, Tiles::kStage, Tiles::kDS;
   static constexpr int kBias = BT * BT * 4;                  // pair-bias tile [128 i][128 j], unswizzled (fp32; half of it for a 16-bit bias)
   static constexpr int kOutWarp = 2048;                      // per compute warp: staging of a d_bias chunk or a dQ block
   static constexpr int offKV = 0;                            // [g][K, V], resident for the whole item
@@ -75,21 +57,6 @@ struct SmemT {
   static_assert(offDS % 1024 == 0 && kStage % 1024 == 0 && offStage % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static_assert(bytes <= 232448, "shared memory budget of one CTA");
 };
-
-struct StepT {
-  int b, h, s, it, g, j0;
-};
-
-// An mbarrier named by its 32-bit shared-window address (8 bytes apart in the barrier array).
-struct Bar {
-  uint32_t a;
-};
-__device__ __forceinline__ Bar operator+(Bar b, int i) { return Bar{b.a + 8u * static_cast<uint32_t>(i)}; }
-__device__ __forceinline__ void mbar_wait(Bar b, uint32_t parity, uint32_t abort_s, int code) {
-  mbar_wait_s(b.a, parity, abort_s, code);
-}
-__device__ __forceinline__ void mbar_arrive(Bar b) { mbar_arrive_s(b.a); }
-__device__ __forceinline__ void mbar_expect_tx(Bar b, uint32_t bytes) { mbar_expect_tx_s(b.a, bytes); }
 
 // The first pass of a backward call: delta[b,h,s,i] = <dO_i, O_i> (evoformer.py:299-326), nl = -lse*log2e,
 // and zeros in the buffers that the fused kernel adds to (the fp32 dQ accumulator, d(pair_bias)).
@@ -209,17 +176,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
                 const __grid_constant__ CUtensorMap tmDB, const __grid_constant__ CUtensorMap tmDQ,
                 const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL) {
   using L = SmemT<DP>;
-  constexpr int RB = L::RB;
-  constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
-  constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-  static_assert(DP == 16 || DP == 32 || DP == 64, "padded head dimension");
-  static_assert(kStages == 2, "steps alternate between two stages");
-  constexpr int G = RowsPerItem<DP>::G;
-  constexpr int kTmemCols = 512;
-  // TMEM: two (S^T, dP^T) half-tile buffers, the per-row dV and dK accumulators, two dQ partials
-  constexpr int colS0 = 0, colDP0 = HT, colS1 = 2 * HT, colDP1 = 3 * HT;
-  constexpr int colDV = 4 * HT, colDK = colDV + G * DP, colDQ = colDK + G * DP;
-  static_assert(colDQ + 2 * DP <= kTmemCols, "TMEM budget");
+  constexpr int G = L::G;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -252,37 +209,9 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
-  const int NT = (a.R + BT - 1) / BT;
-  const int NC = (a.S + G - 1) / G;
   constexpr int kBRow = kBias16 ? BT * 2 : BT * 4;  // bytes per row (one query, 128 keys) of the staged bias tile
-  // Persistent CTAs: CTA c owns the items c, c + gridDim.x, ..., SPI steps per item.  A short last
-  // row group (S % G != 0) is padded with rows >= S: their tiles and statistics arrive as zeros and
-  // their mask is -inf, so P = dS = 0, and nothing of them is stored.
-  const int SPI = NT * G;
-  const int my_items = (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int total_steps = my_items * SPI;
-  auto decode = [&](int N) {
-    StepT d;
-    const int k = N / SPI, n = N - k * SPI;
-    d.it = n / G;
-    d.g = n - d.it * G;
-    int idx = (int)blockIdx.x + k * (int)gridDim.x;
-    const int chunk = idx % NC; idx /= NC;
-    d.j0 = (idx % NT) * BT; idx /= NT;
-    d.h = idx % a.H;
-    d.b = idx / a.H;
-    d.s = chunk * G + d.g;
-    return d;
-  };
-  auto advance = [&](const StepT& c, int n) {  // position of step n = the one after c (no divisions inside an item)
-    StepT d = c;
-    if (++d.g == G) {
-      d.g = 0;
-      if (++d.it == NT) return decode(n);
-    }
-    d.s = c.s - c.g + d.g;
-    return d;
-  };
+  const Steps<G> steps(a, n_items);
+  const int NT = steps.NT, my_items = steps.items, total_steps = steps.total;
 
   grid_dependency_wait();
   grid_launch_dependents();
@@ -306,7 +235,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     prefetch_tmap(&tmB); prefetch_tmap(&tmDB);
   }
   if (warp == 0) {
-    tmem_alloc(tmem_slot, kTmemCols);
+    tmem_alloc(tmem_slot, L::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -317,102 +246,12 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   if (warp >= kCW) {
     setmaxnreg_dec<kServiceRegs>();
     if (warp <= kCW + 1) {
-      // =============================== tensor-core issuers: warp 16 (S^T, dV), warp 17 (dP^T, dK) ==========
-      // Issuing a tcgen05.mma costs the issuing warp fifty cycles and more, so the 32 MMAs of a step
-      // are spread over three warps on three schedulers.  A thread's MMAs run in issue order, MMAs of
-      // different threads in no particular order, so the split follows the data: warp 16 owns the
-      // S^T columns of both buffers (S^T = K_j Q_i^T in, dV_j += P^T dO_i out), warp 17 the dP^T columns
-      // (dP^T = V_j dO_i^T in, dK_j += dS^T Q_i out): the MMA that overwrites a buffer is always issued
-      // by the thread that issued the MMAs reading it.  Warp 18 issues dQ_i = dS K_j, which depends on
-      // neither.  The warps walk their loops converged (see elect_one).
-      const bool isA = (warp == kCW);
-      constexpr uint32_t kIdescSD = make_idesc(kBf16, false, false, BT, HT);   // S^T, dP^T: K-major operands, N = 64
-      constexpr uint32_t kIdescOut = make_idesc(kBf16, false, true, BT, DP);   // dV, dK: A from TMEM, B MN-major
-      constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
-      constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
-      constexpr uint32_t kRowBlk = (16 * RB) >> 4;  // 16 tile rows, in descriptor address units
-      // warp 16 reads K (A operand) and Q (B), then dO (B of dV); warp 17 reads V and dO, then Q (B of dK)
-      const uint32_t kv_lo = (smem_u32(sKV) >> 4) + (isA ? 0 : (L::kTile >> 4));
-      const uint32_t in_lo = (smem_u32(sStage) >> 4) + (isA ? 0 : (L::kTile >> 4));
-      const uint32_t out_lo = (smem_u32(sStage) >> 4) + (isA ? (L::kTile >> 4) : 0);
-      const uint32_t col_in0 = isA ? colS0 : colDP0, col_in1 = isA ? colS1 : colDP1;
-      const uint32_t col_acc = isA ? colDV : colDK;
-
-      // Position of a step inside this CTA's list, advanced without divisions: row g of the group,
-      // query tile it, ring stage and the parities of the stage ring and of the item.
-      struct Pos { int g, it; uint32_t stg, ring_par, item_par; };
-      auto after = [&](Pos p) {
-        if (++p.g == G) { p.g = 0; if (++p.it == NT) { p.it = 0; p.item_par ^= 1u; } }
-        if (++p.stg == (uint32_t)kStages) { p.stg = 0; p.ring_par ^= 1u; }
-        return p;
-      };
-      // Everything an MMA group needs is computed before the wait it follows: this thread shares its
-      // scheduler with four arithmetic warps, so every instruction between the wake-up and the MMA is
-      // paid several times over, and it sits on the critical path of the half that waits for it.
-      auto issue_in = [&](const Pos& p, uint32_t ka, uint32_t qb, int h) {
-        // (the second commit: the item's last read of this warp's K or V tile of row g)
-        const uint32_t bar2 = (h == 1 && p.it == NT - 1) ? (kv_empty + p.g).a : 0u;
-        const uint32_t tD = tmem + (h ? col_in1 : col_in0), qa = qb + h * HT * (RB >> 4);
-        const uint32_t el = elect_one();
-#pragma unroll
-        for (int kk = 0; kk < DP / 16; ++kk)
-          mma_ss_e(el, tD, pack_desc(ka + 2 * kk, kHiOp), pack_desc(qa + 2 * kk, kHiOp), kIdescSD, kk > 0 ? 1u : 0u);
-        mma_commit_if_s(el, (sd_full + 2 * h).a);
-        if (bar2) mma_commit_if_s(el, bar2);
-      };
-      Pos cur{0, 0, 0u, 0u, 0u};
-      if (total_steps > 0) {
-        mbar_wait(st_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
-        mbar_wait(kv_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
-        tc_fence_after();
-        const uint32_t ka = (kv_lo + 0) | kLoLbo, qb = in_lo | kLoLbo;
-        issue_in(cur, ka, qb, 0);
-        issue_in(cur, ka, qb, 1);
-      }
-#pragma unroll 1
-      for (int n = 0; n < total_steps; ++n) {
-        const Pos nxt = after(cur);
-        const bool more = n + 1 < total_steps;
-        // this step: dV_j[g] += P^T dO_i (warp 16) or dK_j[g] += dS^T Q_i (warp 17);
-        // A = 16 queries of P^T / dS^T (8 packed TMEM columns), B = their dO / Q rows
-        const uint32_t acc = tmem + col_acc + cur.g * DP;
-        const uint32_t ob = (out_lo + cur.stg * (L::kStage >> 4)) | kLoLbo;
-        const uint32_t first0 = (cur.it == 0) ? 0u : 1u;  // the item's first MMA of row g overwrites
-        const uint32_t st_empty_bar = (st_empty + (int)cur.stg).a;
-        // next step: S^T = K_j Q_i^T (warp 16) or dP^T = V_j dO_i^T (warp 17) into the buffer just read
-        const uint32_t ka = (kv_lo + (2 * nxt.g) * (L::kTile >> 4)) | kLoLbo;
-        const uint32_t qb = (in_lo + nxt.stg * (L::kStage >> 4)) | kLoLbo;
-        const uint32_t st_full_bar = (st_full + (int)nxt.stg).a, kv_full_bar = (kv_full + nxt.g).a;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          mbar_wait(cdone + 2 * h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-          tc_fence_after();
-          const uint32_t tA = tmem + (h ? col_in1 : col_in0);
-          const uint32_t el = elect_one();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_ts_e(el, acc, tA + 16 * kk, pack_desc(ob + (4 * h + kk) * kRowBlk, kHiOp), kIdescOut, h == 0 && kk == 0 ? first0 : 1u);
-          if (h == 1) mma_commit_if_s(el, st_empty_bar);
-          if (more) {
-            if (h == 0) {
-              mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
-              if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, DEV_TIMEOUT_TMA);
-              tc_fence_after();
-            }
-            issue_in(nxt, ka, qb, h);
-          }
-        }
-        cur = nxt;
-      }
+      // tensor-core issuers of S^T and dV (warp 16), dP^T and dK (warp 17)
+      issue_scores_and_outputs<T, DP, false>(warp == kCW, tmem, smem_u32(sKV), smem_u32(sStage), NT, total_steps,
+                                             IssueBars{kv_full, kv_empty, st_full, st_empty, sd_full, cdone}, abort_s);
     } else if (warp == kCW + 2) {
       // =============================== tensor-core issuer of dQ; pair-bias loads ===============================
-      constexpr uint32_t kIdescDQ = make_idesc(kBf16, true, true, BT, DP);     // A = dS^T read MN-major, B = K MN-major
-      constexpr uint32_t kHiOp = static_cast<uint32_t>(make_sdesc_const(16, 8 * RB, SWZ) >> 32);
-      constexpr uint32_t kHiDS = static_cast<uint32_t>(make_sdesc_const(16, 1024, SWZ_128B) >> 32);
-      constexpr uint32_t kLoLbo = static_cast<uint32_t>(make_sdesc_const(16, 0, 0) & 0xffffffffu);
-      constexpr uint32_t kLoLboDS = static_cast<uint32_t>(make_sdesc_const(BT * 128, 0, 0) & 0xffffffffu);
-      constexpr uint32_t kRowBlk = (16 * RB) >> 4;
-      const uint32_t kv_lo = smem_u32(sKV) >> 4, ds_lo = smem_u32(sDS) >> 4;
+      const uint32_t sKV_s = smem_u32(sKV), sDS_s = smem_u32(sDS);
       const uint32_t sBias_s = smem_u32(sBias);
       // The bias tile (i, j) is the same for the G rows of a group; each half (64 queries) is loaded
       // for the group's first step and replaced as soon as the warps of that half have read it for
@@ -425,13 +264,13 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         __syncwarp();
       };
       const int tiles = my_items * NT;
-      if (tiles > 0) { const StepT d0 = decode(0); load_bias(d0, 0); load_bias(d0, 1); }
+      if (tiles > 0) { const StepT d0 = steps.decode(0); load_bias(d0, 0); load_bias(d0, 1); }
       int g = 0, it = 0, t = 0;  // row of the group, query tile, running (item, query tile) index
 #pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const bool turn = g == G - 1 && t + 1 < tiles;  // the group's last step: the halves come back
         StepT nb = StepT{0, 0, 0, 0, 0, 0};
-        if (turn) nb = decode((t + 1) * G);  // (divisions: before the waits, not between them)
+        if (turn) nb = steps.decode((t + 1) * G);  // (divisions: before the waits, not between them)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           mbar_wait(sdone + h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
@@ -441,12 +280,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           }
         }
         tc_fence_after();
-        const uint32_t ka = (kv_lo + (2 * g) * (L::kTile >> 4)) | kLoLbo;
-        // dQ_i partial = dS K_j : A = dS^T tile [key][query] read MN-major (M = query), K runs over the keys
-        const uint32_t el = elect_one();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk)
-          mma_ss_e(el, tmem + colDQ + (n & 1) * DP, pack_desc((ds_lo | kLoLboDS) + 128 * kk, kHiDS), pack_desc(ka + kk * kRowBlk, kHiOp), kIdescDQ, kk > 0 ? 1u : 0u);
+        const uint32_t el = issue_dq<T, DP>(tmem + L::colDQ + (n & 1) * DP, sDS_s, sKV_s + 2 * g * L::kTile);
         mma_commit_if_s(el, (dq_full + (n & 1)).a);
         mma_commit_if_s(el, ds_empty.a);
         if (it == NT - 1) mma_commit_if_s(el, (kv_empty + g).a);
@@ -457,27 +291,17 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       // K/V of row g stay for the whole item and are replaced when the item's last MMAs that read them
       // have completed; Q, dO and the two statistics vectors of a step ride a two-deep ring.
       const uint32_t sKV_s = smem_u32(sKV), sStage_s = smem_u32(sStage), sMask_s = smem_u32(smem + L::offMask);
-      auto mask_of = [&](int b, int s, int j) -> float {
-        if (s >= a.S || j >= a.R) return -__int_as_float(0x7f800000);
-        if (a.mask_kind == EVOATTN_MASK_NONE) return 0.f;
-        const long long mi = (long long)b * a.smask.a + (long long)s * a.smask.b + (long long)j * a.smask.c;
-        if (a.mask_kind == EVOATTN_MASK_BOOL) return reinterpret_cast<const unsigned char*>(a.mask)[mi] ? 0.f : -__int_as_float(0x7f800000);
-        if (a.mask_kind == EVOATTN_MASK_ADD_F32) return reinterpret_cast<const float*>(a.mask)[mi] * kLog2e;
-        return to_float<T>(reinterpret_cast<const T*>(a.mask)[mi]) * kLog2e;
-      };
-      StepT d = decode(0);
+      StepT d = steps.decode(0);
 #pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const int stg = n % kStages;
         if (d.it == 0) {
-          const int k = n / SPI;
-          // The mask of the row: four keys a lane, loaded before the wait.  In the log2 domain it is added to a
-          // score: 0 keeps it, -inf drops it (a dropped score gives P = 0 exactly, as exp(-FLT_MAX - lse)
-          // does in evoformer.py:69,600).  (The last dQ MMA of the row is behind kv_empty, so its last
-          // step has read the mask before.)
+          const int k = n / (NT * G);
+          // The mask of the row: four keys a lane, loaded before the wait.  (The last dQ MMA of the row is behind
+          // kv_empty, so its last step has read the mask before.)
           float mk[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mk[u] = mask_of(d.b, d.s, d.j0 + lane + 32 * u);
+          for (int u = 0; u < 4; ++u) mk[u] = mask_term<T>(a, d.b, d.s, d.j0 + lane + 32 * u);
           mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
 #pragma unroll
           for (int u = 0; u < 4; ++u) sts_f32(sMask_s + (d.g * BT + lane + 32 * u) * 4, mk[u]);
@@ -502,7 +326,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           tma_load_3d_s(dst + 2 * L::kTile + L::kVec, &tmDL, bar, d.it * BT, d.s, d.b * a.H + d.h);
         }
         __syncwarp();
-        d = advance(d, n + 1);
+        d = steps.advance(d, n + 1);
       }
     }
   } else {
@@ -519,11 +343,10 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     const int q4 = warp & 3, cb2 = (warp >> 2) & 1, H = warp >> 3;
     const int jrow = q4 * 32 + lane;
     const uint32_t t_lane = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
-    const uint32_t cS = t_lane + (H ? colS1 : colS0) + QT * cb2, cP = t_lane + (H ? colDP1 : colDP0) + QT * cb2;
-    const float scale = a.scale;
+    const uint32_t cS = t_lane + (H ? L::colS1 : L::colS0) + QT * cb2, cP = t_lane + (H ? L::colDP1 : L::colDP0) + QT * cb2;
     const float inv_r = 1.f / (float)a.R;
     const float kInf = __int_as_float(0x7f800000);
-    const float c1 = scale * kLog2e;
+    const float c1 = a.scale * kLog2e;
     // 32-bit shared-window addresses: every access below stays a shared-memory instruction
     const uint32_t sStage_s = smem_u32(sStage), sDS_s = smem_u32(sDS);
     const uint32_t out_s = smem_u32(sOut) + warp * L::kOutWarp;  // this warp's private staging area
@@ -536,41 +359,6 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       __syncwarp();
     };
 
-    // dK, dV of row-group slot g (MSA row s of (b,h), keys j0..): TMEM -> registers -> global.
-    // Done by the warps of half 0 (half of the DP columns each, 16 at a time): they are the ones
-    // whose arrival lets the next item's first MMAs overwrite the slot.
-    auto drain_dkdv = [&](int b, int h, int s, int j0, int g) {
-      const int j = j0 + jrow;
-      constexpr int W = DP == 16 ? 8 : 16;  // columns at a time
-#pragma unroll
-      for (int part = 0; part < DP / 2 / W; ++part) {
-        const int c0 = cb2 * (DP / 2) + part * W;
-        uint32_t kr[W], vr[W];
-        tmem_ld<W>(t_lane + colDK + g * DP + c0, kr);
-        tmem_ld<W>(t_lane + colDV + g * DP + c0, vr);
-        tmem_wait_ld();
-        if (j < a.R && s < a.S) {
-          T* kd = reinterpret_cast<T*>(a.dk) + off4(a.sdk, b, h, s, j) + c0;
-          T* vd = reinterpret_cast<T*>(a.dv) + off4(a.sdv, b, h, s, j) + c0;
-#pragma unroll
-          for (int d8 = 0; d8 < W / 8; ++d8) {
-            if (c0 + d8 * 8 < a.D) {
-              uint4 pk, pv;
-              pk.x = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 0]) * scale, __uint_as_float(kr[d8 * 8 + 1]) * scale);
-              pk.y = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 2]) * scale, __uint_as_float(kr[d8 * 8 + 3]) * scale);
-              pk.z = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 4]) * scale, __uint_as_float(kr[d8 * 8 + 5]) * scale);
-              pk.w = Pack2<T>::pack(__uint_as_float(kr[d8 * 8 + 6]) * scale, __uint_as_float(kr[d8 * 8 + 7]) * scale);
-              pv.x = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 0]), __uint_as_float(vr[d8 * 8 + 1]));
-              pv.y = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 2]), __uint_as_float(vr[d8 * 8 + 3]));
-              pv.z = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 4]), __uint_as_float(vr[d8 * 8 + 5]));
-              pv.w = Pack2<T>::pack(__uint_as_float(vr[d8 * 8 + 6]), __uint_as_float(vr[d8 * 8 + 7]));
-              *reinterpret_cast<uint4*>(kd + d8 * 8) = pk;
-              *reinterpret_cast<uint4*>(vd + d8 * 8) = pv;
-            }
-          }
-        }
-      }
-    };
     // The dQ partial of step m at position d (TMEM lanes = queries): this warp's DP/4 columns of its 32
     // query rows go through its staging area ([32 rows][DP/4 floats]) into the fp32 accumulator in global
     // memory, as one small bulk tensor reduction that the warp issues itself.  It happens after the
@@ -582,7 +370,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       mbar_wait(dq_full + (m & 1), (m >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
       uint32_t qr[QC];
-      tmem_ld<QC>(t_lane + colDQ + (m & 1) * DP + colblk * QC, qr);
+      tmem_ld<QC>(t_lane + L::colDQ + (m & 1) * DP + colblk * QC, qr);
       staging_free();
       tmem_wait_ld();
 #pragma unroll
@@ -604,7 +392,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     // row the unconditional form is the faster one ([1,128,768,8,64] 1 092 instead of 1 160).
     const bool flush = G == 1 || a.dbias != nullptr;
     const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
-    const F2 l2e2 = f2_make(kLog2e, kLog2e), c12 = f2_make(c1, c1), neg1 = f2_make(-1.f, -1.f);
+    const F2 c12 = f2_make(c1, c1);
     F2 bacc[16];  // d(pair_bias) of this thread's key and its 32 queries, summed over the rows of a group
 #pragma unroll
     for (int e = 0; e < 16; ++e) bacc[e] = f2_make(0.f, 0.f);
@@ -613,7 +401,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     uint32_t tile = 0;  // running (item, query tile)
 #pragma unroll 1
     for (int k = 0; k < my_items; ++k) {
-    const StepT cur = decode(n);
+    const StepT cur = steps.decode(n);
 #pragma unroll 1
     for (int it = 0; it < NT; ++it, ++tile)
 #pragma unroll 1
@@ -645,41 +433,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tmem_wait_ld();
         uint32_t pk[8];
         if (!deadstep) {
-#pragma unroll
-          for (int c4 = 0; c4 < 4; ++c4) {
-            const float4 nl = lds_v4f(vnl + 16 * c4);
-            const float4 dl = lds_v4f(vdl + 16 * c4);
-            // two queries per instruction (the pairs lie side by side in every operand)
-            F2 t[2] = {f2_make(nl.x, nl.y), f2_make(nl.z, nl.w)};
-            const F2 de[2] = {f2_make(dl.x, dl.y), f2_make(dl.z, dl.w)};
-            float bv[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              if constexpr (kBias16) {
-                const uint16_t raw = lds_u16(brow + (4 * c4 + u) * kBRow);
-                bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
-              } else {
-                bv[u] = lds_f32(brow + (4 * c4 + u) * kBRow);
-              }
-            }
-            t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
-            t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int e = 4 * c4 + 2 * u;
-              // x = S*(scale*log2e) + (bias*log2e - lse*log2e) + mask
-              float x0, x1;
-              f2_get(f2_add(f2_fma(f2_from_bits(sr[e], sr[e + 1]), c12, t[u]), mj2), x0, x1);
-              const float p0 = ex2(x0), p1 = ex2(x1);
-              // dS = P (dP - delta); d_bias_acc += dS
-              const F2 ds = f2_mul(f2_make(p0, p1), f2_fma(de[u], neg1, f2_from_bits(dr[e], dr[e + 1])));
-              bacc[(sub * 16 + e) / 2] = f2_add(bacc[(sub * 16 + e) / 2], ds);
-              float d0, d1;
-              f2_get(ds, d0, d1);
-              pk[2 * c4 + u] = Pack2<T>::pack(p0, p1);
-              dk[sub * 8 + 2 * c4 + u] = Pack2<T>::pack(d0, d1);
-            }
-          }
+          score_chunk<T, kBias16 ? BIAS_16 : BIAS_F32, kBRow>(sr, dr, vnl, vdl, brow, c12, mj2, pk, dk + 8 * sub,
+                                                              [&](int e, F2 ds) { bacc[8 * sub + e] = f2_add(bacc[8 * sub + e], ds); });
         } else {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);
@@ -698,7 +453,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
             mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
             tc_fence_after();
           }
-          drain_dkdv(pb, ph, ps0 + g, pj0, g);
+          drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
         }
         if (sub == 1) {
           tmem_wait_st();
@@ -753,17 +508,15 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         const int last = total_steps - 1;
         mbar_wait(st_empty + (last & 1), (last >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
-        for (int g = 0; g < G; ++g) drain_dkdv(pb, ph, ps0 + g, pj0, g);
+        for (int g = 0; g < G; ++g) drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
       }
     }
     if (lane == 0) tma_wait_group0();  // this warp's reductions have completed before the CTA may exit
   }
 
   end_of_cta(abort_flag, a.status);
-  if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+  if (warp == 0) tmem_dealloc(tmem, L::kTmemCols);
 }
-
-#include "bwd_nodbias.cuh"
 
 size_t align_up(size_t x, size_t al) { return (x + al - 1) / al * al; }
 
