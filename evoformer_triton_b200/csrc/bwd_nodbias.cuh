@@ -5,9 +5,9 @@
 // staging area and issue a reduction of its own; and the bias has a third half tile.  The compute warps wait three
 // times a step (S^T and dP^T with the statistics; the bias; dQ of the step before with the place for it) instead of
 // five.  Bound, as the other form, by the instructions and hand-overs of the compute warps.  Backward calls, us,
-// against that form: [4,1,2048,32,64] 742 -> 570, [4,1,300,32,64] 46 -> 42, [1,128,384,8,32] without a bias 148 -> 139.
+// against that form: [4,1,2048,32,64] 742 -> 576, [4,1,300,32,64] 46 -> 42, [1,128,384,8,32] without a bias 148 -> 139.
 // With a d(pair_bias) it is the slower of the two: the bulk reductions of both leave at some 16 bytes a cycle and SM
-// one after another ([1,128,384,8,32] 195 and 199, [1,128,768,8,64] 1 148 and 1 182).
+// one after another ([1,128,384,8,32] 195 and 199, [1,128,768,8,64] 1 148 and 1 182, both before the former came to 1 096).
 #pragma once
 
 #include "bwd_common.cuh"

@@ -1,5 +1,5 @@
 // Evoformer attention backward for sm_100a: the fused dQ/dK/dV/d(pair_bias) kernel with TRANSPOSED
-// score tiles, for head dimensions up to 64 (padded to 32 or 64).
+// score tiles, for head dimensions up to 64 (padded to 16, 32 or 64).
 //
 // Replaces dsevoformer-triton/evoformer.py:299-326 (_attn_bwd_preprocess), :479-630
 // (_attn_bwd_dk_dv) and :329-476 (_attn_bwd_dq).  The reference recomputes S and dP in two kernels
@@ -15,8 +15,8 @@
 //   * The shared memory this frees holds the K/V tiles of a work item for its whole life and the
 //     pair-bias tile of a whole row group.
 //
-// Work item = one 128-key tile j of G consecutive MSA rows of one (b,h): G = 3 at a padded head
-// dimension of 32, G = 1 at 64 (the dK/dV accumulators of a row take 2*DP of the 512 TMEM columns).
+// Work item = one 128-key tile j of G consecutive MSA rows of one (b,h): G = 7 at a padded head
+// dimension of 16, 3 at 32 and 1 at 64 (the dK/dV accumulators of a row take 2*DP of the 512 TMEM columns).
 // A persistent CTA walks its items as a flat list of steps (query tile i, row g); a step is two
 // halves of 64 queries, each with its own TMEM score buffer and its own eight warps: while one half
 // computes, the tensor core finishes the other half's dV/dK MMAs and its next S^T/dP^T.
@@ -338,7 +338,7 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     // a scheduler, no wait of any length): positions are loop counters and the mask of a key comes staged.
     // Backward calls with that, the issue loops walked by converged warps and the waits in one short sequence,
     // before and after, us: [1,128,384,8,32] 211 -> 195, [1,384,384,4,32] 348 -> 306, [1,1024,384,8,8] fp16
-    // 1251 -> 1083, [1,128,768,8,64] 1195 -> 1148, [4,1,2048,32,64] without d(pair_bias) 819 -> 742.
+    // 1251 -> 1083, [1,128,768,8,64] 1195 -> 1148 (1 096 now), [4,1,2048,32,64] without d(pair_bias) 819 -> 742.
     setmaxnreg_inc<kComputeRegs>();
     const int q4 = warp & 3, cb2 = (warp >> 2) & 1, H = warp >> 3;
     const int jrow = q4 * 32 + lane;

@@ -23,7 +23,7 @@
 // Per warpgroup and key tile n:  S_n = Q K_n^T lands in TMEM; the warpgroup turns it into P_n (rounded to
 // the storage type as evoformer.py:84 does) and writes it back over S_n in TMEM, from where it feeds the P V
 // MMA as the A operand; O accumulates in TMEM over the item.  With two warpgroups S is double buffered; with
-// three or four (168 to 112 registers a thread) it is not, and the other warpgroups hide the hand-over.
+// three or four (152 and 112 registers a thread) it is not, and the other warpgroups hide the hand-over.
 //
 // The exponentials of a tile do not wait for its maximum: they are taken against the running maximum m of the
 // tiles before (of the first tile, its own), straight from the scores: load, two FMAs, ex2, row sum, pack.  Only
@@ -33,9 +33,9 @@
 // (Lag), the next tile's maximum is taken first, and its exponentials only once.
 //
 // Bound by the issue slots and hand-overs around the exponentials (16 a cycle and SM: [1,256,1024,4,32] would
-// take 236 us).  That shape takes 379 us with four warpgroups, and 540 with the form before, which had the
+// take 236 us).  That shape takes 378 us with four warpgroups, and 540 with the form before, which had the
 // maximum in line, two warpgroups taking turns, one TMA copy per row and MMAs issued from a single-lane branch;
-// [1,128,384,8,32] 97 -> 77, [1,1024,384,8,8] fp16 703 -> 507, [1,128,768,8,64] 349 -> 309 us.
+// [1,128,384,8,32] 97 -> 77, [1,1024,384,8,8] fp16 703 -> 505, [1,128,768,8,64] 349 -> 295 us.
 #include <type_traits>
 
 #include "common.cuh"
@@ -79,8 +79,8 @@ struct Cfg {
   // Query pairs with an fp32 bias: a stage of V and the bias is 64 KB and more, so there are two of them, and at
   // DP = 64 two of K, which leaves room for the masks of every length.  Bound by reading the bias (332 us of it at
   // 2 048).  Forward of [4,1,R,32,D] bf16, us, as query pairs and as items of two rows, the second of which does not
-  // exist: R = 2048, D = 8 343 and 426, D = 32 354 and 447, D = 64 376 and 538; R = 300 18.5 and 22.6, 20.6 and 22.6,
-  // 24.1 (either way, a third K stage made no difference).
+  // exist: R = 2048, D = 8 343 and 426, D = 32 354 and 447, D = 64 376 and 538; R = 300, D = 8 18.5 and 22.6, D = 32
+  // 20.6 and 22.6.  (At D = 64 up to 1 472 query pairs fitted with three stages of K as well: 24 and 114 either way.)
   static constexpr bool kWide = QP && BIAS == BIAS_F32;
   static constexpr int NK = DP == 64 && NW > 2 ? 1 : DP == 64 && kWide ? 2 : SB + 1;  // K stages (S is through with one early in a tile)
   static constexpr int NV = (DP == 64 || NW > 2 || kWide) ? 2 : 3;  // stages of V and the pair bias
