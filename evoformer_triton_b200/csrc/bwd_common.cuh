@@ -112,14 +112,18 @@ __device__ __forceinline__ float mask_term(const Args& a, int b, int s, int j) {
 // (dP^T = V_j dO_i^T in, dK_j += dS^T Q_i out): the MMA that overwrites a buffer is always issued
 // by the thread that issued the MMAs reading it.  Warp 18 issues dQ_i = dS K_j, which depends on
 // neither.  The warps walk their loops converged (see elect_one).
+// The compute warps wait for S^T, dP^T and the statistics at once, and warp 16, which has seen these land, arrives on
+// their barrier for them.
+// With one row per item (G = 1) every item boundary would be a gap of a load and more: K and V have a barrier each
+// (kv_full, kv_empty: [0] K, [1] V).  V is replaced as soon as the item's last dP^T is through, by load_v() of warp 17;
+// K, which dQ reads too, by warp 18.  The outputs of an item's last step do not wait for the next K, and the compute
+// warps read dK and dV meanwhile; `drained` lets the next item's first outputs overwrite them.
 struct IssueBars {
-  Bar kv_full, kv_empty, st_full, st_empty, sd_full, cdone;
+  Bar kv_full, kv_empty, st_full, st_empty, sd_full, cdone, drained;
 };
-// STATS: the compute warps wait for S^T, dP^T and the statistics at once, and warp 16, which has seen these land,
-// arrives on their barrier for them.
-template <class T, int DP, bool STATS>
+template <class T, int DP, class LoadV>
 __device__ __forceinline__ void issue_scores_and_outputs(bool isA, uint32_t tmem, uint32_t sKV_s, uint32_t sStage_s, int NT,
-                                                         int total_steps, const IssueBars& bar, uint32_t abort_s) {
+                                                         int total_steps, const IssueBars& bar, uint32_t abort_s, LoadV load_v) {
   using L = TilesT<DP>;
   constexpr int G = L::G, RB = L::RB;
   constexpr uint32_t SWZ = swizzle_code_for_row_bytes(RB);
@@ -149,7 +153,7 @@ __device__ __forceinline__ void issue_scores_and_outputs(bool isA, uint32_t tmem
   // paid several times over, and it sits on the critical path of the half that waits for it.
   auto issue_in = [&](const Pos& p, uint32_t ka, uint32_t qb, int h) {
     // (the second commit: the item's last read of this warp's K or V tile of row g)
-    const uint32_t bar2 = (h == 1 && p.it == NT - 1) ? (bar.kv_empty + p.g).a : 0u;
+    const uint32_t bar2 = (h == 1 && p.it == NT - 1 && !(G == 1 && isA)) ? (bar.kv_empty + (G == 1 ? 1 : p.g)).a : 0u;
     const uint32_t tD = tmem + (h ? col_in1 : col_in0), qa = qb + h * HT * (RB >> 4);
     const uint32_t el = elect_one();
 #pragma unroll
@@ -157,15 +161,16 @@ __device__ __forceinline__ void issue_scores_and_outputs(bool isA, uint32_t tmem
       mma_ss_e(el, tD, pack_desc(ka + 2 * kk, kHiOp), pack_desc(qa + 2 * kk, kHiOp), kIdescSD, kk > 0 ? 1u : 0u);
     mma_commit_if_s(el, (bar.sd_full + 2 * h).a);
     if (bar2) mma_commit_if_s(el, bar2);
-    if (STATS && isA) {
+    if (isA) {
       if (el) mbar_arrive(bar.sd_full + 2 * h);
       __syncwarp();
     }
+    if (G == 1 && !isA && bar2) load_v();
   };
   Pos cur{0, 0, 0u, 0u, 0u};
   if (total_steps > 0) {
     mbar_wait(bar.st_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
-    mbar_wait(bar.kv_full + 0, 0, abort_s, DEV_TIMEOUT_TMA);
+    mbar_wait(bar.kv_full + (G == 1 && !isA ? 1 : 0), 0, abort_s, DEV_TIMEOUT_TMA);
     tc_fence_after();
     const uint32_t ka = (kv_lo + 0) | kLoLbo, qb = in_lo | kLoLbo;
     issue_in(cur, ka, qb, 0);
@@ -184,10 +189,10 @@ __device__ __forceinline__ void issue_scores_and_outputs(bool isA, uint32_t tmem
     // next step: S^T = K_j Q_i^T (warp 16) or dP^T = V_j dO_i^T (warp 17) into the buffer just read
     const uint32_t ka = (kv_lo + (2 * nxt.g) * (L::kTile >> 4)) | kLoLbo;
     const uint32_t qb = (in_lo + nxt.stg * (L::kStage >> 4)) | kLoLbo;
-    const uint32_t st_full_bar = (bar.st_full + (int)nxt.stg).a, kv_full_bar = (bar.kv_full + nxt.g).a;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
+    const uint32_t st_full_bar = (bar.st_full + (int)nxt.stg).a, kv_full_bar = (bar.kv_full + (G == 1 ? (isA ? 0 : 1) : nxt.g)).a;
+    auto outputs = [&](int h) {
       mbar_wait(bar.cdone + 2 * h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+      if (G == 1 && h == 0 && cur.it == 0 && n > 0) mbar_wait(bar.drained, cur.item_par ^ 1u, abort_s, DEV_TIMEOUT_SYNC);
       tc_fence_after();
       const uint32_t tA = tmem + (h ? col_in1 : col_in0);
       const uint32_t el = elect_one();
@@ -195,15 +200,26 @@ __device__ __forceinline__ void issue_scores_and_outputs(bool isA, uint32_t tmem
       for (int kk = 0; kk < 4; ++kk)
         mma_ts_e(el, acc, tA + 16 * kk, pack_desc(ob + (4 * h + kk) * kRowBlk, kHiOp), kIdescOut, h == 0 && kk == 0 ? first0 : 1u);
       if (h == 1) mma_commit_if_s(el, st_empty_bar);
-      if (more) {
-        if (h == 0) {
-          mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
-          if (nxt.it == 0) mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, DEV_TIMEOUT_TMA);
-          tc_fence_after();
-        }
-        issue_in(nxt, ka, qb, h);
+    };
+    auto inputs = [&](int h) {
+      if (!more) return;
+      if (h == 0 && nxt.it == 0) {
+        mbar_wait_s(kv_full_bar, nxt.item_par, abort_s, DEV_TIMEOUT_TMA);
+        tc_fence_after();
       }
+      issue_in(nxt, ka, qb, h);
+    };
+    // (the next step's tiles are long there as a rule: waited for here, where nobody waits for this warp)
+    if (more) mbar_wait_s(st_full_bar, nxt.ring_par, abort_s, DEV_TIMEOUT_TMA);
+    outputs(0);
+    if (G == 1 && nxt.it == 0) {
+      outputs(1);
+      inputs(0);
+    } else {
+      inputs(0);
+      outputs(1);
     }
+    inputs(1);
     cur = nxt;
   }
 }
@@ -229,30 +245,34 @@ __device__ __forceinline__ uint32_t issue_dq(uint32_t d_tmem, uint32_t sDS_s, ui
   return el;
 }
 
+// A pair-bias value of a staged tile, widened.
+template <class T, bool BIAS16>
+__device__ __forceinline__ float staged_bias(uint32_t at) {
+  if constexpr (BIAS16) {
+    const uint16_t raw = lds_u16(at);
+    return to_float<T>(*reinterpret_cast<const T*>(&raw));
+  } else {
+    return lds_f32(at);
+  }
+}
+
 // P^T and dS^T of a key and 16 queries, packed, from S^T and dP^T: x = S*(scale*log2e) + (bias*log2e - lse*log2e) +
 // mask, P = 2^x, dS = P (dP - delta), two queries per instruction (the pairs lie side by side in every operand).
-// vnl, vdl: the queries' statistics; brow: their bias values, BROW bytes apart; take(e, dS): the dS of pair e.
-template <class T, int BIAS, int BROW, class Take>
+// vnl, vdl: the queries' statistics; bias_at(e): the bias value of query e; take(e, dS): the dS of pair e.
+template <class T, bool HAS_BIAS, class BiasAt, class Take>
 __device__ __forceinline__ void score_chunk(const uint32_t (&sr)[16], const uint32_t (&dr)[16], uint32_t vnl, uint32_t vdl,
-                                            uint32_t brow, F2 c12, F2 mj2, uint32_t (&pk)[8], uint32_t* dk, Take take) {
-  const F2 l2e2 = f2_make(kLog2e, kLog2e), neg1 = f2_make(-1.f, -1.f);
+                                            BiasAt bias_at, F2 c12, F2 mj2, uint32_t (&pk)[8], uint32_t* dk, Take take) {
+  const F2 l2e2 = f2_make(kLog2e, kLog2e);
 #pragma unroll
   for (int c4 = 0; c4 < 4; ++c4) {
     const float4 nl = lds_v4f(vnl + 16 * c4);
     const float4 dl = lds_v4f(vdl + 16 * c4);
     F2 t[2] = {f2_make(nl.x, nl.y), f2_make(nl.z, nl.w)};
     const F2 de[2] = {f2_make(dl.x, dl.y), f2_make(dl.z, dl.w)};
-    if constexpr (BIAS != BIAS_NONE) {
+    if constexpr (HAS_BIAS) {
       float bv[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if constexpr (BIAS == BIAS_16) {
-          const uint16_t raw = lds_u16(brow + (4 * c4 + u) * BROW);
-          bv[u] = to_float<T>(*reinterpret_cast<const T*>(&raw));
-        } else {
-          bv[u] = lds_f32(brow + (4 * c4 + u) * BROW);
-        }
-      }
+      for (int u = 0; u < 4; ++u) bv[u] = bias_at(4 * c4 + u);
       t[0] = f2_fma(f2_make(bv[0], bv[1]), l2e2, t[0]);
       t[1] = f2_fma(f2_make(bv[2], bv[3]), l2e2, t[1]);
     }
@@ -262,7 +282,7 @@ __device__ __forceinline__ void score_chunk(const uint32_t (&sr)[16], const uint
       float x0, x1;
       f2_get(f2_add(f2_fma(f2_from_bits(sr[e], sr[e + 1]), c12, t[u]), mj2), x0, x1);
       const float p0 = ex2(x0), p1 = ex2(x1);
-      const F2 ds = f2_mul(f2_make(p0, p1), f2_fma(de[u], neg1, f2_from_bits(dr[e], dr[e + 1])));
+      const F2 ds = f2_mul(f2_make(p0, p1), f2_add(f2_from_bits(dr[e], dr[e + 1]), de[u]));
       take(e / 2, ds);
       float d0, d1;
       f2_get(ds, d0, d1);
@@ -308,6 +328,23 @@ __device__ __forceinline__ void drain_dkdv(const Args& a, uint32_t t_lane, int c
         }
       }
     }
+  }
+}
+
+// The same with one row per item, where all sixteen warps do it: 32 columns of dK (half 0) or dV (half 1) each, to the
+// swizzled tile at dst, which leaves by one bulk store.  (Sixteen bytes a lane straight to global memory, 32 rows an
+// instruction, took 3 800 cycles at every item boundary.)
+template <class T>
+__device__ __forceinline__ void stage_dk_or_dv(uint32_t t_src, uint32_t dst, float f, int jrow, int cb2) {
+  uint32_t r[32];
+  tmem_ld32(t_src, r);
+  tmem_wait_ld();
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) w[u] = Pack2<T>::pack(__uint_as_float(r[8 * c + 2 * u]) * f, __uint_as_float(r[8 * c + 2 * u + 1]) * f);
+    sts_v4(dst + jrow * 128 + (((4 * cb2 + c) ^ (jrow & 7)) << 4), w[0], w[1], w[2], w[3]);
   }
 }
 

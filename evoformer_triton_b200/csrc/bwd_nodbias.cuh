@@ -23,7 +23,7 @@ struct SmemN : TilesT<DP> {
   static constexpr int kHalfF32 = HT * BT * 4, kHalf = BIAS == BIAS_16 ? kHalfF32 / 2 : kHalfF32;
   static constexpr int kBufs = BIAS == BIAS_NONE ? 0 : DP == 64 && BIAS == BIAS_F32 ? 2 : 3;
   static constexpr int kOut = BT * DP * 4;                   // a step's dQ partial
-  static constexpr int kMaskRows = DP == 32 && BIAS == BIAS_F32 ? 0 : G;  // (in registers where a kilobyte is missing)
+  static constexpr int kMaskRows = DP == 64 || (DP == 32 && BIAS == BIAS_F32) ? 0 : G;  // (in registers where a kilobyte is missing, or one row's is waited for anyway)
   static constexpr int offKV = 0;                            // [g][K, V], resident for the whole item
   static constexpr int offStage = offKV + 2 * G * kTile;
   static constexpr int offDS = offStage + kStages * kStage;
@@ -47,7 +47,8 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
                 const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                 const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmDQ,
-                const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL) {
+                const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL,
+                const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV) {
   using L = SmemN<DP, BIAS>;
   constexpr int G = L::G;
 
@@ -64,7 +65,9 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBars);
   const uint32_t bars_s = smem_u32(bars);
   const Bar kv_full{bars_s + 8 * 0};     // [G] K and V of row g of the current item landed
-  const Bar kv_empty{bars_s + 8 * 7};    // [G] ... and every MMA that reads them has completed
+  const Bar kv_empty{bars_s + 8 * 7};    // [G] ... and every MMA that reads them has completed (G = 1: [0] K, [1] V)
+  const Bar drained{bars_s + 8 * 44};    // (G = 1) dK and dV of the item before are in shared memory, over its last dS
+  const Bar dkv_sent{bars_s + 8 * 45};   // (G = 1) ... have left it
   const Bar st_full{bars_s + 8 * 32};     // [2] Q, dO and the statistics vectors of a step landed
   const Bar st_empty{bars_s + 8 * 40};    // [2] ... the step's last dV/dK MMAs have completed
   const Bar sd_full{bars_s + 8 * 48};    // [2], two apart: S^T and dP^T of half h of a step are in TMEM, its statistics landed
@@ -72,7 +75,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
   const Bar sdone{bars_s + 8 * 23};      // [2] ... and dS in shared memory (for the dQ MMAs), with the dQ partial of the step before
   const Bar b_full{bars_s + 8 * 56};     // [kBufs] a half (64 queries) of a pair-bias tile landed
   const Bar b_done{bars_s + 8 * 60};     // [kBufs] ... has been read for the last time
-  const Bar dq_full{bars_s + 8 * 19};    // [2] the dQ partial of a step is complete in TMEM, the dS tile read, and the place for it free
+  const Bar dq_full{bars_s + 8 * 36};    // [2] the dQ partial of a step is complete in TMEM, the dS tile read, and the place for it free (DP = 64: [2 halves][2], for what the half takes of it)
   const Bar mk_full{bars_s + 8 * 25};    // [G] the mask of row g of the current item is in shared memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 22);  // (bars 23, 24: sdone; 25..31: mk_full)
@@ -96,11 +99,13 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
   if (*abort_flag) return;
 
   if (tid == 0) {
-    for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); mbar_init(bars + 25 + i, 1); }  // kv_full; kv_empty: three MMA warps read K/V
+    for (int i = 0; i < (G == 1 ? 2 : G); ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, G == 1 ? 1 : 3); }  // kv_full; kv_empty: three MMA warps read K/V
+    for (int i = 0; i < G; ++i) mbar_init(bars + 25 + i, 1);  // mk_full
+    mbar_init(bars + 44, kCW); mbar_init(bars + 45, 1);  // drained, dkv_sent
     for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + 48 + 2 * i, 3); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full: two commits, one warp; cdone
-      mbar_init(bars + 19 + i, 2);                                     // dq_full: the commit, and the loader
+      mbar_init(bars + 36 + i, 2); mbar_init(bars + 38 + i, 2);                // dq_full: the commit, and the loader
     }
     for (int i = 0; i < kBufs; ++i) { mbar_init(bars + 56 + i, 1); mbar_init(bars + 60 + i, kCW / 2); }  // b_full, b_done
     for (int i = 0; i < 2; ++i) mbar_init(bars + 23 + i, kCW / 2);  // sdone
@@ -123,8 +128,21 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     setmaxnreg_dec<kServiceRegs>();
     if (warp <= kCW + 1) {
       // tensor-core issuers of S^T and dV (warp 16), dP^T and dK (warp 17)
-      issue_scores_and_outputs<T, DP, true>(warp == kCW, tmem, smem_u32(sKV), smem_u32(sStage), NT, total_steps,
-                                            IssueBars{kv_full, kv_empty, st_full, st_empty, sd_full, cdone}, abort_s);
+      int item = 0;  // whose V is loaded next
+      auto load_v = [&] {
+        if (item >= my_items) return;
+        const StepT d = steps.decode(item * (NT * G));
+        mbar_wait(kv_empty + 1, (item & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
+        if (elect_one()) {
+          mbar_expect_tx(kv_full + 1, L::kTile);
+          tma_load_5d_s(smem_u32(sKV) + L::kTile, &tmV, (kv_full + 1).a, 0, d.j0, d.s, d.h, d.b);
+        }
+        __syncwarp();
+        ++item;
+      };
+      if (G == 1 && warp == kCW + 1) load_v();
+      issue_scores_and_outputs<T, DP>(warp == kCW, tmem, smem_u32(sKV), smem_u32(sStage), NT, total_steps,
+                                      IssueBars{kv_full, kv_empty, st_full, st_empty, sd_full, cdone, drained}, abort_s, load_v);
     } else if (warp == kCW + 2) {
       // =============================== tensor-core issuer of dQ; pair-bias loads ===============================
       const uint32_t sKV_s = smem_u32(sKV), sDS_s = smem_u32(sDS);
@@ -132,39 +150,77 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       // The bias tile (i, j) is the same for the G rows of a group.  Its halves (64 queries) go round the
       // buffers: half q = 2 * tile + h is loaded into buffer q % kBufs when the warps that read half q - kBufs
       // there have done so for the last time.
-      auto load_bias = [&](uint32_t q) {
-        const StepT d = steps.decode((int)(q >> 1) * G);
-        const uint32_t buf = q % kBufs;
+      const uint32_t halves = has_bias ? 2u * my_items * NT : 0u;
+      uint32_t lq = 0;             // half that is loaded next
+      StepT lp = steps.decode(0);  // and its tile
+      auto load_bias = [&] {
+        const uint32_t buf = lq % kBufs;
         if (elect_one()) {
           mbar_expect_tx(b_full + (int)buf, kHalf);
-          tma_load_4d_s(sBias_s + buf * kHalf, &tmB, (b_full + (int)buf).a, d.j0, d.it * BT + (int)(q & 1) * HT, d.h, d.b);
+          tma_load_4d_s(sBias_s + buf * kHalf, &tmB, (b_full + (int)buf).a, lp.j0, lp.it * BT + (int)(lq & 1) * HT, lp.h, lp.b);
         }
         __syncwarp();
+        if (++lq % 2 == 0 && ++lp.it == NT && lq < halves) lp = steps.decode((int)(lq >> 1) * G);  // (divisions: here, not before a load)
       };
-      const uint32_t halves = has_bias ? 2u * my_items * NT : 0u;
 #pragma unroll 1
-      for (uint32_t q = 0; q < kBufs && q < halves; ++q) load_bias(q);
+      while (lq < (uint32_t)kBufs && lq < halves) load_bias();
       int g = 0, it = 0;  // row of the group, query tile
-      uint32_t q = 0;     // half tile that is read next for the last time
+      int item = 0;       // (G = 1) whose K is loaded next
+      StepT kp = steps.decode(0);
+      auto load_k = [&] {
+        if (item >= my_items) return;
+        mbar_wait(kv_empty + 0, (item & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
+        if (elect_one()) {
+          mbar_expect_tx(kv_full + 0, L::kTile);
+          tma_load_5d_s(sKV_s, &tmK, kv_full.a, 0, kp.j0, kp.s, kp.h, kp.b);
+        }
+        __syncwarp();
+        if (++item < my_items) kp = steps.decode(item * (NT * G));
+      };
+      if (G == 1) load_k();
+      int item_out = 0;  // (G = 1) whose dK and dV leave next
+      StepT op = steps.decode(0);
+      uint32_t q = 0;  // half tile that is read next for the last time
 #pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
+        if (has_bias && g == G - 1) {  // the group's last step: its halves are free well before its dS is stored
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-          mbar_wait(sdone + h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-          if (has_bias && g == G - 1) {  // the group's last step
-            if (q + kBufs < halves) {
+          for (int h = 0; h < 2; ++h, ++q) {
+            if (lq < halves) {
               mbar_wait(b_done + (int)(q % kBufs), (q / kBufs) & 1, abort_s, DEV_TIMEOUT_SYNC);
-              load_bias(q + kBufs);
+              load_bias();
             }
-            ++q;
           }
         }
+        mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+        mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+        // With one row per item the halves end a step together and wait for the next S^T and dP^T, so these go first.
+        // (At the end of an item they need the next K, which waits for this dQ.)
+        if (G == 1 && it < NT - 1) mbar_wait(sd_full + 2, (n + 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
         const uint32_t el = issue_dq<T, DP>(tmem + L::colDQ + (n & 1) * DP, sDS_s, sKV_s + 2 * g * L::kTile);
         mma_commit_if_s(el, (dq_full + (n & 1)).a);
-        if (it == NT - 1) mma_commit_if_s(el, (kv_empty + g).a);
+        if (DP == 64) mma_commit_if_s(el, (dq_full + 2 + (n & 1)).a);
+        if (it == NT - 1) {
+          mma_commit_if_s(el, (kv_empty + g).a);  // (G = 1: S^T of these keys is long through)
+          if (G == 1) {
+            load_k();
+            mbar_wait(drained, (item_out & 1), abort_s, DEV_TIMEOUT_SYNC);
+            if (elect_one()) {
+              tma_store_5d_s(&tmDK, sDS_s, 0, op.j0, op.s, op.h, op.b);
+              tma_store_5d_s(&tmDV, sDS_s + L::kTile, 0, op.j0, op.s, op.h, op.b);
+              tma_commit_group();
+              tma_wait_group_read0();
+              mbar_arrive(dkv_sent);
+            }
+            __syncwarp();
+            if (++item_out < my_items) op = steps.decode(item_out * (NT * G));
+          }
+        }
         if (++g == G) { g = 0; if (++it == NT) it = 0; }
       }
+      if (G == 1 && elect_one()) tma_wait_group0();
+      __syncwarp();
     } else {
       // =============================== tile loader ===============================
       // K/V of row g stay for the whole item and are replaced when the item's last MMAs that read them
@@ -174,20 +230,24 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       // reduction has read the place, the next one may be stored there, for which the compute warps wait on
       // dq_full (so sdone of a step cannot come before this warp has seen that of the step before).
       const uint32_t sOut_s = smem_u32(smem + L::offOut);
-      auto send_dq = [&](int row0, int slab) {
+      // At DP = 64 it is two tiles of 32 columns, one from each half, that leave one after the other.
+      constexpr int kBoxes = DP == 64 ? 2 : 1;
+      auto send_dq = [&](int box, int row0, int slab) {
         if (elect_one()) {
-          if (slab >= 0) {
-            tma_reduce_add_3d_s(&tmDQ, sOut_s, 0, row0, slab);
-            if (DP == 64 && a.D > 32) tma_reduce_add_3d_s(&tmDQ, sOut_s + BT * 128, 32, row0, slab);
-          }
+          if (slab >= 0 && 32 * box < a.D) tma_reduce_add_3d_s(&tmDQ, sOut_s + box * (BT * 128), 32 * box, row0, slab);
           tma_commit_group();
         }
         __syncwarp();
       };
       auto dq_place_free = [&](int m) {  // for the partial of step m
         if (elect_one()) {
-          tma_wait_group_read0();
+          if constexpr (kBoxes == 2) tma_wait_group_read1();
+          else tma_wait_group_read0();
           mbar_arrive(dq_full + (m & 1));
+          if constexpr (kBoxes == 2) {
+            tma_wait_group_read0();
+            mbar_arrive(dq_full + 2 + (m & 1));
+          }
         }
         __syncwarp();
       };
@@ -220,8 +280,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       for (int n = 0; n < total_steps + 2; ++n) {
         const int stg = n % kStages;
         const bool load = n < total_steps;
-        // (with one row per item, kv_empty waits for the step before, which waits for dq_place_free)
-        if (G > 1 && load && d.it == 0) load_kv(n);
+          if (G > 1 && load && d.it == 0) load_kv(n);
         mbar_wait(st_empty + stg, ((n / kStages) & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);  // (of step n - 2)
         if (load) {
           if (elect_one()) {
@@ -238,8 +297,9 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         {
           if (n >= 2) {
             mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+            if (kBoxes == 2 && n >= 3) send_dq(0, row3, slab3);
             mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-            if (n >= 3) send_dq(row3, slab3);
+            if (n >= 3) send_dq(kBoxes - 1, row3, slab3);
             dq_place_free(n - 2);
           }
           row3 = row2; slab3 = slab2;
@@ -247,13 +307,12 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
           row1 = d.it * BT;
           slab1 = d.s < a.S ? (d.b * a.H + d.h) * a.S + d.s : -1;
         }
-        if (G == 1 && load && d.it == 0) load_kv(n);
         if (load) d = steps.advance(d, n + 1);
       }
       if (total_steps > 0) {  // the last step's partial: the compute warps arrive once more
         mbar_wait(sdone + 0, total_steps & 1, abort_s, DEV_TIMEOUT_SYNC);
         mbar_wait(sdone + 1, total_steps & 1, abort_s, DEV_TIMEOUT_SYNC);
-        send_dq(row3, slab3);
+        for (int box = 0; box < kBoxes; ++box) send_dq(box, row3, slab3);
         if (elect_one()) tma_wait_group0();
         __syncwarp();
       }
@@ -296,7 +355,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     };
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
     const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
-    float mreg[DP == 32 ? G : 1];
+    float mreg[L::kMaskRows == 0 ? G : 1];
     const F2 c12 = f2_make(c1, c1);
     int n = 0;            // running step
     uint32_t tile = 0;    // running (item, query tile)
@@ -317,10 +376,20 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       const bool last_of_group = (g == G - 1);
       float mj;
       if constexpr (L::kMaskRows == 0) {
-        mj = g == 0 ? mreg[0] : g == 1 ? mreg[1] : mreg[2];
+        mj = G == 1 || g == 0 ? mreg[0] : g == 1 ? mreg[1] : mreg[2];
       } else {
         if (it == 0) mbar_wait(mk_full + g, k & 1, abort_s, DEV_TIMEOUT_TMA);
         mj = lds_f32(mask_s + g * (BT * 4));
+      }
+      if (G == 1 && it == 0 && k > 0) {  // dK and dV of the item before, while this one's K is on its way
+        mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+        mbar_wait(kv_empty + 0, (k - 1) & 1, abort_s, DEV_TIMEOUT_MMA);  // (dQ of the item's last step: its dS has been read)
+        tc_fence_after();
+        stage_dk_or_dv<T>(t_lane + (H ? L::colDV : L::colDK) + 32 * cb2, sDS_s + H * L::kTile, H ? 1.f : a.scale, jrow, cb2);
+        fence_async_shared();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(drained);
       }
       if (has_bias && g == 0) {
         const uint32_t q = 2 * tile + H;
@@ -347,7 +416,8 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         tmem_wait_ld();
         uint32_t pk[8];
         if (!deadstep) {
-          score_chunk<T, BIAS, kBRow>(sr, dr, vnl, vdl, brow, c12, mj2, pk, dk + 8 * sub, [](int, F2) {});
+          score_chunk<T, has_bias>(sr, dr, vnl, vdl, [&](int e) { return staged_bias<T, kBias16>(brow + e * kBRow); }, c12, mj2, pk,
+                                   dk + 8 * sub, [](int, F2) {});
         } else {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);
@@ -359,15 +429,13 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         tmem_st8(cS + 16 * sub, pk);
         tmem_st8(cP + 16 * sub, *reinterpret_cast<uint32_t(*)[8]>(&dk[sub * 8]));
       }
-      if (H == 0 && it == 0 && k > 0) {  // before this step's dV / dK MMAs overwrite them
-        // With one row per item the other half's MMAs of the step before belong to them too; with more rows, all of
-        // theirs were issued before the S^T and dP^T of this step.
-        if constexpr (G == 1) {
-          mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
-          tc_fence_after();
-        }
-        drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
+      if (has_bias && last_of_group) {  // (every value read has been worked on, so the loads are through)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bdone);
       }
+      if (G > 1 && H == 0 && it == 0 && k > 0)  // before this step's dV / dK MMAs overwrite them
+        // (All of the other half's MMAs into them were issued before the S^T and dP^T of this step.)
+        drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
       // P^T and dS^T are in tensor memory: the dV / dK MMAs and the next S^T and dP^T may go, under what follows
       if constexpr (EARLY) {
         tmem_wait_st();
@@ -376,8 +444,9 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         if (lane == 0) mbar_arrive(cdone + 2 * H);
       }
       // dQ of the previous step is complete, and the place it leaves from is free
-      if (n > 0) mbar_wait(dq_full + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+      if (n > 0) mbar_wait(dq_full + (DP == 64 ? 2 * H : 0) + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
+      if (G == 1 && it == 0 && k > 0) mbar_wait(dkv_sent, (k - 1) & 1, abort_s, DEV_TIMEOUT_SYNC);
       if (n > 0) store_dq(n - 1);
       // dS^T -> shared memory, [key][query] rows of 128 bytes per half, 128-byte swizzle
 #pragma unroll
@@ -390,25 +459,33 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       if (lane == 0) {
         if constexpr (!EARLY) mbar_arrive(cdone + 2 * H);
         mbar_arrive(sdone + H);
-        if (has_bias && last_of_group) mbar_arrive(bdone);
       }
     }
     pb = cur.b; ph = cur.h; ps0 = cur.s; pj0 = cur.j0;
     }
 
     if (total_steps > 0) {
-      mbar_wait(dq_full + ((total_steps - 1) & 1), ((total_steps - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+      mbar_wait(dq_full + (DP == 64 ? 2 * H : 0) + ((total_steps - 1) & 1), ((total_steps - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
       store_dq(total_steps - 1);
       fence_async_shared();
       __syncwarp();
       if (lane == 0) mbar_arrive(sdone + H);
-      if (H == 0) {
+      if (H == 0 || G == 1) {
         // every dV / dK MMA of this CTA has completed once the last step's tile stage has been released
         const int last = total_steps - 1;
         mbar_wait(st_empty + (last & 1), (last >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
-        for (int g = 0; g < G; ++g) drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
+        if constexpr (G == 1) {
+          mbar_wait(kv_empty + 0, (my_items - 1) & 1, abort_s, DEV_TIMEOUT_MMA);
+          tc_fence_after();
+          stage_dk_or_dv<T>(t_lane + (H ? L::colDV : L::colDK) + 32 * cb2, sDS_s + H * L::kTile, H ? 1.f : a.scale, jrow, cb2);
+          fence_async_shared();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(drained);
+        } else {
+          for (int g = 0; g < G; ++g) drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
+        }
       }
     }
   }

@@ -26,6 +26,7 @@
 // Warps: 0-15 compute (warp w: keys 32*(w%4).., queries 32*((w/4)%2).. of half w/8), 16-18 issue the
 // tcgen05.mma (18 also loads the pair-bias tiles), 19 loads the other tiles.
 #include "bwd_common.cuh"
+#include "bwd_dbias.cuh"
 #include "bwd_nodbias.cuh"
 #include "common.cuh"
 #include "launch.h"
@@ -37,28 +38,37 @@ namespace {
 
 template <int DP>
 struct SmemT : TilesT<DP> {
+  static_assert(DP < 64, "above 32 columns d(pair_bias) has a kernel of its own");
   using Tiles = TilesT<DP>;
   using Tiles::G, Tiles::kTile, Tiles::kStage, Tiles::kDS;
   static constexpr int kBias = BT * BT * 4;                  // pair-bias tile [128 i][128 j], unswizzled (fp32; half of it for a 16-bit bias)
-  static constexpr int kOutWarp = 2048;                      // per compute warp: staging of a d_bias chunk or a dQ block
+  // Staging areas, each with a place of its own so that a warp hardly waits for a reduction to have read it:
+  // d(pair_bias) of every compute warp (16 queries x 32 keys at a time), and the dQ partial (32 queries, QC columns)
+  // of the warps of half 1.
+  static constexpr int kOutB = 16 * 32 * 4;
+  static constexpr int QC = DP / 2;
+  static constexpr int kOutQ = 32 * QC * 4;
+  static constexpr int kMaskRows = DP == 32 ? 0 : G;         // (in registers where a kilobyte is missing)
   static constexpr int offKV = 0;                            // [g][K, V], resident for the whole item
   static constexpr int offStage = offKV + 2 * G * kTile;
   static constexpr int offDS = offStage + kStages * kStage;
   static constexpr int offBias = offDS + kDS;
-  static constexpr int offOut = offBias + kBias;
-  static constexpr int offMask = offOut + kCW * kOutWarp;    // [G][128 keys]: what the mask adds to a score
-  static constexpr int offBars = offMask + G * BT * 4;
-  // 64 barrier slots (see the kernel) and the slack for aligning the tiles to 1024 bytes.  At DP = 64
-  // none fits: the kernel checks what the base address needs and gives up with a status code if that is
-  // anything (the dynamic shared memory of a kernel without static shared memory starts on a 1024-byte
-  // boundary on this architecture, so it needs none).
-  static constexpr int kSlack = (DP == 64) ? 0 : 1024;
+  static constexpr int offOutB = offBias + kBias;
+  static constexpr int offOutQ = offOutB + kCW * kOutB;
+  static constexpr int offMask = offOutQ + kCW / 2 * kOutQ;      // [kMaskRows][128 keys]: what the mask adds to a score
+  static constexpr int offBars = offMask + kMaskRows * BT * 4;
+  // 64 barrier slots (see the kernel) and the slack for aligning the tiles to 1024 bytes, where it fits: the
+  // kernel checks what the base address needs and gives up with a status code if that is more (the dynamic
+  // shared memory of a kernel without static shared memory starts on a 1024-byte boundary on this
+  // architecture, so it needs none).
+  static constexpr int kSlack = offBars + 512 + 1024 <= 232448 ? 1024 : 0;
   static constexpr size_t bytes = offBars + 512 + kSlack;
   static_assert(offDS % 1024 == 0 && kStage % 1024 == 0 && offStage % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static_assert(bytes <= 232448, "shared memory budget of one CTA");
 };
 
-// The first pass of a backward call: delta[b,h,s,i] = <dO_i, O_i> (evoformer.py:299-326), nl = -lse*log2e,
+// The first pass of a backward call: delta[b,h,s,i] = -<dO_i, O_i> (evoformer.py:299-326; negated, so that it is
+// added), nl = -lse*log2e,
 // and zeros in the buffers that the fused kernel adds to (the fp32 dQ accumulator, d(pair_bias)).
 // A row whose keys were all dropped carries lse = -FLT_MAX from the forward; its nl is +inf, which
 // the fused kernel recognises.  With a gate (Og = sigmoid(gate) O is the output, G its gradient):
@@ -121,7 +131,7 @@ __global__ void __launch_bounds__(256) prep_kernel(const Args a, float* __restri
   for (int o = (1 << LG) >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (ok && c == 0) {
     const size_t at = (size_t)slab * a.delta_ld + i;
-    a.delta[at] = acc;
+    a.delta[at] = -acc;
     const float lse = a.lse[row];
     nl[at] = (lse == -FLT_MAX) ? __int_as_float(0x7f800000) : -lse * kLog2e;
   }
@@ -188,20 +198,18 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
   uint8_t* sStage = smem + L::offStage;
   uint8_t* sDS = smem + L::offDS;
   uint8_t* sBias = smem + L::offBias;
-  uint8_t* sOut = smem + L::offOut;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::offBars);
   const uint32_t bars_s = smem_u32(bars);
   const Bar kv_full{bars_s + 8 * 0};     // [G] K and V of row g of the current item landed
   const Bar kv_empty{bars_s + 8 * 7};    // [G] ... and every MMA that reads them has completed
   const Bar st_full{bars_s + 8 * 32};     // [2] Q, dO and the statistics vectors of a step landed
   const Bar st_empty{bars_s + 8 * 40};    // [2] ... the step's last dV/dK MMAs have completed
-  const Bar sd_full{bars_s + 8 * 48};    // [2], two apart: S^T and dP^T of half h of a step are in TMEM
+  const Bar sd_full{bars_s + 8 * 48};    // [2], two apart: S^T and dP^T of half h of a step are in TMEM, its statistics landed
   const Bar cdone{bars_s + 8 * 52};      // [2], two apart: the warps of that half have its P^T and dS^T in TMEM (for the dV/dK MMAs)
-  const Bar sdone{bars_s + 8 * 23};      // [2] ... and have stored their half of dS in shared memory (for the dQ MMAs)
+  const Bar sdone{bars_s + 8 * 23};      // [2] ... and have stored their half of dS in shared memory (for the dQ MMAs) and read dQ of the step before
   const Bar b_full{bars_s + 8 * 14};     // [2] half h (64 queries) of the pair-bias tile landed
   const Bar b_done{bars_s + 8 * 16};     // [2] ... has been read for the last time
-  const Bar ds_empty{bars_s + 8 * 18};   // the dQ MMAs of a step have read the dS tile
-  const Bar dq_full{bars_s + 8 * 19};    // [2] the dQ partial of a step is complete in TMEM
+  const Bar dq_full{bars_s + 8 * 19};    // the dQ partial of the step before is complete in TMEM (and the dS tile has been read)
   const Bar mk_full{bars_s + 8 * 25};    // [G] the mask of row g of the current item is in shared memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 21);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 22);  // (bars 23, 24: sdone; 25..31: mk_full)
@@ -223,12 +231,11 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     for (int i = 0; i < G; ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, 3); mbar_init(bars + 25 + i, 1); }  // kv_full; kv_empty: three MMA warps read K/V
     for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bars + 48 + 2 * i, 2); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full, cdone
+      mbar_init(bars + 48 + 2 * i, 3); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full: two commits, one warp; cdone
       mbar_init(bars + 14 + i, 1); mbar_init(bars + 16 + i, kCW / 2);  // b_full, b_done
-      mbar_init(bars + 19 + i, 1);                                     // dq_full
       mbar_init(bars + 23 + i, kCW / 2);                               // sdone
     }
-    mbar_init(bars + 18, 1);  // ds_empty
+    mbar_init(bars + 19, 1);  // dq_full
     fence_mbar_init();
     prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmDO);
     prefetch_tmap(&tmNL); prefetch_tmap(&tmDL); prefetch_tmap(&tmDQ);
@@ -247,8 +254,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     setmaxnreg_dec<kServiceRegs>();
     if (warp <= kCW + 1) {
       // tensor-core issuers of S^T and dV (warp 16), dP^T and dK (warp 17)
-      issue_scores_and_outputs<T, DP, false>(warp == kCW, tmem, smem_u32(sKV), smem_u32(sStage), NT, total_steps,
-                                             IssueBars{kv_full, kv_empty, st_full, st_empty, sd_full, cdone}, abort_s);
+      issue_scores_and_outputs<T, DP>(warp == kCW, tmem, smem_u32(sKV), smem_u32(sStage), NT, total_steps,
+                                      IssueBars{kv_full, kv_empty, st_full, st_empty, sd_full, cdone, Bar{0}}, abort_s, [] {});
     } else if (warp == kCW + 2) {
       // =============================== tensor-core issuer of dQ; pair-bias loads ===============================
       const uint32_t sKV_s = smem_u32(sKV), sDS_s = smem_u32(sDS);
@@ -265,24 +272,26 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       };
       const int tiles = my_items * NT;
       if (tiles > 0) { const StepT d0 = steps.decode(0); load_bias(d0, 0); load_bias(d0, 1); }
+      if (elect_one()) mbar_arrive(dq_full);  // (for the first step, which has none before it)
+      __syncwarp();
       int g = 0, it = 0, t = 0;  // row of the group, query tile, running (item, query tile) index
 #pragma unroll 1
       for (int n = 0; n < total_steps; ++n) {
         const bool turn = g == G - 1 && t + 1 < tiles;  // the group's last step: the halves come back
         StepT nb = StepT{0, 0, 0, 0, 0, 0};
         if (turn) nb = steps.decode((t + 1) * G);  // (divisions: before the waits, not between them)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          mbar_wait(sdone + h, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-          if (turn) {
+        if (turn) {
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
             mbar_wait(b_done + h, t & 1, abort_s, DEV_TIMEOUT_SYNC);
             load_bias(nb, h);
           }
         }
+        mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+        mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
         tc_fence_after();
-        const uint32_t el = issue_dq<T, DP>(tmem + L::colDQ + (n & 1) * DP, sDS_s, sKV_s + 2 * g * L::kTile);
-        mma_commit_if_s(el, (dq_full + (n & 1)).a);
-        mma_commit_if_s(el, ds_empty.a);
+        const uint32_t el = issue_dq<T, DP>(tmem + L::colDQ, sDS_s, sKV_s + 2 * g * L::kTile);
+        mma_commit_if_s(el, dq_full.a);
         if (it == NT - 1) mma_commit_if_s(el, (kv_empty + g).a);
         if (++g == G) { g = 0; ++t; if (++it == NT) it = 0; }
       }
@@ -300,13 +309,17 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
           // The mask of the row: four keys a lane, loaded before the wait.  (The last dQ MMA of the row is behind
           // kv_empty, so its last step has read the mask before.)
           float mk[4];
+          if constexpr (L::kMaskRows > 0) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) mk[u] = mask_term<T>(a, d.b, d.s, d.j0 + lane + 32 * u);
+            for (int u = 0; u < 4; ++u) mk[u] = mask_term<T>(a, d.b, d.s, d.j0 + lane + 32 * u);
+          }
           mbar_wait(kv_empty + d.g, (k & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
+          if constexpr (L::kMaskRows > 0) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) sts_f32(sMask_s + (d.g * BT + lane + 32 * u) * 4, mk[u]);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(mk_full + d.g);
+            for (int u = 0; u < 4; ++u) sts_f32(sMask_s + (d.g * BT + lane + 32 * u) * 4, mk[u]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(mk_full + d.g);
+          }
           if (elect_one()) {
             const uint32_t dst = sKV_s + (2 * d.g) * L::kTile;
             mbar_expect_tx(kv_full + d.g, 2 * L::kTile);
@@ -349,70 +362,95 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     const float c1 = a.scale * kLog2e;
     // 32-bit shared-window addresses: every access below stays a shared-memory instruction
     const uint32_t sStage_s = smem_u32(sStage), sDS_s = smem_u32(sDS);
-    const uint32_t out_s = smem_u32(sOut) + warp * L::kOutWarp;  // this warp's private staging area
+    const uint32_t outB_s = smem_u32(smem + L::offOutB) + warp * L::kOutB;  // this warp's own staging areas
+    const uint32_t outQ_s = smem_u32(smem + L::offOutQ) + (warp & 7) * L::kOutQ;
     const uint32_t brow0 = smem_u32(sBias) + (H * HT + QT * cb2) * kBRow + jrow * (kBias16 ? 2 : 4);
     const uint32_t drow = sDS_s + H * (L::kDS / 2) + jrow * 128;
 
-    // This warp's staging area is free again once its previous bulk reduction has read it.
+    // Every step has one bulk group per warp with its dQ partial (empty in a warp that takes none), and the last of a
+    // row group two with d(pair_bias), one before and one after it.  So that staging area is free once all but the
+    // last group have been read.
     auto staging_free = [&]() {
-      if (lane == 0) tma_wait_group_read0();
+      if (lane == 0) tma_wait_group_read1();
       __syncwarp();
     };
-
-    // The dQ partial of step m at position d (TMEM lanes = queries): this warp's DP/4 columns of its 32
-    // query rows go through its staging area ([32 rows][DP/4 floats]) into the fp32 accumulator in global
-    // memory, as one small bulk tensor reduction that the warp issues itself.  It happens after the
-    // warp's arrival, underneath the tensor core's turnaround for its half.
-    constexpr int QC = DP / 4;       // dQ columns per warp (4, 8 or 16)
-    const int colblk = 2 * H + cb2;  // which of the four column blocks this warp drains
-    // (row0: the first of the 32 query rows; slab: (b,h,s), negative for a padded row)
-    auto send_dq = [&](int m, int row0, int slab) {
-      mbar_wait(dq_full + (m & 1), (m >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
-      tc_fence_after();
-      uint32_t qr[QC];
-      tmem_ld<QC>(t_lane + L::colDQ + (m & 1) * DP + colblk * QC, qr);
-      staging_free();
-      tmem_wait_ld();
+    // dQ of a step (TMEM lanes = queries): the warps of half 1 take QC columns of 32 query rows each to their staging
+    // areas, from where they are added to the fp32 accumulator in global memory by one small bulk tensor reduction per
+    // warp.  (Half 0 takes dK and dV.  Rows of 64 bytes instead of 32: 5.1 TB/s of reductions instead of 3.6, the chip
+    // over, and half as many instructions.)
+    constexpr int QC = L::QC;
+    const bool takes_dq = H == 1;
+    const int qcol = cb2 * QC;
+    auto store_dq = [&](const uint32_t (&qr)[QC]) {  // (rows of 32 or 64 bytes, swizzled as wide: no bank conflicts)
+      const int x = QC == 8 ? (lane >> 2) & 1 : (lane >> 1) & 3;
 #pragma unroll
       for (int c = 0; c < QC / 4; ++c)
-        sts_v4(out_s + lane * (QC * 4) + 16 * c, qr[4 * c], qr[4 * c + 1], qr[4 * c + 2], qr[4 * c + 3]);
-      fence_async_shared();
-      __syncwarp();
-      if (lane == 0 && slab >= 0 && colblk * QC < a.D) {
-        tma_reduce_add_3d_s(&tmDQ, out_s, colblk * QC, row0, slab);
-        tma_commit_group();
-      }
+        sts_v4(outQ_s + lane * (QC * 4) + ((c ^ x) << 4), qr[4 * c], qr[4 * c + 1], qr[4 * c + 2], qr[4 * c + 3]);
+    };
+    // (row0: the first of the 32 query rows; slab: (b,h,s), negative for a padded row)
+    auto send_dq = [&](int row0, int slab) {
+      if (takes_dq && slab >= 0 && qcol < a.D) tma_reduce_add_3d_s(&tmDQ, outQ_s, qcol, row0, slab);
+      tma_commit_group();
     };
 
     int p_row0 = 0, p_slab = -1;           // the step whose dQ partial has not left yet
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
     // Always true.  With more than one row it has to be looked at all the same, which the compiler cannot know: given
     // last_of_group alone it makes two copies of a step, whose registers do not fit (8 to 24 bytes of spills; the
-    // backward of [1,128,384,8,32] took 210 us instead of 195, [1,1024,384,8,8] fp16 1177 instead of 1083).  With one
-    // row the unconditional form is the faster one ([1,128,768,8,64] 1 092 instead of 1 160).
-    const bool flush = G == 1 || a.dbias != nullptr;
+    // backward of [1,128,384,8,32] took 210 us instead of 195, [1,1024,384,8,8] fp16 1177 instead of 1083).
+    const bool flush = a.dbias != nullptr;
     const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
+    float mreg[L::kMaskRows == 0 ? G : 1];
     const F2 c12 = f2_make(c1, c1);
     F2 bacc[16];  // d(pair_bias) of this thread's key and its 32 queries, summed over the rows of a group
 #pragma unroll
     for (int e = 0; e < 16; ++e) bacc[e] = f2_make(0.f, 0.f);
-
+    // Half a sum (16 queries x 32 keys of a warp) to the staging area and from there, by a bulk tensor reduction that
+    // the warp issues itself, to d(pair_bias).  The first half leaves as soon as the group's last row has been added
+    // to it, the second at the end of that step, by when the staging area has been read.
+    auto flush_half = [&](int sub, int i0, int j0, int h, int b) {
+      staging_free();
+#pragma unroll
+      for (int c = 0; c < 16; c += 2) {
+        F2& acc = bacc[(sub * 16 + c) / 2];
+        float b0, b1;
+        f2_get(acc, b0, b1);
+        sts_f32(outB_s + c * 128 + lane * 4, b0);
+        sts_f32(outB_s + (c + 1) * 128 + lane * 4, b1);
+        acc = f2_make(0.f, 0.f);
+      }
+      fence_async_shared();
+      __syncwarp();
+      if (lane == 0) {
+        tma_reduce_add_4d_s(&tmDB, outB_s, j0 + q4 * 32, i0 + H * HT + QT * cb2 + 16 * sub, h, b);
+        tma_commit_group();
+      }
+    };
     int n = 0;          // running step
     uint32_t tile = 0;  // running (item, query tile)
 #pragma unroll 1
     for (int k = 0; k < my_items; ++k) {
     const StepT cur = steps.decode(n);
+    if constexpr (L::kMaskRows == 0) {
+#pragma unroll
+      for (int r = 0; r < G; ++r) mreg[r] = mask_term<T>(a, cur.b, cur.s + r, cur.j0 + jrow);
+    }
 #pragma unroll 1
     for (int it = 0; it < NT; ++it, ++tile)
 #pragma unroll 1
     for (int g = 0; g < G; ++g, ++n) {
       const uint32_t vec_s = sStage_s + (n & 1) * L::kStage + 2 * L::kTile;
       const bool last_of_group = (g == G - 1);
-      if (it == 0) mbar_wait(mk_full + g, k & 1, abort_s, DEV_TIMEOUT_TMA);
-      const float mj = lds_f32(mask_s + g * (BT * 4));
-      // the statistics vectors of this step are read with ordinary loads: observe their arrival here
-      mbar_wait(st_full + (n & 1), (n >> 1) & 1, abort_s, DEV_TIMEOUT_TMA);
+      float mj;
+      if constexpr (L::kMaskRows == 0) {
+        mj = g == 0 ? mreg[0] : g == 1 ? mreg[1] : mreg[2];
+      } else {
+        if (it == 0) mbar_wait(mk_full + g, k & 1, abort_s, DEV_TIMEOUT_TMA);
+        mj = lds_f32(mask_s + g * (BT * 4));
+      }
       if (g == 0) mbar_wait(b_full + H, tile & 1, abort_s, DEV_TIMEOUT_TMA);
+      mbar_wait(sd_full + 2 * H, n & 1, abort_s, DEV_TIMEOUT_MMA);  // S^T and dP^T, statistics
+      tc_fence_after();
       // a row whose keys are all dropped has nl = +inf for every query (the mask row is shared by
       // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
       const bool deadstep = (lds_f32(vec_s) == kInf);
@@ -421,10 +459,6 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 #pragma unroll
       for (int sub = 0; sub < 2; ++sub) {
         // this warp's queries of the half: 32*cb2 + 16*sub .. +16
-        if (sub == 0) {
-          mbar_wait(sd_full + 2 * H, n & 1, abort_s, DEV_TIMEOUT_MMA);
-          tc_fence_after();
-        }
         uint32_t sr[16], dr[16];
         tmem_ld16(cS + 16 * sub, sr);
         tmem_ld16(cP + 16 * sub, dr);
@@ -433,8 +467,10 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tmem_wait_ld();
         uint32_t pk[8];
         if (!deadstep) {
-          score_chunk<T, kBias16 ? BIAS_16 : BIAS_F32, kBRow>(sr, dr, vnl, vdl, brow, c12, mj2, pk, dk + 8 * sub,
-                                                              [&](int e, F2 ds) { bacc[8 * sub + e] = f2_add(bacc[8 * sub + e], ds); });
+          score_chunk<T, true>(
+              sr, dr, vnl, vdl,
+              [&](int e) { return staged_bias<T, kBias16>(brow + e * kBRow); }, c12, mj2, pk, dk + 8 * sub,
+              [&](int e, F2 ds) { bacc[8 * sub + e] = f2_add(bacc[8 * sub + e], ds); });
         } else {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);
@@ -445,56 +481,46 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         // the A operands of the dV and dK MMAs (16 queries = 8 packed columns each)
         tmem_st8(cS + 16 * sub, pk);
         tmem_st8(cP + 16 * sub, *reinterpret_cast<uint32_t(*)[8]>(&dk[sub * 8]));
-        // P^T and dS^T of this warp's score buffer are in tensor memory: its dV / dK MMAs may go
-        if (sub == 1 && H == 0 && it == 0 && k > 0) {  // before those MMAs overwrite it
-          // With one row per item the other half's MMAs of the step before belong to this slot too: wait until they
-          // are through.  With more rows, all of theirs were issued before the S^T and dP^T of this step.
-          if constexpr (G == 1) {
-            mbar_wait(st_empty + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
-            tc_fence_after();
-          }
-          drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
-        }
-        if (sub == 1) {
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(cdone + 2 * H);
-        }
-        if (last_of_group && flush) {
-          // The group's last row: this thread's 16 d_bias values of the chunk (one key, 16 queries) go
-          // through the warp's staging area ([16 queries][32 keys]) and are added to d_bias in global
-          // memory by a bulk tensor reduction that the warp issues itself.
-          staging_free();
-#pragma unroll
-          for (int c = 0; c < 16; c += 2) {
-            float b0, b1;
-            f2_get(bacc[(sub * 16 + c) / 2], b0, b1);
-            sts_f32(out_s + c * 128 + lane * 4, b0);
-            sts_f32(out_s + (c + 1) * 128 + lane * 4, b1);
-            bacc[(sub * 16 + c) / 2] = f2_make(0.f, 0.f);
-          }
-          fence_async_shared();
-          __syncwarp();
-          if (lane == 0) {
-            tma_reduce_add_4d_s(&tmDB, out_s, cur.j0 + q4 * 32, it * BT + H * HT + QT * cb2 + 16 * sub, cur.h, cur.b);
-            tma_commit_group();
-          }
-        }
+        if (sub == 0 && last_of_group && flush) flush_half(0, it * BT, cur.j0, cur.h, cur.b);
       }
-      // dS^T -> shared memory, [key][query] rows of 128 bytes per half, 128-byte swizzle; the tile is
-      // free once the dQ MMAs of the previous step have read it
-      mbar_wait(ds_empty, (n & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);
+      if (last_of_group) {  // (every value read has been worked on, so the loads are through)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_done + H);
+      }
+      if (H == 0 && it == 0 && k > 0)  // before this step's dV / dK MMAs overwrite them
+        // (All of the other half's MMAs into them were issued before the S^T and dP^T of this step.)
+        drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
+      // P^T and dS^T are in tensor memory: the dV / dK MMAs and the next S^T and dP^T may go, under what follows
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(cdone + 2 * H);
+      // dQ of the step before is complete, so the dS tile has been read as well.  Its MMAs ran underneath this step.
+      mbar_wait(dq_full, n & 1, abort_s, DEV_TIMEOUT_MMA);
+      tc_fence_after();
+      // dS^T -> shared memory, [key][query] rows of 128 bytes per half, 128-byte swizzle
 #pragma unroll
       for (int c = 0; c < 4; ++c)  // dk[4 * c ..]: queries 32 * cb2 + 8 * c .. of this half
         sts_v4(drow + (((4 * cb2 + c) ^ (jrow & 7)) << 4), dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
+      if (takes_dq) {
+        uint32_t qr[QC];
+        tmem_ld<QC>(t_lane + L::colDQ + qcol, qr);
+        if (lane == 0) {
+          if (last_of_group || g == 0) tma_wait_group_read1();  // (d(pair_bias) left since the last dQ)
+          else tma_wait_group_read0();
+        }
+        __syncwarp();
+        tmem_wait_ld();
+        store_dq(qr);
+      }
       fence_async_shared();
+      tc_fence_before();  // (the next MMAs into the dQ columns just read follow from this arrival)
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(sdone + H);
-        if (last_of_group) mbar_arrive(b_done + H);
+        send_dq(p_row0, p_slab);
       }
-      if (n > 0) send_dq(n - 1, p_row0, p_slab);  // its MMAs ran underneath this step
+      if (last_of_group && flush) flush_half(1, it * BT, cur.j0, cur.h, cur.b);
       p_row0 = it * BT + q4 * 32;
       p_slab = cur.s + g < a.S ? (cur.b * a.H + cur.h) * a.S + cur.s + g : -1;
     }
@@ -502,7 +528,19 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     }
 
     if (total_steps > 0) {
-      send_dq(total_steps - 1, p_row0, p_slab);
+      mbar_wait(dq_full, total_steps & 1, abort_s, DEV_TIMEOUT_MMA);
+      tc_fence_after();
+      if (takes_dq) {
+        uint32_t qr[QC];
+        tmem_ld<QC>(t_lane + L::colDQ + qcol, qr);
+        if (lane == 0) tma_wait_group_read0();
+        __syncwarp();
+        tmem_wait_ld();
+        store_dq(qr);
+        fence_async_shared();
+        __syncwarp();
+        if (lane == 0) send_dq(p_row0, p_slab);
+      }
       if (H == 0) {
         // every dV / dK MMA of this CTA has completed once the last step's tile stage has been released
         const int last = total_steps - 1;
@@ -526,7 +564,6 @@ size_t stats_bytes(const Args& a) { return align_up((size_t)a.B * a.H * a.S * a.
 template <class T, int DP>
 int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* launches) {
   constexpr int G = RowsPerItem<DP>::G;
-  using L = SmemT<DP>;
   Args a = a0;
   const size_t rows = (size_t)a.B * a.H * a.S * a.R;
   const size_t vec_bytes = stats_bytes(a);
@@ -541,20 +578,25 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
     launch_prep<T, false>(a, nl, dq_acc, st);
   }
 
-  CUtensorMap tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl;
+  CUtensorMap tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl, tdk, tdv;
   if (!make_qkv_map(&tq, a.q, a.sq, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tk, a.k, a.sk, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tv, a.v, a.sv, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tdo, a.d_o, a.sdo, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
-  const bool nodbias = !a.dbias;
+  constexpr bool kApart = DP == 64;  // d(pair_bias) has a kernel of its own
+  const bool nodbias = kApart || !a.dbias;
   const long long slabs = (long long)a.B * a.H * a.S;
   if (!(nodbias ? make_rows_f32_map(&tdq, dq_acc, a.D, a.R, slabs, DP < 32 ? DP : 32, BT, /*swizzle=*/true)
-                : make_rows_f32_map(&tdq, dq_acc, a.D, a.R, slabs, DP / 4, 32, /*swizzle=*/false)))
+                : make_rows_f32_map(&tdq, dq_acc, a.D, a.R, slabs, DP / 2, 32, /*swizzle=*/true)))
     return EVOATTN_ERR_CUDA;
   if (!make_stats_map(&tnl, nl, a.B * a.H, a.S, a.R, a.delta_ld, BT)) return EVOATTN_ERR_CUDA;
   if (!make_stats_map(&tdl, a.delta, a.B * a.H, a.S, a.R, a.delta_ld, BT)) return EVOATTN_ERR_CUDA;
   tb = tq;
   tdb = tq;
+  tdk = tdv = tq;
+  if (G == 1 && (!make_qkv_map(&tdk, a.dk, a.sdk, a.B, a.H, a.S, a.R, a.D, DP, BT) ||
+                 !make_qkv_map(&tdv, a.dv, a.sdv, a.B, a.H, a.S, a.R, a.D, DP, BT)))
+    return EVOATTN_ERR_CUDA;
   if (a.bias) {
     const bool ok = a.bias16 ? make_bias16_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT, /*swizzle=*/false)
                              : make_bias_plain_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT);
@@ -568,18 +610,35 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   const int sms = sm_count();
   if (sms <= 0) return EVOATTN_ERR_CUDA;
   const long long ctas = items < sms ? items : sms;
-  const auto kern = a.bias16 ? evo_bwd_sm100_kernel<T, DP, true> : evo_bwd_sm100_kernel<T, DP, false>;
   const auto kern_n = !a.bias ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_NONE>
                       : (a.bias16 ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_16> : evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_F32>);
-  const void* entry = nodbias ? reinterpret_cast<const void*>(kern_n) : reinterpret_cast<const void*>(kern);
-  const size_t smem = !nodbias ? L::bytes : !a.bias ? SmemN<DP, BIAS_NONE>::bytes : a.bias16 ? SmemN<DP, BIAS_16>::bytes : SmemN<DP, BIAS_F32>::bytes;
+  const void* entry = reinterpret_cast<const void*>(kern_n);
+  size_t smem = !a.bias ? SmemN<DP, BIAS_NONE>::bytes : a.bias16 ? SmemN<DP, BIAS_16>::bytes : SmemN<DP, BIAS_F32>::bytes;
+  if constexpr (!kApart) {
+    if (!nodbias) {
+      entry = a.bias16 ? reinterpret_cast<const void*>(evo_bwd_sm100_kernel<T, DP, true>) : reinterpret_cast<const void*>(evo_bwd_sm100_kernel<T, DP, false>);
+      smem = SmemT<DP>::bytes;
+    }
+  }
   // setmaxnreg.inc waits until the scheduler's register pool (five warps at the launch-time count)
   // has what it asks for: never launch a build whose pool cannot hold the warps' requests.
   int num_regs = 0;
   if (!kernel_ready(entry, (int)smem, &num_regs)) return EVOATTN_ERR_CUDA;
   if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
-  if (nodbias) launch_dependent(kern_n, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdq, tnl, tdl);
-  else launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
+  if (nodbias) launch_dependent(kern_n, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdq, tnl, tdl, tdk, tdv);
+  if constexpr (kApart) {
+    if (a.dbias) {
+      const auto kern_b = a.bias16 ? evo_bwd_dbias_sm100_kernel<T, DP, true> : evo_bwd_dbias_sm100_kernel<T, DP, false>;
+      if (!kernel_ready(reinterpret_cast<const void*>(kern_b), (int)SmemB<DP>::bytes, &num_regs)) return EVOATTN_ERR_CUDA;
+      if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
+      const WalkB walk = walk_b(a, sms);
+      launch_dependent(kern_b, dim3((unsigned)(walk.n_items < sms ? walk.n_items : sms)), kThreadsT, SmemB<DP>::bytes, st, a, walk, tq, tk, tv, tdo, tnl, tdl);
+      *launches += 1;
+    }
+  } else {
+    const auto kern = a.bias16 ? evo_bwd_sm100_kernel<T, DP, true> : evo_bwd_sm100_kernel<T, DP, false>;
+    if (!nodbias) launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
+  }
   if (a.dbias_out) {
     const int rc = launch_dbias_out(a, st, launches);
     if (rc) return rc;

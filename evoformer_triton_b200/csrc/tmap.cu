@@ -72,7 +72,8 @@ bool make_rows_f32_map(CUtensorMap* out, const float* base, int D, int R, long l
   cuuint32_t estr[3] = {1, 1, 1};
   const CUtensorMapSwizzle swz = !swizzle ? CU_TENSOR_MAP_SWIZZLE_NONE
                                  : box_d == 32 ? CU_TENSOR_MAP_SWIZZLE_128B
-                                               : CU_TENSOR_MAP_SWIZZLE_64B;
+                                 : box_d == 16 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                               : CU_TENSOR_MAP_SWIZZLE_32B;
   CUresult r = g_encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
