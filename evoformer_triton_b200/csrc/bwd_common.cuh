@@ -60,6 +60,11 @@ struct StepT {
 // Persistent CTAs: CTA c owns the items c, c + gridDim.x, ..., NT * G steps per item.  A short last
 // row group (S % G != 0) is padded with rows >= S: their tiles and statistics arrive as zeros and
 // their mask is -inf, so P = dS = 0, and nothing of them is stored.
+// Key tiles are the fastest: the CTAs that work side by side share Q, dO and the dQ accumulator of the same rows, which
+// come from DRAM once.  With row groups the fastest a large (b,h) came back for every key tile (four times the bytes
+// at [1,512,768,2,64]; forward and backward of [1,512,768,8,32] 3 514 us, now 3 384, [2,512,768,8,64] 12 580, now
+// 12 000).  Padded to sixteen columns a (b,h) is small, and there the shared bias tile is what counts:
+// [1,1024,384,8,8] 1 475 us with row groups the fastest and 1 489 with key tiles, [1,1024,1024,8,8] 9 352 and 9 520.
 template <int G>
 struct Steps {
   int NT, NC, H;   // query (and key) tiles, row groups, heads
@@ -73,8 +78,10 @@ struct Steps {
     d.it = n / G;
     d.g = n - d.it * G;
     int idx = (int)blockIdx.x + k * (int)gridDim.x;
-    const int chunk = idx % NC; idx /= NC;
+    int chunk = 0;
+    if constexpr (G == 7) { chunk = idx % NC; idx /= NC; }
     d.j0 = (idx % NT) * BT; idx /= NT;
+    if constexpr (G != 7) { chunk = idx % NC; idx /= NC; }
     d.h = idx % H;
     d.b = idx / H;
     d.s = chunk * G + d.g;

@@ -128,7 +128,8 @@ __device__ __forceinline__ uint32_t div_mod(uint32_t n, const FastDiv& f, uint32
   rem = n - q * f.d;
   return q;
 }
-// Work items (b, h, outer, inner), inner fastest.  Row mode: warpgroup w works on MSA row NW * inner + w,
+// Work items (b, h, inner, outer), outer fastest: the CTAs that work side by side take the query tiles of the same rows,
+// whose K and V come from DRAM once (with the rows fastest, once for every query tile of a large (b,h)).  Row mode: warpgroup w works on MSA row NW * inner + w,
 // query tile `outer`.  Query-pair mode: on row `inner`, query tile 2 * outer + w.
 struct Walk {
   int n_items;
@@ -139,8 +140,8 @@ struct Item {
 };
 __device__ __forceinline__ Item decode_item(int idx, const Walk& wk) {
   Item it;
-  uint32_t n = div_mod(static_cast<uint32_t>(idx), wk.inner, it.inner);
-  n = div_mod(n, wk.outer, it.outer);
+  uint32_t n = div_mod(static_cast<uint32_t>(idx), wk.outer, it.outer);
+  n = div_mod(n, wk.inner, it.inner);
   it.b = div_mod(n, wk.heads, it.h);
   return it;
 }
