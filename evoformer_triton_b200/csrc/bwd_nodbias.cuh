@@ -84,9 +84,6 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // (uniform, and known to be)
   constexpr bool has_bias = BIAS != BIAS_NONE, kBias16 = BIAS == BIAS_16;
-  // Whether the dV / dK MMAs of a half may go before its dS is stored, or all go at once ([4,1,2048,32,64] 597 us
-  // and 570; [1,128,384,8,32] without a bias 139 and 150).
-  constexpr bool EARLY = DP < 64;
   constexpr int kBufs = has_bias ? L::kBufs : 1, kHalf = L::kHalf;
   constexpr int kBRow = kBias16 ? BT * 2 : BT * 4;  // bytes per row (one query, 128 keys) of the staged bias tile
   const Steps<G> steps(a, n_items);
@@ -437,12 +434,10 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         // (All of the other half's MMAs into them were issued before the S^T and dP^T of this step.)
         drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
       // P^T and dS^T are in tensor memory: the dV / dK MMAs and the next S^T and dP^T may go, under what follows
-      if constexpr (EARLY) {
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(cdone + 2 * H);
-      }
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(cdone + 2 * H);
       // dQ of the previous step is complete, and the place it leaves from is free
       if (n > 0) mbar_wait(dq_full + (DP == 64 ? 2 * H : 0) + ((n - 1) & 1), ((n - 1) >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
@@ -453,11 +448,9 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       for (int c = 0; c < 4; ++c)  // dk[4 * c ..]: queries 32 * cb2 + 8 * c .. of this half
         sts_v4(drow + (((4 * cb2 + c) ^ (jrow & 7)) << 4), dk[4 * c], dk[4 * c + 1], dk[4 * c + 2], dk[4 * c + 3]);
       fence_async_shared();
-      if constexpr (!EARLY) tmem_wait_st();
       tc_fence_before();  // (the next MMAs into the dQ columns just read follow from this arrival)
       __syncwarp();
       if (lane == 0) {
-        if constexpr (!EARLY) mbar_arrive(cdone + 2 * H);
         mbar_arrive(sdone + H);
       }
     }
