@@ -184,7 +184,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
                 const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                 const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmDB, const __grid_constant__ CUtensorMap tmDQ,
-                const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL) {
+                const __grid_constant__ CUtensorMap tmNL, const __grid_constant__ CUtensorMap tmDL,
+                const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV) {
   using L = SmemT<DP>;
   constexpr int G = L::G;
 
@@ -367,11 +368,13 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     const uint32_t brow0 = smem_u32(sBias) + (H * HT + QT * cb2) * kBRow + jrow * (kBias16 ? 2 : 4);
     const uint32_t drow = sDS_s + H * (L::kDS / 2) + jrow * 128;
 
-    // Every step has one bulk group per warp with its dQ partial (empty in a warp that takes none), and the last of a
-    // row group two with d(pair_bias), one before and one after it.  So that staging area is free once all but the
-    // last group have been read.
-    auto staging_free = [&]() {
-      if (lane == 0) tma_wait_group_read1();
+    // Every step has one bulk group per warp with its dQ partial (empty in a warp that takes none).  Before that one
+    // there may be one with dK or dV, then one with half of a d(pair_bias).
+    auto staging_free = [&](bool all) {  // all groups have been read, or all but the last
+      if (lane == 0) {
+        if (all) tma_wait_group_read0();
+        else tma_wait_group_read1();
+      }
       __syncwarp();
     };
     // dQ of a step (TMEM lanes = queries): the warps of half 1 take QC columns of 32 query rows each to their staging
@@ -407,9 +410,10 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     for (int e = 0; e < 16; ++e) bacc[e] = f2_make(0.f, 0.f);
     // Half a sum (16 queries x 32 keys of a warp) to the staging area and from there, by a bulk tensor reduction that
     // the warp issues itself, to d(pair_bias).  The first half leaves as soon as the group's last row has been added
-    // to it, the second at the end of that step, by when the staging area has been read.
-    auto flush_half = [&](int sub, int i0, int j0, int h, int b) {
-      staging_free();
+    // to it, the second a step later, by when the staging area has been read (at the end of the same step it was
+    // waited for, 900 cycles in three steps).
+    auto flush_half = [&](int sub, int i0, int j0, int h, int b, bool all) {
+      staging_free(all);
 #pragma unroll
       for (int c = 0; c < 16; c += 2) {
         F2& acc = bacc[(sub * 16 + c) / 2];
@@ -426,6 +430,32 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tma_commit_group();
       }
     };
+    // dK (cb2 = 0) or dV (1) of row-group slot g, 32 keys, by a bulk store from the staging area.  Done by the warps of
+    // half 0: they are the ones whose arrival lets the next item's first MMAs overwrite the slot.  (Straight from
+    // registers, sixteen bytes of 32 rows an instruction, it took 900 to 1 700 cycles at each of an item's first steps.)
+    auto send_dk_or_dv = [&](int g, bool all) {
+      uint32_t r[DP];
+      tmem_ld<DP>(t_lane + (cb2 ? L::colDV : L::colDK) + g * DP, r);
+      staging_free(all);
+      tmem_wait_ld();
+      const float f = cb2 ? 1.f : a.scale;
+      const int x = DP == 16 ? (lane >> 2) & 1 : (lane >> 1) & 3;  // (swizzled as wide as a row)
+#pragma unroll
+      for (int c = 0; c < DP / 8; ++c) {
+        uint32_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = Pack2<T>::pack(__uint_as_float(r[8 * c + 2 * u]) * f, __uint_as_float(r[8 * c + 2 * u + 1]) * f);
+        sts_v4(outB_s + lane * (DP * 2) + ((c ^ x) << 4), w[0], w[1], w[2], w[3]);
+      }
+      fence_async_shared();
+      __syncwarp();
+      if (lane == 0) {
+        const int j = pj0 + q4 * 32, s = ps0 + g;
+        if (j < a.R && s < a.S) tma_store_5d_s(cb2 ? &tmDV : &tmDK, outB_s, 0, j, s, ph, pb);
+        tma_commit_group();
+      }
+    };
+
     int n = 0;          // running step
     uint32_t tile = 0;  // running (item, query tile)
 #pragma unroll 1
@@ -455,6 +485,10 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
       // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
       const bool deadstep = (lds_f32(vec_s) == kInf);
       const F2 mj2 = f2_make(mj, mj);
+      // dK and dV of the item before, ahead of this step's MMAs into them.  (All of the other half's MMAs into them were
+      // issued before the S^T and dP^T of this step.)
+      const bool drain = H == 0 && it == 0 && k > 0;
+      if (drain) send_dk_or_dv(g, false);
       uint32_t dk[16];
 #pragma unroll
       for (int sub = 0; sub < 2; ++sub) {
@@ -481,15 +515,18 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         // the A operands of the dV and dK MMAs (16 queries = 8 packed columns each)
         tmem_st8(cS + 16 * sub, pk);
         tmem_st8(cP + 16 * sub, *reinterpret_cast<uint32_t(*)[8]>(&dk[sub * 8]));
-        if (sub == 0 && last_of_group && flush) flush_half(0, it * BT, cur.j0, cur.h, cur.b);
+        if (sub == 0) {
+          if (last_of_group && flush) flush_half(0, it * BT, cur.j0, cur.h, cur.b, drain);
+          if (g == 0 && tile > 0 && flush) {
+            const bool turn = it == 0;
+            flush_half(1, (turn ? NT - 1 : it - 1) * BT, turn ? pj0 : cur.j0, turn ? ph : cur.h, turn ? pb : cur.b, drain);
+          }
+        }
       }
       if (last_of_group) {  // (every value read has been worked on, so the loads are through)
         __syncwarp();
         if (lane == 0) mbar_arrive(b_done + H);
       }
-      if (H == 0 && it == 0 && k > 0)  // before this step's dV / dK MMAs overwrite them
-        // (All of the other half's MMAs into them were issued before the S^T and dP^T of this step.)
-        drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
       // P^T and dS^T are in tensor memory: the dV / dK MMAs and the next S^T and dP^T may go, under what follows
       tmem_wait_st();
       tc_fence_before();
@@ -520,7 +557,6 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         mbar_arrive(sdone + H);
         send_dq(p_row0, p_slab);
       }
-      if (last_of_group && flush) flush_half(1, it * BT, cur.j0, cur.h, cur.b);
       p_row0 = it * BT + q4 * 32;
       p_slab = cur.s + g < a.S ? (cur.b * a.H + cur.h) * a.S + cur.s + g : -1;
     }
@@ -528,13 +564,13 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
     }
 
     if (total_steps > 0) {
+      flush_half(1, (NT - 1) * BT, pj0, ph, pb, true);
       mbar_wait(dq_full, total_steps & 1, abort_s, DEV_TIMEOUT_MMA);
       tc_fence_after();
       if (takes_dq) {
         uint32_t qr[QC];
         tmem_ld<QC>(t_lane + L::colDQ + qcol, qr);
-        if (lane == 0) tma_wait_group_read0();
-        __syncwarp();
+        staging_free(true);
         tmem_wait_ld();
         store_dq(qr);
         fence_async_shared();
@@ -546,7 +582,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         const int last = total_steps - 1;
         mbar_wait(st_empty + (last & 1), (last >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
-        for (int g = 0; g < G; ++g) drain_dkdv<T, DP>(a, t_lane, cb2, jrow, pb, ph, ps0 + g, pj0, g);
+#pragma unroll 1
+        for (int g = 0; g < G; ++g) send_dk_or_dv(g, true);
       }
     }
     if (lane == 0) tma_wait_group0();  // this warp's reductions have completed before the CTA may exit
@@ -594,8 +631,9 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   tb = tq;
   tdb = tq;
   tdk = tdv = tq;
-  if (G == 1 && (!make_qkv_map(&tdk, a.dk, a.sdk, a.B, a.H, a.S, a.R, a.D, DP, BT) ||
-                 !make_qkv_map(&tdv, a.dv, a.sdv, a.B, a.H, a.S, a.R, a.D, DP, BT)))
+  const int box_kv = nodbias ? BT : 32;
+  if ((G == 1 || !nodbias) && (!make_qkv_map(&tdk, a.dk, a.sdk, a.B, a.H, a.S, a.R, a.D, DP, box_kv) ||
+                               !make_qkv_map(&tdv, a.dv, a.sdv, a.B, a.H, a.S, a.R, a.D, DP, box_kv)))
     return EVOATTN_ERR_CUDA;
   if (a.bias) {
     const bool ok = a.bias16 ? make_bias16_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT, /*swizzle=*/false)
@@ -637,7 +675,7 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
     }
   } else {
     const auto kern = a.bias16 ? evo_bwd_sm100_kernel<T, DP, true> : evo_bwd_sm100_kernel<T, DP, false>;
-    if (!nodbias) launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl);
+    if (!nodbias) launch_dependent(kern, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdb, tdq, tnl, tdl, tdk, tdv);
   }
   if (a.dbias_out) {
     const int rc = launch_dbias_out(a, st, launches);
