@@ -211,7 +211,6 @@ evo_bwd_dbias_sm100_kernel(const Args a, const WalkB walk, const __grid_constant
     const int q4 = warp & 3, kg = warp >> 2;
     const int row = q4 * 32 + lane;
     const uint32_t t_base = tmem + (static_cast<uint32_t>(q4 * 32) << 16) + 32 * kg;
-    const float kInf = __int_as_float(0x7f800000);
     const float c1 = a.scale * kLog2e;
     const F2 c12 = f2_make(c1, c1), l2e2 = f2_make(kLog2e, kLog2e);
     uint32_t n = 0;
@@ -268,9 +267,8 @@ evo_bwd_dbias_sm100_kernel(const Args a, const WalkB walk, const __grid_constant
         mbar_wait(sd_full + buf, (n >> 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
         const float nl = lds_f32(vec_s + row * 4), dl = lds_f32(vec_s + BT * 4 + row * 4);
-        const uint32_t dirty = lds_u32(smem_s + L::offDirty + 4 * slot);
-        // a row whose keys are all dropped has nl = +inf for every query: replaced scores are constants, dS = 0
-        const bool dead = lds_f32(vec_s) == kInf;
+        const uint32_t dirty = __shfl_sync(0xffffffffu, lds_u32(smem_s + L::offDirty + 4 * slot), 0);
+        // (of a row whose keys are all dropped dS comes out 0, see kDeadRow)
         const F2 nl2 = f2_make(nl, nl), dl2 = f2_make(dl, dl);
         auto accumulate = [&](auto masked) {
           const uint32_t mk_s = smem_s + L::offMask + (slot * BT + 32 * kg) * 4;
@@ -299,11 +297,7 @@ evo_bwd_dbias_sm100_kernel(const Args a, const WalkB walk, const __grid_constant
             }
           }
         };
-        if (dead) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(t_empty + buf);
-        } else if ((dirty >> kg) & 1u) {
+        if ((dirty >> kg) & 1u) {
           accumulate(std::true_type{});
         } else {
           accumulate(std::false_type{});

@@ -326,7 +326,6 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
     const uint32_t t_lane = tmem + (static_cast<uint32_t>(q4 * 32) << 16);
     const uint32_t cS = t_lane + (H ? L::colS1 : L::colS0) + QT * cb2, cP = t_lane + (H ? L::colDP1 : L::colDP0) + QT * cb2;
     const float inv_r = 1.f / (float)a.R;
-    const float kInf = __int_as_float(0x7f800000);
     const float c1 = a.scale * kLog2e;
     // 32-bit shared-window addresses: every access below stays a shared-memory instruction
     const uint32_t sStage_s = smem_u32(sStage), sDS_s = smem_u32(sDS);
@@ -373,7 +372,10 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       const bool last_of_group = (g == G - 1);
       float mj;
       if constexpr (L::kMaskRows == 0) {
-        mj = G == 1 || g == 0 ? mreg[0] : g == 1 ? mreg[1] : mreg[2];
+        mj = mreg[0];  // (the rows take turns)
+#pragma unroll
+        for (int r = 0; r + 1 < G; ++r) mreg[r] = mreg[r + 1];
+        mreg[G - 1] = mj;
       } else {
         if (it == 0) mbar_wait(mk_full + g, k & 1, abort_s, DEV_TIMEOUT_TMA);
         mj = lds_f32(mask_s + g * (BT * 4));
@@ -397,9 +399,9 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       const uint32_t brow0 = bias_s + QT * cb2 * kBRow + jrow * (kBias16 ? 2 : 4);
       mbar_wait(sd_full + 2 * H, n & 1, abort_s, DEV_TIMEOUT_MMA);  // S^T and dP^T, statistics
       tc_fence_after();
-      // a row whose keys are all dropped has nl = +inf for every query (the mask row is shared by
-      // all queries of the MSA row): the whole step is uniform, P = 1/N_res, dS = 0
-      const bool deadstep = (lds_f32(vec_s) == kInf);
+      // a row whose keys are all dropped has this nl for every query (the mask row is shared by all queries of the
+      // MSA row): dS comes out 0, and P is 1/N_res
+      const bool dead = __any_sync(0xffffffffu, lds_f32(vec_s) == kDeadRow);
       const F2 mj2 = f2_make(mj, mj);
       uint32_t dk[16];
 #pragma unroll
@@ -412,14 +414,13 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         const uint32_t brow = brow0 + (16 * sub) * kBRow;
         tmem_wait_ld();
         uint32_t pk[8];
-        if (!deadstep) {
-          score_chunk<T, has_bias>(sr, dr, vnl, vdl, [&](int e) { return staged_bias<T, kBias16>(brow + e * kBRow); }, c12, mj2, pk,
-                                   dk + 8 * sub, [](int, F2) {});
-        } else {
+        score_chunk<T, has_bias>(sr, dr, vnl, vdl, [&](int e) { return staged_bias<T, kBias16>(brow + e * kBRow); }, c12, mj2, pk,
+                                 dk + 8 * sub, [](int, F2) {});
+        if (dead) {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) { pk[e] = w; dk[sub * 8 + e] = 0u; }  // replaced scores are constants: dS = 0
+          for (int e = 0; e < 8; ++e) pk[e] = w;
         }
         // P^T and dS^T, two 16-bit values per column, over the columns this thread has just read:
         // the A operands of the dV and dK MMAs (16 queries = 8 packed columns each)
