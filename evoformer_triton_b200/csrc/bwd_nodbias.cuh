@@ -1,13 +1,13 @@
 // The fused backward kernel for calls that want no d(pair_bias) (inference-like fine tuning, a frozen bias, no
-// bias at all): the same items, steps and halves as evo_bwd_sm100_kernel.  What the
-// missing gradient makes room for in shared memory changes how dQ leaves: a step's partial is one swizzled tile
-// that the loader adds to global memory by one bulk reduction, where every compute warp had to wait for its own
-// staging area and issue a reduction of its own; and the bias has a third half tile.  The compute warps wait three
-// times a step (S^T and dP^T with the statistics; the bias; dQ of the step before with the place for it) instead of
-// five.  Bound, as the other form, by the instructions and hand-overs of the compute warps.  Backward calls, us,
-// against that form: [4,1,2048,32,64] 742 -> 576, [4,1,300,32,64] 46 -> 42, [1,128,384,8,32] without a bias 148 -> 139.
-// With a d(pair_bias) it is the slower of the two: the bulk reductions of both leave at some 16 bytes a cycle and SM
-// one after another ([1,128,384,8,32] 195 and 199, [1,128,768,8,64] 1 148 and 1 182, both before the former came to 1 096).
+// bias at all), and above a head dimension of 32 for all (d(pair_bias) then comes from bwd_dbias.cuh): the same items,
+// steps and halves as evo_bwd_sm100_kernel.  What the missing gradient makes room for in shared memory changes how dQ
+// leaves: a step's partial is one swizzled tile that the loader adds to global memory by one bulk reduction (two at
+// DP = 64, a half each), where the other form's warps have staging areas and reductions of their own; and the bias has
+// a third half tile where it fits.  Bound, as the other form, by the hand-overs and the chain of the compute warps; at
+// DP = 64 also by the gap at an item boundary (a load of K, some 4 000 cycles).  Forward and backward of
+// [4,1,2048,32,64] 1 024 us, 928 since K and V have a barrier each, dK and dV leave by bulk stores and P and dS are
+// handed over before dS is stored.  With a d(pair_bias) of its own it would be the slower of the two at DP = 32: the bulk
+// reductions of both leave one after another.
 #pragma once
 
 #include "bwd_common.cuh"
@@ -191,9 +191,6 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         }
         mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
         mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-        // With one row per item the halves end a step together and wait for the next S^T and dP^T, so these go first.
-        // (At the end of an item they need the next K, which waits for this dQ.)
-        if (G == 1 && it < NT - 1) mbar_wait(sd_full + 2, (n + 1) & 1, abort_s, DEV_TIMEOUT_MMA);
         tc_fence_after();
         const uint32_t el = issue_dq<T, DP>(tmem + L::colDQ + (n & 1) * DP, sDS_s, sKV_s + 2 * g * L::kTile);
         mma_commit_if_s(el, (dq_full + (n & 1)).a);

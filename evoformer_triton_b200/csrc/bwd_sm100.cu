@@ -1,5 +1,6 @@
 // Evoformer attention backward for sm_100a: the fused dQ/dK/dV/d(pair_bias) kernel with TRANSPOSED
-// score tiles, for head dimensions up to 64 (padded to 16, 32 or 64).
+// score tiles, for head dimensions up to 32 (padded to 16 or 32); above, and without a d(pair_bias), see
+// bwd_nodbias.cuh and bwd_dbias.cuh, which are launched from here too.
 //
 // Replaces dsevoformer-triton/evoformer.py:299-326 (_attn_bwd_preprocess), :479-630
 // (_attn_bwd_dk_dv) and :329-476 (_attn_bwd_dq).  The reference recomputes S and dP in two kernels
@@ -16,7 +17,7 @@
 //     pair-bias tile of a whole row group.
 //
 // Work item = one 128-key tile j of G consecutive MSA rows of one (b,h): G = 7 at a padded head
-// dimension of 16, 3 at 32 and 1 at 64 (the dK/dV accumulators of a row take 2*DP of the 512 TMEM columns).
+// dimension of 16 and 3 at 32 (the dK/dV accumulators of a row take 2*DP of the 512 TMEM columns).
 // A persistent CTA walks its items as a flat list of steps (query tile i, row g); a step is two
 // halves of 64 queries, each with its own TMEM score buffer and its own eight warps: while one half
 // computes, the tensor core finishes the other half's dV/dK MMAs and its next S^T/dP^T.
@@ -152,30 +153,26 @@ void launch_prep(const Args& a, float* nl, float* dq_acc, cudaStream_t st) {
   }
 }
 
-// dq = scale * dq_acc, cast to the storage type (dq_acc: contiguous fp32 [B,H,S,R,D]).
-template <class T>
+// dq = scale * dq_acc, cast to the storage type (dq_acc: contiguous fp32 [B,H,S,R,D]).  Bound by memory; the position is
+// found in 32 bits where that is enough (Index): 64-bit divisions were 400 instructions a warp (forward and backward of
+// [1,203,203,4,32] 112.6 us, now 111.0).
+template <class T, class Index>
 __global__ void __launch_bounds__(256) dq_store_kernel(Args a, const float* __restrict__ acc) {
   grid_dependency_wait();
   grid_launch_dependents();
-  const int d8n = a.D / 8;
-  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-  const long long total = (long long)a.B * a.H * a.S * a.R * d8n;
+  const Index d8n = a.D / 8, total = (Index)a.B * a.H * a.S * a.R * d8n;
+  const Index idx = (Index)blockIdx.x * 256 + threadIdx.x;
   if (idx >= total) return;
-  const int d8 = (int)(idx % d8n);
-  const long long row = idx / d8n;
-  const int i = (int)(row % a.R);
-  long long sl = row / a.R;
-  const int s = (int)(sl % a.S); sl /= a.S;
-  const int h = (int)(sl % a.H);
-  const int b = (int)(sl / a.H);
-  const float4* src = reinterpret_cast<const float4*>(acc + row * a.D + d8 * 8);
+  const float4* src = reinterpret_cast<const float4*>(acc) + 2 * (size_t)idx;
   const float4 x = src[0], y = src[1];
+  const Index row = idx / d8n, slab = row / (Index)a.R, bh = slab / (Index)a.S, b = bh / (Index)a.H;
+  const int d = (int)(idx - row * d8n) * 8, i = (int)(row - slab * a.R), s = (int)(slab - bh * a.S), h = (int)(bh - b * a.H);
   uint4 pk;
   pk.x = Pack2<T>::pack(x.x * a.scale, x.y * a.scale);
   pk.y = Pack2<T>::pack(x.z * a.scale, x.w * a.scale);
   pk.z = Pack2<T>::pack(y.x * a.scale, y.y * a.scale);
   pk.w = Pack2<T>::pack(y.z * a.scale, y.w * a.scale);
-  *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.dq) + off4(a.sdq, b, h, s, i) + d8 * 8) = pk;
+  *reinterpret_cast<uint4*>(reinterpret_cast<T*>(a.dq) + off4(a.sdq, (int)b, h, s, i) + d) = pk;
 }
 
 template <class T, int DP, bool kBias16>
@@ -696,8 +693,9 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   }
   const long long n8 = (long long)rows * (a.D / 8);
   const dim3 store_grid((unsigned)((n8 + 255) / 256));
-  if (a.exchange) dq_store_kernel<T><<<store_grid, 256, 0, st>>>(a, dq_acc);  // (another launch lies between)
-  else launch_dependent(dq_store_kernel<T>, store_grid, 256, 0, st, a, static_cast<const float*>(dq_acc));
+  const auto store = n8 <= 0x7fffffffLL ? dq_store_kernel<T, uint32_t> : dq_store_kernel<T, unsigned long long>;
+  if (a.exchange) store<<<store_grid, 256, 0, st>>>(a, dq_acc);  // (another launch lies between)
+  else launch_dependent(store, store_grid, 256, 0, st, a, static_cast<const float*>(dq_acc));
   if (a.exchange && cudaStreamWaitEvent(st, join, 0) != cudaSuccess) return EVOATTN_ERR_CUDA;
   *launches += 3;
   return cudaGetLastError() == cudaSuccess ? EVOATTN_OK : EVOATTN_ERR_CUDA;
