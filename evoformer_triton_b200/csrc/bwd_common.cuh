@@ -25,8 +25,9 @@ constexpr int kComputeRegs = 112, kServiceRegs = 32;  // after setmaxnreg; the l
 constexpr int kStages = 2;  // (three or four stages measured no faster: the loads are not what a step waits for)
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int BIAS_NONE = 0, BIAS_F32 = 1, BIAS_16 = 2;
-// -lse*log2e of the queries of an MSA row whose keys are all dropped: 2^x of any score is 0 with it, so dS is 0 without
-// a branch (replaced scores are constants), and P is set to 1/N_res afterwards.
+// -lse*log2e of the queries of an MSA row whose keys are all dropped.  Its scores are constants: P is 1/N_res and dS 0
+// whatever its Q, K, V and dO hold, which may be memory that was never written.  2^x of a finite score is 0 with it
+// already; for the others each kernel says how.
 constexpr float kDeadRow = -FLT_MAX;
 
 template <int DP>

@@ -268,7 +268,6 @@ evo_bwd_dbias_sm100_kernel(const Args a, const WalkB walk, const __grid_constant
         tc_fence_after();
         const float nl = lds_f32(vec_s + row * 4), dl = lds_f32(vec_s + BT * 4 + row * 4);
         const uint32_t dirty = __shfl_sync(0xffffffffu, lds_u32(smem_s + L::offDirty + 4 * slot), 0);
-        // (of a row whose keys are all dropped dS comes out 0, see kDeadRow)
         const F2 nl2 = f2_make(nl, nl), dl2 = f2_make(dl, dl);
         auto accumulate = [&](auto masked) {
           const uint32_t mk_s = smem_s + L::offMask + (slot * BT + 32 * kg) * 4;
@@ -297,7 +296,11 @@ evo_bwd_dbias_sm100_kernel(const Args a, const WalkB walk, const __grid_constant
             }
           }
         };
-        if ((dirty >> kg) & 1u) {
+        if (__all_sync(0xffffffffu, nl == kDeadRow || i >= a.R)) {  // a row whose keys are all dropped adds nothing
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(t_empty + buf);
+        } else if ((dirty >> kg) & 1u) {
           accumulate(std::true_type{});
         } else {
           accumulate(std::false_type{});

@@ -397,7 +397,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       mbar_wait(sd_full + 2 * H, n & 1, abort_s, DEV_TIMEOUT_MMA);  // S^T and dP^T, statistics
       tc_fence_after();
       // a row whose keys are all dropped has this nl for every query (the mask row is shared by all queries of the
-      // MSA row): dS comes out 0, and P is 1/N_res
+      // MSA row): what its scores gave is replaced
       const bool dead = __any_sync(0xffffffffu, lds_f32(vec_s) == kDeadRow);
       const F2 mj2 = f2_make(mj, mj);
       uint32_t dk[16];
@@ -417,7 +417,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) pk[e] = w;
+          for (int e = 0; e < 8; ++e) { pk[e] = w; dk[8 * sub + e] = 0u; }
         }
         // P^T and dS^T, two 16-bit values per column, over the columns this thread has just read:
         // the A operands of the dV and dK MMAs (16 queries = 8 packed columns each)
