@@ -128,20 +128,24 @@ __device__ __forceinline__ uint32_t div_mod(uint32_t n, const FastDiv& f, uint32
   rem = n - q * f.d;
   return q;
 }
-// Work items (b, h, inner, outer), outer fastest: the CTAs that work side by side take the query tiles of the same rows,
-// whose K and V come from DRAM once (with the rows fastest, once for every query tile of a large (b,h)).  Row mode: warpgroup w works on MSA row NW * inner + w,
-// query tile `outer`.  Query-pair mode: on row `inner`, query tile 2 * outer + w.
+// Work items (b, h, inner, outer) in one of two orders (see rows_first).  Row mode: warpgroup w works on MSA row
+// NW * inner + w, query tile `outer`.  Query-pair mode: on row `inner`, query tile 2 * outer + w.
 struct Walk {
   int n_items;
-  FastDiv inner, outer, heads;
+  bool rows_first;               // inner is the fastest, else outer
+  FastDiv first, second, heads;  // (the fastest and the other one)
 };
 struct Item {
   uint32_t b, h, outer, inner;
 };
+// (Two selects: query tiles fastest without a choice is 1 % faster at D = 64; a branch, or divisions by strides, 1 % slower.)
 __device__ __forceinline__ Item decode_item(int idx, const Walk& wk) {
   Item it;
-  uint32_t n = div_mod(static_cast<uint32_t>(idx), wk.outer, it.outer);
-  n = div_mod(n, wk.inner, it.inner);
+  uint32_t fast, slow;
+  uint32_t n = div_mod(static_cast<uint32_t>(idx), wk.first, fast);
+  n = div_mod(n, wk.second, slow);
+  it.outer = wk.rows_first ? slow : fast;
+  it.inner = wk.rows_first ? fast : slow;
   it.b = div_mod(n, wk.heads, it.h);
   return it;
 }
@@ -728,6 +732,22 @@ evo_fwd_sm100_kernel(const Args a, const Walk wk, const __grid_constant__ CUtens
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
 }
 
+// The order of the items.  With the query tiles fastest the CTAs that work side by side share the K and V of few rows,
+// which then come from DRAM once; with the MSA rows fastest they share the bias tile and spread over the K and V of many
+// rows, all of which come back for every query tile.  That is the better way where they are still in L2 then (126 MB, next
+// to everything else) and there are more than a few query tiles.  Us, query tiles fastest and rows fastest, by the K and
+// V of a (b,h):
+//   64 MB and more: [1,1024,1024,8,32] fp32 bias 2 904 and 3 063, [1,512,1024,4,64] bf16 982 and 1 103,
+//     [1,512,2048,4,64] 3 524 and 4 089, [1,128,2048,4,64] without a bias 842 and 895
+//   48 MB: [1,512,768,8,32] bf16 856 and 877, [1,512,1024,8,24] 1 590 and 1 585, [1,128,2048,4,48] 1 011 and 992
+//   32 MB and less, from six tiles on: [1,1024,1024,8,8] fp32 2 938 and 2 838, [1,128,1024,4,48] bf16 286 and 269,
+//     [1,128,2048,8,8] fp32 1 439 and 1 369, [1,128,768,8,32] 236 and 230, [1,32,2048,4,64] without a bias 240 and 234
+//   up to three tiles: [1,128,384,8,32] fp32 75 and 77, [1,1024,384,4,64] 354 and 381, [1,1024,384,8,8] 478 and 475,
+//     [1,512,256,8,24] 143 and 141
+bool rows_first(const Args& a, int query_tiles) {
+  return query_tiles > 4 && 4LL * a.S * a.R * a.D < 40LL << 20;
+}
+
 template <class T, int DP, int BIAS, int NW, bool QP>
 int launch_t(const Args& a, cudaStream_t st, int* launches) {
   using C = Cfg<DP, NW, QP, BIAS>;
@@ -749,7 +769,8 @@ int launch_t(const Args& a, cudaStream_t st, int* launches) {
   const size_t smem = C::bytes(T_TILES * BN);
   const int inner = QP ? a.S : (a.S + NW - 1) / NW, outer = QP ? (NQT + NW - 1) / NW : NQT;
   const long long items = (long long)a.B * a.H * outer * inner;
-  const Walk wk{(int)items, fast_div((uint32_t)inner), fast_div((uint32_t)outer), fast_div((uint32_t)a.H)};
+  const bool rf = rows_first(a, NQT);
+  const Walk wk{(int)items, rf, fast_div((uint32_t)(rf ? inner : outer)), fast_div((uint32_t)(rf ? outer : inner)), fast_div((uint32_t)a.H)};
   const int grid = (int)(items < sms ? items : sms);
   const bool add = a.mask_kind == EVOATTN_MASK_ADD_F32 || a.mask_kind == EVOATTN_MASK_ADD_SAME;
   auto kern = add ? evo_fwd_sm100_kernel<T, DP, MASK_ADD, BIAS, NW, QP> : evo_fwd_sm100_kernel<T, DP, MASK_MIN, BIAS, NW, QP>;
