@@ -1,4 +1,5 @@
-// d(pair_bias) by itself, for head dimensions above 32: the sum over the MSA rows of dS, from S and dP computed again.
+// d(pair_bias) by itself, for head dimensions above 32 and many MSA rows (apart_pays): the sum over the rows of dS, from S
+// and dP computed again.
 //
 // In the fused kernel (bwd_sm100.cu) d(pair_bias) leaves as fp32 reductions, 64 KB a tile and row group.  Above a head
 // dimension of 32 tensor memory holds the dK and dV of one row only, so that is 64 KB a step next to 32 KB of dQ, at

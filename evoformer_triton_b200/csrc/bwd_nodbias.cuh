@@ -1,13 +1,17 @@
 // The fused backward kernel for calls that want no d(pair_bias) (inference-like fine tuning, a frozen bias, no
-// bias at all), and above a head dimension of 32 for all (d(pair_bias) then comes from bwd_dbias.cuh): the same items,
-// steps and halves as evo_bwd_sm100_kernel.  What the missing gradient makes room for in shared memory changes how dQ
-// leaves: a step's partial is one swizzled tile that the loader adds to global memory by one bulk reduction (two at
-// DP = 64, a half each), where the other form's warps have staging areas and reductions of their own; and the bias has
-// a third half tile where it fits.  Bound, as the other form, by the hand-overs and the chain of the compute warps; at
-// DP = 64 also by the gap at an item boundary (a load of K, some 4 000 cycles).  Forward and backward of
-// [4,1,2048,32,64] 1 024 us, 928 since K and V have a barrier each, dK and dV leave by bulk stores and P and dS are
-// handed over before dS is stored.  With a d(pair_bias) of its own it would be the slower of the two at DP = 32: the bulk
-// reductions of both leave one after another.
+// bias at all), and above a head dimension of 32 for all: the same items, steps and halves as evo_bwd_sm100_kernel.  What
+// the missing gradient makes room for in shared memory changes how dQ leaves: a step's partial is one swizzled tile that
+// the loader adds to global memory by one bulk reduction (two at DP = 64, a half each), where the other form's warps have
+// staging areas and reductions of their own; and the bias has a third half tile where it fits.  Bound, as the other form,
+// by the hand-overs and the chain of the compute warps; at DP = 64 also by the gap at an item boundary (a load of K, some
+// 4 000 cycles).  Forward and backward of [4,1,2048,32,64] 1 024 us, 928 since K and V have a barrier each, dK and dV leave
+// by bulk stores and P and dS are handed over before dS is stored.  With a d(pair_bias) of its own it would be the slower of
+// the two at DP = 32: the bulk reductions of both leave one after another.
+//
+// A d(pair_bias) above a head dimension of 32 comes from bwd_dbias.cuh where there are many rows, else from here (DBIAS,
+// see apart_pays): each dS is added to global memory from its register as it is formed, a warp's 32 keys side by side in
+// one instruction, since no shared memory is left for staging.  (Staged and reduced in bulk, before this kernel took over
+// at DP = 64: [1,4,768,8,64] 79 us, now 76; [4,1,2048,32,64] 1 989 and 1 973; [1,128,128,8,64] 98 and 86.)
 #pragma once
 
 #include "bwd_common.cuh"
@@ -41,7 +45,7 @@ struct SmemN : TilesT<DP> {
   static_assert(bytes <= 232448, "shared memory budget of one CTA");
 };
 
-template <class T, int DP, int BIAS>
+template <class T, int DP, int BIAS, bool DBIAS>
 __global__ void __launch_bounds__(kThreadsT, 1)
 evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CUtensorMap tmQ,
                 const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -51,6 +55,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
                 const __grid_constant__ CUtensorMap tmDK, const __grid_constant__ CUtensorMap tmDV) {
   using L = SmemN<DP, BIAS>;
   constexpr int G = L::G;
+  static_assert(!DBIAS || (G == 1 && BIAS != BIAS_NONE), "d(pair_bias) leaves from here with one row per item only");
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -400,6 +405,14 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       // MSA row): what its scores gave is replaced
       const bool dead = __any_sync(0xffffffffu, lds_f32(vec_s) == kDeadRow);
       const F2 mj2 = f2_make(mj, mj);
+      // (DBIAS) d(pair_bias) of this thread's key and its warp's first query; queries left from there, none in a dead row
+      float* db = nullptr;
+      int db_left = 0;
+      if constexpr (DBIAS) {
+        const int i = it * BT + H * HT + QT * cb2, j = cur.j0 + jrow;
+        db = a.dbias + (((long long)cur.b * a.H + cur.h) * a.R + i) * a.dbias_ld + j;
+        db_left = j < a.R && !dead ? a.R - i : 0;
+      }
       uint32_t dk[16];
 #pragma unroll
       for (int sub = 0; sub < 2; ++sub) {
@@ -412,7 +425,15 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
         tmem_wait_ld();
         uint32_t pk[8];
         score_chunk<T, has_bias>(sr, dr, vnl, vdl, [&](int e) { return staged_bias<T, kBias16>(brow + e * kBRow); }, c12, mj2, pk,
-                                 dk + 8 * sub, [](int, F2) {});
+                                 dk + 8 * sub, [&](int e, F2 ds) {
+                                   if constexpr (DBIAS) {  // (32 neighbouring keys an instruction)
+                                     const int q = 16 * sub + 2 * e;
+                                     float d0, d1;
+                                     f2_get(ds, d0, d1);
+                                     red_add_if(db + (long long)q * a.dbias_ld, d0, q < db_left);
+                                     red_add_if(db + (long long)(q + 1) * a.dbias_ld, d1, q + 1 < db_left);
+                                   }
+                                 });
         if (dead) {
           const float pu = (cur.j0 + jrow < a.R) ? inv_r : 0.f;
           const uint32_t w = Pack2<T>::pack(pu, pu);

@@ -39,7 +39,7 @@ namespace {
 
 template <int DP>
 struct SmemT : TilesT<DP> {
-  static_assert(DP < 64, "above 32 columns d(pair_bias) has a kernel of its own");
+  static_assert(DP < 64, "above 32 columns bwd_nodbias.cuh serves calls with a d(pair_bias) too");
   using Tiles = TilesT<DP>;
   using Tiles::G, Tiles::kTile, Tiles::kStage, Tiles::kDS;
   static constexpr int kBias = BT * BT * 4;                  // pair-bias tile [128 i][128 j], unswizzled (fp32; half of it for a 16-bit bias)
@@ -615,6 +615,22 @@ size_t align_up(size_t x, size_t al) { return (x + al - 1) / al * al; }
 // One vector of row statistics: [B,H,S,delta_ld] fp32.
 size_t stats_bytes(const Args& a) { return align_up((size_t)a.B * a.H * a.S * a.delta_ld * sizeof(float), 256); }
 
+// Above a head dimension of 32: whether d(pair_bias) comes from a kernel that computes S and dP again (bwd_dbias.cuh), or
+// leaves the kernel that gives dQ, dK and dV as reductions, 64 KB a step.  An item of the former costs its rows and about
+// two more, so it takes many rows (and tiles, for there to be an item for every SM without cutting the rows up) to save
+// what the reductions cost.  Forward and backward, us, apart and as reductions, fp32 bias:
+//   one row:    [4,1,2048,32,64] 3 192 and 1 973, [4,1,300,32,64] 124 and 84, [1,1,300,8,64] 39 and 33
+//   few:        [1,4,768,8,64] 86 and 76, [1,8,2048,8,64] 635 and 579, [1,16,512,8,64] 107 and 101
+//   about even: [1,64,384,8,64] 219 and 219, [1,64,300,8,64] 198 and 197, [1,96,640,4,64] 378 and 376, [1,24,1536,4,64] 480
+//               and 479
+//   many:       [1,32,768,8,64] 352 and 364, [1,128,384,8,64] 401 and 405, [1,512,257,8,64] 1 277 and 1 310,
+//               [1,56,1536,4,64] 1 027 and 1 083
+//   two tiles:  [1,512,128,8,64] 330 and 304, [1,128,200,4,64] 115 and 107, [2,512,256,8,64] 1 564 and 1 553
+bool apart_pays(const Args& a) {
+  const long long NT = (a.R + BT - 1) / BT;
+  return NT > 2 && a.S * NT >= 192;
+}
+
 template <class T, int DP>
 int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* launches) {
   constexpr int G = RowsPerItem<DP>::G;
@@ -637,7 +653,7 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   if (!make_qkv_map(&tk, a.k, a.sk, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tv, a.v, a.sv, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
   if (!make_qkv_map(&tdo, a.d_o, a.sdo, a.B, a.H, a.S, a.R, a.D, DP, BT)) return EVOATTN_ERR_CUDA;
-  constexpr bool kApart = DP == 64;  // d(pair_bias) has a kernel of its own
+  constexpr bool kApart = DP == 64;  // d(pair_bias) may have a kernel of its own
   const bool nodbias = kApart || !a.dbias;
   const long long slabs = (long long)a.B * a.H * a.S;
   if (!(nodbias ? make_rows_f32_map(&tdq, dq_acc, a.D, a.R, slabs, DP < 32 ? DP : 32, BT, /*swizzle=*/true)
@@ -665,8 +681,13 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   const int sms = sm_count();
   if (sms <= 0) return EVOATTN_ERR_CUDA;
   const long long ctas = items < sms ? items : sms;
-  const auto kern_n = !a.bias ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_NONE>
-                      : (a.bias16 ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_16> : evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_F32>);
+  auto kern_n = !a.bias ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_NONE, false>
+                : a.bias16 ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_16, false> : evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_F32, false>;
+  bool apart = false;
+  if constexpr (kApart) {
+    apart = a.dbias && apart_pays(a);
+    if (a.dbias && !apart) kern_n = a.bias16 ? evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_16, true> : evo_bwd_nodbias_sm100_kernel<T, DP, BIAS_F32, true>;
+  }
   const void* entry = reinterpret_cast<const void*>(kern_n);
   size_t smem = !a.bias ? SmemN<DP, BIAS_NONE>::bytes : a.bias16 ? SmemN<DP, BIAS_16>::bytes : SmemN<DP, BIAS_F32>::bytes;
   if constexpr (!kApart) {
@@ -682,7 +703,7 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
   if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;
   if (nodbias) launch_dependent(kern_n, dim3((unsigned)ctas), kThreadsT, smem, st, a, (int)items, tq, tk, tv, tdo, tb, tdq, tnl, tdl, tdk, tdv);
   if constexpr (kApart) {
-    if (a.dbias) {
+    if (apart) {
       const auto kern_b = a.bias16 ? evo_bwd_dbias_sm100_kernel<T, DP, true> : evo_bwd_dbias_sm100_kernel<T, DP, false>;
       if (!kernel_ready(reinterpret_cast<const void*>(kern_b), (int)SmemB<DP>::bytes, &num_regs)) return EVOATTN_ERR_CUDA;
       if ((kThreadsT / 128) * num_regs < 4 * kComputeRegs + kServiceRegs) return EVOATTN_ERR_UNSUPPORTED;

@@ -262,6 +262,10 @@ __device__ __forceinline__ uint32_t ldg_u8_if(const void* p, bool pred) {
 __device__ __forceinline__ void red_add_v4(float* p, float x, float y, float z, float w) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
+// Adds a float to global memory where pred holds.
+__device__ __forceinline__ void red_add_if(float* p, float x, bool pred) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q red.global.add.f32 [%0], %1;\n\t}" ::"l"(p), "f"(x), "r"((int)pred) : "memory");
+}
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

@@ -17,8 +17,8 @@ pytestmark = pytest.mark.gpu
 ROWS = (1, 4)  # of five: a whole row group of three, a short one, and items of one row
 
 
-def poisoned(D, name, value, frozen=False, R=203):
-    x = rand_inputs(1, 5, R, 2, D, torch.bfloat16, seed=D + R, mask="bool", bias=True)
+def poisoned(D, name, value, frozen=False, R=203, S=5):
+    x = rand_inputs(1, S, R, 2, D, torch.bfloat16, seed=D + R, mask="bool", bias=True)
     if frozen:
         x["pair_bias"] = None
     for s in ROWS:
@@ -56,5 +56,12 @@ def test_with_a_pair_bias_gradient(D, name, value):
 @pytest.mark.parametrize("D", [16, 32, 64])
 def test_without_a_pair_bias(D, name):
     x = poisoned(D, name, "nan", frozen=True, R=264)
+    got, _ = run_op(x, want_path=_lib().PATH_TCGEN05)
+    finite_values_agree(got, x)
+
+
+@pytest.mark.parametrize("name", ["Q", "K", "V", "dO"])
+def test_many_rows_above_a_head_dimension_of_32(name):
+    x = poisoned(64, name, "nan", R=261, S=64)
     got, _ = run_op(x, want_path=_lib().PATH_TCGEN05)
     finite_values_agree(got, x)
