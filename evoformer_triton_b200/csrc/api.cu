@@ -127,6 +127,9 @@ bool use_sm100_bwd(const evoattn_bwd_params* p, const evo::Args& a) {
       !stride_ok16(p->dv_stride, es))
     return false;
   if (p->fwd.gate && ((((uintptr_t)p->dgate) & 15) || !stride_ok16(p->dgate_stride, es))) return false;
+  // dK and dV leave through tensor maps, which know no backward steps.
+  for (int i = 0; i < 4; ++i)
+    if (p->dk_stride[i] < 0 || p->dv_stride[i] < 0) return false;
   // Of the odd lengths with a d(pair_bias), the smallest calls keep the dispatch that all of them once had:
   // the CUDA cores, with P and dS in fp32.  The line does not separate the faster kernels.  Backward calls in
   // us, tensor / CUDA cores, [B,S,R,H]: D = 8: [1,1,33,1] 15.7 / 9.6, [1,5,51,2] 16.5 / 12.8, [1,1,511,1]
