@@ -303,7 +303,8 @@ __device__ __forceinline__ void score_chunk(const uint32_t (&sr)[16], const uint
   }
 }
 
-// dK, dV of row-group slot g (MSA row s of (b,h), keys j0..): TMEM -> registers -> global.
+// dK, dV of row-group slot g (MSA row s of (b,h), keys j0..): TMEM -> registers -> global.  For the kernel without a
+// d(pair_bias) up to DP = 32: with an fp32 bias its shared memory is full, so that nothing can be staged for bulk stores.
 // Done by the warps of half 0 (half of the DP columns each, 16 at a time): they are the ones
 // whose arrival lets the next item's first MMAs overwrite the slot.
 template <class T, int DP>

@@ -12,7 +12,8 @@
 //
 // Work item = (b, h, run of rows, query tile, key tile), tiles fastest, so that the CTAs that work side by side read
 // the same rows out of L2.  Warps 0-15 compute (warp w: queries 32*(w%4).., keys 32*(w/4)..; a thread owns a query, its
-// TMEM lane, and 32 keys), 16 loads tiles, 17 issues the MMAs, 18 stages the residue mask.
+// TMEM lane, and 32 keys), 16 loads tiles, 17 issues the MMAs, 18 stages the residue mask.  Bias and sum are 64 of a
+// compute thread's 112 registers, and eight bytes of the rest are spilled.
 #pragma once
 
 #include "bwd_common.cuh"
@@ -22,9 +23,10 @@ namespace {
 
 template <int DP>
 struct SmemB {
+  static_assert(DP == 64, "up to 32 columns d(pair_bias) leaves the fused kernel");
   static constexpr int kTile = BT * DP * 2;
   static constexpr int kStage = 4 * kTile;                   // Q, dO, K, V of a row
-  static constexpr int kStages3 = DP == 64 ? 3 : 5;
+  static constexpr int kStages3 = 3;
   static constexpr int kSlots = 8;                           // of statistics and masks: more than the steps in flight
   static constexpr int kVecs = 2 * BT * 4;                   // -lse*log2e and -delta of the row's queries
   static constexpr int offStage = 0;

@@ -103,11 +103,12 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
   if (tid == 0) {
     for (int i = 0; i < (G == 1 ? 2 : G); ++i) { mbar_init(bars + 0 + i, 1); mbar_init(bars + 7 + i, G == 1 ? 1 : 3); }  // kv_full; kv_empty: three MMA warps read K/V
     for (int i = 0; i < G; ++i) mbar_init(bars + 25 + i, 1);  // mk_full
-    mbar_init(bars + 44, kCW); mbar_init(bars + 45, 1);  // drained, dkv_sent
+    if (G == 1) { mbar_init(bars + 44, kCW); mbar_init(bars + 45, 1); }  // drained, dkv_sent
     for (int i = 0; i < kStages; ++i) { mbar_init(bars + 32 + i, 1); mbar_init(bars + 40 + i, 2); }  // st_full, st_empty
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + 48 + 2 * i, 3); mbar_init(bars + 52 + 2 * i, kCW / 2);  // sd_full: two commits, one warp; cdone
-      mbar_init(bars + 36 + i, 2); mbar_init(bars + 38 + i, 2);                // dq_full: the commit, and the loader
+      mbar_init(bars + 36 + i, 2);                                     // dq_full: the commit, and the loader
+      if (DP == 64) mbar_init(bars + 38 + i, 2);
     }
     for (int i = 0; i < kBufs; ++i) { mbar_init(bars + 56 + i, 1); mbar_init(bars + 60 + i, kCW / 2); }  // b_full, b_done
     for (int i = 0; i < 2; ++i) mbar_init(bars + 23 + i, kCW / 2);  // sdone
@@ -279,7 +280,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       for (int n = 0; n < total_steps + 2; ++n) {
         const int stg = n % kStages;
         const bool load = n < total_steps;
-          if (G > 1 && load && d.it == 0) load_kv(n);
+        if (G > 1 && load && d.it == 0) load_kv(n);
         mbar_wait(st_empty + stg, ((n / kStages) & 1) ^ 1, abort_s, DEV_TIMEOUT_MMA);  // (of step n - 2)
         if (load) {
           if (elect_one()) {
@@ -293,19 +294,17 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
           }
           __syncwarp();
         }
-        {
-          if (n >= 2) {
-            mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-            if (kBoxes == 2 && n >= 3) send_dq(0, row3, slab3);
-            mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
-            if (n >= 3) send_dq(kBoxes - 1, row3, slab3);
-            dq_place_free(n - 2);
-          }
-          row3 = row2; slab3 = slab2;
-          row2 = row1; slab2 = slab1;
-          row1 = d.it * BT;
-          slab1 = d.s < a.S ? (d.b * a.H + d.h) * a.S + d.s : -1;
+        if (n >= 2) {
+          mbar_wait(sdone + 0, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+          if (kBoxes == 2 && n >= 3) send_dq(0, row3, slab3);
+          mbar_wait(sdone + 1, n & 1, abort_s, DEV_TIMEOUT_SYNC);
+          if (n >= 3) send_dq(kBoxes - 1, row3, slab3);
+          dq_place_free(n - 2);
         }
+        row3 = row2; slab3 = slab2;
+        row2 = row1; slab2 = slab1;
+        row1 = d.it * BT;
+        slab1 = d.s < a.S ? (d.b * a.H + d.h) * a.S + d.s : -1;
         if (load) d = steps.advance(d, n + 1);
       }
       if (total_steps > 0) {  // the last step's partial: the compute warps arrive once more
@@ -469,9 +468,7 @@ evo_bwd_nodbias_sm100_kernel(const Args a, const int n_items, const __grid_const
       fence_async_shared();
       tc_fence_before();  // (the next MMAs into the dQ columns just read follow from this arrival)
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(sdone + H);
-      }
+      if (lane == 0) mbar_arrive(sdone + H);
     }
     pb = cur.b; ph = cur.h; ps0 = cur.s; pj0 = cur.j0;
     }

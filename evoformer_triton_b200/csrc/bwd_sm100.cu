@@ -22,7 +22,8 @@
 // halves of 64 queries, each with its own TMEM score buffer and its own eight warps: while one half
 // computes, the tensor core finishes the other half's dV/dK MMAs and its next S^T/dP^T.
 // dS is summed over the G rows in registers and leaves once per (i, j) tile as bulk tensor
-// reductions; the dQ partial of a step goes to an fp32 accumulator in global memory the same way.
+// reductions, half a tile a warp and step; the dQ partial of a step goes to an fp32 accumulator in
+// global memory the same way, by the eight warps of half 1, while those of half 0 take dK and dV.
 //
 // Warps: 0-15 compute (warp w: keys 32*(w%4).., queries 32*((w/4)%2).. of half w/8), 16-18 issue the
 // tcgen05.mma (18 also loads the pair-bias tiles), 19 loads the other tiles.
@@ -395,10 +396,6 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
 
     int p_row0 = 0, p_slab = -1;           // the step whose dQ partial has not left yet
     int pb = 0, ph = 0, ps0 = 0, pj0 = 0;  // the item whose dK/dV still sit in TMEM
-    // Always true.  With more than one row it has to be looked at all the same, which the compiler cannot know: given
-    // last_of_group alone it makes two copies of a step, whose registers do not fit (8 to 24 bytes of spills; the
-    // backward of [1,128,384,8,32] took 210 us instead of 195, [1,1024,384,8,8] fp16 1177 instead of 1083).
-    const bool flush = a.dbias != nullptr;
     const uint32_t mask_s = smem_u32(smem + L::offMask) + jrow * 4;
     float mreg[L::kMaskRows == 0 ? G : 1];
     const F2 c12 = f2_make(c1, c1);
@@ -519,8 +516,8 @@ evo_bwd_sm100_kernel(const Args a, const int n_items, const __grid_constant__ CU
         tmem_st8(cS + 16 * sub, pk);
         tmem_st8(cP + 16 * sub, *reinterpret_cast<uint32_t(*)[8]>(&dk[sub * 8]));
         if (sub == 0) {
-          if (last_of_group && flush) flush_half(0, it * BT, cur.j0, cur.h, cur.b, drain);
-          if (g == 0 && tile > 0 && flush) {
+          if (last_of_group) flush_half(0, it * BT, cur.j0, cur.h, cur.b, drain);
+          if (g == 0 && tile > 0) {
             const bool turn = it == 0;
             flush_half(1, (turn ? NT - 1 : it - 1) * BT, turn ? pj0 : cur.j0, turn ? ph : cur.h, turn ? pb : cur.b, drain);
           }
@@ -673,7 +670,7 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
                              : make_bias_plain_map(&tb, a.bias, a.sbias, a.B, a.H, a.R, HT, BT);
     if (!ok) return EVOATTN_ERR_CUDA;
     const Str3 dense{(long long)a.H * a.R * a.dbias_ld, (long long)a.R * a.dbias_ld, (long long)a.dbias_ld};
-    if (a.dbias && !make_bias_plain_map(&tdb, a.dbias, dense, a.B, a.H, a.R, 16, 32)) return EVOATTN_ERR_CUDA;
+    if (!nodbias && !make_bias_plain_map(&tdb, a.dbias, dense, a.B, a.H, a.R, 16, 32)) return EVOATTN_ERR_CUDA;
   }
   const int NT = (a.R + BT - 1) / BT;
   const long long items = (long long)a.B * a.H * NT * ((a.S + G - 1) / G);
@@ -745,13 +742,13 @@ int launch_t(const Args& a0, void* ws, size_t ws_bytes, cudaStream_t st, int* la
 // tile every seventh step instead of every third, but there are fewer of them and the last group of rows is
 // padded further.  They are taken where the CTA with the most steps gets no more than 15 % more of them, or 5 % with
 // an fp32 bias that wants no gradient (whose third half tile then pays for itself at three rows already).  Time of
-// the backward call, seven rows over three, by how many more steps that CTA gets (D = 8 and 16, N_res 200 to 1000;
-// at 128 and 256 an fp32 bias without a gradient is 0.05 to 0.1 above):
+// the backward call, seven rows over three, by how many more steps that CTA gets (D = 8 and 16, N_res 200 to 1000, 26
+// shapes):
 //                                as many    5 % more   10 %       17 %       27 %
-//   with d(pair_bias):           0.86-0.89  0.89-0.92  0.93-0.97  0.98-1.00  1.06-1.09
-//   with an fp32 bias alone:     0.89-0.91  0.94-0.96  0.95-0.99  1.03-1.05  1.08-1.14
-//   with a 16-bit bias alone:    0.85-0.90  0.89-0.92  0.93-0.95  1.00-1.01  1.05-1.10
-//   without a bias:              0.80-0.86  0.86-0.89  0.89-0.92  0.95-0.98  1.02-1.06
+//   with d(pair_bias):           0.86-0.89  0.91-0.94  0.94-0.98  0.99-1.03  1.11-1.12
+//   with an fp32 bias alone:     0.90-0.95  0.95-0.99  0.97-1.03  1.03-1.09  1.15-1.18
+//   with a 16-bit bias alone:    0.83-0.87  0.89-0.92  0.88-0.95  0.96-1.01  1.09-1.10
+//   without a bias:              0.80-0.85  0.85-0.91  0.88-0.92  0.94-0.98  1.03-1.05
 bool seven_rows_pay(const Args& a, int sms) {
   const auto steps = [&](int G) {
     const long long items = (long long)a.B * a.H * ((a.R + BT - 1) / BT) * ((a.S + G - 1) / G);
