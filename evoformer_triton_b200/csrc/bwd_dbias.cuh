@@ -1,12 +1,14 @@
 // d(pair_bias) by itself, for head dimensions above 32 and many MSA rows (apart_pays): the sum over the rows of dS, from S
 // and dP computed again.
 //
-// In the fused kernel (bwd_sm100.cu) d(pair_bias) leaves as fp32 reductions, 64 KB a tile and row group.  Above a head
-// dimension of 32 tensor memory holds the dK and dV of one row only, so that is 64 KB a step next to 32 KB of dQ, at
-// the 21 bytes a cycle and SM that reductions leave at (5.9 TB/s, the chip over): 4 600 cycles of a step's 7 200.
-// Here a CTA keeps a 128 x 128 tile of d(pair_bias) in registers while it walks the MSA rows, and so does its tile of the
-// bias: dS costs two products, two FMAs, an exponential and a third FMA an element, and nothing is written before the
-// last row.  dQ, dK and dV come from the kernel without a d(pair_bias) (bwd_nodbias.cuh).
+// Up to a head dimension of 32 d(pair_bias) leaves the fused kernel (bwd_sm100.cu) as fp32 reductions, 64 KB a tile and row
+// group.  Above, tensor memory holds the dK and dV of one row only, so that is 64 KB a step next to 32 KB of dQ, at the 21
+// bytes a cycle and SM that reductions leave at (5.9 TB/s, the chip over): 4 600 cycles of a step's 7 200 when the fused
+// kernel served these too.  Here a CTA keeps a 128 x 128 tile of d(pair_bias) in registers while it walks the MSA rows, and
+// so does its tile of the bias: dS costs two products, two FMAs, an exponential and a third FMA an element, and nothing is
+// written before the last row.  dQ, dK and dV come from the kernel without a d(pair_bias) (bwd_nodbias.cuh).  Bound by the
+// exponentials (68 % of their unit's rate, 1 500 cycles a step).  Forward and backward, us, fused and now:
+// [1,128,384,8,64] 446 and 401, [1,512,257,8,64] 1 464 and 1 277, [1,32,768,8,64] 389 and 352.
 //
 // Replaces the d_pair_bias half of dsevoformer-triton/evoformer.py:329-476 (the atomic of :458).
 //
